@@ -655,9 +655,9 @@ extern "C" int bsg_cnn_create(const bsg_cnn_config* cfg, bsg_cnn** out) {
     if (e == cudaSuccess) e = cudaMalloc(&c->d_m, sizeof(float) * off);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_v, sizeof(float) * off);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_lossmean, sizeof(float) * 1);
-    if (e == cudaSuccess) e = cudaMemcpy(c->d_w, w.data(), sizeof(float) * off, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(c->d_m, 0, sizeof(float) * off);
-    if (e == cudaSuccess) e = cudaMemset(c->d_v, 0, sizeof(float) * off);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_w, w.data(), sizeof(float) * off, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_m, 0, sizeof(float) * off, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_v, 0, sizeof(float) * off, c->stream);
     if (e == cudaSuccess) {
         round_bf16_kernel<<<grid_for(off), 256, 0, c->stream>>>(c->d_w, c->d_weff, off);
         e = cudaGetLastError();
@@ -703,11 +703,11 @@ extern "C" int bsg_cnn_set_params(bsg_cnn* h, const float* in) {
     Cnn* c = reinterpret_cast<Cnn*>(h);
     if (!c || !in) return cfail(BSG_ERR_ARG, "bsg_cnn_set_params: null argument");
     CCK(cudaSetDevice(c->device));
-    CCK(cudaMemcpy(c->d_w, in, sizeof(float) * c->nparams, cudaMemcpyHostToDevice));
+    CCK(cudaMemcpyAsync(c->d_w, in, sizeof(float) * c->nparams, cudaMemcpyHostToDevice, c->stream));
     round_bf16_kernel<<<grid_for(c->nparams), 256, 0, c->stream>>>(c->d_w, c->d_weff, c->nparams);
     CCK(cudaGetLastError());
-    CCK(cudaMemset(c->d_m, 0, sizeof(float) * c->nparams));
-    CCK(cudaMemset(c->d_v, 0, sizeof(float) * c->nparams));
+    CCK(cudaMemsetAsync(c->d_m, 0, sizeof(float) * c->nparams, c->stream));
+    CCK(cudaMemsetAsync(c->d_v, 0, sizeof(float) * c->nparams, c->stream));
     c->step = 0;
     CCK(cudaStreamSynchronize(c->stream));
     return BSG_OK;
