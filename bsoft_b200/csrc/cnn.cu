@@ -14,14 +14,12 @@
 //          R = [b1 b2 b3] (columns), t = shift (pixels)
 //   loss   mean over the batch of |R - R*|_F^2 + lambda |t - t*|^2
 //
-// Convolutions are GEMMs over im2col rows (M = batch x output pixels,
-// K = 9 x input channels, N = output channels): forward C = X_col W^T,
-// weight gradient W' = dY^T X_col (split over M, partial sums reduced in a
-// fixed order), input gradient dX_col = dY W gathered back by col2im.  One
-// tensor-core GEMM kernel (BF16 mma.sync with the operands split into two
-// BF16 terms, FP32 accumulation, 128 x 64 tiles) serves all of them.  Every
-// reduction has a fixed order, so training is bitwise reproducible for a
-// given seed.
+// Convolutions are implicit GEMMs on the tensor cores (BF16 mma.sync with the
+// operands split into two BF16 terms, FP32 accumulation): the operand rows
+// are fetched from the activation planes as a tap needs them, in the forward
+// pass, the input gradient and the weight gradient (over pixel ranges whose
+// partial sums are added in order).  Every reduction has a fixed order, so
+// training is bitwise reproducible for a given seed.
 #include "common.cuh"
 
 #include <cuda_bf16.h>
@@ -43,22 +41,20 @@ constexpr int NCONV = 6;
 constexpr int NOUT = 8;     // a1, a2, shift
 constexpr int NRES = 11;    // R (9, row-major) and shift (2)
 
-// ---- GEMM: C[m][n] (+)= sum_k A(m, k) B(n, k) ------------------------------
-// A(m, k) = AT ? A[k * lda + m] : A[m * lda + k]
-// B(n, k) = BT ? B[k * ldb + n] : B[n * ldb + k]
-// blockIdx.z splits k into `splits` ranges; with splits > 1 each range
-// writes its own partial product C + z * M * N (reduced afterwards).
-// On the tensor cores:
-// mma.sync m16n8k16, BF16 operands, FP32 accumulation.  Every FP32 operand
-// value v is split into hi = bf16(v) and lo = bf16(v - hi) while its tile is
-// staged in shared memory, and each 16-deep step adds Ahi Bhi + Ahi Blo +
-// Alo Bhi (the lo x lo term is below 2^-16 of the product), so a product
-// keeps ~17 significant bits and the weights, which are BF16 values already,
-// enter exactly (their lo parts are zero).  Block tile 128 x 64, eight warps
-// of 32 x 32 (2 x 4 mma tiles); shared rows of 24 BF16 (12 words) so the
-// fragment loads of the 8 row groups x 4 lanes fall on distinct banks.  The
-// mma accumulation order is fixed, so results are bitwise reproducible.
-constexpr int TBM = 128, TBN = 64, TBK = 16, TROW = 24;
+using bf16 = __nv_bfloat16;
+
+// ---- operands ---------------------------------------------------------------
+//
+// Every value that enters a product is held as two BF16 terms, hi = bf16(v)
+// and lo = bf16(v - hi), in two planes; a product adds hi hi, hi lo and lo hi
+// (the lo x lo term is below 2^-16 of it), so it keeps ~17 significant bits.
+// The weights are BF16 values already: their lo terms are zero and left out.
+// The planes are written by the kernel that produces the value (32 bits a
+// value, as the float would take), so no consumer splits again, and they are
+// NHWC with the channels padded to a multiple of 32 (zeros), so every operand
+// row is copied in aligned 16-byte pieces.
+constexpr int CPAD = 32;
+__host__ __device__ constexpr int cpad(int c) { return (c + CPAD - 1) / CPAD * CPAD; }
 
 __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, const uint32_t* b) {
     asm volatile(
@@ -68,187 +64,240 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, const uint
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-__device__ __forceinline__ void split_bf16(float v, __nv_bfloat16& hi, __nv_bfloat16& lo) {
+__device__ __forceinline__ void ldsm4(uint32_t* r, uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t* r, uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// 16 bytes global -> shared, zeros when !ok
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void split_bf16(float v, bf16& hi, bf16& lo) {
     hi = __float2bfloat16_rn(v);
     lo = __float2bfloat16_rn(v - __bfloat162float(hi));
 }
+__device__ __forceinline__ uint32_t pack2(bf16 a, bf16 b) {
+    return (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
+}
+__device__ __forceinline__ void split2(float v0, float v1, uint32_t& hi, uint32_t& lo) {
+    bf16 h0, h1, l0, l1;
+    split_bf16(v0, h0, l0);
+    split_bf16(v1, h1, l1);
+    hi = pack2(h0, h1);
+    lo = pack2(l0, l1);
+}
 
-template <bool AT, bool BT>
-__global__ void __launch_bounds__(256) tgemm_kernel(int M, int N, int K, const float* __restrict__ A, int lda,
-                                                    const float* __restrict__ B, int ldb, float* __restrict__ C,
-                                                    int splits, int accumulate) {
-    __shared__ __align__(16) __nv_bfloat16 Ah[TBM * TROW], Al[TBM * TROW], Bh[TBN * TROW], Bl[TBN * TROW];
+// ---- convolution as an implicit GEMM ----------------------------------------
+//
+// C[m][n] = sum over taps and channels of A(m, tap, c) W(n, tap, c): row m is
+// an output pixel (b, y, x), A its input pixel (stride y + dy, stride x + dx)
+// of the tap (zero outside the image), fetched straight from the activation
+// planes by cp.async, so no column matrix is written.  The forward pass is
+// stride 2 with nine taps; the input gradient is one GEMM per parity class
+// of the input pixel (stride 1 over the output gradient, 4, 2, 2 and 1 taps,
+// blockIdx.z the class); a dense layer is one tap on a 1 x 1 image.
+// The epilogue adds the bias and applies the ReLU (forward) or the ReLU's
+// mask (gradient) and writes the two planes of the result.
+//
+// Column matrices and separate bias, ReLU and mask passes bounded this path
+// before (a K-deep FP32 copy of every input pixel: 302 MB for the second
+// layer of 256 images of 128^2, written, read and split again); a layer now
+// reads its input about 9 / 4 times through L2 and writes its output once.
+// 2,048 images of 128^2: 14.5 -> 1.66 ms, the same bits; loss and gradient of
+// 256 images 11.3 -> 2.1 ms, of which 1.0 ms is the host copies.  Block tile BM x BN with K-steps of 32 in a 4-deep ring, 8 warps of
+// 32 rows.  mma.sync keeps the accumulation order of every product sum (k in
+// steps of 16; hi, then lo), so results do not depend on the tile.
+// Column j of a warp's n-tile t is channel 2 NT (j / 2) + 2 t + (j & 1): a
+// lane's accumulators are then 2 NT consecutive channels of its row and
+// leave in 16-byte stores.
+struct ConvClass {
+    int ntap;
+    signed char dy[9], dx[9], w[9];   // input offset and weight slice of each tap
+    int oy, ox;                       // output pixel = ostride (y, x) + (oy, ox)
+};
+
+struct ConvArgs {
+    const bf16 *ah, *al;              // input planes, pitch C
+    const bf16* w;                    // weights: n wrow + slice wtap + c
+    long wrow, wtap;
+    int M, N, logw, logh;             // rows: m = (b, y, x), 2^logh x 2^logw per image
+    int H, W, C, stride;              // input image
+    bf16 *oh, *ol;                    // output planes, pitch N
+    int OH, OW, ostride;
+    const float* bias;                // or null
+    int nbias;
+    int relu;
+    const bf16* mask;                 // output kept where mask > 0 (laid out as the output), or null
+    ConvClass cls[4];
+};
+
+constexpr int CBK = 32, CST = 4;
+
+template <int BM, int BN>
+constexpr int conv_smem() { return CST * (2 * BM + BN) * CBK * 2; }
+
+template <int BM, int BN>
+__global__ void __launch_bounds__(256) conv_gemm_kernel(const __grid_constant__ ConvArgs a) {
+    constexpr int WMS = BM / 32, WNS = 8 / WMS, WN = BN / WNS, NT = WN / 8;
+    constexpr int LOGR = NT == 8 ? 4 : NT == 4 ? 3 : 2;            // log2(2 NT)
+    static_assert(NT == 2 || NT == 4 || NT == 8, "warp tile");
+    constexpr int APL = BM * CBK * 2, STAGE = 2 * APL + BN * CBK * 2;
+    extern __shared__ __align__(128) unsigned char csm[];
+    const uint32_t base = smem_addr(csm);
+    const ConvClass& k = a.cls[blockIdx.z];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int m0 = blockIdx.y * TBM, n0 = blockIdx.x * TBN;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    const int kper = (K + splits - 1) / splits;
-    const int kb = blockIdx.z * kper, ke = min(K, kb + kper);
-    float acc[2][4][4];
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int wm = (warp / WNS) * 32, wn = (warp % WNS) * WN;
+
+    // this thread's copies: 16-byte piece ch of rows r0 + 64 i
+    const int ch = tid & 3, r0 = tid >> 2;
+    constexpr int AR = (BM + 63) / 64, BR = (BN + 63) / 64;
+    int iy[AR], ix[AR];
+    long ib[AR];
+    bool iv[AR];
+#pragma unroll
+    for (int i = 0; i < AR; ++i) {
+        const int r = r0 + 64 * i, m = m0 + r;
+        iv[i] = r < BM && m < a.M;
+        const int x = m & ((1 << a.logw) - 1), y = (m >> a.logw) & ((1 << a.logh) - 1), b = m >> (a.logw + a.logh);
+        iy[i] = y * a.stride;
+        ix[i] = x * a.stride;
+        ib[i] = (long)b * a.H * a.W;
+    }
+    const int kch = a.C / CBK, T = k.ntap * kch;
+    auto load = [&](int it) {
+        const int tap = it / kch, c0 = (it - tap * kch) * CBK + ch * 8;
+        const uint32_t st = base + (it % CST) * STAGE;
+        const int dy = k.dy[tap], dx = k.dx[tap];
+#pragma unroll
+        for (int i = 0; i < AR; ++i) {
+            const int r = r0 + 64 * i;
+            if (BM >= 64 || r < BM) {
+                const int yy = iy[i] + dy, xx = ix[i] + dx;
+                const bool ok = iv[i] && (unsigned)yy < (unsigned)a.H && (unsigned)xx < (unsigned)a.W;
+                const long off = ok ? (ib[i] + (long)yy * a.W + xx) * a.C + c0 : 0;
+                const uint32_t d = st + r * 64 + ((ch ^ ((r >> 1) & 3)) << 4);
+                cp16(d, a.ah + off, ok);
+                cp16(d + APL, a.al + off, ok);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < BR; ++i) {
+            const int r = r0 + 64 * i;
+            if (BN >= 64 || r < BN)
+                cp16(st + 2 * APL + r * 64 + ((ch ^ ((r >> LOGR) & 3)) << 4),
+                     a.w + (n0 + r) * a.wrow + k.w[tap] * a.wtap + c0, true);
+        }
+    };
+
+    float acc[2][NT][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NT; ++j)
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
-    for (int k0 = kb; k0 < ke; k0 += TBK) {
-        // A tile: TBM x TBK = 2048 values, 8 per thread
+
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const int idx = tid + r * 256;
-            int mm, kk;
-            if (AT) { kk = idx / TBM; mm = idx % TBM; } else { mm = idx / TBK; kk = idx % TBK; }
-            const int gm = m0 + mm, gk = k0 + kk;
-            float v = 0.f;
-            if (gm < M && gk < ke) v = AT ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            split_bf16(v, Ah[mm * TROW + kk], Al[mm * TROW + kk]);
-        }
-        // B tile: TBN x TBK = 1024 values, 4 per thread
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int idx = tid + r * 256;
-            int nn, kk;
-            if (BT) { kk = idx / TBN; nn = idx % TBN; } else { nn = idx / TBK; kk = idx % TBK; }
-            const int gn = n0 + nn, gk = k0 + kk;
-            float v = 0.f;
-            if (gn < N && gk < ke) v = BT ? B[(size_t)gk * ldb + gn] : B[(size_t)gn * ldb + gk];
-            split_bf16(v, Bh[nn * TROW + kk], Bl[nn * TROW + kk]);
-        }
-        __syncthreads();
-        uint32_t ah[2][4], al[2][4], bh[4][2], bl[4][2];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            const int r0 = (wm + mt * 16 + g) * TROW, r8 = r0 + 8 * TROW;
-            ah[mt][0] = *reinterpret_cast<const uint32_t*>(&Ah[r0 + 2 * t]);
-            ah[mt][1] = *reinterpret_cast<const uint32_t*>(&Ah[r8 + 2 * t]);
-            ah[mt][2] = *reinterpret_cast<const uint32_t*>(&Ah[r0 + 2 * t + 8]);
-            ah[mt][3] = *reinterpret_cast<const uint32_t*>(&Ah[r8 + 2 * t + 8]);
-            al[mt][0] = *reinterpret_cast<const uint32_t*>(&Al[r0 + 2 * t]);
-            al[mt][1] = *reinterpret_cast<const uint32_t*>(&Al[r8 + 2 * t]);
-            al[mt][2] = *reinterpret_cast<const uint32_t*>(&Al[r0 + 2 * t + 8]);
-            al[mt][3] = *reinterpret_cast<const uint32_t*>(&Al[r8 + 2 * t + 8]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int c0 = (wn + nt * 8 + g) * TROW;
-            bh[nt][0] = *reinterpret_cast<const uint32_t*>(&Bh[c0 + 2 * t]);
-            bh[nt][1] = *reinterpret_cast<const uint32_t*>(&Bh[c0 + 2 * t + 8]);
-            bl[nt][0] = *reinterpret_cast<const uint32_t*>(&Bl[c0 + 2 * t]);
-            bl[nt][1] = *reinterpret_cast<const uint32_t*>(&Bl[c0 + 2 * t + 8]);
-        }
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                mma_bf16(acc[mt][nt], ah[mt], bh[nt]);
-                mma_bf16(acc[mt][nt], ah[mt], bl[nt]);
-                mma_bf16(acc[mt][nt], al[mt], bh[nt]);
-            }
-        __syncthreads();
+    for (int s = 0; s < CST - 1; ++s) {
+        if (s < T) load(s);
+        cp_commit();
     }
-    float* Cz = C + (splits > 1 ? (size_t)blockIdx.z * M * N : 0);
+    for (int it = 0; it < T; ++it) {
+        cp_wait<CST - 2>();
+        __syncthreads();
+        if (it + CST - 1 < T) load(it + CST - 1);
+        cp_commit();
+        const uint32_t st = base + (it % CST) * STAGE;
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+            uint32_t ah[2][4], al[2][4], b[NT][2];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                const int r = wm + mt * 16 + (lane & 15), c = kk * 2 + (lane >> 4);
+                const uint32_t ad = st + r * 64 + ((c ^ ((r >> 1) & 3)) << 4);
+                ldsm4(ah[mt], ad);
+                ldsm4(al[mt], ad + APL);
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; nt += 2) {
+                const int q = lane >> 3, j = lane & 7;
+                const int r = wn + 2 * NT * (j >> 1) + 2 * (nt + (q >> 1)) + (j & 1), c = kk * 2 + (q & 1);
+                ldsm4(b[nt], st + 2 * APL + r * 64 + ((c ^ ((r >> LOGR) & 3)) << 4));
+            }
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    mma_bf16(acc[mt][nt], ah[mt], b[nt]);
+                    mma_bf16(acc[mt][nt], al[mt], b[nt]);
+                }
+        }
+    }
+    cp_wait<0>();
+
+    const int g = lane >> 2, t = lane & 3;
+    const int nc = n0 + wn + 2 * NT * t;                      // this lane's first channel
+    float bias[2 * NT];
+#pragma unroll
+    for (int j = 0; j < 2 * NT; ++j) bias[j] = a.bias && nc + j < a.nbias ? a.bias[nc + j] : 0.f;
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int hr = 0; hr < 2; ++hr) {
+            const int m = m0 + wm + mt * 16 + hr * 8 + g;
+            if (m >= a.M) continue;
+            const int x = m & ((1 << a.logw) - 1), y = (m >> a.logw) & ((1 << a.logh) - 1), bb = m >> (a.logw + a.logh);
+            const long o = (((long)bb * a.OH + y * a.ostride + k.oy) * a.OW + x * a.ostride + k.ox) * a.N + nc;
+            uint32_t h[NT], l[NT], mk[NT];
+            if (a.mask) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int gm = m0 + wm + mt * 16 + g + (q >= 2 ? 8 : 0);
-                const int gn = n0 + wn + nt * 8 + 2 * t + (q & 1);
-                if (gm >= M || gn >= N) continue;
-                float* c = Cz + (size_t)gm * N + gn;
-                *c = (accumulate && splits == 1) ? *c + acc[mt][nt][q] : acc[mt][nt][q];
+                for (int j = 0; j < NT; j += 2) {
+                    const uint2 v = *reinterpret_cast<const uint2*>(a.mask + o + 2 * j);
+                    mk[j] = v.x;
+                    mk[j + 1] = v.y;
+                }
             }
-}
-
-// sum of `splits` partial products into C (fixed order)
-__global__ void split_reduce_kernel(const float* __restrict__ part, long count, int splits, float* __restrict__ C,
-                                    int accumulate) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count; i += (long)gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int z = 0; z < splits; ++z) s += part[(size_t)z * count + i];
-        C[i] = accumulate ? C[i] + s : s;
-    }
-}
-
-// ---- layers ------------------------------------------------------------------
-
-// im2col for a 3x3, stride 2, padding 1 convolution over NHWC input:
-// row (b, yo, xo), column (ky * 3 + kx) * Cin + ci
-__global__ void im2col_kernel(const float* __restrict__ x, int B, int H, int W, int Cin, int Ho, int Wo,
-                              float* __restrict__ col) {
-    const long K = 9L * Cin, total = (long)B * Ho * Wo * K;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const long row = i / K;
-        const int kk = (int)(i - row * K);
-        const int ci = kk % Cin, kyx = kk / Cin, ky = kyx / 3, kx = kyx % 3;
-        const int xo = (int)(row % Wo), yo = (int)((row / Wo) % Ho), b = (int)(row / ((long)Wo * Ho));
-        const int yi = 2 * yo + ky - 1, xi = 2 * xo + kx - 1;
-        float v = 0.f;
-        if (yi >= 0 && yi < H && xi >= 0 && xi < W) v = x[(((size_t)b * H + yi) * W + xi) * Cin + ci];
-        col[i] = v;
-    }
-}
-
-// input gradient: every input value gathers the column entries it fed
-// (at most 2 x 2 taps for stride 2), in a fixed order
-__global__ void col2im_kernel(const float* __restrict__ gcol, int B, int H, int W, int Cin, int Ho, int Wo,
-                              float* __restrict__ gx) {
-    const long total = (long)B * H * W * Cin;
-    const long K = 9L * Cin;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int ci = (int)(i % Cin);
-        const int xi = (int)((i / Cin) % W), yi = (int)((i / ((long)Cin * W)) % H), b = (int)(i / ((long)Cin * W * H));
-        float s = 0.f;
-        for (int ky = 0; ky < 3; ++ky) {
-            const int t = yi + 1 - ky;
-            if (t < 0 || (t & 1)) continue;
-            const int yo = t >> 1;
-            if (yo >= Ho) continue;
-            for (int kx = 0; kx < 3; ++kx) {
-                const int u = xi + 1 - kx;
-                if (u < 0 || (u & 1)) continue;
-                const int xo = u >> 1;
-                if (xo >= Wo) continue;
-                s += gcol[(((size_t)b * Ho + yo) * Wo + xo) * K + (ky * 3 + kx) * Cin + ci];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                float v0 = acc[mt][j][2 * hr] + bias[2 * j], v1 = acc[mt][j][2 * hr + 1] + bias[2 * j + 1];
+                if (a.relu) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
+                if (a.mask) {
+                    // BF16 terms of a ReLU output: positive or zero
+                    if (!(mk[j] & 0xffffu)) v0 = 0.f;
+                    if (!(mk[j] >> 16)) v1 = 0.f;
+                }
+                split2(v0, v1, h[j], l[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < NT; j += 4) {
+                if (NT >= 4) {
+                    *reinterpret_cast<uint4*>(a.oh + o + 2 * j) = make_uint4(h[j], h[j + 1], h[j + 2], h[j + 3]);
+                    *reinterpret_cast<uint4*>(a.ol + o + 2 * j) = make_uint4(l[j], l[j + 1], l[j + 2], l[j + 3]);
+                } else {
+                    *reinterpret_cast<uint2*>(a.oh + o) = make_uint2(h[0], h[1]);
+                    *reinterpret_cast<uint2*>(a.ol + o) = make_uint2(l[0], l[1]);
+                }
             }
         }
-        gx[i] = s;
-    }
 }
 
-// rows idx[b] of a (n x width) table
-__global__ void gather_rows_kernel(const float* __restrict__ src, const int* __restrict__ idx, int rows, int width,
-                                   float* __restrict__ dst) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * width) return;
-    const int r = i / width, c = i - r * width;
-    dst[i] = src[(long)idx[r] * width + c];
-}
+// ---- first convolution: one input channel -----------------------------------
 
-__global__ void fill_kernel(float* __restrict__ p, long n, float v) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) p[i] = v;
-}
-
-// y[m][n] = relu?(y[m][n] + bias[n])
-__global__ void bias_act_kernel(float* __restrict__ y, long M, int N, const float* __restrict__ bias, int relu) {
-    const long total = M * N;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        float v = y[i] + bias[i % N];
-        y[i] = relu ? fmaxf(v, 0.f) : v;
-    }
-}
-
-// g *= (a > 0)
-__global__ void relu_back_kernel(float* __restrict__ g, const float* __restrict__ a, long count) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count; i += (long)gridDim.x * blockDim.x)
-        if (!(a[i] > 0.f)) g[i] = 0.f;
-}
-
-// batch input: images idx[b] of the data set, normalised per image
-// (population mean and standard deviation, FP64 sums in a fixed order)
-__global__ void __launch_bounds__(256) gather_norm_kernel(const float* __restrict__ data, const int* __restrict__ idx,
-                                                          int npix, float* __restrict__ out) {
+// per image: mean and 1 / population standard deviation (FP64 sums in a
+// fixed order); idx: the images of the batch within the data set, or null
+__global__ void __launch_bounds__(256) image_norm_kernel(const float* __restrict__ data, const int* __restrict__ idx,
+                                                         int npix, float2* __restrict__ norm) {
     __shared__ double s1[256], s2[256];
     const long src = idx ? idx[blockIdx.x] : blockIdx.x;
     const float* p = data + src * (long)npix;
@@ -261,12 +310,469 @@ __global__ void __launch_bounds__(256) gather_norm_kernel(const float* __restric
         if (threadIdx.x < o) { s1[threadIdx.x] += s1[threadIdx.x + o]; s2[threadIdx.x] += s2[threadIdx.x + o]; }
         __syncthreads();
     }
-    const double mean = s1[0] / npix;
-    double var = s2[0] / npix - mean * mean;
-    const float inv = var > 1e-30 ? (float)(1.0 / sqrt(var)) : 1.f;
-    const float mu = (float)mean;
-    float* q = out + (long)blockIdx.x * npix;
-    for (int i = threadIdx.x; i < npix; i += 256) q[i] = (p[i] - mu) * inv;
+    if (threadIdx.x == 0) {
+        const double mean = s1[0] / npix;
+        const double var = s2[0] / npix - mean * mean;
+        norm[blockIdx.x] = make_float2((float)mean, var > 1e-30 ? (float)(1.0 / sqrt(var)) : 1.f);
+    }
+}
+
+// A CTA's patch of the normalised image: output pixels [p0, p0 + 256) of the
+// wo x wo grid and their 3 x 3 input pixels, row pitch 2 wo + 4, column 0
+// holding x = -1 (zeros outside the image).  Rows of wo are split when wo
+// exceeds 256 (never: wo <= 256).
+constexpr int C1PIX = 256;
+__device__ __forceinline__ int c1_rows(int wo) { return 2 * (C1PIX / wo) + 1; }
+__device__ __forceinline__ int c1_pitch(int wo) { return 2 * wo + 4; }
+
+__device__ __forceinline__ void c1_load(float* patch, const float* img, float2 nm, int wo, int y0) {
+    const int rows = c1_rows(wo), pitch = c1_pitch(wo), w = 2 * wo;
+    for (int i = threadIdx.x; i < rows * pitch; i += blockDim.x) {
+        const int r = i / pitch, x = i - r * pitch - 1, y = 2 * y0 - 1 + r;
+        float v = 0.f;
+        if (y >= 0 && y < w && x >= 0 && x < w) v = (img[(long)y * w + x] - nm.x) * nm.y;
+        patch[i] = v;
+    }
+}
+
+// input value of output pixel p (relative to the CTA's first) at tap (ky, kx)
+__device__ __forceinline__ float c1_tap(const float* patch, int pitch, int logw, int p, int tap) {
+    const int y = p >> logw, x = p & ((1 << logw) - 1);
+    const int ky = tap / 3, kx = tap - 3 * ky;
+    return patch[(2 * y + ky) * pitch + 2 * x + kx];
+}
+
+// 256 output pixels of one image per CTA; the nine taps are one K-step of 16
+// whose A fragments are built from the patch in registers.  Bound by its
+// output (two BF16 planes).  w: [cout padded][16] BF16, blockIdx.y the block
+// of 32 channels.
+__global__ void __launch_bounds__(256) conv1_kernel(const float* __restrict__ data, const int* __restrict__ idx,
+                                                    const float2* __restrict__ norm, int logw,
+                                                    const bf16* __restrict__ w, const float* __restrict__ bias,
+                                                    int nbias, int pitch_out, bf16* __restrict__ oh,
+                                                    bf16* __restrict__ ol) {
+    extern __shared__ float patch[];
+    const int wo = 1 << logw, pitch = c1_pitch(wo);
+    const int perimg = (wo * wo) / C1PIX;
+    const int b = blockIdx.x / perimg, p0 = (blockIdx.x - b * perimg) * C1PIX;
+    const long src = idx ? idx[b] : b;
+    c1_load(patch, data + src * (4L << (2 * logw)), norm[b], wo, p0 >> logw);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int n0 = blockIdx.y * 32;
+    // weight fragments: column j of n-tile q is channel 8 (j / 2) + 2 q + (j & 1)
+    uint32_t bw[4][2];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint32_t* r = reinterpret_cast<const uint32_t*>(w + (n0 + 8 * (g >> 1) + 2 * q + (g & 1)) * 16);
+        bw[q][0] = r[t];
+        bw[q][1] = r[t + 4];
+    }
+    float bs[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) bs[j] = n0 + 8 * t + j < nbias ? bias[n0 + 8 * t + j] : 0.f;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+        const int pr = warp * 32 + mt * 16 + g;
+        uint32_t ah[4], al[4];
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+            const int p = pr + 8 * hr;
+            split2(c1_tap(patch, pitch, logw, p, 2 * t), c1_tap(patch, pitch, logw, p, 2 * t + 1), ah[hr], al[hr]);
+            split2(t == 0 ? c1_tap(patch, pitch, logw, p, 8) : 0.f, 0.f, ah[2 + hr], al[2 + hr]);
+        }
+        float acc[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[q][e] = 0.f;
+            mma_bf16(acc[q], ah, bw[q]);
+            mma_bf16(acc[q], al, bw[q]);
+        }
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+            const long o = (((long)b << (2 * logw)) + p0 + pr + 8 * hr) * pitch_out + n0 + 8 * t;
+            uint32_t h[4], l[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                split2(fmaxf(acc[q][2 * hr] + bs[2 * q], 0.f), fmaxf(acc[q][2 * hr + 1] + bs[2 * q + 1], 0.f), h[q], l[q]);
+            *reinterpret_cast<uint4*>(oh + o) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(ol + o) = make_uint4(l[0], l[1], l[2], l[3]);
+        }
+    }
+}
+
+// ---- weight gradients ---------------------------------------------------------
+//
+// dW[n][tap][c] = sum over output pixels of gY(pixel, n) X(pixel's input at
+// tap, c): a GEMM over the pixels whose operands are rows of the planes
+// (fragments by ldmatrix.trans), one tap per CTA.  Three products per step
+// (both operands are split).  The pixels are divided over blockIdx.z ranges
+// whose partial sums are added in a fixed order afterwards; the bias gradient
+// (the column sums of gY) is one more product with a fragment of ones, in the
+// CTAs of the centre tap.
+struct WgradArgs {
+    const bf16 *yh, *yl;              // gY planes: pixels x N
+    const bf16 *xh, *xl;              // X planes, pitch C
+    int M, N, C, logw, logh, H, W, stride, ntap;
+    int steps, per;                   // K-steps of 32 pixels, steps per range
+    float* part;                      // ranges x (N x ntap x C), then ranges x N bias sums
+    float* bpart;
+};
+
+constexpr int GST = 3;
+
+template <int BN>
+constexpr int wgrad_smem() { return GST * 32 * (64 + BN) * 2 * 2; }
+
+// 16-byte piece c of row r in a tile of rows of RB bytes
+template <int RB>
+__device__ __forceinline__ int tswz(int r, int c) {
+    return r * RB + ((RB == 128 ? c ^ (r & 7) : c ^ ((r >> 1) & 3)) << 4);
+}
+
+// grid: x = tap, y = (block of 64 of N) + (blocks of N) (block of BN of C), z = range
+template <int BN>
+__global__ void __launch_bounds__(128) wgrad_kernel(const __grid_constant__ WgradArgs a) {
+    constexpr int NT = BN / 16;                          // n-tiles per warp (2 x 2 warps)
+    constexpr int YB = 128, XB = BN * 2;                 // row bytes
+    constexpr int YPL = 32 * YB, XPL = 32 * XB, STAGE = 2 * (YPL + XPL);
+    extern __shared__ __align__(128) unsigned char gsm[];
+    const uint32_t base = smem_addr(gsm);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tap = blockIdx.x, nb = (a.N + 63) / 64;
+    const int n0 = (blockIdx.y % nb) * 64, c0 = (blockIdx.y / nb) * BN;
+    const int dy = a.ntap == 9 ? tap / 3 - 1 : 0, dx = a.ntap == 9 ? tap % 3 - 1 : 0;
+    const int s0 = blockIdx.z * a.per, s1 = min(a.steps, s0 + a.per);
+    const bool dobias = tap == a.ntap / 2 && c0 == 0;
+    const int wm = (warp >> 1) * 32, wn = (warp & 1) * (BN / 2);
+    auto load = [&](int s, int slot) {
+        const uint32_t st = base + slot * STAGE;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {                    // gY: 32 rows x 8 pieces
+            const int e = tid + 128 * i, r = e >> 3, c = e & 7, m = s * 32 + r;
+            const bool ok = m < a.M && n0 + c * 8 < a.N;
+            const long off = ok ? (long)m * a.N + n0 + c * 8 : 0;
+            cp16(st + tswz<YB>(r, c), a.yh + off, ok);
+            cp16(st + YPL + tswz<YB>(r, c), a.yl + off, ok);
+        }
+#pragma unroll
+        for (int i = 0; i < BN / 32; ++i) {              // X: 32 rows x BN / 8 pieces
+            const int e = tid + 128 * i, r = e / (BN / 8), c = e % (BN / 8), m = s * 32 + r;
+            const int x = m & ((1 << a.logw) - 1), y = (m >> a.logw) & ((1 << a.logh) - 1), b = m >> (a.logw + a.logh);
+            const int yy = y * a.stride + dy, xx = x * a.stride + dx;
+            const bool ok = m < a.M && (unsigned)yy < (unsigned)a.H && (unsigned)xx < (unsigned)a.W && c0 + c * 8 < a.C;
+            const long off = ok ? (((long)b * a.H + yy) * a.W + xx) * a.C + c0 + c * 8 : 0;
+            cp16(st + 2 * YPL + tswz<XB>(r, c), a.xh + off, ok);
+            cp16(st + 2 * YPL + XPL + tswz<XB>(r, c), a.xl + off, ok);
+        }
+    };
+    float acc[2][NT][4], bacc[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) bacc[i][q] = 0.f;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
+    }
+    const uint32_t ones[2] = {0x3f803f80u, 0x3f803f80u};
+#pragma unroll
+    for (int s = 0; s < GST - 1; ++s) {
+        if (s0 + s < s1) load(s0 + s, s);
+        cp_commit();
+    }
+    int slot = 0;
+    for (int s = s0; s < s1; ++s) {
+        cp_wait<GST - 2>();
+        __syncthreads();
+        if (s + GST - 1 < s1) load(s + GST - 1, slot == 0 ? GST - 1 : slot - 1);
+        cp_commit();
+        const uint32_t st = base + slot * STAGE;
+        slot = slot + 1 == GST ? 0 : slot + 1;
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+            uint32_t ah[2][4], al[2][4], bh[NT][2], bl[NT][2];
+            const int q = lane >> 3, j = lane & 7;
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                // matrices (k, m): (lo, lo), (lo, hi), (hi, lo), (hi, hi) of 8 pixels x 8 channels
+                const int r = kk * 16 + (q >> 1) * 8 + j, c = (wm + mt * 16) / 8 + (q & 1);
+                ldsm4t(ah[mt], st + tswz<YB>(r, c));
+                ldsm4t(al[mt], st + YPL + tswz<YB>(r, c));
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; nt += 2) {
+                const int r = kk * 16 + (q & 1) * 8 + j, c = wn / 8 + nt + (q >> 1);
+                ldsm4t(bh[nt], st + 2 * YPL + tswz<XB>(r, c));
+                ldsm4t(bl[nt], st + 2 * YPL + XPL + tswz<XB>(r, c));
+            }
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    mma_bf16(acc[mt][nt], ah[mt], bh[nt]);
+                    mma_bf16(acc[mt][nt], ah[mt], bl[nt]);
+                    mma_bf16(acc[mt][nt], al[mt], bh[nt]);
+                }
+                if (dobias) { mma_bf16(bacc[mt], ah[mt], ones); mma_bf16(bacc[mt], al[mt], ones); }
+            }
+        }
+    }
+    cp_wait<0>();
+    const int g = lane >> 2, t = lane & 3;
+    float* out = a.part + (long)blockIdx.z * a.N * a.ntap * a.C;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+            const int n = n0 + wm + mt * 16 + hr * 8 + g;
+            if (n >= a.N) continue;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const int c = c0 + wn + nt * 8 + 2 * t;
+                if (c < a.C)
+                    *reinterpret_cast<float2*>(out + ((long)n * a.ntap + tap) * a.C + c) =
+                        make_float2(acc[mt][nt][2 * hr], acc[mt][nt][2 * hr + 1]);
+            }
+            if (dobias && t == 0 && (warp & 1) == 0) a.bpart[(long)blockIdx.z * a.N + n] = bacc[mt][2 * hr];
+        }
+}
+
+// The first layer's gradient: 32 channels (blockIdx.y) x (nine taps and a
+// column of ones, the bias) over the pixels of C1PER CTA patches per block.
+// Bound by reading the gradient planes once.  part: blocks x N x 16.
+__global__ void __launch_bounds__(256) wgrad1_kernel(const float* __restrict__ data, const int* __restrict__ idx,
+                                                     const float2* __restrict__ norm, int logw,
+                                                     const bf16* __restrict__ yh, const bf16* __restrict__ yl, int N,
+                                                     int patches, int per, float* __restrict__ part) {
+    extern __shared__ __align__(16) float patch[];
+    __shared__ __align__(16) bf16 ys[2][C1PIX * 32];
+    float (*red)[32 * 16] = reinterpret_cast<float (*)[32 * 16]>(&ys[0][0]);   // the warps' sums, at the end
+    const int wo = 1 << logw, pitch = c1_pitch(wo), perimg = (wo * wo) / C1PIX;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int n0 = blockIdx.y * 32;
+    const uint32_t yb = smem_addr(ys);
+    float acc[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
+    const int q0 = blockIdx.x * per, q1 = min(patches, q0 + per);
+    for (int pt = q0; pt < q1; ++pt) {
+        const int b = pt / perimg, p0 = (pt - b * perimg) * C1PIX;
+        const long src = idx ? idx[b] : b;
+        __syncthreads();
+        const long row = ((long)b << (2 * logw)) + p0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = tid + 256 * i, r = e >> 2, c = e & 3;
+            const long off = (row + r) * N + n0 + c * 8;
+            cp16(yb + tswz<64>(r, c), yh + off, true);
+            cp16(yb + C1PIX * 64 + tswz<64>(r, c), yl + off, true);
+        }
+        cp_commit();
+        c1_load(patch, data + src * (4L << (2 * logw)), norm[b], wo, p0 >> logw);
+        cp_wait<0>();
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < 2; ++kk) {
+            const int k0 = warp * 32 + kk * 16;
+            uint32_t ah[2][4], al[2][4], bh[2][2], bl[2][2];
+            const int q = lane >> 3, j = lane & 7;
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                const int r = k0 + (q >> 1) * 8 + j, c = mt * 2 + (q & 1);
+                ldsm4t(ah[mt], yb + tswz<64>(r, c));
+                ldsm4t(al[mt], yb + C1PIX * 64 + tswz<64>(r, c));
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int p = k0 + 8 * h + 2 * t;
+                split2(c1_tap(patch, pitch, logw, p, g), c1_tap(patch, pitch, logw, p + 1, g), bh[0][h], bl[0][h]);
+                float v0 = 0.f, v1 = 0.f;
+                if (g == 0) { v0 = c1_tap(patch, pitch, logw, p, 8); v1 = c1_tap(patch, pitch, logw, p + 1, 8); }
+                else if (g == 1) v0 = v1 = 1.f;
+                split2(v0, v1, bh[1][h], bl[1][h]);
+            }
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    mma_bf16(acc[mt][nt], ah[mt], bh[nt]);
+                    mma_bf16(acc[mt][nt], ah[mt], bl[nt]);
+                    mma_bf16(acc[mt][nt], al[mt], bh[nt]);
+                }
+        }
+    }
+    // the warps' sums, in warp order
+    __syncthreads();
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                red[warp][(mt * 16 + g + (q >> 1) * 8) * 16 + nt * 8 + 2 * t + (q & 1)] = acc[mt][nt][q];
+    __syncthreads();
+    for (int i = tid; i < 512; i += 256) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += red[w][i];
+        part[((long)blockIdx.x * N + n0) * 16 + i] = s;
+    }
+}
+
+// ---- the last dense layer -----------------------------------------------------
+
+// o = h W^T + bias: one warp per 16 rows, the eight outputs one n-tile
+__global__ void __launch_bounds__(32) fc2_kernel(const bf16* __restrict__ hh, const bf16* __restrict__ hl, int B, int K,
+                                                 const bf16* __restrict__ w, const float* __restrict__ bias,
+                                                 float* __restrict__ o) {
+    const int lane = threadIdx.x, g = lane >> 2, t = lane & 3;
+    const int r0 = blockIdx.x * 16 + g, r1 = r0 + 8;
+    const uint32_t* h0 = reinterpret_cast<const uint32_t*>(hh + (long)min(r0, B - 1) * K);
+    const uint32_t* h1 = reinterpret_cast<const uint32_t*>(hh + (long)min(r1, B - 1) * K);
+    const uint32_t* l0 = reinterpret_cast<const uint32_t*>(hl + (long)min(r0, B - 1) * K);
+    const uint32_t* l1 = reinterpret_cast<const uint32_t*>(hl + (long)min(r1, B - 1) * K);
+    const uint32_t* wr = reinterpret_cast<const uint32_t*>(w + (long)g * K);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int k = t; k < K / 2; k += 8) {
+        const uint32_t ah[4] = {h0[k], h1[k], h0[k + 4], h1[k + 4]};
+        const uint32_t al[4] = {l0[k], l1[k], l0[k + 4], l1[k + 4]};
+        const uint32_t b[2] = {wr[k], wr[k + 4]};
+        mma_bf16(acc, ah, b);
+        mma_bf16(acc, al, b);
+    }
+    const float b0 = bias[2 * t], b1 = bias[2 * t + 1];
+    if (r0 < B) { o[r0 * NOUT + 2 * t] = acc[0] + b0; o[r0 * NOUT + 2 * t + 1] = acc[1] + b1; }
+    if (r1 < B) { o[r1 * NOUT + 2 * t] = acc[2] + b0; o[r1 * NOUT + 2 * t + 1] = acc[3] + b1; }
+}
+
+// its gradients in FP32: dh = go W masked by the ReLU (planes of pitch Kp),
+// one thread per (row, hidden unit)
+__global__ void __launch_bounds__(256) fc2_dgrad_kernel(const float* __restrict__ go, int B, int K, int Kp,
+                                                        const float* __restrict__ w, const bf16* __restrict__ hh,
+                                                        bf16* __restrict__ gh, bf16* __restrict__ gl) {
+    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (i >= (long)B * Kp) return;
+    const int b = (int)(i / Kp), j = (int)(i - (long)b * Kp);
+    float s = 0.f;
+    if (j < K && __bfloat162float(hh[i]) > 0.f)
+#pragma unroll
+        for (int q = 0; q < NOUT; ++q) s = fmaf(go[b * NOUT + q], w[(long)q * K + j], s);
+    split_bf16(s, gh[i], gl[i]);
+}
+
+// dW = go^T h and db = sum go: 32 hidden units per CTA, the rows over 8
+// groups of lanes that are added in order
+__global__ void __launch_bounds__(256) fc2_wgrad_kernel(const float* __restrict__ go, int B, int K, int Kp,
+                                                        const bf16* __restrict__ hh, const bf16* __restrict__ hl,
+                                                        float* __restrict__ dw, float* __restrict__ db) {
+    __shared__ float red[8][NOUT][33];
+    const int jl = threadIdx.x & 31, sl = threadIdx.x >> 5, j = blockIdx.x * 32 + jl;
+    float s[NOUT], sb = 0.f;
+#pragma unroll
+    for (int q = 0; q < NOUT; ++q) s[q] = 0.f;
+#pragma unroll 4
+    for (int b = sl; b < B; b += 8) {
+        const long i = (long)b * Kp + j;
+        const float h = __bfloat162float(hh[i]) + __bfloat162float(hl[i]);
+#pragma unroll
+        for (int q = 0; q < NOUT; ++q) s[q] = fmaf(go[b * NOUT + q], h, s[q]);
+        if (jl < NOUT) sb += go[b * NOUT + jl];
+    }
+#pragma unroll
+    for (int q = 0; q < NOUT; ++q) red[sl][q][jl] = s[q];
+    if (jl < NOUT) red[sl][jl][32] = sb;
+    __syncthreads();
+    float v = 0.f;
+#pragma unroll
+    for (int z = 0; z < 8; ++z) v += red[z][sl][jl];      // warp sl takes output sl
+    if (j < K) dw[(long)sl * K + j] = v;
+    if (blockIdx.x == 0 && jl == 0) {
+        float u = 0.f;
+#pragma unroll
+        for (int z = 0; z < 8; ++z) u += red[z][sl][32];
+        db[sl] = u;
+    }
+}
+
+// ---- packed weights and gradient sums -----------------------------------------
+
+// A layer's weights in the parameter vector, [cout][taps][cin], and the
+// packed forms: forward [coutp][tapsp][cinp] (row n, K contiguous) and, for
+// the input gradient, [taps][cinp][coutp].
+struct PackLayer {
+    long woff, boff;
+    int cin, cout, cinp, coutp, taps, tapsp;
+    long f, fn, b, bn;                // offset and count of the two forms (bn = 0: none)
+    const float* part;                // weight-gradient partials: [ranges][coutp][tapsp][cinp]
+    const float* bpart;               // bias partials: [ranges][coutp] (null: column cin of the weights')
+    int ranges;
+};
+constexpr int NPACK = NCONV + 2;
+struct PackArgs {
+    PackLayer l[NPACK];
+    int n;
+};
+
+__global__ void pack_kernel(const __grid_constant__ PackArgs p, const float* __restrict__ weff, bf16* __restrict__ out) {
+    const PackLayer& L = p.l[blockIdx.y];
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < L.fn + L.bn; i += (long)gridDim.x * blockDim.x) {
+        int n, tap, c;
+        long at;
+        if (i < L.fn) {
+            c = (int)(i % L.cinp);
+            tap = (int)(i / L.cinp % L.tapsp);
+            n = (int)(i / ((long)L.cinp * L.tapsp));
+            at = L.f + i;
+        } else {
+            const long k = i - L.fn;
+            n = (int)(k % L.coutp);
+            c = (int)(k / L.coutp % L.cinp);
+            tap = (int)(k / ((long)L.coutp * L.cinp));
+            at = L.b + k;
+        }
+        const bool ok = n < L.cout && tap < L.taps && c < L.cin;
+        out[at] = __float2bfloat16_rn(ok ? weff[L.woff + ((long)n * L.taps + tap) * L.cin + c] : 0.f);
+    }
+}
+
+// the layers' partial sums, ranges in order, into the gradient vector
+__global__ void grad_sum_kernel(const __grid_constant__ PackArgs p, float* __restrict__ g) {
+    const PackLayer& L = p.l[blockIdx.y];
+    const long nw = (long)L.cout * L.taps * L.cin, slab = (long)L.coutp * L.tapsp * L.cinp;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nw + L.cout; i += (long)gridDim.x * blockDim.x) {
+        float s = 0.f;
+        if (i < nw) {
+            const int c = (int)(i % L.cin), tap = (int)(i / L.cin % L.taps), n = (int)(i / ((long)L.cin * L.taps));
+            const float* q = L.part + ((long)n * L.tapsp + tap) * L.cinp + c;
+#pragma unroll 4
+            for (int z = 0; z < L.ranges; ++z) s += q[z * slab];
+            g[L.woff + i] = s;
+        } else {
+            const int n = (int)(i - nw);
+            if (L.bpart)
+                for (int z = 0; z < L.ranges; ++z) s += L.bpart[(long)z * L.coutp + n];
+            else
+                for (int z = 0; z < L.ranges; ++z) s += L.part[z * slab + n * 16 + 9];
+            g[L.boff + n] = s;
+        }
+    }
+}
+
+// rows idx[b] of a (n x width) table
+__global__ void gather_rows_kernel(const float* __restrict__ src, const int* __restrict__ idx, int rows, int width,
+                                   float* __restrict__ dst) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows * width) return;
+    const int r = i / width, c = i - r * width;
+    dst[i] = src[(long)idx[r] * width + c];
 }
 
 __device__ __forceinline__ void cross3(const float* a, const float* b, float* c) {
@@ -383,28 +889,24 @@ struct Cnn {
     Layer conv[NCONV], fc1, fc2;
     long nparams = 0;
     float *d_w = nullptr, *d_weff = nullptr, *d_g = nullptr, *d_m = nullptr, *d_v = nullptr;
-    int cap = 0;                       // batch capacity of the buffers
-    float* d_in = nullptr;             // cap x box^2
-    float* d_act[NCONV + 1] = {};      // NHWC activations after ReLU (act[0] = input)
-    float* d_h = nullptr;              // fc1 output
+    int cap = 0;                       // images the forward buffers hold
+    int gcap = 0;                      // images the gradient buffers hold
+    float2* d_norm = nullptr;          // mean and 1 / standard deviation of each image
+    bf16 *d_ah[NCONV + 1] = {}, *d_al[NCONV + 1] = {};   // activation planes after ReLU, NHWC (1 .. NCONV)
+    bf16 *d_hh = nullptr, *d_hl = nullptr;               // fc1 output planes
     float* d_o = nullptr;              // fc2 output
-    float* d_col = nullptr;            // im2col scratch
-    float* d_gcol = nullptr;
-    float* d_ga = nullptr;             // activation gradient scratch (two halves)
-    float* d_gb = nullptr;
-    float* d_gh = nullptr;
+    bf16 *d_gh[2] = {}, *d_gl[2] = {}; // activation gradient planes (two, in turn)
+    bf16 *d_dh = nullptr, *d_dl = nullptr;               // gradient of the fc1 output
     float* d_go = nullptr;
-    float* d_part = nullptr;           // split-K partials
-    float* d_ones = nullptr;           // column sums as a GEMM with a ones row
-    long ones_elems = 0;
-    size_t part_elems = 0;
+    float* d_part = nullptr;           // weight-gradient partial sums of every layer
+    bf16* d_pack = nullptr;            // packed weights
+    PackArgs pack{};
+    float* d_src = nullptr;            // host images' copy
+    size_t src_elems = 0;
     float* d_res = nullptr;            // cap x 11
     float* d_tgt = nullptr;            // cap x 11
     float* d_loss = nullptr;           // cap
-    float* d_lossmean = nullptr;       // per step
-    int* d_idx = nullptr;
     long step = 0;                     // Adam steps taken
-    size_t col_elems = 0, act_max = 0;
 };
 
 }  // namespace bsg
@@ -432,160 +934,360 @@ int cfail(int code, const char* fmt, ...) {
 
 unsigned grid_for(long n) { return (unsigned)std::max(1L, std::min(148L * 16, (n + 255) / 256)); }
 
-cudaError_t gemm(Cnn& c, bool at, bool bt, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
-                 float* C, int accumulate, cudaStream_t s);
+int ilog2(int v) { int l = 0; while ((1 << l) < v) ++l; return l; }
 
-// column sums of g (M x N), as ones(1 x M) g: fixed-order split reduction
-cudaError_t colsum(Cnn& c, const float* g, long M, int N, float* out, cudaStream_t s) {
-    return gemm(c, false, true, 1, N, (int)M, c.d_ones, (int)M, g, N, out, 0, s);
+template <int BM, int BN>
+cudaError_t launch_conv(const ConvArgs& a, int nclass, cudaStream_t s) {
+    const dim3 grid((unsigned)((a.M + BM - 1) / BM), (unsigned)(a.N / BN), (unsigned)nclass);
+    conv_gemm_kernel<BM, BN><<<grid, 256, conv_smem<BM, BN>(), s>>>(a);
+    return cudaGetLastError();
 }
 
-cudaError_t gemm(Cnn& c, bool at, bool bt, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
-                 float* C, int accumulate, cudaStream_t s) {
-    dim3 grid((N + TBN - 1) / TBN, (M + TBM - 1) / TBM, 1);
-    int splits = 1;
-    const long tiles = (long)grid.x * grid.y;
-    if (tiles < 148 && K > 4096) {
-        splits = (int)std::min<long>(64, std::max<long>(1, (296 + tiles - 1) / tiles));
-        splits = std::min(splits, std::max(1, K / 1024));
-        if ((size_t)splits * M * N > c.part_elems) splits = std::max(1, (int)(c.part_elems / ((size_t)M * N)));
+// Widest column tile that divides the channels; then the tallest row tile
+// that still gives every SM a block (the deep layers have few pixels: at 256
+// images of 128^2 the last convolution has 1,024 rows, 8 blocks of 128 but
+// 32 of 32).
+cudaError_t conv_gemm(const ConvArgs& a, int nclass, cudaStream_t s) {
+    const long n128 = a.N / 128, rows = a.M;
+    if (a.N % 128 == 0) {
+        if ((rows + 127) / 128 * n128 * nclass >= 148) return launch_conv<128, 128>(a, nclass, s);
+        if ((rows + 63) / 64 * n128 * nclass >= 148) return launch_conv<64, 128>(a, nclass, s);
+        return launch_conv<32, 128>(a, nclass, s);
     }
-    grid.z = splits;
-    float* out = splits > 1 ? c.d_part : C;
-    if (!at && !bt) tgemm_kernel<false, false><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, out, splits, accumulate);
-    else if (!at && bt) tgemm_kernel<false, true><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, out, splits, accumulate);
-    else if (at && !bt) tgemm_kernel<true, false><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, out, splits, accumulate);
-    else tgemm_kernel<true, true><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, out, splits, accumulate);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && splits > 1) {
-        const long cnt = (long)M * N;
-        split_reduce_kernel<<<grid_for(cnt), 256, 0, s>>>(c.d_part, cnt, splits, C, accumulate);
-        e = cudaGetLastError();
+    if (a.N % 64 == 0) {
+        if ((rows + 127) / 128 * (a.N / 64) * nclass >= 148) return launch_conv<128, 64>(a, nclass, s);
+        return launch_conv<64, 64>(a, nclass, s);
     }
+    return launch_conv<128, 32>(a, nclass, s);
+}
+
+template <int BM, int BN>
+cudaError_t conv_attr() {
+    return cudaFuncSetAttribute(conv_gemm_kernel<BM, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem<BM, BN>());
+}
+
+cudaError_t cnn_attributes() {
+    cudaError_t e = conv_attr<128, 128>();
+    if (e == cudaSuccess) e = conv_attr<64, 128>();
+    if (e == cudaSuccess) e = conv_attr<32, 128>();
+    if (e == cudaSuccess) e = conv_attr<128, 64>();
+    if (e == cudaSuccess) e = conv_attr<64, 64>();
+    if (e == cudaSuccess) e = conv_attr<128, 32>();
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(wgrad_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<64>());
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(wgrad_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, wgrad_smem<32>());
     return e;
+}
+
+// forward and input-gradient forms of the layers' weights
+cudaError_t pack_weights(Cnn& c, cudaStream_t s) {
+    pack_kernel<<<dim3(148, NPACK), 256, 0, s>>>(c.pack, c.d_weff, c.d_pack);
+    return cudaGetLastError();
+}
+
+void plan_pack(Cnn& c) {
+    long off = 0;
+    auto take = [&](long n) { const long o = off; off += (n + 7) / 8 * 8; return o; };
+    c.pack.n = NPACK;
+    for (int l = 0; l < NPACK; ++l) {
+        PackLayer& P = c.pack.l[l];
+        const Layer& L = l < NCONV ? c.conv[l] : l == NCONV ? c.fc1 : c.fc2;
+        P.woff = L.woff;
+        P.boff = L.boff;
+        P.cout = L.cout;
+        P.coutp = l == NCONV + 1 ? NOUT : cpad(L.cout);
+        if (l < NCONV) {
+            P.cin = L.cin;
+            P.taps = 9;
+            P.cinp = l ? cpad(L.cin) : 1;
+            P.tapsp = l ? 9 : 16;
+        } else if (l == NCONV) {
+            // (pixel, channel) of the last activation
+            P.cin = c.conv[NCONV - 1].cout;
+            P.cinp = cpad(P.cin);
+            P.taps = P.tapsp = (int)(L.k / P.cin);
+        } else {
+            P.cin = (int)L.k;
+            P.cinp = cpad(P.cin);
+            P.taps = P.tapsp = 1;
+        }
+        P.fn = (long)P.coutp * P.tapsp * P.cinp;
+        P.f = take(P.fn);
+        P.bn = l > 0 && l <= NCONV ? P.fn : 0;
+        P.b = take(P.bn);
+    }
+}
+
+long pack_elems(const Cnn& c) {
+    const PackLayer& P = c.pack.l[NPACK - 1];
+    return P.b + P.bn + 8;
+}
+
+// planes of one image's activations, in elements of one plane
+size_t act_elems(const Cnn& c, int l) { return (size_t)c.conv[l].ho * c.conv[l].wo * cpad(c.conv[l].cout); }
+
+size_t image_bytes(const Cnn& c) {
+    size_t b = 4 * (size_t)cpad(c.cfg.hidden);
+    for (int l = 0; l < NCONV; ++l) b += 4 * act_elems(c, l);
+    return b;
+}
+
+void free_forward(Cnn& c) {
+    auto F = [](auto*& p) { cudaFree(p); p = nullptr; };
+    for (int l = 1; l <= NCONV; ++l) { F(c.d_ah[l]); F(c.d_al[l]); }
+    F(c.d_hh); F(c.d_hl); F(c.d_o); F(c.d_norm); F(c.d_res);
+    c.cap = 0;
 }
 
 int ensure_batch(Cnn& c, int B) {
     if (B <= c.cap) return BSG_OK;
-    auto F = [](float*& p) { cudaFree(p); p = nullptr; };
-    F(c.d_in); for (auto& a : c.d_act) F(a);
-    F(c.d_h); F(c.d_o); F(c.d_col); F(c.d_gcol); F(c.d_ga); F(c.d_gb); F(c.d_gh); F(c.d_go); F(c.d_part);
-    F(c.d_res); F(c.d_tgt); F(c.d_loss); F(c.d_ones);
-    cudaFree(c.d_idx); c.d_idx = nullptr;
-    const int box = c.cfg.box;
-    size_t col = 0, act = (size_t)box * box;
+    free_forward(c);
+    const size_t n = (size_t)B;
     for (int l = 0; l < NCONV; ++l) {
-        const Layer& L = c.conv[l];
-        col = std::max(col, (size_t)L.ho * L.wo * L.k);
-        act = std::max(act, (size_t)L.ho * L.wo * L.cout);
+        CCK(cudaMalloc(&c.d_ah[l + 1], sizeof(bf16) * act_elems(c, l) * n));
+        CCK(cudaMalloc(&c.d_al[l + 1], sizeof(bf16) * act_elems(c, l) * n));
     }
-    c.col_elems = col * B;
-    c.act_max = act * B;
-    CCK(cudaMalloc(&c.d_in, sizeof(float) * (size_t)box * box * B));
-    c.d_act[0] = c.d_in;
-    for (int l = 0; l < NCONV; ++l) {
-        const Layer& L = c.conv[l];
-        CCK(cudaMalloc(&c.d_act[l + 1], sizeof(float) * (size_t)L.ho * L.wo * L.cout * B));
-    }
-    CCK(cudaMalloc(&c.d_h, sizeof(float) * (size_t)c.cfg.hidden * B));
-    CCK(cudaMalloc(&c.d_o, sizeof(float) * NOUT * B));
-    CCK(cudaMalloc(&c.d_col, sizeof(float) * c.col_elems));
-    CCK(cudaMalloc(&c.d_gcol, sizeof(float) * c.col_elems));
-    CCK(cudaMalloc(&c.d_ga, sizeof(float) * c.act_max));
-    CCK(cudaMalloc(&c.d_gb, sizeof(float) * c.act_max));
-    CCK(cudaMalloc(&c.d_gh, sizeof(float) * (size_t)c.cfg.hidden * B));
-    CCK(cudaMalloc(&c.d_go, sizeof(float) * NOUT * B));
-    c.part_elems = std::max<size_t>((size_t)1 << 22, (size_t)c.cfg.hidden * 1024 * 4);
-    CCK(cudaMalloc(&c.d_part, sizeof(float) * c.part_elems));
-    CCK(cudaMalloc(&c.d_res, sizeof(float) * NRES * B));
-    CCK(cudaMalloc(&c.d_tgt, sizeof(float) * NRES * B));
-    CCK(cudaMalloc(&c.d_loss, sizeof(float) * B));
-    CCK(cudaMalloc(&c.d_idx, sizeof(int) * B));
-    c.ones_elems = (long)B * (box / 2) * (box / 2);
-    CCK(cudaMalloc(&c.d_ones, sizeof(float) * c.ones_elems));
-    fill_kernel<<<grid_for(c.ones_elems), 256>>>(c.d_ones, c.ones_elems, 1.f);
-    CCK(cudaGetLastError());
-    CCK(cudaDeviceSynchronize());
+    CCK(cudaMalloc(&c.d_hh, sizeof(bf16) * cpad(c.cfg.hidden) * n));
+    CCK(cudaMalloc(&c.d_hl, sizeof(bf16) * cpad(c.cfg.hidden) * n));
+    CCK(cudaMalloc(&c.d_o, sizeof(float) * NOUT * n));
+    CCK(cudaMalloc(&c.d_norm, sizeof(float2) * n));
+    CCK(cudaMalloc(&c.d_res, sizeof(float) * NRES * n));
     c.cap = B;
     return BSG_OK;
 }
 
-// forward pass of B images already in c.d_in (normalised)
-cudaError_t forward(Cnn& c, int B, cudaStream_t s) {
-    cudaError_t e = cudaSuccess;
-    for (int l = 0; l < NCONV && e == cudaSuccess; ++l) {
-        const Layer& L = c.conv[l];
-        const long M = (long)B * L.ho * L.wo;
-        im2col_kernel<<<grid_for(M * L.k), 256, 0, s>>>(c.d_act[l], B, L.h, L.w, L.cin, L.ho, L.wo, c.d_col);
-        e = cudaGetLastError();
-        if (e == cudaSuccess)
-            e = gemm(c, false, false, (int)M, L.cout, (int)L.k, c.d_col, (int)L.k, c.d_weff + L.woff, (int)L.k,
-                     c.d_act[l + 1], 0, s);
-        if (e == cudaSuccess) {
-            bias_act_kernel<<<grid_for(M * L.cout), 256, 0, s>>>(c.d_act[l + 1], M, L.cout, c.d_weff + L.boff, 1);
-            e = cudaGetLastError();
-        }
-    }
-    const Layer& F1 = c.fc1;
-    const Layer& F2 = c.fc2;
-    if (e == cudaSuccess)
-        e = gemm(c, false, false, B, F1.cout, (int)F1.k, c.d_act[NCONV], (int)F1.k, c.d_weff + F1.woff, (int)F1.k, c.d_h,
-                 0, s);
-    if (e == cudaSuccess) {
-        bias_act_kernel<<<grid_for((long)B * F1.cout), 256, 0, s>>>(c.d_h, B, F1.cout, c.d_weff + F1.boff, 1);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess)
-        e = gemm(c, false, false, B, F2.cout, (int)F2.k, c.d_h, (int)F2.k, c.d_weff + F2.woff, (int)F2.k, c.d_o, 0, s);
-    if (e == cudaSuccess) {
-        bias_act_kernel<<<grid_for((long)B * F2.cout), 256, 0, s>>>(c.d_o, B, F2.cout, c.d_weff + F2.boff, 0);
-        e = cudaGetLastError();
-    }
-    return e;
+// pixel ranges of a layer's weight gradient: about four CTAs per SM, each
+// with at least eight K-steps (a function of the sizes only: the sums'
+// order is fixed)
+int wgrad_ranges(long ctas, int steps) {
+    return (int)std::max<long>(1, std::min<long>((4 * 148 + ctas - 1) / ctas, steps / 8));
 }
 
-// gradients of the batch loss into c.d_g (overwritten), from c.d_go
-cudaError_t backward(Cnn& c, int B, cudaStream_t s) {
-    const Layer& F1 = c.fc1;
-    const Layer& F2 = c.fc2;
-    const int H = c.cfg.hidden;
-    // fc2: dW2 = go^T h, db2 = sum go, dh = go W2
-    cudaError_t e = gemm(c, true, true, F2.cout, H, B, c.d_go, NOUT, c.d_h, H, c.d_g + F2.woff, 0, s);
-    if (e == cudaSuccess) e = colsum(c, c.d_go, B, NOUT, c.d_g + F2.boff, s);
-    if (e == cudaSuccess) e = gemm(c, false, true, B, H, NOUT, c.d_go, NOUT, c.d_weff + F2.woff, H, c.d_gh, 0, s);
-    if (e == cudaSuccess) { relu_back_kernel<<<grid_for((long)B * H), 256, 0, s>>>(c.d_gh, c.d_h, (long)B * H); e = cudaGetLastError(); }
-    // fc1: dW1 = gh^T a6, db1, da6 = gh W1
-    const int K1 = (int)F1.k;
-    if (e == cudaSuccess) e = gemm(c, true, true, H, K1, B, c.d_gh, H, c.d_act[NCONV], K1, c.d_g + F1.woff, 0, s);
-    if (e == cudaSuccess) e = colsum(c, c.d_gh, B, H, c.d_g + F1.boff, s);
-    float* ga = c.d_ga;   // gradient w.r.t. act[l+1]
-    float* gb = c.d_gb;
-    if (e == cudaSuccess) e = gemm(c, false, true, B, K1, H, c.d_gh, H, c.d_weff + F1.woff, K1, ga, 0, s);
-    for (int l = NCONV - 1; l >= 0 && e == cudaSuccess; --l) {
-        const Layer& L = c.conv[l];
-        const long M = (long)B * L.ho * L.wo;
-        relu_back_kernel<<<grid_for(M * L.cout), 256, 0, s>>>(ga, c.d_act[l + 1], M * L.cout);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = colsum(c, ga, M, L.cout, c.d_g + L.boff, s);
-        if (e == cudaSuccess) {
-            im2col_kernel<<<grid_for(M * L.k), 256, 0, s>>>(c.d_act[l], B, L.h, L.w, L.cin, L.ho, L.wo, c.d_col);
-            e = cudaGetLastError();
+struct WgradPlan {
+    int steps, per, ranges, bn;
+    unsigned gy;
+};
+
+WgradPlan wgrad_plan(long M, int N, int C, int ntap) {
+    WgradPlan p;
+    p.steps = (int)((M + 31) / 32);
+    p.bn = C % 64 == 0 ? 64 : 32;
+    p.gy = (unsigned)((N + 63) / 64) * (unsigned)((C + p.bn - 1) / p.bn);
+    const int want = wgrad_ranges((long)ntap * p.gy, p.steps);
+    p.per = (p.steps + want - 1) / want;
+    p.ranges = (p.steps + p.per - 1) / p.per;
+    return p;
+}
+
+constexpr int W1_PER = 8;      // first layer: patches of 256 pixels per CTA
+
+void free_grad(Cnn& c) {
+    auto F = [](auto*& p) { cudaFree(p); p = nullptr; };
+    for (int i = 0; i < 2; ++i) { F(c.d_gh[i]); F(c.d_gl[i]); }
+    F(c.d_dh); F(c.d_dl); F(c.d_go); F(c.d_tgt); F(c.d_loss); F(c.d_part);
+    c.gcap = 0;
+}
+
+// gradient buffers, and room for the layers' partial sums
+int ensure_grad(Cnn& c, int B) {
+    if (B > c.gcap) {
+        free_grad(c);
+        size_t act = 0;
+        for (int l = 0; l < NCONV; ++l) act = std::max(act, act_elems(c, l));
+        for (int i = 0; i < 2; ++i) {
+            CCK(cudaMalloc(&c.d_gh[i], sizeof(bf16) * act * B));
+            CCK(cudaMalloc(&c.d_gl[i], sizeof(bf16) * act * B));
         }
-        // dW = dY^T X_col  (Cout x K, reduced over M)
-        if (e == cudaSuccess)
-            e = gemm(c, true, true, L.cout, (int)L.k, (int)M, ga, L.cout, c.d_col, (int)L.k, c.d_g + L.woff, 0, s);
-        if (l > 0 && e == cudaSuccess) {
-            // dX_col = dY W  (M x K), then col2im into the previous activation's gradient
-            e = gemm(c, false, true, (int)M, (int)L.k, L.cout, ga, L.cout, c.d_weff + L.woff, (int)L.k, c.d_gcol, 0, s);
-            if (e == cudaSuccess) {
-                const long nx = (long)B * L.h * L.w * L.cin;
-                col2im_kernel<<<grid_for(nx), 256, 0, s>>>(c.d_gcol, B, L.h, L.w, L.cin, L.ho, L.wo, gb);
-                e = cudaGetLastError();
+        CCK(cudaMalloc(&c.d_dh, sizeof(bf16) * cpad(c.cfg.hidden) * (size_t)B));
+        CCK(cudaMalloc(&c.d_dl, sizeof(bf16) * cpad(c.cfg.hidden) * (size_t)B));
+        CCK(cudaMalloc(&c.d_go, sizeof(float) * NOUT * B));
+        CCK(cudaMalloc(&c.d_tgt, sizeof(float) * NRES * B));
+        CCK(cudaMalloc(&c.d_loss, sizeof(float) * B));
+        // the most any batch up to B needs: the ranges grow with the batch
+        size_t elems = 0;
+        for (int l = 0; l <= NCONV; ++l) {
+            const PackLayer& P = c.pack.l[l];
+            if (l == 0) {
+                const long patches = (long)B * ((c.conv[0].ho * c.conv[0].wo) / C1PIX);
+                elems += (size_t)((patches + W1_PER - 1) / W1_PER) * P.coutp * 16;
+                continue;
             }
-            std::swap(ga, gb);
+            const long M = l < NCONV ? (long)B * c.conv[l].ho * c.conv[l].wo : B;
+            const int ntap = l < NCONV ? 9 : 1, C = l < NCONV ? P.cinp : P.tapsp * P.cinp;
+            const WgradPlan w = wgrad_plan(M, P.coutp, C, ntap);
+            elems += (size_t)wgrad_ranges((long)ntap * w.gy, w.steps) * (P.fn + P.coutp);
         }
+        CCK(cudaMalloc(&c.d_part, sizeof(float) * elems));
+        c.gcap = B;
     }
-    return e;
+    return BSG_OK;
+}
+
+int ensure_src(Cnn& c, size_t elems) {
+    if (elems <= c.src_elems) return BSG_OK;
+    cudaFree(c.d_src);
+    c.d_src = nullptr;
+    c.src_elems = 0;
+    CCK(cudaMalloc(&c.d_src, sizeof(float) * elems));
+    c.src_elems = elems;
+    return BSG_OK;
+}
+
+size_t patch_bytes(int wo) { return sizeof(float) * (2 * (C1PIX / wo) + 1) * (2 * wo + 4); }
+
+// forward pass of B images: data (and idx, the batch's images within it, or
+// null) on the device; outputs in c.d_o
+cudaError_t forward(Cnn& c, const float* data, const int* idx, int B, cudaStream_t s) {
+    const int box = c.cfg.box;
+    image_norm_kernel<<<B, 256, 0, s>>>(data, idx, box * box, c.d_norm);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    {
+        const Layer& L = c.conv[0];
+        const PackLayer& P = c.pack.l[0];
+        const dim3 grid((unsigned)((long)B * ((L.ho * L.wo) / C1PIX)), (unsigned)(P.coutp / 32));
+        conv1_kernel<<<grid, 256, patch_bytes(L.wo), s>>>(data, idx, c.d_norm, ilog2(L.wo), c.d_pack + P.f,
+                                                          c.d_weff + L.boff, L.cout, P.coutp, c.d_ah[1], c.d_al[1]);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    for (int l = 1; l <= NCONV; ++l) {
+        const PackLayer& P = c.pack.l[l];
+        const bool fc = l == NCONV;
+        const Layer& L = fc ? c.fc1 : c.conv[l];
+        ConvArgs a{};
+        a.ah = c.d_ah[l];
+        a.al = c.d_al[l];
+        a.w = c.d_pack + P.f;
+        a.C = fc ? P.tapsp * P.cinp : P.cinp;
+        a.wrow = (long)P.tapsp * P.cinp;
+        a.wtap = P.cinp;
+        a.M = B * L.ho * L.wo;
+        a.N = P.coutp;
+        a.logw = a.logh = ilog2(L.wo);
+        a.H = a.W = L.h;
+        a.stride = fc ? 1 : 2;
+        a.oh = fc ? c.d_hh : c.d_ah[l + 1];
+        a.ol = fc ? c.d_hl : c.d_al[l + 1];
+        a.OH = a.OW = L.ho;
+        a.ostride = 1;
+        a.bias = c.d_weff + P.boff;
+        a.nbias = P.cout;
+        a.relu = 1;
+        ConvClass& k = a.cls[0];
+        k.ntap = fc ? 1 : 9;
+        for (int t = 0; t < k.ntap; ++t) {
+            k.dy[t] = (signed char)(fc ? 0 : t / 3 - 1);
+            k.dx[t] = (signed char)(fc ? 0 : t % 3 - 1);
+            k.w[t] = (signed char)t;
+        }
+        if ((e = conv_gemm(a, 1, s)) != cudaSuccess) return e;
+    }
+    const PackLayer& P = c.pack.l[NCONV + 1];
+    fc2_kernel<<<(B + 15) / 16, 32, 0, s>>>(c.d_hh, c.d_hl, B, P.cinp, c.d_pack + P.f, c.d_weff + P.boff, c.d_o);
+    return cudaGetLastError();
+}
+
+// gradients of the batch loss into c.d_g (overwritten), from c.d_go; the
+// batch as given to forward
+cudaError_t backward(Cnn& c, const float* data, const int* idx, int B, cudaStream_t s) {
+    const int Hp = cpad(c.cfg.hidden);
+    const PackLayer& P2 = c.pack.l[NCONV + 1];
+    fc2_wgrad_kernel<<<Hp / 32, 256, 0, s>>>(c.d_go, B, c.cfg.hidden, Hp, c.d_hh, c.d_hl, c.d_g + P2.woff,
+                                             c.d_g + P2.boff);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    fc2_dgrad_kernel<<<(unsigned)(((long)B * Hp + 255) / 256), 256, 0, s>>>(c.d_go, B, c.cfg.hidden, Hp,
+                                                                            c.d_weff + P2.woff, c.d_hh, c.d_dh, c.d_dl);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    PackArgs sums = c.pack;
+    float* part = c.d_part;
+    const bf16 *yh = c.d_dh, *yl = c.d_dl;                    // gradient of layer l's output
+    for (int l = NCONV; l >= 1; --l) {
+        PackLayer& P = sums.l[l];
+        const bool fc = l == NCONV;
+        const Layer& L = fc ? c.fc1 : c.conv[l];
+        WgradArgs w{};
+        w.yh = yh;
+        w.yl = yl;
+        w.xh = c.d_ah[l];
+        w.xl = c.d_al[l];
+        w.M = B * L.ho * L.wo;
+        w.N = P.coutp;
+        w.C = fc ? P.tapsp * P.cinp : P.cinp;
+        w.logw = w.logh = ilog2(L.wo);
+        w.H = w.W = L.h;
+        w.stride = fc ? 1 : 2;
+        w.ntap = fc ? 1 : 9;
+        const WgradPlan p = wgrad_plan(w.M, w.N, w.C, w.ntap);
+        w.steps = p.steps;
+        w.per = p.per;
+        w.part = part;
+        w.bpart = part + (size_t)p.ranges * P.fn;
+        part = w.bpart + (size_t)p.ranges * P.coutp;
+        P.part = w.part;
+        P.bpart = w.bpart;
+        P.ranges = p.ranges;
+        const dim3 grid((unsigned)w.ntap, p.gy, (unsigned)p.ranges);
+        if (p.bn == 64) wgrad_kernel<64><<<grid, 128, wgrad_smem<64>(), s>>>(w);
+        else wgrad_kernel<32><<<grid, 128, wgrad_smem<32>(), s>>>(w);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        // input gradient, masked by the ReLU of the layer below
+        ConvArgs a{};
+        a.ah = yh;
+        a.al = yl;
+        a.w = c.d_pack + P.b;
+        a.wrow = P.coutp;
+        a.wtap = (long)P.cinp * P.coutp;
+        a.C = P.coutp;
+        a.N = fc ? P.tapsp * P.cinp : P.cinp;
+        a.M = B * L.ho * L.wo;
+        a.logw = a.logh = ilog2(L.wo);
+        a.H = a.W = L.ho;
+        a.stride = 1;
+        a.oh = c.d_gh[l & 1];
+        a.ol = c.d_gl[l & 1];
+        a.OH = a.OW = fc ? 1 : L.h;
+        a.ostride = fc ? 1 : 2;
+        a.mask = c.d_ah[l];
+        int ncls = 0;
+        if (fc) {
+            a.cls[0].ntap = 1;
+            ncls = 1;
+        } else {
+            // input pixel 2 y + py takes the taps ky = py + 1 (mod 2) from
+            // output row y + (py + 1 - ky) / 2; the class with most taps first
+            for (int py = 1; py >= 0; --py)
+                for (int px = 1; px >= 0; --px) {
+                    ConvClass& k = a.cls[ncls++];
+                    k.oy = py;
+                    k.ox = px;
+                    for (int ky = 0; ky < 3; ++ky)
+                        for (int kx = 0; kx < 3; ++kx) {
+                            if (((py + 1 - ky) & 1) || ((px + 1 - kx) & 1)) continue;
+                            k.dy[k.ntap] = (signed char)((py + 1 - ky) / 2);
+                            k.dx[k.ntap] = (signed char)((px + 1 - kx) / 2);
+                            k.w[k.ntap++] = (signed char)(ky * 3 + kx);
+                        }
+                }
+        }
+        if ((e = conv_gemm(a, ncls, s)) != cudaSuccess) return e;
+        yh = a.oh;
+        yl = a.ol;
+    }
+    {
+        PackLayer& P = sums.l[0];
+        const Layer& L = c.conv[0];
+        const int patches = B * ((L.ho * L.wo) / C1PIX);
+        P.ranges = (patches + W1_PER - 1) / W1_PER;
+        P.part = part;
+        P.bpart = nullptr;
+        wgrad1_kernel<<<dim3((unsigned)P.ranges, (unsigned)(P.coutp / 32)), 256, patch_bytes(L.wo), s>>>(
+            data, idx, c.d_norm, ilog2(L.wo), yh, yl, P.coutp, patches, W1_PER, part);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    grad_sum_kernel<<<dim3(148, NCONV + 1), 256, 0, s>>>(sums, c.d_g);
+    return cudaGetLastError();
 }
 
 uint64_t splitmix(uint64_t& x) {
@@ -654,7 +1356,9 @@ extern "C" int bsg_cnn_create(const bsg_cnn_config* cfg, bsg_cnn** out) {
     if (e == cudaSuccess) e = cudaMalloc(&c->d_g, sizeof(float) * off);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_m, sizeof(float) * off);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_v, sizeof(float) * off);
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_lossmean, sizeof(float) * 1);
+    plan_pack(*c);
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_pack, sizeof(bf16) * pack_elems(*c));
+    if (e == cudaSuccess) e = cnn_attributes();
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_w, w.data(), sizeof(float) * off, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_m, 0, sizeof(float) * off, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->d_v, 0, sizeof(float) * off, c->stream);
@@ -662,6 +1366,7 @@ extern "C" int bsg_cnn_create(const bsg_cnn_config* cfg, bsg_cnn** out) {
         round_bf16_kernel<<<grid_for(off), 256, 0, c->stream>>>(c->d_w, c->d_weff, off);
         e = cudaGetLastError();
     }
+    if (e == cudaSuccess) e = pack_weights(*c, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         bsg_cnn_destroy(reinterpret_cast<bsg_cnn*>(c));
@@ -676,12 +1381,11 @@ extern "C" void bsg_cnn_destroy(bsg_cnn* h) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    float* fp[] = {c->d_w, c->d_weff, c->d_g, c->d_m, c->d_v, c->d_in, c->d_h, c->d_o, c->d_col, c->d_gcol,
-                   c->d_ga, c->d_gb, c->d_gh, c->d_go, c->d_part, c->d_res, c->d_tgt, c->d_loss, c->d_lossmean,
-                   c->d_ones};
+    free_forward(*c);
+    free_grad(*c);
+    float* fp[] = {c->d_w, c->d_weff, c->d_g, c->d_m, c->d_v, c->d_src};
     for (float* p : fp) if (p) cudaFree(p);
-    for (int l = 1; l <= NCONV; ++l) if (c->d_act[l]) cudaFree(c->d_act[l]);
-    if (c->d_idx) cudaFree(c->d_idx);
+    if (c->d_pack) cudaFree(c->d_pack);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -706,6 +1410,7 @@ extern "C" int bsg_cnn_set_params(bsg_cnn* h, const float* in) {
     CCK(cudaMemcpyAsync(c->d_w, in, sizeof(float) * c->nparams, cudaMemcpyHostToDevice, c->stream));
     round_bf16_kernel<<<grid_for(c->nparams), 256, 0, c->stream>>>(c->d_w, c->d_weff, c->nparams);
     CCK(cudaGetLastError());
+    CCK(pack_weights(*c, c->stream));
     CCK(cudaMemsetAsync(c->d_m, 0, sizeof(float) * c->nparams, c->stream));
     CCK(cudaMemsetAsync(c->d_v, 0, sizeof(float) * c->nparams, c->stream));
     c->step = 0;
@@ -717,39 +1422,43 @@ extern "C" int bsg_cnn_predict(bsg_cnn* h, const float* images, long n, float* o
     Cnn* c = reinterpret_cast<Cnn*>(h);
     if (!c || !images || !out || n < 1) return cfail(BSG_ERR_ARG, "bsg_cnn_predict: bad argument");
     CCK(cudaSetDevice(c->device));
-    const int B = std::max(1, std::min<int>(c->cfg.batch > 0 ? c->cfg.batch : 256, (int)std::min<long>(n, 1 << 20)));
-    int rc = ensure_batch(*c, B);
-    if (rc) return rc;
+    // images per pass: at least the context's batch; as many as 1.5 GB of
+    // activations hold when they fit (each image's result is its own).  2,048
+    // images of 128^2 in passes of 256 leave the deep layers with 8 to 32
+    // blocks for 148 SMs.
+    int B = std::max(1, std::min<int>(c->cfg.batch > 0 ? c->cfg.batch : 256, (int)std::min<long>(n, 1 << 20)));
+    const long wide = std::min<long>(std::min<long>(n, 16384), (long)(1500000000 / image_bytes(*c)));
+    int rc = BSG_OK;
+    if (wide > B && ensure_batch(*c, (int)wide) == BSG_OK) {
+        B = (int)wide;
+    } else {
+        cudaGetLastError();                      // the wide buffers did not fit
+        rc = ensure_batch(*c, B);
+        if (rc) return rc;
+    }
     const int npix = c->cfg.box * c->cfg.box;
     cudaStream_t s = c->stream;
-    float* d_src = nullptr;
-    float* d_out = nullptr;
-    if (!(flags & BSG_DEVICE_PTR)) {
-        CCK(cudaMalloc(&d_src, sizeof(float) * (size_t)npix * B));
-        CCK(cudaMalloc(&d_out, sizeof(float) * NRES * B));
-    }
+    const bool dev = (flags & BSG_DEVICE_PTR) != 0;
+    if (!dev && (rc = ensure_src(*c, (size_t)npix * B))) return rc;
     cudaError_t e = cudaSuccess;
     for (long b0 = 0; e == cudaSuccess && b0 < n; b0 += B) {
         const int cnt = (int)std::min<long>(B, n - b0);
         const float* src = images + (size_t)b0 * npix;
-        if (!(flags & BSG_DEVICE_PTR)) {
-            e = cudaMemcpyAsync(d_src, src, sizeof(float) * (size_t)npix * cnt, cudaMemcpyHostToDevice, s);
-            src = d_src;
+        if (!dev) {
+            e = cudaMemcpyAsync(c->d_src, src, sizeof(float) * (size_t)npix * cnt, cudaMemcpyHostToDevice, s);
+            src = c->d_src;
         }
-        if (e == cudaSuccess) { gather_norm_kernel<<<cnt, 256, 0, s>>>(src, nullptr, npix, c->d_in); e = cudaGetLastError(); }
-        if (e == cudaSuccess) e = forward(*c, cnt, s);
-        float* res = (flags & BSG_DEVICE_PTR) ? out + (size_t)b0 * NRES : d_out;
+        if (e == cudaSuccess) e = forward(*c, src, nullptr, cnt, s);
+        float* res = dev ? out + (size_t)b0 * NRES : c->d_res;
         if (e == cudaSuccess) {
             head_kernel<<<(cnt + 127) / 128, 128, 0, s>>>(c->d_o, cnt, nullptr, 0.f, res, nullptr, nullptr);
             e = cudaGetLastError();
         }
-        if (e == cudaSuccess && !(flags & BSG_DEVICE_PTR))
-            e = cudaMemcpyAsync(out + (size_t)b0 * NRES, d_out, sizeof(float) * NRES * cnt, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && !(flags & BSG_DEVICE_PTR)) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess && !dev)
+            e = cudaMemcpyAsync(out + (size_t)b0 * NRES, res, sizeof(float) * NRES * cnt, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess && !dev) e = cudaStreamSynchronize(s);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_src);
-    cudaFree(d_out);
     if (e != cudaSuccess) return cfail(BSG_ERR_CUDA, "bsg_cnn_predict: %s", cudaGetErrorString(e));
     return BSG_OK;
 }
@@ -761,25 +1470,23 @@ extern "C" int bsg_cnn_loss_grad(bsg_cnn* h, const float* images, const float* t
     CCK(cudaSetDevice(c->device));
     const int B = (int)n;
     int rc = ensure_batch(*c, B);
+    if (!rc) rc = ensure_grad(*c, B);
     if (rc) return rc;
     const int npix = c->cfg.box * c->cfg.box;
     cudaStream_t s = c->stream;
-    float* d_src = nullptr;
-    CCK(cudaMalloc(&d_src, sizeof(float) * (size_t)npix * B));
-    cudaError_t e = cudaMemcpyAsync(d_src, images, sizeof(float) * (size_t)npix * B, cudaMemcpyHostToDevice, s);
+    if ((rc = ensure_src(*c, (size_t)npix * B))) return rc;
+    cudaError_t e = cudaMemcpyAsync(c->d_src, images, sizeof(float) * (size_t)npix * B, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(c->d_tgt, targets, sizeof(float) * NRES * B, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) { gather_norm_kernel<<<B, 256, 0, s>>>(d_src, nullptr, npix, c->d_in); e = cudaGetLastError(); }
-    if (e == cudaSuccess) e = forward(*c, B, s);
+    if (e == cudaSuccess) e = forward(*c, c->d_src, nullptr, B, s);
     if (e == cudaSuccess) {
         head_kernel<<<(B + 127) / 128, 128, 0, s>>>(c->d_o, B, c->d_tgt, c->cfg.shift_weight, c->d_res, c->d_go, c->d_loss);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = backward(*c, B, s);
+    if (e == cudaSuccess) e = backward(*c, c->d_src, nullptr, B, s);
     std::vector<float> l(B);
     if (e == cudaSuccess) e = cudaMemcpyAsync(l.data(), c->d_loss, sizeof(float) * B, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && grads) e = cudaMemcpyAsync(grads, c->d_g, sizeof(float) * c->nparams, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_src);
     if (e != cudaSuccess) return cfail(BSG_ERR_CUDA, "bsg_cnn_loss_grad: %s", cudaGetErrorString(e));
     if (loss) {
         double t = 0;
@@ -799,8 +1506,8 @@ extern "C" int bsg_cnn_train(bsg_cnn* h, const float* images, const float* targe
     CCK(cudaSetDevice(c->device));
     const int B = std::max(1, c->cfg.batch > 0 ? c->cfg.batch : 256);
     int rc = ensure_batch(*c, B);
+    if (!rc) rc = ensure_grad(*c, B);
     if (rc) return rc;
-    const int npix = c->cfg.box * c->cfg.box;
     cudaStream_t s = c->stream;
     // mini-batch indices for every step (seeded, sampled without replacement
     // within each pass over the data)
@@ -824,23 +1531,23 @@ extern "C" int bsg_cnn_train(bsg_cnn* h, const float* images, const float* targe
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     for (int t = 0; e == cudaSuccess && t < steps; ++t) {
         const int* bi = d_all + (size_t)t * B;
-        gather_norm_kernel<<<B, 256, 0, s>>>(images, bi, npix, c->d_in);
         gather_rows_kernel<<<(B * NRES + 255) / 256, 256, 0, s>>>(targets, bi, B, NRES, c->d_tgt);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = forward(*c, B, s);
+        if (e == cudaSuccess) e = forward(*c, images, bi, B, s);
         if (e == cudaSuccess) {
             head_kernel<<<(B + 127) / 128, 128, 0, s>>>(c->d_o, B, c->d_tgt, c->cfg.shift_weight, c->d_res, c->d_go,
                                                         c->d_loss);
             mean_kernel<<<1, 32, 0, s>>>(c->d_loss, B, d_losses + t);
             e = cudaGetLastError();
         }
-        if (e == cudaSuccess) e = backward(*c, B, s);
+        if (e == cudaSuccess) e = backward(*c, images, bi, B, s);
         if (e == cudaSuccess) {
             ++c->step;
             const float c1 = 1.f / (1.f - powf(b1, (float)c->step)), c2 = 1.f / (1.f - powf(b2, (float)c->step));
             adam_kernel<<<grid_for(c->nparams), 256, 0, s>>>(c->d_w, c->d_weff, c->d_g, c->d_m, c->d_v, c->nparams, lr,
                                                              b1, b2, eps, c1, c2);
             e = cudaGetLastError();
+            if (e == cudaSuccess) e = pack_weights(*c, s);
         }
     }
     if (e == cudaSuccess && losses) e = cudaMemcpyAsync(losses, d_losses, sizeof(float) * steps, cudaMemcpyDeviceToHost, s);
