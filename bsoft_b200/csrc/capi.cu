@@ -27,8 +27,6 @@ void set_error(const char* fmt, ...) {
 
 cudaError_t prepare_fft2d_attributes();
 cudaError_t prepare_finish_attributes();
-cudaError_t launch_weigh(const Context& c, int imap, cudaStream_t s);
-cudaError_t launch_ifft3(const Context& c, float2* vol, float* real_out, bool sinc, cudaStream_t s);
 int insert_num_shapes();
 void insert_shape(int i, int* tx, int* ty, int* tz);
 cudaError_t prepare_insert_attributes();
@@ -280,7 +278,6 @@ static void free_all(Recon* r) {
     for (int i = 0; i < 2; ++i) {
         F(r->d_imgbuf[i]); F(r->d_vol[i]); F(r->d_w[i]); F(r->d_pow[i]); F(r->d_w2[i]);
         F(r->d_evol[i]); F(r->d_ew[i]);
-        F(r->d_half_weighed[i]);
         F(r->d_partbuf[i]); F(r->d_psymbuf[i]); F(r->d_specbuf[i]);
         if (r->h_partbuf[i]) cudaFreeHost(r->h_partbuf[i]);
         if (r->copy_done[i]) cudaEventDestroy(r->copy_done[i]);
@@ -288,7 +285,7 @@ static void free_all(Recon* r) {
         if (r->compute_done[i]) cudaEventDestroy(r->compute_done[i]);
     }
     F(r->d_bkg); F(r->d_phase); F(r->d_rows); F(r->d_tw); F(r->d_twmap);
-    F(r->d_work); F(r->d_map); F(r->d_fom); F(r->d_fsc); F(r->d_tile_order); F(r->d_part_sums); F(r->d_symtmp);
+    F(r->d_work); F(r->d_map); F(r->d_fom); F(r->d_sinc); F(r->d_fsc); F(r->d_tile_order); F(r->d_part_sums); F(r->d_symtmp);
     if (r->h_status) cudaFreeHost(r->h_status);
     for (auto& t : r->timed) { cudaEventDestroy(t.a); cudaEventDestroy(t.b); }
     r->timed.clear();
@@ -659,12 +656,19 @@ int bsg_recon_finish(bsg_recon* h, int imap, float* map_out, float* fom_out, int
     const bool dev = (flags & BSG_DEVICE_PTR) != 0;
     float* dst = dev ? map_out : r->d_map;
     const bool symz = !r->symz_orders.empty(), resc = r->rescale_std > 0;
-    CK(launch_weigh(*r, imap, r->stream));
     // with symmetrization after reconstruction (mode 1) and rescaling, the
     // sinc weight follows them, as breconstruct applies filter_sinc to the
     // written map (breconstruct.cpp:332-346, 360)
-    CK(launch_ifft3(*r, r->d_work, dst, sinc && !symz && !resc, r->stream));
-    r->stats.launches += 4;
+    const bool weight = sinc && !symz && !resc;
+    if (weight && !r->d_sinc) {
+        rc = alloc((void**)&r->d_sinc, sizeof(double) * (3 * (size_t)(r->g.map / 2) * (r->g.map / 2) + 1));
+        if (rc) return rc;
+        CK(launch_sinc_table(r->d_sinc, r->g.map, r->stream));
+        r->stats.launches += 1;
+    }
+    int launches = 0;
+    CK(launch_finish(*r, imap, dst, weight, &launches, r->stream));
+    r->stats.launches += launches;
     if (symz) {
         if (!r->d_symtmp) {
             int rc = alloc((void**)&r->d_symtmp, sizeof(float) * r->vol_elems());
@@ -801,15 +805,18 @@ int bsg_recon_fsc(bsg_recon* h, int nshell, double* fsc_out) {
     if (!r || !fsc_out || nshell < 1) return fail(BSG_ERR_ARG, "bsg_recon_fsc: bad argument");
     if (r->nhalves < 2) return fail(BSG_ERR_STATE, "bsg_recon_fsc: needs half maps (nmaps >= 2)");
     CK(cudaSetDevice(r->device));
-    const size_t N3 = r->vol_elems();
-    for (int i = 0; i < 2; ++i)
-        if (!r->d_half_weighed[i]) { int rc = alloc((void**)&r->d_half_weighed[i], sizeof(float2) * N3); if (rc) return rc; }
-    if (r->d_fsc) { cudaFree(r->d_fsc); r->d_fsc = nullptr; }
-    int rc = alloc((void**)&r->d_fsc, sizeof(double) * 3 * (size_t)r->g.map * nshell + sizeof(double) * nshell);
-    if (rc) return rc;
-    double* d_out = r->d_fsc + 3 * (size_t)r->g.map * nshell;
-    CK(launch_fsc(*r, nshell, d_out, r->stream));
-    r->stats.launches += 4;
+    const size_t parts = fsc_part_elems(*r, nshell), need = parts + nshell;
+    if (need > r->fsc_elems) {
+        if (r->d_fsc) cudaFree(r->d_fsc);
+        r->d_fsc = nullptr;
+        r->fsc_elems = 0;
+        int rc = alloc((void**)&r->d_fsc, sizeof(double) * need);
+        if (rc) return rc;
+        r->fsc_elems = need;
+    }
+    double* d_out = r->d_fsc + parts;
+    CK(launch_fsc(*r, nshell, r->d_fsc, d_out, r->stream));
+    r->stats.launches += 2;
     CK(cudaMemcpyAsync(fsc_out, d_out, sizeof(double) * nshell, cudaMemcpyDeviceToHost, r->stream));
     CK(cudaStreamSynchronize(r->stream));
     return BSG_OK;

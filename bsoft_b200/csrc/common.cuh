@@ -81,8 +81,10 @@ cudaError_t launch_rows(const Context& c, const float* img, int nimg, cudaStream
 cudaError_t launch_cols(const Context& c, int nimg, float2* spectra, cudaStream_t s);
 cudaError_t launch_insert(const Context& c, const float2* spectra, const DevParticle* parts, int np, int half,
                           cudaStream_t s);
-cudaError_t launch_finish(const Context& c, int imap, float* map_out, float* fom_out, bool sinc, cudaStream_t s);
-cudaError_t launch_fsc(const Context& c, int nshell, double* out_dev, cudaStream_t s);
+cudaError_t launch_finish(const Context& c, int imap, float* map_out, bool sinc, int* launches, cudaStream_t s);
+cudaError_t launch_sinc_table(double* t, int N, cudaStream_t s);
+size_t fsc_part_elems(const Context& c, int nshell);
+cudaError_t launch_fsc(const Context& c, int nshell, double* part, double* out_dev, cudaStream_t s);
 cudaError_t launch_symmetrize(const Context& c, float* map, float* tmp, bool sinc, cudaStream_t s);
 cudaError_t launch_rescale(const Context& c, float* map, double nuavg, double nustd, bool sinc, cudaStream_t s);
 

@@ -47,11 +47,12 @@ struct Context {
     double* d_w2[2] = {nullptr, nullptr};
 
     // finishing buffers (allocated on first use)
-    float2* d_work = nullptr;        // N^3 complex
+    float2* d_work = nullptr;        // N^3 complex (the finish uses the half volume)
     float* d_map = nullptr;          // N^3 real
     float* d_fom = nullptr;          // N^3 real
-    float2* d_half_weighed[2] = {nullptr, nullptr};
-    double* d_fsc = nullptr;         // FSC partial sums
+    double* d_sinc = nullptr;        // sinc weight by squared distance from the map centre
+    double* d_fsc = nullptr;         // FSC partial sums and result (grow-only)
+    size_t fsc_elems = 0;
 
     int shape = 0;                   // gridding tile shape (insert.cu kShapes)
     int* d_tile_order = nullptr;     // tile visiting order for `shape`

@@ -7,28 +7,38 @@
 //   fft_back (1/sqrt(N^3)), real  img/Bimage.h:903-908, Bimage_complex.cpp:170-186
 //   filter_sinc (trilinear)       img/Bimage_filter.cpp:484-509
 //
-// weigh_kernel is one pass over the voxels; the 3-D inverse transform is
-// three passes of warp FFTs (x lines contiguous; y and z lines staged 16 at
-// a time through shared memory so global accesses stay coalesced).  The last
-// pass writes only the real part, scaled and sinc-weighted.
+// Only the real part of the inverse transform is kept, and the real part of
+// a transform is the transform of the Hermitian part G(v) = (F(v) +
+// conj(F(-v))) / 2.  So the finish works on the half volume x = 0 .. N/2 of
+// G: y lines (weighing the sums as it loads them), z lines, then x lines as
+// a complex-to-real transform of half the length with the scale and the sinc
+// weight.  One pass over the sums, then 8 N^3 bytes a pass.
 #include "context.cuh"
-#include "fft_dev.cuh"
+#include "fft_tile.cuh"
 
 #include <math.h>
 
+#include <algorithm>
+
 namespace bsg {
 
-#define SMALLFLOAT_F 1e-30f
+// Sums of one half map (vol, w), their unpaired pixels' sums below zsplit
+// (e, ew; half-space accumulators) and the FOM channels (p, q).
+struct HalfSums {
+    const double2* vol;
+    const double* w;
+    const double2* e;
+    const double* ew;
+    const double* p;
+    const double* q;
+};
 
 struct WeighArgs {
-    const double2* v0; const double* w0; const double* p0; const double* q0;
-    const double2* v1; const double* w1; const double* p1; const double* q1;   // second half or null
-    float2* out;      // weighed, centre-shifted complex volume
-    float* fom;       // optional SNR map
+    HalfSums h[2];
+    int nh;           // halves that are added
     int N;
     int zsplit;       // > 0: half-space accumulators (insert.cu walk_edges)
-    const double2* e0; const double* ew0;   // their unpaired pixels' sums below zsplit
-    const double2* e1; const double* ew1;
+    float* fom;       // SNR map (snr_kernel)
 };
 
 // Index of the voxel at minus the frequency of voxel (x, y, z) (wrap-around).
@@ -60,217 +70,253 @@ __device__ __forceinline__ void read_sums(const double2* vol, const double* w, c
     }
 }
 
-__global__ void weigh_kernel(WeighArgs a) {
+// A voxel's sums over the halves that are added.
+__device__ __forceinline__ void voxel_sums(const WeighArgs& a, size_t i, double2& v, double& w) {
+    read_sums(a.h[0].vol, a.h[0].w, a.h[0].e, a.h[0].ew, i, a.N, a.zsplit, v, w);
+    if (a.nh > 1) {
+        double2 v1;
+        double w1;
+        read_sums(a.h[1].vol, a.h[1].w, a.h[1].e, a.h[1].ew, i, a.N, a.zsplit, v1, w1);
+        v.x += v1.x;
+        v.y += v1.y;
+        w += w1;
+    }
+}
+
+// fspace_reconstruction_weigh: the sum over the weight, as float
+__device__ __forceinline__ float2 weighed(double2 v, double w) {
+    if (!(w > 1e-30)) return make_float2(0.f, 0.f);
+    return make_float2((float)(v.x / w), (float)(v.y / w));
+}
+
+// fspace_reconstruction_snr on the weighed channels (full-map sums: the FOM
+// channels switch half-space gridding off)
+__global__ void snr_kernel(WeighArgs a) {
     const size_t N = a.N, N3 = N * N * N;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N3; i += (size_t)gridDim.x * blockDim.x) {
         double2 v;
         double w;
-        read_sums(a.v0, a.w0, a.e0, a.ew0, i, N, a.zsplit, v, w);
-        double p = a.p0 ? a.p0[i] : 0.0, q = a.q0 ? a.q0[i] : 0.0;
-        if (a.v1) {
-            double2 v1;
-            double w1;
-            read_sums(a.v1, a.w1, a.e1, a.ew1, i, N, a.zsplit, v1, w1);
-            v.x += v1.x; v.y += v1.y;
-            w += w1;
-            if (a.p1) { p += a.p1[i]; q += a.q1[i]; }
-        }
-        float2 F = make_float2(0.f, 0.f);
+        voxel_sums(a, i, v, w);
+        double p = a.h[0].p[i], q = a.h[0].q[i];
+        if (a.nh > 1) { p += a.h[1].p[i]; q += a.h[1].q[i]; }
+        const float2 F = weighed(v, w);
         if (w > 1e-30) {
             q = w - q / w;
-            F = make_float2((float)(v.x / w), (float)(v.y / w));
             if (q > 1.0) p /= q;
             else if (w > 1.0) p /= w;
             if (p < 0.0) p = 0.0;
         } else {
             p = 0.0;
-            w = q = 1e-30;
+            w = 1e-30;
         }
-        if (a.fom) {
-            // fspace_reconstruction_snr on the weighed channels
-            const double signal = (double)F.x * F.x + (double)F.y * F.y;
-            double noise = p - signal;
-            if (noise < signal) noise = signal;
-            float f = 0.f;
-            if (w > 1.0 && signal > 1e-30 && noise > 1e-30) f = (float)((w * signal - p) / noise);
-            a.fom[i] = (i == 0) ? 1.f : f;
-        }
-        // (-1)^(h+k+l): signed and unsigned indices share parity for even N
-        const size_t x = i % N, y = (i / N) % N, z = i / (N * N);
-        if ((x + y + z) & 1) { F.x = -F.x; F.y = -F.y; }
-        a.out[i] = F;
+        const double signal = (double)F.x * F.x + (double)F.y * F.y;
+        double noise = p - signal;
+        if (noise < signal) noise = signal;
+        float f = 0.f;
+        if (w > 1.0 && signal > 1e-30 && noise > 1e-30) f = (float)((w * signal - p) / noise);
+        a.fom[i] = (i == 0) ? 1.f : f;
     }
 }
 
-// Radix plan of a map edge: power of two -> in-place radix-2/4 DIT on
-// bit-reversed input; otherwise mixed-radix Stockham (needs N scratch).
-struct Radix {
-    int mixed;
-    int nstage;
-    int r[16];
-};
+// ---- 3-D inverse transform ----------------------------------------------------
+//
+// 384^3, both half maps and their FSC: 24.8 -> 5.5 ms; the passes were
+// full complex volumes through runtime-radix line transforms (an index
+// division per element and local-memory butterflies) at 1.4 TB/s.
 
-// x-lines: one warp per line, 8 lines per CTA
-constexpr int XW = 8;
-__global__ void __launch_bounds__(XW * 32) fft_x_kernel(float2* data, const float2* tw, int N, int logN, Radix rp) {
-    extern __shared__ float2 sm[];
-    float2* stw = sm;                              // N roots
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int per = rp.mixed ? 2 * N : N;
-    float2* buf = sm + N + warp * per;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) stw[i] = tw[i];
-    __syncthreads();
-    const size_t line = (size_t)blockIdx.x * XW + warp;
-    if (line >= (size_t)N * N) return;
-    float2* p = data + line * N;
-    if (rp.mixed) {
-        for (int i = lane; i < N; i += 32) buf[i] = p[i];
-        __syncwarp();
-        warp_fft_mixed<true>(buf, buf + N, N, rp.r, rp.nstage, stw);
-    } else {
-        for (int i = lane; i < N; i += 32) buf[bitrev(i, logN)] = p[i];
-        __syncwarp();
-        warp_fft<true>(buf, N, logN, stw);
-    }
-    for (int i = lane; i < N; i += 32) p[i] = buf[i];
-}
+constexpr int FIN_THREADS = 256;
+// float2 between the elements of a strided tile (16 lines side by side) and
+// of a transposed x tile (odd, so that a warp's consecutive elements of one
+// line fall in distinct banks)
+constexpr int YZ_PITCH = TILE_LINES, X_PITCH = TILE_LINES + 1;
 
-// strided lines (y: stride N, z: stride N*N): 16 adjacent x per CTA.
-constexpr int SW = 16;
-struct StridedArgs {
-    float2* data;
-    const float2* tw;
-    int N, logN;
-    int axis;          // 1 = y, 2 = z
-    float* real_out;   // when set: write the real part * scale (* sinc) instead
+struct IfftArgs {
+    float2* g;         // N x N x pitch: the half volume
+    const float2* tw;  // N roots
+    int N, pitch;
+    TilePlan plan;     // N (y, z) or N / 2 (x)
+    float* out;        // x pass: the real map
     float scale;
-    int sinc;
-    Radix rp;
+    const double* sinc;   // weight by squared distance from the map centre, or null
 };
 
-__global__ void __launch_bounds__(SW * 32) fft_strided_kernel(StridedArgs a) {
+// y lines: 16 adjacent x of one z, G formed from the sums on the way in
+__global__ void __launch_bounds__(FIN_THREADS) weigh_y_kernel(const __grid_constant__ WeighArgs w,
+                                                              const __grid_constant__ IfftArgs a) {
     extern __shared__ float2 sm[];
-    const int N = a.N;
-    const int per = a.rp.mixed ? 2 * N : N;
-    float2* stw = sm;                 // N roots
-    float2* tile = sm + N;            // SW lines of `per`
-    for (int i = threadIdx.x; i < N; i += blockDim.x) stw[i] = a.tw[i];
-    // blockIdx.x: x-chunk, blockIdx.y: the remaining coordinate (z for axis y, y for axis z)
-    const int x0 = blockIdx.x * SW;
-    const int other = blockIdx.y;
-    const size_t stride = a.axis == 1 ? (size_t)N : (size_t)N * N;
-    const size_t obase = a.axis == 1 ? (size_t)other * N * N : (size_t)other * N;
-    for (int i = threadIdx.x; i < SW * N; i += blockDim.x) {
-        const int c = i % SW, j = i / SW;
-        const int x = x0 + c;
-        float2 v = make_float2(0.f, 0.f);
-        if (x < N) v = a.data[obase + (size_t)j * stride + x];
-        tile[c * per + (a.rp.mixed ? j : (int)bitrev(j, a.logN))] = v;
+    const int N = a.N, XH = N / 2 + 1;
+    float2* roots = sm;
+    float2* t0 = sm + N;
+    float2* t1 = t0 + N * YZ_PITCH;
+    for (int i = threadIdx.x; i < N; i += FIN_THREADS) roots[i] = a.tw[i];
+    const int x0 = blockIdx.x * TILE_LINES, z = blockIdx.y, zm = z ? N - z : 0;
+    for (int i = threadIdx.x; i < N * TILE_LINES; i += FIN_THREADS) {
+        const int c = i & (TILE_LINES - 1), y = i / TILE_LINES, x = x0 + c;
+        float2 g = make_float2(0.f, 0.f);
+        if (x < XH) {
+            const int ym = y ? N - y : 0, xm = x ? N - x : 0;
+            double2 v;
+            double wt;
+            voxel_sums(w, ((size_t)z * N + y) * N + x, v, wt);
+            const float2 f = weighed(v, wt);
+            voxel_sums(w, ((size_t)zm * N + ym) * N + xm, v, wt);
+            const float2 m = weighed(v, wt);
+            // half the sum; phase_shift_to_center is (-1)^(h+k+l), the same
+            // for both (signed and unsigned indices share parity for even N)
+            const float s = ((x + y + z) & 1) ? -0.5f : 0.5f;
+            g = make_float2(s * (f.x + m.x), s * (f.y - m.y));
+        }
+        t0[y * YZ_PITCH + c] = g;
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5;
-    if (x0 + warp < N) {
-        if (a.rp.mixed) warp_fft_mixed<true>(tile + warp * per, tile + warp * per + N, N, a.rp.r, a.rp.nstage, stw);
-        else warp_fft<true>(tile + warp * N, N, a.logN, stw);
+    const float2* r = tile_fft<true>(t0, t1, a.plan, roots, 1, YZ_PITCH);
+    for (int i = threadIdx.x; i < N * TILE_LINES; i += FIN_THREADS) {
+        const int c = i & (TILE_LINES - 1), y = i / TILE_LINES, x = x0 + c;
+        if (x < XH) a.g[((size_t)z * N + y) * a.pitch + x] = r[y * YZ_PITCH + c];
+    }
+}
+
+// z lines: 16 adjacent x of one y, in place
+__global__ void __launch_bounds__(FIN_THREADS) fft_z_kernel(const __grid_constant__ IfftArgs a) {
+    extern __shared__ float2 sm[];
+    const int N = a.N, XH = N / 2 + 1;
+    float2* roots = sm;
+    float2* t0 = sm + N;
+    float2* t1 = t0 + N * YZ_PITCH;
+    for (int i = threadIdx.x; i < N; i += FIN_THREADS) roots[i] = a.tw[i];
+    const int x0 = blockIdx.x * TILE_LINES, y = blockIdx.y;
+    const size_t zs = (size_t)N * a.pitch;
+    float2* g = a.g + (size_t)y * a.pitch + x0;
+    for (int i = threadIdx.x; i < N * TILE_LINES; i += FIN_THREADS) {
+        const int c = i & (TILE_LINES - 1), z = i / TILE_LINES;
+        t0[z * YZ_PITCH + c] = x0 + c < XH ? g[z * zs + c] : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < SW * N; i += blockDim.x) {
-        const int c = i % SW, j = i / SW;
-        const int x = x0 + c;
-        if (x >= N) continue;
-        const size_t idx = obase + (size_t)j * stride + x;
-        const float2 v = tile[c * per + j];
-        if (a.real_out) {
-            float r = v.x * a.scale;
+    const float2* r = tile_fft<true>(t0, t1, a.plan, roots, 1, YZ_PITCH);
+    for (int i = threadIdx.x; i < N * TILE_LINES; i += FIN_THREADS) {
+        const int c = i & (TILE_LINES - 1), z = i / TILE_LINES;
+        if (x0 + c < XH) g[z * zs + c] = r[z * YZ_PITCH + c];
+    }
+}
+
+// x lines, complex to real: x[2j] + i x[2j+1] is the N/2-point transform of
+// E_k + i O_k, E_k = G_k + conj(G_{N/2-k}), O_k = (G_k - conj(G_{N/2-k}))
+// exp(2 pi i k / N); then the scale and the sinc weight.  16 consecutive rows
+// (z, y) per CTA, a warp reading and writing one row at a time.
+__global__ void __launch_bounds__(FIN_THREADS) fft_x_real_kernel(const __grid_constant__ IfftArgs a) {
+    extern __shared__ float2 sm[];
+    const int N = a.N, M = N / 2;
+    float2* roots = sm;
+    float2* t0 = sm + N;
+    float2* t1 = t0 + (M + 1) * X_PITCH;
+    for (int i = threadIdx.x; i < N; i += FIN_THREADS) roots[i] = a.tw[i];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long rows = (long)N * N, r0 = (long)blockIdx.x * TILE_LINES;
+    for (int c = warp; c < TILE_LINES; c += FIN_THREADS / 32) {
+        const float2* src = a.g + (r0 + c) * a.pitch;
+        for (int k = lane; k <= M; k += 32) {
+            float2 v = r0 + c < rows ? src[k] : make_float2(0.f, 0.f);
+            if (k == 0 || k == M) v.y = 0.f;       // real up to rounding
+            t1[k * X_PITCH + c] = v;
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < M * TILE_LINES; i += FIN_THREADS) {
+        const int c = i & (TILE_LINES - 1), k = i / TILE_LINES;
+        const float2 p = t1[k * X_PITCH + c], q = t1[(M - k) * X_PITCH + c], w = roots[k];
+        const float2 e = make_float2(p.x + q.x, p.y - q.y), d = make_float2(p.x - q.x, p.y + q.y);
+        const float2 o = make_float2(d.x * w.x + d.y * w.y, d.y * w.x - d.x * w.y);   // d conj(w)
+        t0[k * X_PITCH + c] = make_float2(e.x - o.y, e.y + o.x);
+    }
+    __syncthreads();
+    const float2* r = tile_fft<true>(t0, t1, a.plan, roots, 2, X_PITCH);
+    for (int c = warp; c < TILE_LINES; c += FIN_THREADS / 32) {
+        const long row = r0 + c;
+        if (row >= rows) break;
+        const int z = (int)(row / N), y = (int)(row - (long)z * N);
+        const int dy = y - M, dz = z - M, d2 = dy * dy + dz * dz;
+        float2* dst = reinterpret_cast<float2*>(a.out + row * N);
+        for (int j = lane; j < M; j += 32) {
+            float2 v = r[j * X_PITCH + c];
+            v.x *= a.scale;
+            v.y *= a.scale;
             if (a.sinc) {
-                // filter_sinc: r = pi |d|, d = (index - N/2) / N, weight (r / sin r)^2
-                const int yy = a.axis == 1 ? j : other;
-                const int zz = a.axis == 1 ? other : j;
-                const double o = (double)(N / 2);
-                const double dx = (x - o) / N, dy = (yy - o) / N, dz = (zz - o) / N;
-                const double rr = 3.14159265358979323846 * sqrt(dx * dx + dy * dy + dz * dz);
-                if (rr != 0.0) { const double w = rr / sin(rr); r = (float)(w * w * r); }
+                const int x = 2 * j - M;
+                v.x = (float)(a.sinc[d2 + x * x] * v.x);
+                v.y = (float)(a.sinc[d2 + (x + 1) * (x + 1)] * v.y);
             }
-            a.real_out[idx] = r;
-        } else {
-            a.data[idx] = v;
+            dst[j] = v;
         }
     }
 }
 
-cudaError_t launch_weigh(const Context& c, int imap, cudaStream_t s) {
-    WeighArgs a{};
-    const int N = c.g.map;
-    int h0 = 0;
-    bool both = false;
-    if (c.nhalves == 2) {
-        if (imap == 0) both = true;
-        else h0 = imap - 1;
+// filter_sinc: r = pi |d|, d = (index - N/2) / N, weight (r / sin r)^2, by
+// the squared distance in voxels (0 .. 3 (N/2)^2)
+__global__ void sinc_table_kernel(double* t, int N) {
+    const int n = 3 * (N / 2) * (N / 2) + 1;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double rr = 3.14159265358979323846 * (sqrt((double)i) / N);
+        const double w = i ? rr / sin(rr) : 1.0;
+        t[i] = w * w;
     }
-    a.v0 = c.d_vol[h0]; a.w0 = c.d_w[h0]; a.p0 = c.d_pow[h0]; a.q0 = c.d_w2[h0];
-    if (both) { a.v1 = c.d_vol[1]; a.w1 = c.d_w[1]; a.p1 = c.d_pow[1]; a.q1 = c.d_w2[1]; }
-    a.out = c.d_work;
-    a.fom = c.g.fom ? c.d_fom : nullptr;
+}
+
+cudaError_t launch_sinc_table(double* t, int N, cudaStream_t s) {
+    sinc_table_kernel<<<64, 256, 0, s>>>(t, N);
+    return cudaGetLastError();
+}
+
+static HalfSums half_sums(const Context& c, int h) {
+    return HalfSums{c.d_vol[h], c.d_w[h], c.d_evol[h], c.d_ew[h], c.d_pow[h], c.d_w2[h]};
+}
+
+static WeighArgs weigh_args(const Context& c, int imap) {
+    WeighArgs w{};
+    w.N = c.g.map;
+    w.zsplit = c.zsplit;
+    w.nh = 1;
+    w.h[0] = half_sums(c, c.nhalves == 2 && imap > 0 ? imap - 1 : 0);
+    if (c.nhalves == 2 && imap == 0) {
+        w.h[1] = half_sums(c, 1);
+        w.nh = 2;
+    }
+    return w;
+}
+
+static size_t yz_smem(int N) { return sizeof(float2) * ((size_t)N + 2 * (size_t)N * YZ_PITCH); }
+static size_t x_smem(int N) { return sizeof(float2) * ((size_t)N + 2 * (size_t)(N / 2 + 1) * X_PITCH); }
+
+// Map imap (0: the halves added) of the context's sums: weighed, transformed,
+// scaled and, with sinc, weighted, into map_out; the SNR map into d_fom when
+// the context keeps its channels.  *launches: kernels launched.
+cudaError_t launch_finish(const Context& c, int imap, float* map_out, bool sinc, int* launches, cudaStream_t s) {
+    const int N = c.g.map, XH = N / 2 + 1;
+    WeighArgs w = weigh_args(c, imap);
+    *launches = 3;
+    cudaError_t e;
+    if (c.g.fom) {
+        w.fom = c.d_fom;
+        snr_kernel<<<148 * 8, 256, 0, s>>>(w);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        *launches = 4;
+    }
+    IfftArgs a{};
+    a.g = c.d_work;
+    a.tw = c.d_twmap;
     a.N = N;
-    a.zsplit = c.zsplit;
-    a.e0 = c.d_evol[h0]; a.ew0 = c.d_ew[h0];
-    if (both) { a.e1 = c.d_evol[1]; a.ew1 = c.d_ew[1]; }
-    weigh_kernel<<<148 * 8, 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-static Radix radix_plan(int N) {
-    Radix rp{};
-    rp.mixed = (N & (N - 1)) != 0;
-    if (rp.mixed) rp.nstage = factor_radices(N, rp.r);
-    return rp;
-}
-
-cudaError_t launch_ifft3(const Context& c, float2* vol, float* real_out, bool sinc, cudaStream_t s) {
-    const int N = c.g.map, logN = ilog2i(N);
-    const Radix rp = radix_plan(N);
-    const size_t per = rp.mixed ? 2 * (size_t)N : (size_t)N;
-    {
-        const size_t lines = (size_t)N * N;
-        const size_t smem = sizeof(float2) * ((size_t)N + XW * per);
-        fft_x_kernel<<<(unsigned)((lines + XW - 1) / XW), XW * 32, smem, s>>>(vol, c.d_twmap, N, logN, rp);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    const size_t smem = sizeof(float2) * ((size_t)N + SW * per);
-    dim3 grid((N + SW - 1) / SW, N);
-    StridedArgs a{};
-    a.data = vol; a.tw = c.d_twmap; a.N = N; a.logN = logN; a.rp = rp;
-    a.axis = 1;
-    fft_strided_kernel<<<grid, SW * 32, smem, s>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    a.axis = 2;
-    a.real_out = real_out;
+    // whole 32-byte sectors per row
+    a.pitch = (XH + 3) / 4 * 4;
+    if (!tile_plan(N, &a.plan)) return cudaErrorInvalidValue;
+    const dim3 grid((unsigned)((XH + TILE_LINES - 1) / TILE_LINES), (unsigned)N);
+    weigh_y_kernel<<<grid, FIN_THREADS, yz_smem(N), s>>>(w, a);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    fft_z_kernel<<<grid, FIN_THREADS, yz_smem(N), s>>>(a);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (!tile_plan(N / 2, &a.plan)) return cudaErrorInvalidValue;
+    a.out = map_out;
     a.scale = (float)(1.0 / sqrt((double)N * N * N));
-    a.sinc = sinc ? 1 : 0;
-    fft_strided_kernel<<<grid, SW * 32, smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_finish(const Context& c, int imap, float* map_out, float* fom_out, bool sinc, cudaStream_t s) {
-    (void)fom_out;
-    cudaError_t e = launch_weigh(c, imap, s);
-    if (e != cudaSuccess) return e;
-    return launch_ifft3(c, c.d_work, map_out, sinc, s);
-}
-
-// Weighed (not centre-shifted) half map for the FSC: reuse weigh_kernel and
-// undo nothing - the FSC only uses products F1 conj(F2) and |F|^2, which the
-// (-1)^(h+k+l) factor leaves unchanged.
-cudaError_t launch_weigh_into(const Context& c, int imap, float2* out, cudaStream_t s) {
-    WeighArgs a{};
-    const int h0 = imap - 1;
-    a.v0 = c.d_vol[h0]; a.w0 = c.d_w[h0]; a.p0 = nullptr; a.q0 = nullptr;
-    a.out = out; a.fom = nullptr; a.N = c.g.map;
-    a.zsplit = c.zsplit;
-    a.e0 = c.d_evol[h0]; a.ew0 = c.d_ew[h0];
-    weigh_kernel<<<148 * 8, 256, 0, s>>>(a);
+    a.sinc = sinc ? c.d_sinc : nullptr;
+    fft_x_real_kernel<<<(unsigned)(((long)N * N + TILE_LINES - 1) / TILE_LINES), FIN_THREADS, x_smem(N), s>>>(a);
     return cudaGetLastError();
 }
 
@@ -318,10 +364,18 @@ cudaError_t launch_map_sums(double2* dv, double* dw, const double2* vol, const d
 // (bsoft/src/img/Bimage_resolution.cpp:330-406 with fspace_radial_power,
 // Bimage_fspace.cpp:848-958): radius = real * |index / real| (wrapped at
 // (N-1)/2), a voxel adds (1 - f) to shell floor(radius) and f to the next,
-// only voxels with floor(radius) < maxrad count.  One CTA per z-plane;
-// thread r accumulates shell r of that plane in a fixed order (rows, then
-// |h|, then sign), fsc_reduce sums the planes in order - deterministic,
-// FP64 throughout.
+// only voxels with floor(radius) < maxrad count.  The weighed values come
+// straight from the sums (the centre shift's sign leaves F1 conj(F2) and
+// |F|^2 unchanged).
+//
+// A warp takes rows (z, y), 32 values of h >= 0 at a time with their mates
+// -(h, k, l), which have the same radius.  Along a row the radius grows by
+// less than 1 a step, so the lanes of a shell are consecutive: a segmented
+// scan sums them and the last lane of a run adds it to the warp's shells in
+// shared memory.  Rows, warps and CTAs in fixed order: deterministic, FP64
+// throughout.  Bound by the FP64 pipe and the reads of the sums; a thread per
+// shell scanning a whole plane (384 CTAs, every voxel's square root two to
+// four times) took 5.4 ms at 384^3 after 2.0 ms of weighing.
 __device__ __forceinline__ double fsc_radius(int h, int k, int l, double real) {
     const double fs = 1.0 / real;
     double rx = h * fs, ry = k * fs, rz = l * fs;
@@ -329,57 +383,102 @@ __device__ __forceinline__ double fsc_radius(int h, int k, int l, double real) {
     return real * sqrt(rx + ry + rz);
 }
 
-__global__ void fsc_plane_kernel(const float2* v1, const float2* v2, int N, int nshell, int maxrad, double real,
-                                 double* part) {
-    const int z = blockIdx.x;
-    const int l = sfreq(z, N);
-    for (int r = threadIdx.x; r < nshell; r += blockDim.x) {
-        double num = 0, d1 = 0, d2 = 0;
-        if (r < maxrad) {
-            // voxels with floor(radius) in {r - 1, r}: radius in [r - 1, r + 1)
-            const double rlo = r - 1.5, rhi = r + 1.5;      // index-space bounds with margin
-            for (int y = 0; y < N; ++y) {
-                const int k = sfreq(y, N);
-                const double kl = (double)k * k + (double)l * l;
-                if (kl >= rhi * rhi) continue;
-                const int hlo = (rlo > 0 && rlo * rlo > kl) ? (int)floor(sqrt(rlo * rlo - kl)) : 0;
-                const int hhi = min(N / 2, (int)ceil(sqrt(rhi * rhi - kl)));
-                for (int hh = hlo; hh <= hhi; ++hh) {
-                    for (int sgn = 0; sgn < 2; ++sgn) {
-                        if (sgn && (hh == 0 || hh == N / 2)) continue;
-                        const int x = sgn ? (N - hh) % N : hh;
-                        const int h = sfreq(x, N);
-                        const double rad = fsc_radius(h, k, l, real);
-                        const int ir = (int)rad;
-                        if (ir >= maxrad) continue;
-                        double w;
-                        if (ir == r) w = 1.0 - (rad - ir);
-                        else if (ir + 1 == r) w = rad - ir;
-                        else continue;
-                        const size_t i = ((size_t)z * N + y) * N + x;
-                        const float2 a = v1[i], b = v2[i];
-                        num += w * ((double)a.x * b.x + (double)a.y * b.y);
-                        d1 += w * ((double)a.x * a.x + (double)a.y * a.y);
-                        d2 += w * ((double)b.x * b.x + (double)b.y * b.y);
-                    }
+constexpr int FSC_WARPS = 8;
+
+struct FscArgs {
+    WeighArgs w[2];
+    int N, ns, maxrad;     // ns: shells kept
+    double real;
+    double* part;          // CTAs x ns x 3
+};
+
+__global__ void __launch_bounds__(FSC_WARPS * 32) fsc_rows_kernel(const __grid_constant__ FscArgs a) {
+    extern __shared__ double shells[];        // FSC_WARPS x ns x 3
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double* my = shells + (size_t)warp * a.ns * 3;
+    for (int i = lane; i < a.ns * 3; i += 32) my[i] = 0.0;
+    __syncwarp();
+    const int N = a.N, rows = N * N, H = N / 2;
+    for (int row = blockIdx.x * FSC_WARPS + warp; row < rows; row += gridDim.x * FSC_WARPS) {
+        const int z = row / N, y = row - z * N, zm = z ? N - z : 0, ym = y ? N - y : 0;
+        const int k = sfreq(y, N), l = sfreq(z, N);
+        for (int h0 = 0; h0 <= H; h0 += 32) {
+            const int h = h0 + lane;
+            const double rad = fsc_radius(h, k, l, a.real);
+            int ir = (int)rad;
+            const bool in = h <= H && ir < a.maxrad;
+            if (!__any_sync(0xffffffffu, in)) break;            // the radius only grows
+            double num = 0, d1 = 0, d2 = 0;
+            if (in) {
+                for (int m = 0; m < 2; ++m) {
+                    if (m && (h == 0 || h == H)) continue;       // its mate is another row's
+                    const size_t i = m ? ((size_t)zm * N + ym) * N + (N - h) : ((size_t)z * N + y) * N + h;
+                    double2 v;
+                    double w;
+                    voxel_sums(a.w[0], i, v, w);
+                    const float2 f1 = weighed(v, w);
+                    voxel_sums(a.w[1], i, v, w);
+                    const float2 f2 = weighed(v, w);
+                    num += (double)f1.x * f2.x + (double)f1.y * f2.y;
+                    d1 += (double)f1.x * f1.x + (double)f1.y * f1.y;
+                    d2 += (double)f2.x * f2.x + (double)f2.y * f2.y;
+                }
+            } else {
+                ir = -1;
+            }
+            const double f = rad - ir;
+            double s[6] = {num * (1.0 - f), d1 * (1.0 - f), d2 * (1.0 - f), num * f, d1 * f, d2 * f};
+            if (!in)
+#pragma unroll
+                for (int q = 0; q < 6; ++q) s[q] = 0.0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int other = __shfl_up_sync(0xffffffffu, ir, o);
+                const bool add = lane >= o && other == ir;
+#pragma unroll
+                for (int q = 0; q < 6; ++q) {
+                    const double t = __shfl_up_sync(0xffffffffu, s[q], o);
+                    if (add) s[q] += t;
                 }
             }
+            const int next = __shfl_down_sync(0xffffffffu, ir, 1);
+            const bool last = in && (lane == 31 || next != ir);
+            if (last && ir < a.ns)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) my[ir * 3 + q] += s[q];
+            __syncwarp();
+            if (last && ir + 1 < a.ns)
+#pragma unroll
+                for (int q = 0; q < 3; ++q) my[(ir + 1) * 3 + q] += s[3 + q];
+            __syncwarp();
         }
-        double* o = part + ((size_t)z * nshell + r) * 3;
-        o[0] = num; o[1] = d1; o[2] = d2;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.ns * 3; i += FSC_WARPS * 32) {
+        double t = 0;
+        for (int w = 0; w < FSC_WARPS; ++w) t += shells[(size_t)w * a.ns * 3 + i];
+        a.part[(size_t)blockIdx.x * a.ns * 3 + i] = t;
     }
 }
 
 // FSC[0] = 1 (the reference sets it), FSC[r] = num / sqrt(d1 d2), 0 where
-// not finite or beyond maxrad
-__global__ void fsc_reduce_kernel(const double* part, int N, int nshell, int maxrad, double* fsc) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+// not finite or beyond maxrad.  One warp per shell: the CTAs' sums lane by
+// lane, then a fixed tree.
+__global__ void fsc_reduce_kernel(const double* part, int parts, int ns, int nshell, int maxrad, double* fsc) {
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (r >= nshell) return;
     double num = 0, d1 = 0, d2 = 0;
-    for (int z = 0; z < N; ++z) {
-        const double* o = part + ((size_t)z * nshell + r) * 3;
-        num += o[0]; d1 += o[1]; d2 += o[2];
+    if (r < ns)
+        for (int z = lane; z < parts; z += 32) {
+            const double* o = part + ((size_t)z * ns + r) * 3;
+            num += o[0]; d1 += o[1]; d2 += o[2];
+        }
+    for (int o = 16; o; o >>= 1) {
+        num += __shfl_xor_sync(0xffffffffu, num, o);
+        d1 += __shfl_xor_sync(0xffffffffu, d1, o);
+        d2 += __shfl_xor_sync(0xffffffffu, d2, o);
     }
+    if (lane) return;
     double v = 0;
     if (r == 0) v = 1;
     else if (r < maxrad) {
@@ -389,28 +488,41 @@ __global__ void fsc_reduce_kernel(const double* part, int N, int nshell, int max
     fsc[r] = v;
 }
 
-cudaError_t launch_fsc(const Context& c, int nshell, double* out_dev, cudaStream_t s) {
-    cudaError_t e = launch_weigh_into(c, 1, c.d_half_weighed[0], s);
-    if (e != cudaSuccess) return e;
-    e = launch_weigh_into(c, 2, c.d_half_weighed[1], s);
-    if (e != cudaSuccess) return e;
+// shells that a voxel can reach: at most sqrt(3) N / 2, and the next
+static int fsc_shells(const Context& c, int nshell) { return std::min(nshell, (int)(0.8661 * c.g.map) + 2); }
+static int fsc_ctas(const Context& c) { return std::min(148 * 2, (c.g.map * c.g.map + FSC_WARPS - 1) / FSC_WARPS); }
+
+size_t fsc_part_elems(const Context& c, int nshell) { return (size_t)fsc_ctas(c) * fsc_shells(c, nshell) * 3; }
+
+cudaError_t launch_fsc(const Context& c, int nshell, double* part, double* out_dev, cudaStream_t s) {
+    FscArgs a{};
+    a.w[0] = weigh_args(c, 1);
+    a.w[1] = weigh_args(c, 2);
+    a.N = c.g.map;
+    a.ns = fsc_shells(c, nshell);
     // fspace_maximum_radius (Bimage_fspace.cpp:26-38), sampling ratio 1
-    const double real = c.g.map * c.cfg.map_sampling;
-    const int maxrad = c.cfg.hi_res > 0.1 ? (int)(long)(real / c.cfg.hi_res) : c.g.map / 2;
-    fsc_plane_kernel<<<c.g.map, 128, 0, s>>>(c.d_half_weighed[0], c.d_half_weighed[1], c.g.map, nshell, maxrad, real,
-                                             c.d_fsc);
-    e = cudaGetLastError();
+    a.real = c.g.map * c.cfg.map_sampling;
+    a.maxrad = c.cfg.hi_res > 0.1 ? (int)(long)(a.real / c.cfg.hi_res) : c.g.map / 2;
+    a.part = part;
+    const int ctas = fsc_ctas(c);
+    fsc_rows_kernel<<<ctas, FSC_WARPS * 32, sizeof(double) * 3 * FSC_WARPS * a.ns, s>>>(a);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    fsc_reduce_kernel<<<(nshell + 127) / 128, 128, 0, s>>>(c.d_fsc, c.g.map, nshell, maxrad, out_dev);
+    fsc_reduce_kernel<<<(nshell + 7) / 8, 256, 0, s>>>(part, ctas, a.ns, nshell, a.maxrad, out_dev);
     return cudaGetLastError();
 }
 
 cudaError_t prepare_finish_attributes() {
-    cudaError_t e = cudaFuncSetAttribute(fft_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(float2) * (512 + XW * 1024)));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(fft_strided_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(float2) * (512 + SW * 1024)));
+    const int most = 512;
+    cudaError_t e = cudaFuncSetAttribute(weigh_y_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)yz_smem(most));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fft_z_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)yz_smem(most));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fft_x_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x_smem(most));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fsc_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * 3 * FSC_WARPS * 512));
+    return e;
 }
 
 }  // namespace bsg
