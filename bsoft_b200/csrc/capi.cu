@@ -190,13 +190,16 @@ static int set_shape(Recon* r, int shape) {
     std::vector<int> order(d.size());
     for (size_t i = 0; i < d.size(); ++i) order[i] = d[i].second;
     CK(cudaMemcpy(r->d_tile_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemset(r->d_arrived, 0, sizeof(unsigned) * order.size()));
+    CK(cudaStreamSynchronize(nullptr));
     r->shape = shape;
     // replicas: enough warps to fill the GPU several times over and to split
     // the tiles near the origin, which every particle reaches (at 256^3 two
     // replicas measured 2.5% faster than four, and halve the partial sums)
     const long ntiles = (long)nx * ny * nz;
     int R = (int)std::min<long>(16, std::max<long>(2, (65536 + ntiles - 1) / ntiles));
-    const size_t need = (size_t)R * (r->g.fom ? 5 : 3) * r->vol_elems() * sizeof(double);
+    const size_t need = r->g.fom ? (size_t)R * 5 * r->vol_elems() * sizeof(double)
+                                 : (size_t)R * 3 * ntiles * tx * ty * tz * sizeof(float);
     if (r->d_part_sums) { cudaFree(r->d_part_sums); r->d_part_sums = nullptr; }
     if (cudaMalloc((void**)&r->d_part_sums, need) != cudaSuccess) {
         // not enough memory for replicas: run each tile in one warp
@@ -285,7 +288,7 @@ static void free_all(Recon* r) {
         if (r->compute_done[i]) cudaEventDestroy(r->compute_done[i]);
     }
     F(r->d_bkg); F(r->d_phase); F(r->d_rows); F(r->d_tw); F(r->d_twmap);
-    F(r->d_work); F(r->d_map); F(r->d_fom); F(r->d_sinc); F(r->d_fsc); F(r->d_tile_order); F(r->d_part_sums); F(r->d_symtmp);
+    F(r->d_work); F(r->d_map); F(r->d_fom); F(r->d_sinc); F(r->d_fsc); F(r->d_tile_order); F(r->d_arrived); F(r->d_part_sums); F(r->d_symtmp);
     if (r->h_status) cudaFreeHost(r->h_status);
     for (auto& t : r->timed) { cudaEventDestroy(t.a); cudaEventDestroy(t.b); }
     r->timed.clear();
@@ -316,7 +319,7 @@ static int run_batch_kernels(Recon* r, int buf, const float* d_img, long np, boo
         if (r->nexp > 0) CK(launch_insert(*r, spec_out, r->d_psym, (int)r->nexp, r->nhalves == 2 ? h : -1, s));
         else CK(launch_insert(*r, spec_out, r->d_part, (int)np, r->nhalves == 2 ? h : -1, s));
         if (r->timing) { cudaEventRecord(b, s); r->timed.push_back({a, b, 0}); }
-        r->stats.launches += r->replicas > 1 ? 2 : 1;     // gridding (+ replica combine)
+        r->stats.launches += r->g.fom && r->replicas > 1 ? 2 : 1;     // gridding (+ the FOM path's replica combine)
         r->stats.insert_launches += 1;
     }
     r->stats.particles += np;
@@ -555,7 +558,10 @@ int bsg_recon_create(const bsg_recon_config* cfg, bsg_recon** out) {
     if (!rc && cudaHostGetDevicePointer((void**)&r->d_status, r->h_status, 0) != cudaSuccess)
         rc = fail(BSG_ERR_CUDA, "bsg_recon_create: status word mapping");
     if (!rc) *r->h_status = 0;
-    if (!rc) rc = alloc((void**)&r->d_tile_order, sizeof(int) * (size_t)((N + 7) / 8) * ((N + 7) / 8) * ((N + 7) / 8));
+    // (the shapes' tiles are at least 8 x 8 x 8 or 16 x 16 x 4 voxels)
+    const size_t most_tiles = (size_t)((N + 7) / 8) * ((N + 7) / 8) * ((N + 7) / 8);
+    if (!rc) rc = alloc((void**)&r->d_tile_order, sizeof(int) * most_tiles);
+    if (!rc) rc = alloc((void**)&r->d_arrived, sizeof(unsigned) * most_tiles);
     if (rc) { free_all(r); delete r; return rc; }
     std::vector<float2> tw;
     host_twiddles(ft, tw);

@@ -54,7 +54,9 @@ struct InsertArgs {
     int ntx, nty, ntz;         // tiles per axis
     const int* order;          // tile visiting order (heaviest first)
     int R;                     // replicas per tile (each takes a slice of the particles)
-    double* psum;              // R > 1: replica partial sums, R x channels x N^3
+    float* psum;               // R > 1: replica partial sums, tiles x R x 3 x tile voxels
+    unsigned* arrived;         // per tile: replicas done (bits 0-7) and which stored sums (8 + rep)
+    double* fsum;              // FOM path, R > 1: replica partial sums, R x 5 x N^3
     int zsplit;                // > 0: half-space gridding (walk_edges)
     double2* evol;             // half-space: unpaired pixels' sums below zsplit (zsplit x N^2)
     double* ew;
@@ -118,15 +120,12 @@ struct TileAcc {
     tacc_t* q;
 };
 
-template <bool FOM>
 __device__ __forceinline__ void add_voxel(const TileAcc& A, int i, float2 f, float w) {
     A.re[i] += f.x * w;
     A.im[i] += f.y * w;
     A.w[i] += w;
-    if (FOM) {
-        A.p[i] += w * (f.x * f.x + f.y * f.y);
-        A.q[i] += w * w;
-    }
+    A.p[i] += w * (f.x * f.x + f.y * f.y);
+    A.q[i] += w * w;
 }
 
 // One pixel (h, k) of particle P against the tile at alias origin o.  All
@@ -134,7 +133,7 @@ __device__ __forceinline__ void add_voxel(const TileAcc& A, int i, float2 f, flo
 // __syncwarp after each corner orders the shared-memory updates of
 // different corner offsets, which may touch the same voxel from different
 // lanes.
-template <bool FOM, bool GATE, int TX, int TY, int TZ>
+template <bool GATE, int TX, int TY, int TZ>
 __device__ __forceinline__ void pixel(const InsertArgs& a, const DevParticle& P, const float2* S, const TileAcc& A,
                                       double ox, double oy, double oz, int h, int k, bool act) {
     const int hf = a.ft / 2;
@@ -167,7 +166,7 @@ __device__ __forceinline__ void pixel(const InsertArgs& a, const DevParticle& P,
             w = (float)((double)wt * (1.0 - sqrt(dx * dx + dy * dy + dz * dz)));
         }
         if (act && (unsigned)ix < TX && (unsigned)iy < TY && (unsigned)iz < TZ && w > 0.f)
-            add_voxel<FOM>(A, (iz * TY + iy) * TX + ix, f, w);
+            add_voxel(A, (iz * TY + iy) * TX + ix, f, w);
         __syncwarp();
         return;
     }
@@ -186,7 +185,7 @@ __device__ __forceinline__ void pixel(const InsertArgs& a, const DevParticle& P,
             for (int dx = 0; dx < 2; ++dx) {
                 const int x = ix + dx;
                 if (act && (unsigned)x < TX && (unsigned)y < TY && (unsigned)z < TZ)
-                    add_voxel<FOM>(A, (z * TY + y) * TX + x, f, (dx ? rx : 1.f - rx) * wyz);
+                    add_voxel(A, (z * TY + y) * TX + x, f, (dx ? rx : 1.f - rx) * wyz);
                 __syncwarp();
             }
         }
@@ -309,106 +308,158 @@ __device__ __forceinline__ int floor_div(int x, int d, float inv_d) {
     return q;
 }
 
-// The same walk with the lattice phases of one row block interleaved: lane t
-// takes a group of Lh consecutive pixels of one lattice row (h = g, g + 1,
-// ..., g + Lh - 1 with g = h_lo + sh j + Lh i), one pixel of each column
-// phase, and the warp steps through the phases together: at step ph every
-// lane holds a point of phase (ph, pk), so the conflict-free property of a
-// phase still holds, and pix() ends each step with __syncwarp.  The row
-// search is done once per group instead of once per point, and neighbouring
-// lanes read neighbouring pixels of the spectrum.
-// excl = 1 leaves out the row k = -hf and the column h = -hf (half-space
-// gridding grids them separately, walk_edges).
-template <int TX, int TY, int TZ, class Pix>
-__device__ __forceinline__ void walk_groups(const DevParticle& P, int hf, double ox, double oy, double oz, int lane,
-                                            int* s_row, int excl, Pix&& pix) {
-    const double e = P.ezmax;
+// One (tile, particle, alias) pair of the gridding walk, set up by one lane
+// (setup_pair) and read by the whole warp: pixel ranges, the anchor pixel and
+// its tile-relative map coordinate, and the particle's constants.
+struct __align__(16) Pair {
+    int h_lo, h_hi, k_lo, k_hi;       // edge walk: t0, t1 of line 0 and line 1
+    int hc, kc;                       // anchor pixel
+    int part, lat;
+    float bx, by, bz, pw;             // coordinate of the anchor; particle weight
+    float ax, ay, az, inv_step;       // map step per pixel along h
+    float cx, cy, cz;                 // and along k
+    int spec;
+};
+
+// The FP32 form of a row's pixel bounds: along axis i, a row whose coordinate
+// at h = hc is b has its tents inside the tile for h - hc between
+// -b ia + lo and -b ia + hi, each with its error bound taken off and added on.
+struct __align__(16) RowBounds {
+    float ia[3], lo_a[3], lo_b[3], hi_a[3], hi_b[3];
+    int exact;                        // an axis does not vary along h: the FP64 form only
+};
+constexpr int QN = 8;                 // pairs set up at a time
+
+// The pixels [hmin, hmax] of row k whose tents reach the tile box, in FP64:
+// the set of pixels that a tile grids is defined by these bounds.
+template <int TX, int TY, int TZ>
+__device__ __noinline__ int2 row_bounds(const DevParticle& P, int k, int h_lo, int h_hi, double ox, double oy,
+                                        double oz, double e) {
     const double lo[3] = {ox - 1.0 - e, oy - 1.0 - e, oz - 1.0 - e};
     const double hi[3] = {ox + TX + e, oy + TY + e, oz + TZ + e};
-    double vc = 0, hv = 0, uc = 0, hu = 0;
+    double hl = h_lo, hh = h_hi;
+    bool live = true;
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const double c = 0.5 * (lo[i] + hi[i]), e = 0.5 * (hi[i] - lo[i]);
-        vc += P.bd[i] * c; hv += fabs(P.bd[i]) * e;
-        uc += P.ad[i] * c; hu += fabs(P.ad[i]) * e;
+        const double base = k * P.bd[i], ia = P.iad[i];
+        if (ia != 0.0) {
+            double p0 = (lo[i] - base) * ia, p1 = (hi[i] - base) * ia;
+            if (p0 > p1) { const double t = p0; p0 = p1; p1 = t; }
+            hl = fmax(hl, p0);
+            hh = fmin(hh, p1);
+        } else if (!(base > lo[i] && base < hi[i])) {
+            live = false;
+        }
     }
-    vc *= P.inv_st2; hv *= P.inv_st2; uc *= P.inv_st2; hu *= P.inv_st2;
-    const int k_lo = max((int)ceil(vc - hv), -hf + excl), k_hi = min((int)floor(vc + hv), hf - 1);
-    const int h_lo = max((int)ceil(uc - hu), -hf + excl), h_hi = min((int)floor(uc + hu), hf - 1);
-    if (k_lo > k_hi || h_lo > h_hi) return;
+    return live && hl <= hh ? make_int2((int)ceil(hl), (int)floor(hh)) : make_int2(0, -1);
+}
+
+// Walk the pixels of pair Q that can reach the tile, on the particle's phase
+// lattice: lane t takes a group of Lh consecutive pixels of one lattice row
+// (h = g, g + 1, ..., g + Lh - 1 with g = h_lo + sh j + Lh i), one pixel of
+// each column phase, and the warp steps through the phases together: at step
+// ph every lane holds a point of phase (ph, pk), so the conflict-free property
+// of a phase holds, and pix() ends each step with __syncwarp.  Each pixel's
+// value is fetched one step before it is gridded (fetch(h, k, act), then
+// pix(value, h, k, act)).  (Groups that start at a row's first pixel instead
+// of on the lattice fill the lanes better, 10.5 against 11.4 thousand steps a
+// particle, but add a voxel's contributions in another order.)
+//
+// The rows' bounds are FP32 with an error bound; where that does not settle
+// the integers (1 to 2% of the walks) the warp evaluates them in FP64, so the
+// pixels are the FP64 ones always.  A lane finds its group's row from the
+// groups' starts in a bit mask.  The FP64 bounds, a shuffle scan and a binary
+// search in shared memory took 2.8 of 6.0 ms per 953 particles at 256^3.
+template <int TX, int TY, int TZ, class Fetch, class Pix>
+__device__ __forceinline__ void walk_groups(const DevParticle& P, const Pair& Q, const RowBounds& B, double e,
+                                             double ox, double oy, double oz, int lane, int4* s_row, Fetch&& fetch,
+                                             Pix&& pix) {
+    const int k_lo = Q.k_lo, k_hi = Q.k_hi, h_lo = Q.h_lo, h_hi = Q.h_hi;
     int Lh, Lk, sh;
-    if (P.lat) {
-        Lh = P.lat & 0xfff; Lk = (P.lat >> 12) & 0xfff; sh = (P.lat >> 24) & 0x7f;
+    if (Q.lat) {
+        Lh = Q.lat & 0xfff; Lk = (Q.lat >> 12) & 0xfff; sh = (Q.lat >> 24) & 0x7f;
     } else {
-        const int L = max(1, (int)ceilf(1.7320508f * 1.0001f * P.inv_step));
+        const int L = max(1, (int)ceilf(1.7320508f * 1.0001f * Q.inv_step));
         if (L * L > 12 && 3.6055513f * P.step >= 1.7320508f * 1.0001f) { Lh = 4; Lk = 3; sh = 2; }
         else { Lh = L; Lk = L; sh = 0; }
     }
-    const double* ia = P.iad;
     const float iLh = __fdividef(1.0f, (float)Lh);
+    const unsigned lt = (1u << lane) - 1u;
     for (int pk = 0; pk < Lk; ++pk) {
         const int k0 = k_lo + pk;
         if (k0 > k_hi) break;
         for (int jb = 0; k0 + Lk * jb <= k_hi; jb += 32) {
-            const int j = jb + lane;
-            const int k = k0 + Lk * j;
-            double hl = h_lo, hh = h_hi;
-            bool live = k <= k_hi;
-            if (live) {
-                for (int i = 0; i < 3; ++i) {
-                    const double base = k * P.bd[i];
-                    if (ia[i] != 0.0) {
-                        double p0 = (lo[i] - base) * ia[i], p1 = (hi[i] - base) * ia[i];
-                        if (p0 > p1) { const double t = p0; p0 = p1; p1 = t; }
-                        hl = fmax(hl, p0);
-                        hh = fmin(hh, p1);
-                    } else if (!(base > lo[i] && base < hi[i])) {
-                        live = false;
-                    }
-                }
-                live = live && hl <= hh;
-            }
-            // this row's pixels [hmin, hmax] in groups of Lh from its phase-0
-            // lattice point g0 = h_lo + sh j (mod Lh)
-            int gfirst = 0, cnt = 0, hmin = 0, hmax = -1;
-            if (live) {
-                hmin = (int)ceil(hl);
-                hmax = (int)floor(hh);
-                if (hmax >= hmin) {
-                    const int g0 = h_lo + sh * j;
-                    const int i0 = floor_div(hmin - g0, Lh, iLh);
-                    const int i1 = floor_div(hmax - g0, Lh, iLh);
-                    gfirst = g0 + Lh * i0;
-                    cnt = i1 - i0 + 1;
-                }
-            }
-            int incl = cnt;
+            const int j = jb + lane, k = k0 + Lk * j;
+            const bool row = k <= k_hi;
+            int hmin = 0, hmax = -1;
+            bool sure = !row;
+            if (row && !B.exact) {
+                const float dk = (float)(k - Q.kc);
+                const float b[3] = {fmaf(dk, Q.cx, Q.bx), fmaf(dk, Q.cy, Q.by), fmaf(dk, Q.cz, Q.bz)};
+                float la = -1e9f, lb = -1e9f, ha = 1e9f, hb = 1e9f;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
+                for (int i = 0; i < 3; ++i) {
+                    const float q = -b[i] * B.ia[i];
+                    la = fmaxf(la, q + B.lo_a[i]);
+                    lb = fmaxf(lb, q + B.lo_b[i]);
+                    ha = fminf(ha, q + B.hi_a[i]);
+                    hb = fminf(hb, q + B.hi_b[i]);
+                }
+                hmin = max(h_lo, Q.hc + __float2int_ru(la));
+                hmax = min(h_hi, Q.hc + __float2int_rd(hb));
+                sure = hmin > hmax || (hmin == max(h_lo, Q.hc + __float2int_ru(lb)) &&
+                                       hmax == min(h_hi, Q.hc + __float2int_rd(ha)));
             }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            if (__any_sync(0xffffffffu, !sure) && row) {
+                const int2 r = row_bounds<TX, TY, TZ>(P, k, h_lo, h_hi, ox, oy, oz, e);
+                hmin = r.x;
+                hmax = r.y;
+            }
+            // the row's groups; cnt < 16 in all but extreme geometries
+            int gfirst = 0, cnt = 0;
+            if (hmax >= hmin) {
+                const int g0 = h_lo + sh * j, i0 = floor_div(hmin - g0, Lh, iLh);
+                gfirst = g0 + Lh * i0;
+                cnt = floor_div(hmax - g0, Lh, iLh) - i0 + 1;
+            }
+            int off, total;
+            if (!__any_sync(0xffffffffu, cnt > 15)) {
+                const unsigned b0 = __ballot_sync(0xffffffffu, cnt & 1), b1 = __ballot_sync(0xffffffffu, cnt & 2),
+                               b2 = __ballot_sync(0xffffffffu, cnt & 4), b3 = __ballot_sync(0xffffffffu, cnt & 8);
+                off = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt) + 8 * __popc(b3 & lt);
+                total = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2) + 8 * __popc(b3);
+            } else {
+                int incl = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                off = incl - cnt;
+                total = __shfl_sync(0xffffffffu, incl, 31);
+            }
             if (total == 0) continue;
-            s_row[lane] = incl;                        // inclusive end of row j's groups
-            s_row[32 + lane] = gfirst;
-            s_row[64 + lane] = k;
-            s_row[96 + lane] = hmin;
-            s_row[128 + lane] = hmax;
+            const unsigned some = __ballot_sync(0xffffffffu, cnt > 0);
+            if (cnt > 0) s_row[__popc(some & lt)] = make_int4(gfirst - Lh * off, k, hmin, hmax);
             __syncwarp();
             for (int t0 = 0; t0 < total; t0 += 32) {
+                const bool here = cnt > 0 && (unsigned)(off - t0) < 32u;
+                const unsigned starts = __reduce_or_sync(0xffffffffu, here ? 1u << (off - t0) : 0u);
+                const int before = __popc(__ballot_sync(0xffffffffu, cnt > 0 && off < t0));
                 const int t = t0 + lane;
                 const bool in = t < total;
-                int r = 0;                              // row holding group t
-#pragma unroll
-                for (int sft = 16; sft > 0; sft >>= 1)
-                    if (s_row[r + sft - 1] <= t) r += sft;
-                r = min(r, 31);
-                const int before = r ? s_row[r - 1] : 0;
-                const int g = s_row[32 + r] + Lh * (t - before);
-                const int kr = s_row[64 + r], lo_h = s_row[96 + r], hi_h = s_row[128 + r];
+                const int4 r = s_row[max(0, before + __popc(starts & (lt | (1u << lane))) - 1)];
+                const int g = r.x + Lh * t;
+                bool act = in && g >= r.z && g <= r.w;
+                float2 f = fetch(g, r.y, act);
+#pragma unroll 1
                 for (int ph = 0; ph < Lh; ++ph) {
-                    const int h = g + ph;
-                    pix(h, kr, in && h >= lo_h && h <= hi_h);
+                    const int h = g + ph + 1;
+                    const bool next = in && ph + 1 < Lh && h >= r.z && h <= r.w;
+                    const float2 fn = fetch(h, r.y, next);
+                    pix(f, h - 1, r.y, act);
+                    f = fn;
+                    act = next;
                 }
             }
             __syncwarp();
@@ -431,42 +482,90 @@ __device__ __forceinline__ void walk_groups(const DevParticle& P, int hf, double
 // subtracted, so a voxel that nothing reaches reads exactly zero.
 // walk_edges visits the unpaired pixels whose tents reach the tile, one
 // line at a time, points L pixels apart (L step >= sqrt(3) voxels) so that
-// the lanes of a call touch distinct cells; pix(h, k, act) as walk_groups.
-template <int TX, int TY, int TZ, class Pix>
-__device__ __forceinline__ void walk_edges(const DevParticle& P, int hf, double ox, double oy, double oz, int lane,
-                                           Pix&& pix) {
+// the lanes of a call touch distinct cells; edge_range gives a line's pixels
+// (line 0: (t, -hf), t in [-hf, hf - 1]; line 1: (-hf, t), t in [-hf + 1,
+// hf - 1]; t0 > t1: none).
+template <int TX, int TY, int TZ>
+__device__ __noinline__ void edge_range(const DevParticle& P, int hf, double ox, double oy, double oz, int line,
+                                           int& t0, int& t1) {
     const double lo[3] = {ox - 1.0, oy - 1.0, oz - 1.0};
     const double hi[3] = {ox + TX, oy + TY, oz + TZ};
-    const int L = max(1, (int)ceilf(1.7320508f * 1.0001f * P.inv_step));
-    for (int line = 0; line < 2; ++line) {
-        // 0: (t, -hf), t in [-hf, hf - 1];  1: (-hf, t), t in [-hf + 1, hf - 1]
-        const bool along_h = line == 0;
-        double tl = line == 0 ? -hf : -hf + 1;
-        double th = hf - 1;
-        bool live = true;
-        for (int i = 0; i < 3; ++i) {
-            const double idir = along_h ? P.iad[i] : P.ibd[i];
-            const double base = -hf * (along_h ? P.bd[i] : P.ad[i]);
-            if (idir != 0.0) {
-                double p0 = (lo[i] - base) * idir, p1 = (hi[i] - base) * idir;
-                if (p0 > p1) { const double t = p0; p0 = p1; p1 = t; }
-                tl = fmax(tl, p0);
-                th = fmin(th, p1);
-            } else if (!(base >= lo[i] && base <= hi[i])) {
-                live = false;
-            }
+    const bool along_h = line == 0;
+    double tl = line == 0 ? -hf : -hf + 1;
+    double th = hf - 1;
+    bool live = true;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const double idir = along_h ? P.iad[i] : P.ibd[i];
+        const double base = -hf * (along_h ? P.bd[i] : P.ad[i]);
+        if (idir != 0.0) {
+            double p0 = (lo[i] - base) * idir, p1 = (hi[i] - base) * idir;
+            if (p0 > p1) { const double t = p0; p0 = p1; p1 = t; }
+            tl = fmax(tl, p0);
+            th = fmin(th, p1);
+        } else if (!(base >= lo[i] && base <= hi[i])) {
+            live = false;
         }
-        if (!live) continue;
-        const int t0 = (int)ceil(tl), t1 = (int)floor(th);
+    }
+    t0 = 0;
+    t1 = -1;
+    if (live && tl <= th) {
+        t0 = (int)ceil(tl);
+        t1 = (int)floor(th);
+    }
+}
+
+template <class Fetch, class Pix>
+__device__ __forceinline__ void walk_edges(const Pair& Q, int hf, int lane, Fetch&& fetch, Pix&& pix) {
+    const int L = max(1, (int)ceilf(1.7320508f * 1.0001f * Q.inv_step));
+#pragma unroll 1
+    for (int line = 0; line < 2; ++line) {
+        const int t0 = line ? Q.k_lo : Q.h_lo, t1 = line ? Q.k_hi : Q.h_hi;
         for (int ph = 0; ph < L; ++ph) {
             const int first = t0 + ph;
             if (first > t1) break;
             for (int tb = first; tb <= t1; tb += 32 * L) {
                 const int t = tb + L * lane;
-                pix(along_h ? t : -hf, along_h ? -hf : t, t <= t1);
+                const int h = line ? -hf : t, k = line ? t : -hf;
+                const bool act = t <= t1;
+                pix(fetch(h, k, act), h, k, act);
             }
         }
     }
+}
+
+// Of the aliases in `mask`, those whose tile box (grown by a voxel) comes
+// near a line of unpaired pixels: the box's enclosing sphere against the
+// segment, in FP32 with a margin above its rounding (a superset; edge_range
+// decides).  A plane reaches some 1,400 (tile, alias) pairs below the split of
+// a 256^3 map, its two lines about 130: setting all of them up took 2.9 of
+// 13.3 ms per 2,000 particles.
+template <int TX, int TY, int TZ>
+__device__ __forceinline__ unsigned edge_mask(const DevParticle& P, unsigned mask, int x0, int y0, int z0, int N,
+                                              int ft) {
+    const float hf = 0.5f * ft;
+    const float ex = 0.5f * (TX + 1), ey = 0.5f * (TY + 1), ez = 0.5f * (TZ + 1);
+    const float R = sqrtf(ex * ex + ey * ey + ez * ez) + 0.05f;
+    const float ax = P.af[0], ay = P.af[1], az = P.af[2], bx = P.bf[0], by = P.bf[1], bz = P.bf[2];
+    const float ia = 1.0f / (ax * ax + ay * ay + az * az), ib = 1.0f / (bx * bx + by * by + bz * bz);
+    unsigned out = 0;
+    while (mask) {
+        const int al = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const float cx = x0 - ((al & 1) ? N : 0) + 0.5f * (TX - 1), cy = y0 - ((al & 2) ? N : 0) + 0.5f * (TY - 1),
+                    cz = z0 - ((al & 4) ? N : 0) + 0.5f * (TZ - 1);
+        // d = centre - (the line's offset -hf v); the nearest point is t u
+        float dx = fmaf(hf, bx, cx), dy = fmaf(hf, by, cy), dz = fmaf(hf, bz, cz);
+        float t = fminf(fmaxf((dx * ax + dy * ay + dz * az) * ia, -hf), hf);
+        dx -= t * ax; dy -= t * ay; dz -= t * az;
+        bool near = dx * dx + dy * dy + dz * dz <= R * R;
+        dx = fmaf(hf, ax, cx); dy = fmaf(hf, ay, cy); dz = fmaf(hf, az, cz);
+        t = fminf(fmaxf((dx * bx + dy * by + dz * bz) * ib, -hf), hf);
+        dx -= t * bx; dy -= t * by; dz -= t * bz;
+        near = near || dx * dx + dy * dy + dz * dz <= R * R;
+        if (near) out |= 1u << al;
+    }
+    return out;
 }
 
 // Can an unpaired pixel (at least rmin voxels from the origin, and no pixel
@@ -488,53 +587,52 @@ __device__ __forceinline__ bool tile_reaches_edges(int x0, int y0, int z0, int N
     return false;
 }
 
-template <bool FOM, bool GATE, int TX, int TY, int TZ>
+template <bool GATE, int TX, int TY, int TZ>
 __device__ __forceinline__ void scatter_particle(const InsertArgs& a, const DevParticle& P, const float2* S,
                                                  const TileAcc& A, double ox, double oy, double oz, int lane,
                                                  int* s_row) {
     walk_pair<TX, TY, TZ>(P, a.ft / 2, ox, oy, oz, lane, s_row, [&](int h, int k, bool act) {
-        pixel<FOM, GATE, TX, TY, TZ>(a, P, S, A, ox, oy, oz, h, k, act);
+        pixel<GATE, TX, TY, TZ>(a, P, S, A, ox, oy, oz, h, k, act);
     });
 }
 
 // Tile sums -> HBM: added to the map accumulators (one replica), or stored
 // into this replica's partial buffer (combined later in replica order).
-template <bool FOM, int TX, int TY, int TZ>
+template <int TX, int TY, int TZ>
 __device__ __forceinline__ void fold_tile(const InsertArgs& a, const TileAcc& A, int x0, int y0, int z0, int r,
                                           int lane) {
     const int N = a.N;
     constexpr int TV = TX * TY * TZ;
     const size_t N3 = (size_t)N * N * N;
-    const int nch = FOM ? 5 : 3;
     for (int i = lane; i < TV; i += 32) {
         const int lx = i % TX, ly = (i / TX) % TY, lz = i / (TX * TY);
         const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
         if (x < N && y < N && z < N) {
             const size_t idx = ((size_t)z * N + y) * N + x;
             if (a.R > 1) {
-                double* pb = a.psum + (size_t)r * nch * N3 + idx;
+                double* pb = a.fsum + (size_t)r * 5 * N3 + idx;
                 pb[0] = A.re[i];
                 pb[N3] = A.im[i];
                 pb[2 * N3] = A.w[i];
-                if (FOM) { pb[3 * N3] = A.p[i]; pb[4 * N3] = A.q[i]; }
+                pb[3 * N3] = A.p[i]; pb[4 * N3] = A.q[i];
             } else {
                 double2 o = a.vol[idx];
                 o.x += A.re[i];
                 o.y += A.im[i];
                 a.vol[idx] = o;
                 a.w[idx] += A.w[i];
-                if (FOM) { a.pow[idx] += A.p[i]; a.w2[idx] += A.q[i]; }
+                a.pow[idx] += A.p[i]; a.w2[idx] += A.q[i];
             }
         }
         A.re[i] = 0; A.im[i] = 0; A.w[i] = 0;
-        if (FOM) { A.p[i] = 0; A.q[i] = 0; }
+        A.p[i] = 0; A.q[i] = 0;
     }
     __syncwarp();
 }
 
-template <bool FOM, bool GATE, int TX, int TY, int TZ>
+template <bool GATE, int TX, int TY, int TZ>
 __global__ void __launch_bounds__(WARPS * 32) insert_kernel(InsertArgs a) {
-    constexpr int NCH = FOM ? 5 : 3;
+    constexpr int NCH = 5;
     constexpr int TV = TX * TY * TZ;
     extern __shared__ tacc_t s_dacc[];                 // WARPS x NCH x TV
     tacc_t* const my_acc = s_dacc + (size_t)(threadIdx.x >> 5) * NCH * TV;
@@ -552,7 +650,7 @@ __global__ void __launch_bounds__(WARPS * 32) insert_kernel(InsertArgs a) {
     const size_t spec_stride = (size_t)(2 * hf + 1) * a.pitch;
     TileAcc A;
     A.re = my_acc; A.im = A.re + TV; A.w = A.im + TV;
-    A.p = FOM ? A.w + TV : nullptr; A.q = FOM ? A.p + TV : nullptr;
+    A.p = A.w + TV; A.q = A.p + TV;
     for (int i = lane; i < NCH * TV; i += 32) my_acc[i] = 0;
     __syncwarp();
 
@@ -573,24 +671,25 @@ __global__ void __launch_bounds__(WARPS * 32) insert_kernel(InsertArgs a) {
             const float2* S = a.spec + (size_t)P.spec * spec_stride;
             for (int al = 0; al < 8; ++al)
                 if ((am >> al) & 1u)
-                    scatter_particle<FOM, GATE, TX, TY, TZ>(a, P, S, A, (double)(x0 - ((al & 1) ? N : 0)),
+                    scatter_particle<GATE, TX, TY, TZ>(a, P, S, A, (double)(x0 - ((al & 1) ? N : 0)),
                                                 (double)(y0 - ((al & 2) ? N : 0)),
                                                 (double)(z0 - ((al & 4) ? N : 0)), lane, s_rows[warp]);
         }
     }
-    fold_tile<FOM, TX, TY, TZ>(a, A, x0, y0, z0, rep, lane);
+    fold_tile<TX, TY, TZ>(a, A, x0, y0, z0, rep, lane);
 }
 
-// ---- gridding without the FOM channels: float4 cells --------------------
+// ---- gridding without the FOM channels -----------------------------------
 //
-// The map tile is an array of float4 cells {F re * w, F im * w, w, unused},
-// so a corner's read-modify-write is one 16-byte load, three adds and one
-// 16-byte store.  Cell (x, y, z) of the tile sits at slot x + PX y + PP z:
-// the plane pitch PP (PX TY plus a few unused slots) spreads the cells a
-// warp's lattice points touch over the eight 16-byte bank groups (at 8^3,
-// PP = 68 puts cell (x, y, z) in group (x + 4 z) mod 8; the pitches were
-// chosen by simulating the lattice walk over random orientations), and the
-// corner offsets stay compile-time constants.
+// The map tile is an array of float2 cells {F re * w, F im * w} and one of
+// float weights, so a corner's read-modify-write is an 8-byte and a 4-byte
+// load, three adds and the two stores.  Cell (x, y, z) of the tile sits at
+// index x + PX y + PP z: the plane pitch PP (PX TY plus a few unused cells)
+// spreads the cells that a warp's lattice points touch over the banks, and the
+// corner offsets stay compile-time constants.  The shared-memory pipe is what
+// bounds the scatter: as one float4 cell a corner took 4 + 4 wavefronts at
+// best where this takes 3 + 3 (5.47 -> 4.90 ms per 953 particles at 256^3;
+// pitches 64 to 102 measured between 4.90 and 5.44).
 //
 // Map frequencies are formed in FP32 relative to the tile: per (tile,
 // particle) pair an anchor pixel (hc, kc) near the tile's projection has its
@@ -601,34 +700,40 @@ __global__ void __launch_bounds__(WARPS * 32) insert_kernel(InsertArgs a) {
 // lands on the other side of a cell boundary because of it moves a
 // contribution by that much, and the phase lattices keep a margin above it
 // (lattice.h).
-// One cell's read-modify-write as a single 16-byte shared load and store
-// (the unused fourth word travels with them, so the compiler cannot split the
-// access into narrower ones).
-__device__ __forceinline__ void cell_add(unsigned addr, float2 f, float w) {
-    float x, y, z, u;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x), "=f"(y), "=f"(z), "=f"(u) : "r"(addr) : "memory");
+// One cell's read-modify-write; SLOTS: cells of the tile (the weights follow
+// them).  A corner outside the tile (on = false) loads the tile's first cell
+// and stores nothing: a select and a predicate instead of a branch per corner
+// (as float4 cells, 6.53 -> 5.47 ms per 953 particles at 256^3).
+template <int SLOTS>
+__device__ __forceinline__ void cell_add(unsigned cell0, int index, float2 f, float w, bool on) {
+    const unsigned i = on ? index : 0, at = cell0 + 8u * i, wt = cell0 + 8u * SLOTS + 4u * i;
+    float x, y, z;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(at) : "memory");
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(z) : "r"(wt) : "memory");
     x = fmaf(f.x, w, x);
     y = fmaf(f.y, w, y);
     z += w;
-    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" :: "r"(addr), "f"(x), "f"(y), "f"(z), "f"(u) : "memory");
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t"
+        "@p st.shared.v2.f32 [%0], {%1, %2};\n\t@p st.shared.f32 [%3], %4;\n\t}" ::"r"(at),
+        "f"(x), "f"(y), "r"(wt), "f"(z), "r"((int)on)
+        : "memory");
 }
 
 template <bool GATE, bool EW, int TX, int TY, int TZ, int PX, int PP>
-__device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P, const float2* S, float4* cell,
-                                       unsigned cell0,
-                                       float bx, float by, float bz, int hc, int kc, int h, int k, bool act) {
-    const int hf = a.ft / 2;
-    float wt = P.pw;
+__device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P, const Pair& Q, unsigned cell0,
+                                       float2 f, int h, int k, bool act) {
+    float wt = Q.pw;
     if (GATE && act) {
         bool keep;
         const float tw = pixel_weight_gate(a, P, h, k, keep);
         if (!keep) act = false;
         wt *= tw;
     }
-    const float dh = (float)(h - hc), dk = (float)(k - kc);
-    float mx = fmaf(dh, P.af[0], fmaf(dk, P.bf[0], bx));
-    float my = fmaf(dh, P.af[1], fmaf(dk, P.bf[1], by));
-    float mz = fmaf(dh, P.af[2], fmaf(dk, P.bf[2], bz));
+    const float dh = (float)(h - Q.hc), dk = (float)(k - Q.kc);
+    float mx = fmaf(dh, Q.ax, fmaf(dk, Q.cx, Q.bx));
+    float my = fmaf(dh, Q.ay, fmaf(dk, Q.cy, Q.by));
+    float mz = fmaf(dh, Q.az, fmaf(dk, Q.cz, Q.bz));
     if (EW && P.ewh != 0.0) {
         // Ewald surface: s_z = +-(lambda/2) s2 along R[:,2] (Bimage_reconstruct.cpp:
         // 157-168), at most P.ezmax voxels, added in FP32 to the tile-relative
@@ -638,7 +743,6 @@ __device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P
         my += (float)(sz * P.cd[1]);
         mz += (float)(sz * P.cd[2]);
     }
-    const float2 f = act ? __ldg(S + (size_t)(k + hf) * a.pitch + (h + hf)) : make_float2(0.f, 0.f);
     if (a.interp != 2) {
         const float fx = floorf(mx + 0.5f), fy = floorf(my + 0.5f), fz = floorf(mz + 0.5f);
         const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
@@ -647,164 +751,300 @@ __device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P
             const float dx = mx - fx, dy = my - fy, dz = mz - fz;
             w = wt * (1.0f - sqrtf(dx * dx + dy * dy + dz * dz));
         }
-        if (act && (unsigned)ix < TX && (unsigned)iy < TY && (unsigned)iz < TZ && w > 0.f)
-            cell_add(cell0 + 16u * (unsigned)(ix + PX * iy + PP * iz), f, w);
+        const bool on = act && (unsigned)ix < TX && (unsigned)iy < TY && (unsigned)iz < TZ && w > 0.f;
+        cell_add<PP * TZ>(cell0, ix + PX * iy + PP * iz, f, w, on);
         __syncwarp();
         return;
     }
     const float flx = floorf(mx), fly = floorf(my), flz = floorf(mz);
     const int ix = (int)flx, iy = (int)fly, iz = (int)flz;
     const float rx = mx - flx, ry = my - fly, rz = mz - flz;
-    const bool vx[2] = {(unsigned)ix < TX, (unsigned)(ix + 1) < TX};
+    const bool vx[2] = {act && (unsigned)ix < TX, act && (unsigned)(ix + 1) < TX};
     const bool vy[2] = {(unsigned)iy < TY, (unsigned)(iy + 1) < TY};
     const bool vz[2] = {(unsigned)iz < TZ, (unsigned)(iz + 1) < TZ};
-    const unsigned cell_addr = cell0 + 16u * (unsigned)(ix + PX * iy + PP * iz);
+    const int cell = ix + PX * iy + PP * iz;
 #pragma unroll
     for (int dz = 0; dz < 2; ++dz) {
         const float wz = (dz ? rz : 1.f - rz) * wt;
 #pragma unroll
         for (int dy = 0; dy < 2; ++dy) {
             const float wyz = (dy ? ry : 1.f - ry) * wz;
+            const bool vyz = vy[dy] && vz[dz];
 #pragma unroll
             for (int dx = 0; dx < 2; ++dx) {
-                if (act && vx[dx] && vy[dy] && vz[dz]) {
-                    const float w = (dx ? rx : 1.f - rx) * wyz;
-                    cell_add(cell_addr + 16u * (unsigned)(dx + PX * dy + PP * dz), f, w);
-                }
+                cell_add<PP * TZ>(cell0, cell + dx + PX * dy + PP * dz, f, (dx ? rx : 1.f - rx) * wyz,
+                         vx[dx] && vyz);
                 __syncwarp();
             }
         }
     }
 }
 
-template <bool GATE, bool EW, int TX, int TY, int TZ, int PX, int PP, int NW>
-__global__ void __launch_bounds__(NW * 32, 5) grid4_kernel(InsertArgs a) {
+// The pair's set-up by one lane: the pixels whose tents can reach the tile at
+// alias origin (ox, oy, oz) lie in [h_lo, h_hi] x [k_lo, k_hi] (excl = 1
+// leaves out the row k = -hf and the column h = -hf, which half-space gridding
+// grids separately), or, for the edge walk, the two lines' ranges; the anchor
+// is the tile centre's projection on the plane.  False: no pixel.
+template <int TX, int TY, int TZ>
+__device__ __noinline__ bool setup_pair(const DevParticle& P, int part, int hf, double ox, double oy, double oz,
+                                           bool edge, int excl, Pair& Q, RowBounds& B) {
+    if (edge) {
+        edge_range<TX, TY, TZ>(P, hf, ox, oy, oz, 0, Q.h_lo, Q.h_hi);
+        edge_range<TX, TY, TZ>(P, hf, ox, oy, oz, 1, Q.k_lo, Q.k_hi);
+        if (Q.h_lo > Q.h_hi && Q.k_lo > Q.k_hi) return false;
+    } else {
+        const double e = P.ezmax;
+        const double lo[3] = {ox - 1.0 - e, oy - 1.0 - e, oz - 1.0 - e};
+        const double hi[3] = {ox + TX + e, oy + TY + e, oz + TZ + e};
+        double vc = 0, hv = 0, uc = 0, hu = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double c = 0.5 * (lo[i] + hi[i]), e2 = 0.5 * (hi[i] - lo[i]);
+            vc += P.bd[i] * c; hv += fabs(P.bd[i]) * e2;
+            uc += P.ad[i] * c; hu += fabs(P.ad[i]) * e2;
+        }
+        vc *= P.inv_st2; hv *= P.inv_st2; uc *= P.inv_st2; hu *= P.inv_st2;
+        Q.k_lo = max((int)ceil(vc - hv), -hf + excl);
+        Q.k_hi = min((int)floor(vc + hv), hf - 1);
+        Q.h_lo = max((int)ceil(uc - hu), -hf + excl);
+        Q.h_hi = min((int)floor(uc + hu), hf - 1);
+        if (Q.k_lo > Q.k_hi || Q.h_lo > Q.h_hi) return false;
+    }
+    const double cx = ox + 0.5 * (TX - 1), cy = oy + 0.5 * (TY - 1), cz = oz + 0.5 * (TZ - 1);
+    Q.hc = (int)rint((P.ad[0] * cx + P.ad[1] * cy + P.ad[2] * cz) * P.inv_st2);
+    Q.kc = (int)rint((P.bd[0] * cx + P.bd[1] * cy + P.bd[2] * cz) * P.inv_st2);
+    Q.bx = (float)(Q.hc * P.ad[0] + Q.kc * P.bd[0] - ox);
+    Q.by = (float)(Q.hc * P.ad[1] + Q.kc * P.bd[1] - oy);
+    Q.bz = (float)(Q.hc * P.ad[2] + Q.kc * P.bd[2] - oz);
+    Q.part = part;
+    Q.lat = P.lat;
+    Q.pw = P.pw;
+    Q.inv_step = P.inv_step;
+    Q.ax = P.af[0]; Q.ay = P.af[1]; Q.az = P.af[2];
+    Q.cx = P.bf[0]; Q.cy = P.bf[1]; Q.cz = P.bf[2];
+    Q.spec = P.spec;
+    if (edge) return true;
+    // Errors of -b ia + bound: b is off by its own rounding, the steps' and
+    // the sum's (|b| < 64 voxels: < 1e-5), and each product and sum by 2^-24
+    // of at most 64 |ia|; together < 3e-5 |ia|, and the integers' own sum.
+    B.exact = 0;
+    const int T[3] = {TX, TY, TZ};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float ia = (float)P.iad[i], err = 5e-5f * fabsf(ia) + 1e-5f;
+        const float p0 = (-1.0f - P.ezmax) * ia, p1 = ((float)T[i] + P.ezmax) * ia;
+        if (ia == 0.f) B.exact = 1;
+        B.ia[i] = ia;
+        B.lo_a[i] = fminf(p0, p1) - err;
+        B.lo_b[i] = fminf(p0, p1) + err;
+        B.hi_a[i] = fmaxf(p0, p1) - err;
+        B.hi_b[i] = fmaxf(p0, p1) + err;
+    }
+    return true;
+}
+
+// Work items: R replicas of a tile, each on its slice of the particles, and
+// with half-space gridding one more per tile below the split for the unpaired
+// pixels (all particles).  The pairs that reach the tile are queued QN at a
+// time, in (particle, alias) order, and set up by one lane each: the FP64
+// set-up of a pair cost the warp ~850 instructions of the ~3,900 a pair
+// takes when every lane did it.  One warp per CTA: the items' times differ, and
+// in CTAs of four the early ones' shared memory waited for the last (11 of 20
+// warps resident on average).
+template <bool GATE, bool EW, int TX, int TY, int TZ, int PX, int PP>
+__global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
     constexpr int SLOTS = PP * TZ;
     constexpr int TV = TX * TY * TZ;
-    extern __shared__ float4 s_cells[];                 // NW x SLOTS
-    __shared__ int s_rows[NW][160];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float4* const cell = s_cells + (size_t)warp * SLOTS;
-    const int gw = blockIdx.x * NW + warp;
-    const int slot = gw / a.R, rep = gw % a.R;        // replicas of a tile are adjacent
-    if (slot >= a.ntx * a.nty * a.ntz) return;
+    extern __shared__ float2 s_sum[];                   // SLOTS cells, then their weights
+    float* const s_wt = reinterpret_cast<float*>(s_sum + SLOTS);
+    __shared__ int4 s_rows[32];
+    __shared__ Pair s_pairs[QN];
+    __shared__ RowBounds s_bounds[QN];
+    __shared__ int s_ids[QN];
+    const int lane = threadIdx.x;
+    const bool hs = a.zsplit > 0;
+    const int items = a.R + (hs ? 1 : 0);               // per tile
+    const int slot = blockIdx.x / items, rep = blockIdx.x - slot * items;
     const int tile = a.order[slot];
-    const int p_lo = (int)((long)a.np * rep / a.R), p_hi = (int)((long)a.np * (rep + 1) / a.R);
     const int x0 = (tile % a.ntx) * TX, y0 = ((tile / a.ntx) % a.nty) * TY, z0 = (tile / (a.ntx * a.nty)) * TZ;
     const int N = a.N;
     const int hf = a.ft / 2;
     const size_t spec_stride = (size_t)(2 * hf + 1) * a.pitch;
-    const unsigned cell0 = (unsigned)__cvta_generic_to_shared(cell);
+    const unsigned cell0 = (unsigned)__cvta_generic_to_shared(s_sum);
     // half-space gridding (walk_edges): tiles at or above zsplit grid only
-    // the unpaired pixels; those below it grid the others, and then (one
-    // replica, all particles) the unpaired ones into evol / ew
-    const bool hs = a.zsplit > 0;
+    // the unpaired pixels; those below it grid the others, and the extra item
+    // the unpaired ones into evol / ew
     const bool upper = hs && z0 >= a.zsplit;
-    const bool edges = hs && tile_reaches_edges<TX, TY, TZ>(x0, y0, z0, N, a.edge_rmin, a.edge_rmax);
-    for (int i = lane; i < SLOTS; i += 32) cell[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool extra = rep == a.R;
+    if (extra && upper) return;
+    const bool edge_walk = extra || upper;
+    // (a tile that no unpaired pixel reaches skips the edge walks)
+    const bool none = edge_walk && !tile_reaches_edges<TX, TY, TZ>(x0, y0, z0, N, a.edge_rmin, a.edge_rmax);
+    if (extra && none) return;
+    const int p_lo = extra ? 0 : (int)((long)a.np * rep / a.R);
+    const int p_hi = none ? p_lo : extra ? a.np : (int)((long)a.np * (rep + 1) / a.R);
+    for (int i = lane; i < SLOTS; i += 32) {
+        s_sum[i] = make_float2(0.f, 0.f);
+        s_wt[i] = 0.f;
+    }
     __syncwarp();
 
-    // pass 0: the tile's sums (all pixels; with half-space gridding the
-    // paired ones, or above the split the unpaired ones); pass 1: the
-    // unpaired pixels of a tile below the split
-    for (int pass = 0; pass < 2; ++pass) {
-        if (pass == 1 && !(hs && !upper && edges && rep == 0)) break;
-        const bool edge_walk = pass == 1 || upper;
-        const int b_lo = pass ? 0 : p_lo, b_hi = pass ? a.np : p_hi;
-        // (a tile that no unpaired pixel reaches skips the edge walks)
-        const int b_end = (edge_walk && !edges) ? b_lo : b_hi;
-        for (int base = b_lo; base < b_end; base += 32) {
-            const int p = base + lane;
-            unsigned mask = 0;
-            if (p < b_hi) {
-                const DevParticle& P = a.part[p];
-                if (P.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(P, x0, y0, z0, N, a.ft);
+    bool any = false;                // some pair reached the tile
+    int base = p_lo - 32, qn = 0;
+    unsigned mask = 0;               // this lane's particle's aliases still to be queued
+    for (;;) {
+        const unsigned todo = __ballot_sync(0xffffffffu, mask != 0);
+        if (todo) {
+            const int cnt = __popc(mask);
+            int off = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, off, o);
+                if (lane >= o) off += v;
             }
-            unsigned todo = __ballot_sync(0xffffffffu, mask != 0);
-            while (todo) {
-                const int src = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const unsigned am = __shfl_sync(0xffffffffu, mask, src);
-                const DevParticle& P = a.part[base + src];
-                const float2* S = a.spec + (size_t)P.spec * spec_stride;
-                for (int al = 0; al < 8; ++al) {
-                    if (!((am >> al) & 1u)) continue;
-                    const double ox = (double)(x0 - ((al & 1) ? N : 0));
-                    const double oy = (double)(y0 - ((al & 2) ? N : 0));
-                    const double oz = (double)(z0 - ((al & 4) ? N : 0));
-                    // anchor pixel: the tile centre's projection on the plane
-                    const double cx = ox + 0.5 * (TX - 1), cy = oy + 0.5 * (TY - 1), cz = oz + 0.5 * (TZ - 1);
-                    const int hc = (int)rint((P.ad[0] * cx + P.ad[1] * cy + P.ad[2] * cz) * P.inv_st2);
-                    const int kc = (int)rint((P.bd[0] * cx + P.bd[1] * cy + P.bd[2] * cz) * P.inv_st2);
-                    const float bx = (float)(hc * P.ad[0] + kc * P.bd[0] - ox);
-                    const float by = (float)(hc * P.ad[1] + kc * P.bd[1] - oy);
-                    const float bz = (float)(hc * P.ad[2] + kc * P.bd[2] - oz);
-                    auto pix = [&](int h, int k, bool act) {
-                        pixel4<GATE, EW, TX, TY, TZ, PX, PP>(a, P, S, cell, cell0, bx, by, bz, hc, kc, h, k, act);
-                    };
-                    if (edge_walk) walk_edges<TX, TY, TZ>(P, hf, ox, oy, oz, lane, pix);
-                    else walk_groups<TX, TY, TZ>(P, hf, ox, oy, oz, lane, s_rows[warp], hs ? 1 : 0, pix);
+            const int total = __shfl_sync(0xffffffffu, off, 31);
+            for (int at = qn + off - cnt; mask && at < QN; ++at) {
+                const int al = __ffs(mask) - 1;
+                mask &= mask - 1;
+                s_ids[at] = (base + lane) * 8 + al;
+            }
+            qn = min(QN, qn + total);
+        } else {
+            base += 32;
+            if (base < p_hi) {
+                const int p = base + lane;
+                if (p < p_hi) {
+                    const DevParticle& P = a.part[p];
+                    if (P.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(P, x0, y0, z0, N, a.ft);
+                    if (edge_walk && mask) mask = edge_mask<TX, TY, TZ>(P, mask, x0, y0, z0, N, a.ft);
                 }
+                continue;
             }
+            if (qn == 0) break;
         }
-        // tile sums -> HBM: pass 0 adds to the map (one replica) or stores
-        // this replica's partial sums (combined later in replica order);
-        // pass 1 adds to evol / ew.  The cells are cleared for the next pass.
-        const size_t N3 = (size_t)N * N * N;
-        for (int i = lane; i < TV; i += 32) {
-            const int lx = i % TX, ly = (i / TX) % TY, lz = i / (TX * TY);
-            const int x = x0 + lx, y = y0 + ly, z = z0 + lz;
-            const int ci = lx + PX * ly + PP * lz;
-            const float4 c = cell[ci];
-            if (x < N && y < N && z < N) {
-                const size_t idx = ((size_t)z * N + y) * N + x;
-                if (pass == 1) {
-                    double2 o = a.evol[idx];
-                    o.x += c.x;
-                    o.y += c.y;
-                    a.evol[idx] = o;
-                    a.ew[idx] += c.z;
-                } else if (a.R > 1) {
-                    double* pb = a.psum + (size_t)rep * 3 * N3 + idx;
-                    pb[0] = c.x;
-                    pb[N3] = c.y;
-                    pb[2 * N3] = c.z;
-                } else {
-                    double2 o = a.vol[idx];
-                    o.x += c.x;
-                    o.y += c.y;
-                    a.vol[idx] = o;
-                    a.w[idx] += c.z;
-                }
-            }
-            cell[ci] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        if (qn < QN && base < p_hi) continue;
         __syncwarp();
+        bool ok = false;
+        if (lane < qn) {
+            const int id = s_ids[lane], al = id & 7;
+            ok = setup_pair<TX, TY, TZ>(a.part[id >> 3], id, hf, (double)(x0 - ((al & 1) ? N : 0)),
+                                        (double)(y0 - ((al & 2) ? N : 0)), (double)(z0 - ((al & 4) ? N : 0)),
+                                        edge_walk, hs ? 1 : 0, s_pairs[lane], s_bounds[lane]);
+        }
+        unsigned go = __ballot_sync(0xffffffffu, ok);
+        __syncwarp();
+        any = any || go;
+        while (go) {
+            const int at = __ffs(go) - 1;
+            const Pair Q = s_pairs[at];
+            go &= go - 1;
+            const int al = Q.part & 7;
+            const DevParticle& P = a.part[Q.part >> 3];
+            const float2* S = a.spec + (size_t)Q.spec * spec_stride + (size_t)hf * a.pitch + hf;
+            auto fetch = [&](int h, int k, bool act) {
+                return act ? __ldg(S + (long)k * a.pitch + h) : make_float2(0.f, 0.f);
+            };
+            auto pix = [&](float2 f, int h, int k, bool act) {
+                pixel4<GATE, EW, TX, TY, TZ, PX, PP>(a, P, Q, cell0, f, h, k, act);
+            };
+            if (edge_walk) walk_edges(Q, hf, lane, fetch, pix);
+            else walk_groups<TX, TY, TZ>(P, Q, s_bounds[at], EW ? (double)P.ezmax : 0.0,
+                                          (double)(x0 - ((al & 1) ? N : 0)), (double)(y0 - ((al & 2) ? N : 0)),
+                                          (double)(z0 - ((al & 4) ? N : 0)), lane, s_rows, fetch, pix);
+        }
+        qn = 0;
+        __syncwarp();
+    }
+    // tile sums -> HBM.  One replica (and the unpaired pixels' item) adds to
+    // the map; of several, each stores its FP32 partial sums, and the one that
+    // arrives last adds them in replica order while they are still in L2 (a
+    // separate pass over FP64 partial sums took 0.86 ms of a 256^3 map's
+    // 14.9 ms and 0.93 ms per batch and half map at 384^3).  Replicas that no
+    // pair reached store nothing.
+    const size_t N2 = (size_t)N * N;
+    auto voxel = [&](int i, size_t& idx) {
+        const int x = x0 + i % TX, y = y0 + (i / TX) % TY, z = z0 + i / (TX * TY);
+        idx = (size_t)z * N2 + (size_t)y * N + x;
+        return x < N && y < N && z < N;
+    };
+    if (extra || a.R == 1) {
+        double2* const vol = extra ? a.evol : a.vol;
+        double* const wgt = extra ? a.ew : a.w;
+        if (!any) return;
+#pragma unroll 2
+        for (int i = lane; i < TV; i += 32) {
+            const int ci = i % TX + PX * ((i / TX) % TY) + PP * (i / (TX * TY));
+            size_t idx;
+            if (!voxel(i, idx)) continue;
+            double2 o = vol[idx];
+            o.x += s_sum[ci].x;
+            o.y += s_sum[ci].y;
+            vol[idx] = o;
+            wgt[idx] += s_wt[ci];
+        }
+        return;
+    }
+    float* const mine = a.psum + ((size_t)tile * a.R + rep) * 3 * TV;
+    if (any) {
+#pragma unroll 2
+        for (int i = lane; i < TV; i += 32) {
+            const int ci = i % TX + PX * ((i / TX) % TY) + PP * (i / (TX * TY));
+            mine[i] = s_sum[ci].x;
+            mine[TV + i] = s_sum[ci].y;
+            mine[2 * TV + i] = s_wt[ci];
+        }
+        __threadfence();
+    }
+    __syncwarp();
+    unsigned old = 0;
+    if (lane == 0) old = atomicAdd(&a.arrived[tile], 1u | (any ? 256u << rep : 0u));
+    old = __shfl_sync(0xffffffffu, old, 0);
+    if ((int)(old & 255u) != a.R - 1) return;
+    const unsigned have = (old >> 8) | (any ? 1u << rep : 0u);
+    if (lane == 0) a.arrived[tile] = 0;               // for the next launch
+    if (!have) return;
+    __threadfence();
+    const float* const all = a.psum + (size_t)tile * a.R * 3 * TV;
+#pragma unroll 1
+    for (int i = lane; i < TV; i += 32) {
+        size_t idx;
+        if (!voxel(i, idx)) continue;
+        double re = 0, im = 0, w = 0;
+        for (int r = 0; r < a.R; ++r) {
+            if (!((have >> r) & 1u)) continue;
+            const float* q = all + (size_t)r * 3 * TV + i;
+            re += __ldcg(q);
+            im += __ldcg(q + TV);
+            w += __ldcg(q + 2 * TV);
+        }
+        double2 o = a.vol[idx];
+        o.x += re;
+        o.y += im;
+        a.vol[idx] = o;
+        a.w[idx] += w;
     }
 }
 
-// vol += sum over replicas, in replica order.
-template <bool FOM>
+// FOM path: map += sum over replicas, in replica order.
 __global__ void combine_kernel(InsertArgs a) {
     const size_t N3 = (size_t)a.N * a.N * a.N;
-    const int nch = FOM ? 5 : 3;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N3; i += (size_t)gridDim.x * blockDim.x) {
         double re = 0, im = 0, w = 0, p = 0, q = 0;
         for (int r = 0; r < a.R; ++r) {
-            const double* pb = a.psum + (size_t)r * nch * N3 + i;
+            const double* pb = a.fsum + (size_t)r * 5 * N3 + i;
             re += pb[0]; im += pb[N3]; w += pb[2 * N3];
-            if (FOM) { p += pb[3 * N3]; q += pb[4 * N3]; }
+            p += pb[3 * N3]; q += pb[4 * N3];
         }
         double2 o = a.vol[i];
         o.x += re; o.y += im;
         a.vol[i] = o;
         a.w[i] += w;
-        if (FOM) { a.pow[i] += p; a.w2[i] += q; }
+        a.pow[i] += p; a.w2[i] += q;
     }
 }
 
-// Tile shapes the autotuner chooses from (map voxels per warp).  The float4
-// cell pitches (PX, PP) and warps per block of each shape are the template
+// Tile shapes the autotuner chooses from (map voxels per warp).  The cell
+// pitches (PX, PP) of each shape are the template
 // arguments of its grid4_kernel launch below.
 struct Shape { int tx, ty, tz; };
 static const Shape kShapes[] = {{8, 8, 8}, {16, 16, 4}, {16, 8, 8}, {16, 16, 8}};
@@ -816,37 +1056,32 @@ void insert_shape(int i, int* tx, int* ty, int* tz) { *tx = kShapes[i].tx; *ty =
 template <int TX, int TY, int TZ>
 static cudaError_t set_smem_shape() {
     const int smem = (int)(WARPS * 5 * TX * TY * TZ * sizeof(tacc_t));
-    cudaError_t e;
-    if ((e = cudaFuncSetAttribute(insert_kernel<true, true, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(insert_kernel<true, false, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(insert_kernel<false, true, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(insert_kernel<false, false, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(insert_kernel<true, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(insert_kernel<false, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
-template <int TX, int TY, int TZ, int PX, int PP, int NW>
+static constexpr int cell_bytes(int slots) { return slots * (int)(sizeof(float2) + sizeof(float)); }
+
+template <int TX, int TY, int TZ, int PX, int PP>
 static cudaError_t set_smem_shape4() {
-    const int smem = (int)(NW * PP * TZ * sizeof(float4));
+    const int smem = cell_bytes(PP * TZ);
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(grid4_kernel<true, false, TX, TY, TZ, PX, PP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(grid4_kernel<false, false, TX, TY, TZ, PX, PP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(grid4_kernel<true, true, TX, TY, TZ, PX, PP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(grid4_kernel<false, true, TX, TY, TZ, PX, PP, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if ((e = cudaFuncSetAttribute(grid4_kernel<true, false, TX, TY, TZ, PX, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(grid4_kernel<false, false, TX, TY, TZ, PX, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(grid4_kernel<true, true, TX, TY, TZ, PX, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+    return cudaFuncSetAttribute(grid4_kernel<false, true, TX, TY, TZ, PX, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
 cudaError_t prepare_insert_attributes() {
     cudaError_t e;
-    if ((e = set_smem_shape4<8, 8, 8, 8, 68, 4>()) != cudaSuccess) return e;
-    if ((e = set_smem_shape4<16, 16, 4, 17, 277, 4>()) != cudaSuccess) return e;
-    if ((e = set_smem_shape4<16, 8, 8, 16, 134, 4>()) != cudaSuccess) return e;
-    if ((e = set_smem_shape4<16, 16, 8, 16, 262, 2>()) != cudaSuccess) return e;
+    if ((e = set_smem_shape4<8, 8, 8, 8, 67>()) != cudaSuccess) return e;
+    if ((e = set_smem_shape4<16, 16, 4, 17, 277>()) != cudaSuccess) return e;
+    if ((e = set_smem_shape4<16, 8, 8, 16, 134>()) != cudaSuccess) return e;
+    if ((e = set_smem_shape4<16, 16, 8, 16, 262>()) != cudaSuccess) return e;
     if ((e = set_smem_shape<8, 8, 8>()) != cudaSuccess) return e;
     if ((e = set_smem_shape<16, 16, 4>()) != cudaSuccess) return e;
-    if ((e = set_smem_shape<16, 8, 8>()) != cudaSuccess) return e;
-    // 16 x 16 x 8 with FOM needs 5 x 2048 x 4 B per warp (160 KB for 4
-    // warps); only the non-FOM variants are used
-    const int smem = (int)(WARPS * 3 * 16 * 16 * 8 * sizeof(tacc_t));
-    if ((e = cudaFuncSetAttribute(insert_kernel<false, true, 16, 16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(insert_kernel<false, false, 16, 16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return set_smem_shape<16, 8, 8>();
 }
 
 template <int TX, int TY, int TZ>
@@ -858,22 +1093,16 @@ static cudaError_t launch_shape(const InsertArgs& a0, const Context& c, cudaStre
     a.ntz = (N + TZ - 1) / TZ;
     const int ntiles = a.ntx * a.nty * a.ntz;
     const unsigned blocks = (unsigned)(((long)ntiles * a.R + WARPS - 1) / WARPS);
-    const size_t smem = (size_t)WARPS * (c.g.fom ? 5 : 3) * TX * TY * TZ * sizeof(tacc_t);
-    if (c.g.fom) {
-        if (c.g.gate) insert_kernel<true, true, TX, TY, TZ><<<blocks, WARPS * 32, smem, s>>>(a);
-        else insert_kernel<true, false, TX, TY, TZ><<<blocks, WARPS * 32, smem, s>>>(a);
-    } else {
-        if (c.g.gate) insert_kernel<false, true, TX, TY, TZ><<<blocks, WARPS * 32, smem, s>>>(a);
-        else insert_kernel<false, false, TX, TY, TZ><<<blocks, WARPS * 32, smem, s>>>(a);
-    }
+    const size_t smem = (size_t)WARPS * 5 * TX * TY * TZ * sizeof(tacc_t);
+    if (c.g.gate) insert_kernel<true, TX, TY, TZ><<<blocks, WARPS * 32, smem, s>>>(a);
+    else insert_kernel<false, TX, TY, TZ><<<blocks, WARPS * 32, smem, s>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || a.R == 1) return e;
-    if (c.g.fom) combine_kernel<true><<<148 * 8, 256, 0, s>>>(a);
-    else combine_kernel<false><<<148 * 8, 256, 0, s>>>(a);
+    combine_kernel<<<148 * 8, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-template <int TX, int TY, int TZ, int PX, int PP, int NW>
+template <int TX, int TY, int TZ, int PX, int PP>
 static cudaError_t launch_shape4(const InsertArgs& a0, const Context& c, cudaStream_t s) {
     InsertArgs a = a0;
     const int N = c.g.map;
@@ -881,18 +1110,15 @@ static cudaError_t launch_shape4(const InsertArgs& a0, const Context& c, cudaStr
     a.nty = (N + TY - 1) / TY;
     a.ntz = (N + TZ - 1) / TZ;
     const int ntiles = a.ntx * a.nty * a.ntz;
-    const unsigned blocks = (unsigned)(((long)ntiles * a.R + NW - 1) / NW);
-    const size_t smem = (size_t)NW * PP * TZ * sizeof(float4);
+    const long items = (long)ntiles * (a.R + (a.zsplit > 0 ? 1 : 0));
+    const size_t smem = cell_bytes(PP * TZ);
     if (c.g.ewald) {
-        if (c.g.gate) grid4_kernel<true, true, TX, TY, TZ, PX, PP, NW><<<blocks, NW * 32, smem, s>>>(a);
-        else grid4_kernel<false, true, TX, TY, TZ, PX, PP, NW><<<blocks, NW * 32, smem, s>>>(a);
+        if (c.g.gate) grid4_kernel<true, true, TX, TY, TZ, PX, PP><<<(unsigned)items, 32, smem, s>>>(a);
+        else grid4_kernel<false, true, TX, TY, TZ, PX, PP><<<(unsigned)items, 32, smem, s>>>(a);
     } else {
-        if (c.g.gate) grid4_kernel<true, false, TX, TY, TZ, PX, PP, NW><<<blocks, NW * 32, smem, s>>>(a);
-        else grid4_kernel<false, false, TX, TY, TZ, PX, PP, NW><<<blocks, NW * 32, smem, s>>>(a);
+        if (c.g.gate) grid4_kernel<true, false, TX, TY, TZ, PX, PP><<<(unsigned)items, 32, smem, s>>>(a);
+        else grid4_kernel<false, false, TX, TY, TZ, PX, PP><<<(unsigned)items, 32, smem, s>>>(a);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || a.R == 1) return e;
-    combine_kernel<false><<<148 * 8, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -917,7 +1143,9 @@ cudaError_t launch_insert(const Context& c, const float2* spectra, const DevPart
     a.w2 = c.d_w2[h];
     a.order = c.d_tile_order;
     a.R = c.replicas;
-    a.psum = c.d_part_sums;
+    a.psum = reinterpret_cast<float*>(c.d_part_sums);
+    a.fsum = reinterpret_cast<double*>(c.d_part_sums);
+    a.arrived = c.d_arrived;
     a.zsplit = c.g.fom ? 0 : c.zsplit;
     a.evol = c.d_evol[h];
     a.ew = c.d_ew[h];
@@ -925,16 +1153,15 @@ cudaError_t launch_insert(const Context& c, const float2* spectra, const DevPart
     a.edge_rmax = c.edge_rmax;
     if (!c.g.fom) {
         switch (c.shape) {
-            case 0: return launch_shape4<8, 8, 8, 8, 68, 4>(a, c, s);
-            case 2: return launch_shape4<16, 8, 8, 16, 134, 4>(a, c, s);
-            case 3: return launch_shape4<16, 16, 8, 16, 262, 2>(a, c, s);
-            default: return launch_shape4<16, 16, 4, 17, 277, 4>(a, c, s);
+            case 0: return launch_shape4<8, 8, 8, 8, 67>(a, c, s);
+            case 2: return launch_shape4<16, 8, 8, 16, 134>(a, c, s);
+            case 3: return launch_shape4<16, 16, 8, 16, 262>(a, c, s);
+            default: return launch_shape4<16, 16, 4, 17, 277>(a, c, s);
         }
     }
     switch (c.shape) {
         case 0: return launch_shape<8, 8, 8>(a, c, s);
         case 2: return launch_shape<16, 8, 8>(a, c, s);
-        case 3: if (!c.g.fom) return launch_shape<16, 16, 8>(a, c, s); return launch_shape<16, 16, 4>(a, c, s);
         default: return launch_shape<16, 16, 4>(a, c, s);
     }
 }
