@@ -3,7 +3,6 @@
 // pipeline (image upload, 2-D stage, gridding) and map finishing.
 #include "context.cuh"
 #include "fft_dev.cuh"
-#include "lattice.h"
 
 #include <math.h>
 #include <stdarg.h>
@@ -130,13 +129,11 @@ static void make_dev_particle(const Recon& r, const double* q, DevParticle& d, d
     if (pad_ratio > 1) { pad_ratio *= pad_ratio * 0.6; pw /= pad_ratio; }
     d.pw = (float)pw;
     d.half = (int)q[23];
-    // the curvature bound ewh inv2 mscale |p + q| <= ewh inv2 mscale ft sqrt(2)
-    // per pixel step of a lattice vector, and the surface's largest offset
+    // the Ewald surface's largest offset (its lattice bounds the curvature:
+    // ewh inv2 mscale |p + q| <= ewh inv2 mscale ft sqrt(2) per pixel step)
     d.ewh = ewh;
     const double hf = g.ft / 2.0;
     d.ezmax = (float)(fabs(d.ewh) * 2.0 * hf * hf * d.inv2 * g.mscale * 1.0001);
-    const double curve = fabs(d.ewh) * d.inv2 * g.mscale * g.ft * 1.4142135623730951 * 1.0001;
-    d.lat = pack_lattice(choose_lattice(d.ad, d.bd, 16, curve));
     // particle_reconstruct's rescale_to_avg_std(0, 1) under -rescale
     // (mg_reconstruct.cpp:155): v * scale + shift, scale 0 = none
     d.na = q[24] != 0 ? q[24] : 1.0;
@@ -400,6 +397,9 @@ static int upload_params(Recon* r, int buf, const double* params, long np) {
         CK(cudaMemcpyAsync(r->d_psym, r->h_psym.data(), sizeof(DevParticle) * k, cudaMemcpyHostToDevice,
                            r->fft_stream));
     }
+    // the records that are gridded get their phase lattices on the device
+    CK(launch_lattices(*r, r->nexp > 0 ? r->d_psym : r->d_part, r->nexp > 0 ? r->nexp : np, r->fft_stream));
+    r->stats.launches += 1;
     return BSG_OK;
 }
 

@@ -79,6 +79,7 @@ struct Context;
 cudaError_t launch_background(const Context& c, const float* img, int nimg, cudaStream_t s);
 cudaError_t launch_rows(const Context& c, const float* img, int nimg, cudaStream_t s);
 cudaError_t launch_cols(const Context& c, int nimg, float2* spectra, cudaStream_t s);
+cudaError_t launch_lattices(const Context& c, DevParticle* parts, long n, cudaStream_t s);
 cudaError_t launch_insert(const Context& c, const float2* spectra, const DevParticle* parts, int np, int half,
                           cudaStream_t s);
 cudaError_t launch_finish(const Context& c, int imap, float* map_out, bool sinc, int* launches, cudaStream_t s);
