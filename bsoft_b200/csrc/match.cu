@@ -717,7 +717,7 @@ extern "C" int bsg_match_create(const bsg_match_config* cfg, bsg_match** out) {
                 const double d = (double)r / NDIV + h2 - j, a = M_PI * d / wd;
                 lut[(size_t)r * wd + j] = sin(M_PI * d) / (wd * sin(a)) * pow(cos(a), cfg->kernel_power);
             }
-        lut[(size_t)NDIV * wd + h2 + 1] = 1.0;
+        if (h2 + 1 < wd) lut[(size_t)NDIV * wd + h2 + 1] = 1.0;    // (width 1 has no tap there)
     }
     std::vector<double2> twm, twi;
     twiddles(N, twm);
