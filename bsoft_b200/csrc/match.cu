@@ -342,8 +342,7 @@ __global__ void __launch_bounds__(256) section_kernel(const float2* __restrict__
 struct FomArgs {
     cudaTextureObject_t tex;
     int D, wd;
-    const float* lut;        // FSI table, FP32 (T = float)
-    const double* lutd;      // the same, FP64 (T = double)
+    const float* lut;        // FSI table, FP32 (T = float without psec)
     const MPix* pix;
     int npix;
     const MHypG* hyps;
@@ -358,29 +357,91 @@ struct FomArgs {
     double wf, wc;           // their sums over [0, nf) and [cv0, cv1)
     double* fom;             // per group x MAXORG
     double* cv;
-    const double2* sec;      // gathered sections (npix per view, FP64), or null: gather here
-    const float2* psec;      // FP32 panel sections (npix per panel view, row H.sec; T = float), or null
+    const double2* sec;      // gathered sections (npix per view, row H.sec, FP64; T = double)
+    const float2* psec;      // FP32 panel sections (npix per panel view, row H.sec; T = float), or null: gather here
     int dpr;                 // 1: the DPR form (fom_type 1) instead of the FRC
+    int hmax;                // T = double: largest |h|, |k| of the phase tables; -1: no room, sincos per pixel
 };
+
+constexpr int PHASE_TABLES = 3;     // distinct slopes per axis with a table (a 3 x 3 origin grid has three)
+
+// Sums over the warp of NV values per lane: each step of the fixed tree (xor
+// 16, 8, 4, 2, 1) halves the values a lane holds, so 16 exchanges do what five
+// per value would.  Value o ends in the lanes whose bits 4..1 are o's.
+template <int NV, typename T>
+__device__ __forceinline__ T warp_sums(const T* t, int lane) {
+    static_assert(NV <= 16, "sixteen slots");
+    T a[8];
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const T lo = i < NV ? t[i] : (T)0, hi = i + 8 < NV ? t[i + 8] : (T)0;
+        a[i] = (b4 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b4 ? lo : hi, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = (b3 ? a[i + 4] : a[i]) + __shfl_xor_sync(0xffffffffu, b3 ? a[i] : a[i + 4], 8);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) a[i] = (b2 ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, b2 ? a[i] : a[i + 2], 4);
+    a[0] = (b1 ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, b1 ? a[0] : a[1], 2);
+    return a[0] + __shfl_xor_sync(0xffffffffu, a[0], 1);
+}
 
 // T = float: the search's rescoring (agrees with the reference's figure of
 // merit to ~1e-7); T = double: gather, products and shell sums in FP64, as
 // the reference accumulates (~1e-8), for refinement whose decisions compare
 // figures of merit against a 1e-6 threshold.
+//
+// T = double: the image phase of pixel (h, k) at an origin is exp(i h sx)
+// exp(i k sy), from tables of each distinct slope built once per group (an
+// FP64 sincos per pixel and origin was most of the kernel: refinement of 24
+// images of 128^2 14.6 -> 7.7 ms).  Groups with more distinct slopes than
+// tables evaluate the sincos.
 template <typename T>
 __global__ void __launch_bounds__(FOM_WARPS * 32) fom_kernel(FomArgs a) {
     extern __shared__ __align__(16) unsigned char fom_smem[];
-    T* lut = reinterpret_cast<T*>(fom_smem);                                // (NDIV+1)*wd
-    T* wsum = lut + (NDIV + 1) * MAXW;                                      // FOM_WARPS x nshell x (1+MAXORG)
+    T* wsum = reinterpret_cast<T*>(fom_smem);                               // FOM_WARPS x nshell x (1+MAXORG)
     constexpr int NV = 1 + MAXORG;
+    // T = float, gathering here: the FSI table ((NDIV+1)*wd); T = double: the phase tables
+    T* lut = wsum + FOM_WARPS * a.nshell * NV;
+    double2* phase = reinterpret_cast<double2*>(lut);
+    __shared__ int s_tab[2][MAXORG];      // table of each origin's slope on x, y
+    __shared__ int s_ntab[2];
+    __shared__ double s_slope[2][PHASE_TABLES];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const T* glut;
-    if constexpr (sizeof(T) == 8) glut = a.lutd; else glut = a.lut;
-    for (int i = threadIdx.x; i < (NDIV + 1) * a.wd; i += blockDim.x) lut[i] = glut[i];
+    if (sizeof(T) == 4 && !a.psec)
+        for (int i = threadIdx.x; i < (NDIV + 1) * a.wd; i += blockDim.x) lut[i] = (T)a.lut[i];
     for (int i = threadIdx.x; i < FOM_WARPS * a.nshell * NV; i += blockDim.x) wsum[i] = (T)0;
-    __syncthreads();
     const MHypG& H = a.hyps[blockIdx.x];
     const int norg = H.norg;
+    const int width = 2 * a.hmax + 1;
+    bool tables = false;
+    if constexpr (sizeof(T) == 8) {
+        if (threadIdx.x < 2) {
+            const double* sl = threadIdx.x ? H.sy : H.sx;
+            int n = 0;
+            for (int o = 0; o < norg; ++o) {
+                int t = 0;
+                while (t < n && t < PHASE_TABLES && s_slope[threadIdx.x][t] != sl[o]) ++t;
+                if (t == n || t == PHASE_TABLES) {
+                    if (n < PHASE_TABLES) s_slope[threadIdx.x][n] = sl[o];
+                    t = n++;
+                }
+                s_tab[threadIdx.x][o] = t;
+            }
+            s_ntab[threadIdx.x] = n;
+        }
+        __syncthreads();
+        tables = a.hmax >= 0 && s_ntab[0] <= PHASE_TABLES && s_ntab[1] <= PHASE_TABLES;
+        if (tables)
+            for (int i = threadIdx.x; i < (s_ntab[0] + s_ntab[1]) * width; i += blockDim.x) {
+                const int t = i / width, f = i - t * width - a.hmax;
+                const int ax = t >= s_ntab[0], at = ax ? t - s_ntab[0] : t;
+                double sn, cs;
+                sincos((double)f * s_slope[ax][at], &sn, &cs);
+                phase[(ax * PHASE_TABLES + at) * width + f + a.hmax] = make_double2(cs, sn);
+            }
+    }
+    __syncthreads();
     const long img = H.img;
     const float2* X = a.spec + img * (long)a.D * a.D;
     const float* C = a.ctf + (long)H.ctf * a.npix;
@@ -388,31 +449,32 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) fom_kernel(FomArgs a) {
     for (int base = warp * 32; base < a.npix; base += FOM_WARPS * 32) {
         T Rx = 0, Ry = 0;
         const int cnt = min(32, a.npix - base);
-        if (a.psec) {                                     // the panel's FP32 section, gathered once
-            if (lane < cnt) {
-                const float2 r = a.psec[(long)H.sec * a.npix + base + lane];
-                Rx = (T)r.x;
-                Ry = (T)r.y;
-            }
-        } else if (a.sec) {                               // section gathered once per view
+        if constexpr (sizeof(T) == 8) {                   // section gathered once per view
             if (lane < cnt) {
                 const double2 r = a.sec[(long)H.sec * a.npix + base + lane];
-                Rx = (T)r.x;
-                Ry = (T)r.y;
+                Rx = r.x;
+                Ry = r.y;
             }
-        } else
-        for (int q = 0; q < cnt; ++q) {
-            const MPix pq = a.pix[base + q];
-            if (!pq.insec) continue;                      // warp-uniform
-            const double ix = pq.h * a.inv, iy = pq.k * a.inv;
-            const double mx = (H.m[0] * ix + H.m[1] * iy) * a.real;
-            const double myy = (H.m[3] * ix + H.m[4] * iy) * a.real;
-            const double mz = (H.m[6] * ix + H.m[7] * iy) * a.real;
-            T vr, vi;
-            fsi_gather<T>(TexSrc{a.tex}, a.D, mx, myy, mz, lut, a.wd, lane, vr, vi);
-            if (lane == q) {
-                Rx = vr;
-                Ry = vi;
+        } else if (a.psec) {                              // the panel's FP32 section, gathered once
+            if (lane < cnt) {
+                const float2 r = a.psec[(long)H.sec * a.npix + base + lane];
+                Rx = r.x;
+                Ry = r.y;
+            }
+        } else {
+            for (int q = 0; q < cnt; ++q) {
+                const MPix pq = a.pix[base + q];
+                if (!pq.insec) continue;                  // warp-uniform
+                const double ix = pq.h * a.inv, iy = pq.k * a.inv;
+                const double mx = (H.m[0] * ix + H.m[1] * iy) * a.real;
+                const double myy = (H.m[3] * ix + H.m[4] * iy) * a.real;
+                const double mz = (H.m[6] * ix + H.m[7] * iy) * a.real;
+                float vr, vi;
+                fsi_gather<float>(TexSrc{a.tex}, a.D, mx, myy, mz, lut, a.wd, lane, vr, vi);
+                if (lane == q) {
+                    Rx = vr;
+                    Ry = vi;
+                }
             }
         }
         const int p = base + lane;
@@ -437,11 +499,18 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) fom_kernel(FomArgs a) {
 #pragma unroll
             for (int o = 0; o < MAXORG; ++o) {
                 if (o < norg) {
-                    double phi = pq.h * H.sx[o] + pq.k * H.sy[o];
                     T sn, cs;
                     if constexpr (sizeof(T) == 8) {
-                        sincos(phi, &sn, &cs);
+                        if (tables) {
+                            const double2 ex = phase[s_tab[0][o] * width + pq.h + a.hmax];
+                            const double2 ey = phase[(PHASE_TABLES + s_tab[1][o]) * width + pq.k + a.hmax];
+                            cs = ex.x * ey.x - ex.y * ey.y;
+                            sn = ex.y * ey.x + ex.x * ey.y;
+                        } else {
+                            sincos(pq.h * H.sx[o] + pq.k * H.sy[o], &sn, &cs);
+                        }
                     } else {
+                        double phi = pq.h * H.sx[o] + pq.k * H.sy[o];
                         phi -= 6.283185307179586 * rint(phi * 0.15915494309189535);
                         sincosf((float)phi, &sn, &cs);
                     }
@@ -463,13 +532,22 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) fom_kernel(FomArgs a) {
             const int lead = __ffs(left) - 1;
             const int s = __shfl_sync(0xffffffffu, shell, lead);
             const bool in = shell == s;
+            if (norg == 1) {
 #pragma unroll
-            for (int o = 0; o < NV; ++o) {
-                if (o > norg) break;
-                T t = in ? v[o] : (T)0;
+                for (int o = 0; o < 2; ++o) {
+                    T t = in ? v[o] : (T)0;
 #pragma unroll
-                for (int k = 16; k; k >>= 1) t += __shfl_xor_sync(0xffffffffu, t, k);
-                if (lane == 0) my[s * NV + o] += t;
+                    for (int k = 16; k; k >>= 1) t += __shfl_xor_sync(0xffffffffu, t, k);
+                    if (lane == 0) my[s * NV + o] += t;
+                }
+            } else {
+                T t[NV];
+#pragma unroll
+                for (int o = 0; o < NV; ++o) t[o] = in ? v[o] : (T)0;
+                const T sum = warp_sums<NV>(t, lane);
+                const int o = lane >> 1;
+                // bit 4 of the lane is slot bit 3, and so on
+                if (!(lane & 1) && o < NV) my[s * NV + o] += sum;
             }
             left &= ~__ballot_sync(0xffffffffu, in);
         }
@@ -506,6 +584,123 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) fom_kernel(FomArgs a) {
         if (lane == 0) {
             a.fom[(long)blockIdx.x * MAXORG + o] = a.nf > 0 ? tf / a.wf : 0.0;
             a.cv[(long)blockIdx.x * MAXORG + o] = (a.cv1 > a.cv0) ? tc / a.wc : 0.0;
+        }
+    }
+}
+
+// The figure of merit of one (image, view, origin) under up to TRIALS CTF rows
+// (a refinement's defocus trials, rows H.ctf ..., blockIdx.y the block of
+// them), FP64: the image, section and phase of a pixel are read once for all.
+// One launch of fom_kernel per (view, trial) read them for each, and the host
+// built and copied ten times the groups (5,184 views x 10
+// trials 4.5 -> 2.1 ms).
+constexpr int TRIALS = 5;
+
+template <bool DPR>
+__global__ void __launch_bounds__(FOM_WARPS * 32) fom_trials_kernel(FomArgs a, int max_trials) {
+    extern __shared__ __align__(16) double tsm[];
+    constexpr int NV = 2 * TRIALS;
+    double* wsum = tsm;                                       // FOM_WARPS x nshell x NV: (numerator, denominator)
+    double2* phase = reinterpret_cast<double2*>(wsum + FOM_WARPS * a.nshell * NV);
+    const MHypG& H = a.hyps[blockIdx.x];
+    const int k0 = blockIdx.y * TRIALS, nt = min(TRIALS, H.ntr - k0);
+    if (nt <= 0) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int width = 2 * a.hmax + 1;
+    for (int i = threadIdx.x; i < FOM_WARPS * a.nshell * NV; i += blockDim.x) wsum[i] = 0.0;
+    if (a.hmax >= 0)
+        for (int i = threadIdx.x; i < 2 * width; i += blockDim.x) {
+            const int y = i >= width, f = i - y * width - a.hmax;
+            double sn, cs;
+            sincos((double)f * (y ? H.sy[0] : H.sx[0]), &sn, &cs);
+            phase[i] = make_double2(cs, sn);
+        }
+    __syncthreads();
+    const long img = H.img;
+    const float2* X = a.spec + img * (long)a.D * a.D;
+    const float* C = a.ctf + (long)(H.ctf + k0) * a.npix;
+    double* my = wsum + warp * a.nshell * NV;
+    for (int base = warp * 32; base < a.npix; base += FOM_WARPS * 32) {
+        const int p = base + lane;
+        double v[NV];
+#pragma unroll
+        for (int o = 0; o < NV; ++o) v[o] = 0;
+        int shell = -1;
+        if (p < a.npix) {
+            const MPix pq = a.pix[p];
+            shell = pq.shell;
+            const float2 x = X[pq.idx];
+            const double2 R = a.sec[(long)H.sec * a.npix + p];
+            double sn, cs;
+            if (a.hmax >= 0) {
+                const double2 ex = phase[pq.h + a.hmax], ey = phase[width + pq.k + a.hmax];
+                cs = ex.x * ey.x - ex.y * ey.y;
+                sn = ex.y * ey.x + ex.x * ey.y;
+            } else {
+                sincos(pq.h * H.sx[0] + pq.k * H.sy[0], &sn, &cs);
+            }
+            const double xr = (double)x.x * cs - (double)x.y * sn, xi = (double)x.x * sn + (double)x.y * cs;
+            const double mag = DPR ? sqrt((double)x.x * x.x + (double)x.y * x.y) : 0.0;
+#pragma unroll
+            for (int k = 0; k < TRIALS; ++k) {
+                if (k < nt) {
+                    const double c = C[(long)k * a.npix + p];
+                    const double rr = R.x * c, ri = R.y * c;
+                    if (DPR) {
+                        const double amp = mag + sqrt(rr * rr + ri * ri);
+                        double d = atan2(xi, xr) - atan2(ri, rr);
+                        if (d < -3.14159265358979323846) d += 6.28318530717958647692;
+                        else if (d > 3.14159265358979323846) d -= 6.28318530717958647692;
+                        v[2 * k] = amp * d * d;
+                        v[2 * k + 1] = amp;
+                    } else {
+                        v[2 * k] = xr * rr + xi * ri;
+                        v[2 * k + 1] = rr * rr + ri * ri;
+                    }
+                }
+            }
+        }
+        unsigned left = __ballot_sync(0xffffffffu, shell >= 0);
+        while (left) {
+            const int s = __shfl_sync(0xffffffffu, shell, __ffs(left) - 1);
+            const bool in = shell == s;
+            double t[NV];
+#pragma unroll
+            for (int o = 0; o < NV; ++o) t[o] = in ? v[o] : 0.0;
+            const double sum = warp_sums<NV>(t, lane);
+            if (!(lane & 1) && (lane >> 1) < NV) my[s * NV + (lane >> 1)] += sum;
+            left &= ~__ballot_sync(0xffffffffu, in);
+        }
+    }
+    __syncthreads();
+    const double* ds = a.dsum + img * (long)a.nshell;
+    for (int k = warp; k < nt; k += FOM_WARPS) {
+        double tf = 0, tc = 0;
+        for (int j = lane; j < a.nshell; j += 32) {
+            double fj = 0, mj = 0;
+            for (int w = 0; w < FOM_WARPS; ++w) {
+                mj += wsum[(w * a.nshell + j) * NV + 2 * k + 1];
+                fj += wsum[(w * a.nshell + j) * NV + 2 * k];
+            }
+            double t;
+            const double wj = a.wshell[j];
+            if (DPR) {
+                t = mj != 0.0 ? wj * cos(sqrt(fj / mj)) : 0.0;
+            } else {
+                const double den = ds[j] * mj;
+                t = den > 0 ? wj * fj / sqrt(den) : 0.0;
+            }
+            if (j < a.nf) tf += t;
+            if (j >= a.cv0 && j < a.cv1) tc += t;
+        }
+#pragma unroll
+        for (int i = 16; i; i >>= 1) {
+            tf += __shfl_xor_sync(0xffffffffu, tf, i);
+            tc += __shfl_xor_sync(0xffffffffu, tc, i);
+        }
+        if (lane == 0) {
+            a.fom[(long)blockIdx.x * max_trials + k0 + k] = a.nf > 0 ? tf / a.wf : 0.0;
+            a.cv[(long)blockIdx.x * max_trials + k0 + k] = (a.cv1 > a.cv0) ? tc / a.wc : 0.0;
         }
     }
 }
@@ -562,6 +757,10 @@ void set_attributes() {
         e = cudaFuncSetAttribute(fom_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(fom_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fom_trials_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fom_trials_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     g_attr_err = e;
 }
 
@@ -762,9 +961,9 @@ extern "C" void bsg_match_destroy(bsg_match* h) {
     if (!M) return;
     cudaSetDevice(M->device);
     if (M->stream) cudaStreamSynchronize(M->stream);
-    void* ptrs[] = {M->d_pix, M->d_shell_start, M->d_secpix, M->d_lut, M->d_lutf, M->d_tw_map, M->d_tw_img, M->d_ref,
+    void* ptrs[] = {M->d_pix, M->d_shell_start, M->d_secpix, M->d_lut, M->d_lutf, M->d_tw_map, M->d_tw_img, M->d_ref, M->d_refpad,
                     M->d_spec, M->d_ctf, M->d_dsum, M->d_real, M->d_work, M->d_scale, M->d_shift, M->d_ictf,
-                    M->d_hyp, M->d_out, M->d_full, M->d_grp, M->d_gout, M->d_cpix, M->d_cstart, M->d_secs, M->d_panel, M->d_A, M->d_pscore,
+                    M->d_hyp, M->d_out, M->d_full, M->d_grp, M->d_gout, M->d_rmats, M->d_rsec, M->d_rctf, M->d_rrec, M->d_cpix, M->d_cstart, M->d_secs, M->d_panel, M->d_A, M->d_pscore,
                     M->d_pidx, M->d_csec, M->d_corg, M->d_cscore, M->d_rots, M->d_gA, M->d_slopes,
                     M->d_lprop, M->d_lorg, M->d_nlorg, M->d_lcand, M->d_lcount,
                     M->d_status, M->d_pexact, M->d_wshell};
@@ -833,6 +1032,7 @@ extern "C" int bsg_match_set_reference(bsg_match* h, const float* map, const dou
     const double sx = origin[0] * sc / D * 2 * M_PI, sy = origin[1] * sc / D * 2 * M_PI, sz = origin[2] * sc / D * 2 * M_PI;
     map_cut_kernel<<<148 * 8, 256, 0, s>>>(M->d_work, N, D, 1.0 / sqrt((double)n3), sx, sy, sz, M->d_ref);
     MCK(cudaGetLastError());
+    M->refpad_valid = false;
     if (!M->d_full) MCK(cudaMalloc(&M->d_full, sizeof(float2) * n3));
     {
         const double fx = origin[0] / N * 2 * M_PI, fy = origin[1] / N * 2 * M_PI, fz = origin[2] / N * 2 * M_PI;
@@ -903,33 +1103,142 @@ int match_fail(int code, const char* fmt, ...) {
     return code;
 }
 
+// The cut transform for the FP64 gather: centred on the zero frequency, with
+// HALO wrapped planes on every side, so that the 8^3 taps of any position
+// within HALO - 4 of the transform's edge are plain consecutive addresses.
+// Rows of an even number of values; two copies, the second one value further
+// on, so that every row of eight taps starts on 16 bytes in one of them.
+__host__ __device__ __forceinline__ int pad_edge(int D) { return D + 2 * HALO; }
+__host__ __device__ __forceinline__ size_t pad_elems(int D) {       // one copy, a multiple of 2
+    return (size_t)pad_edge(D) * pad_edge(D) * pad_edge(D) + 2;
+}
+
+__global__ void pad_reference_kernel(const float2* __restrict__ ref, int D, float2* __restrict__ out) {
+    const int P = pad_edge(D);
+    const long total = (long)P * P * P;
+    float2* second = out + pad_elems(D) + 1;
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+        const int off = D / 2 + HALO;
+        const int x = wrap1((int)(i % P) - off, D), y = wrap1((int)(i / P % P) - off, D), z = wrap1((int)(i / ((long)P * P)) - off, D);
+        const float2 v = ref[((size_t)z * D + y) * D + x];
+        out[i] = v;
+        second[i] = v;
+    }
+}
+
+// the padded copies of the current reference (made when first needed)
+static cudaError_t ensure_padded(Match& M, cudaStream_t s) {
+    if (M.refpad_valid) return cudaSuccess;
+    if (!M.d_refpad) {
+        const cudaError_t e = cudaMalloc(&M.d_refpad, sizeof(float2) * 2 * pad_elems(M.D));
+        if (e != cudaSuccess) return e;
+    }
+    pad_reference_kernel<<<148 * 8, 256, 0, s>>>(M.d_ref, M.D, M.d_refpad);
+    const cudaError_t e = cudaGetLastError();
+    M.refpad_valid = e == cudaSuccess;
+    return e;
+}
+
 // The FP64 section values of nv views (9 doubles each, rows 0 and 1
-// scaled as in MHyp) at the figure-of-merit pixels: the same gather, in the
-// same order, as fom_kernel<double> performs for one group, so scores from
-// these values equal the gathering kernel's.
+// scaled as in MHyp) at the figure-of-merit pixels, for fom_kernel<double>.
+//
+// Kernel width 8: the lanes work out 32 pixels' tap positions and table rows
+// at once (the whole warp doing each pixel's cost a third of its FP64
+// operations) and the warp then gathers each: lane = (pair of x taps, y tap),
+// its taps summed over z with the z weights alone in 16-byte loads, the y and
+// x weights applied to the sums, and eight pixels' lane sums added by one
+// exchange tree.  Loads come from the padded copies: the texture unit delivers
+// four 8-byte texels a clock per SM, which bounded the gather through it
+// (5,184 views of 9,900 pixels 25.7 -> 14.3 ms, now the
+// float-to-double conversions').  gridDim.y CTAs share a
+// view's pixels, so that a few hundred views fill the SMs evenly.  Positions
+// beyond the padding, and other kernel widths, take the general gather.
 __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureObject_t tex, int D, int wd,
+                                                                   const float2* __restrict__ pad,
                                                                    const double* __restrict__ lut_g,
                                                                    const MPix* __restrict__ pix, int npix,
                                                                    const double* __restrict__ mats, double inv,
                                                                    double real, double2* __restrict__ out) {
-    __shared__ double lut[(NDIV + 1) * MAXW];
+    __shared__ __align__(16) double lut[(NDIV + 1) * MAXW];
     for (int i = threadIdx.x; i < (NDIV + 1) * wd; i += blockDim.x) lut[i] = lut_g[i];
     __syncthreads();
     const double* m = mats + 9 * (long)blockIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = blockIdx.y * FOM_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int P = pad_edge(D), lim = D / 2 + HALO;
+    const int xp = lane & 3, yl = lane >> 2;
+    const long second = (long)pad_elems(D) + 1, dz = (long)P * P;
     double2* o = out + (long)blockIdx.x * npix;
-    for (int base = warp * 32; base < npix; base += FOM_WARPS * 32) {
+    for (int base = warp * 32; base < npix; base += gridDim.y * FOM_WARPS * 32) {
         double Rx = 0, Ry = 0;
         const int cnt = min(32, npix - base);
-        for (int q = 0; q < cnt; ++q) {
+        // this lane's pixel: first taps' padded address, table rows
+        int at = -1, kxy = 0, kz = 0;
+        bool general = false;
+        if (lane < cnt) {
+            const MPix pq = pix[base + lane];
+            if (pq.insec) {
+                const double ix = pq.h * inv, iy = pq.k * inv;
+                const double mx = (m[0] * ix + m[1] * iy) * real;
+                const double my = (m[3] * ix + m[4] * iy) * real;
+                const double mz = (m[6] * ix + m[7] * iy) * real;
+                const double fx = floor(mx), fy = floor(my), fz = floor(mz);
+                const int bx = (int)fx - 3 + lim, by = (int)fy - 3 + lim, bz = (int)fz - 3 + lim;
+                kxy = (int)((mx - fx) * NDIV + 0.5) | ((int)((my - fy) * NDIV + 0.5) << 16);
+                kz = (int)((mz - fz) * NDIV + 0.5);
+                general = wd != 8 || min(bx, min(by, bz)) < 0 || max(bx, max(by, bz)) > P - 8;
+                at = general ? 0 : (bz * P + by) * P + bx;
+            }
+        }
+        const unsigned far = __ballot_sync(0xffffffffu, general);
+        const unsigned live = __ballot_sync(0xffffffffu, at >= 0) & ~far;
+        for (int q0 = 0; q0 < cnt; q0 += 8) {
+            if (!((live >> q0) & 255u)) continue;
+            double t[16];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                t[2 * u] = t[2 * u + 1] = 0;
+                const int a = __shfl_sync(0xffffffffu, at, q0 + u), rows = __shfl_sync(0xffffffffu, kxy, q0 + u),
+                          rz = __shfl_sync(0xffffffffu, kz, q0 + u);
+                if (!((live >> (q0 + u)) & 1u)) continue;          // warp-uniform
+                // P is even, so the rows of a pixel all start on odd or all on
+                // even values: odd ones are 16-byte aligned in the second copy
+                const float4* src = reinterpret_cast<const float4*>(pad + a + ((a & 1) ? second : 0L) + (long)yl * P + 2 * xp);
+                const double2* wz = reinterpret_cast<const double2*>(lut + rz * 8);
+                double s0x = 0, s0y = 0, s1x = 0, s1y = 0;
+                float4 v[8];
+#pragma unroll
+                for (int z = 0; z < 8; ++z) v[z] = __ldg(src + z * (dz / 2));
+#pragma unroll
+                for (int z = 0; z < 8; ++z) {
+                    const double2 w2 = wz[z / 2];
+                    const double w = (z & 1) ? w2.y : w2.x;
+                    s0x += (double)v[z].x * w;
+                    s0y += (double)v[z].y * w;
+                    s1x += (double)v[z].z * w;
+                    s1y += (double)v[z].w * w;
+                }
+                const double wy = lut[(rows >> 16) * 8 + yl];
+                const double2 wx = reinterpret_cast<const double2*>(lut + (rows & 0xffff) * 8)[xp];
+                t[2 * u] = (s0x * wx.x + s1x * wx.y) * wy;
+                t[2 * u + 1] = (s0y * wx.x + s1y * wx.y) * wy;
+            }
+            const double sum = warp_sums<16>(t, lane);            // slot lane / 2: pixel lane / 4, real or imaginary
+            const int from = ((lane - q0) & 7) * 4;
+            const double re = __shfl_sync(0xffffffffu, sum, from), im = __shfl_sync(0xffffffffu, sum, from + 2);
+            if (lane >= q0 && lane < q0 + 8) {
+                Rx = re;
+                Ry = im;
+            }
+        }
+        for (unsigned left = far; left; left &= left - 1) {
+            const int q = __ffs(left) - 1;
             const MPix pq = pix[base + q];
-            if (!pq.insec) continue;                      // warp-uniform
             const double ix = pq.h * inv, iy = pq.k * inv;
             const double mx = (m[0] * ix + m[1] * iy) * real;
-            const double myy = (m[3] * ix + m[4] * iy) * real;
+            const double my = (m[3] * ix + m[4] * iy) * real;
             const double mz = (m[6] * ix + m[7] * iy) * real;
             double vr, vi;
-            fsi_gather<double>(TexSrc{tex}, D, mx, myy, mz, lut, wd, lane, vr, vi);
+            fsi_gather<double>(TexSrc{tex}, D, mx, my, mz, lut, wd, lane, vr, vi);
             if (lane == q) {
                 Rx = vr;
                 Ry = vi;
@@ -939,11 +1248,17 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureOb
     }
 }
 
-cudaError_t launch_secgather(const Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s) {
-    if (nv > 0)
-        secgather_kernel<<<(unsigned)nv, FOM_WARPS * 32, 0, s>>>(M.ref_tex, M.D, M.wd, M.d_lut, M.d_pix,
-                                                                 (int)M.h_pix.size(), d_mats, 1.0 / M.real_map,
-                                                                 M.real_map, d_out);
+cudaError_t launch_secgather(Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s) {
+    if (nv <= 0) return cudaSuccess;
+    const cudaError_t e = ensure_padded(M, s);
+    if (e != cudaSuccess) return e;
+    // CTAs per view: about eight waves of three CTAs per SM, each with at
+    // least two blocks of 32 pixels per warp
+    const int npix = (int)M.h_pix.size();
+    const long most = std::max(1L, (long)npix / (64 * FOM_WARPS));
+    const unsigned split = (unsigned)std::max(1L, std::min(most, 148L * 3 * 8 / nv));
+    secgather_kernel<<<dim3((unsigned)nv, split), FOM_WARPS * 32, 0, s>>>(
+        M.ref_tex, M.D, M.wd, M.d_refpad, M.d_lut, M.d_pix, npix, d_mats, 1.0 / M.real_map, M.real_map, d_out);
     return cudaGetLastError();
 }
 
@@ -1003,23 +1318,54 @@ cudaError_t launch_ctf_rows(const Match& M, const ImgCtf* d_rec, long nrec, floa
     return cudaGetLastError();
 }
 
-cudaError_t launch_fom(const Match& M, const MHypG* d_groups, long ng, double* d_fom, double* d_cv, cudaStream_t s,
-                       bool fp64, const float* ctf_table, const double2* sec, bool dpr, const float2* psec) {
+static FomArgs fom_args(const Match& M, const MHypG* d_groups, double* d_fom, double* d_cv, const float* ctf_table,
+                        const double2* sec) {
     FomArgs a{};
-    a.dpr = dpr ? 1 : 0;
-    a.psec = fp64 ? nullptr : psec;
-    a.tex = M.ref_tex; a.D = M.D; a.wd = M.wd; a.lut = M.d_lutf; a.lutd = M.d_lut;
+    a.tex = M.ref_tex; a.D = M.D; a.wd = M.wd; a.lut = M.d_lutf;
     a.pix = M.d_pix; a.npix = (int)M.h_pix.size(); a.hyps = d_groups;
     a.spec = M.d_spec; a.ctf = ctf_table ? ctf_table : M.d_ctf; a.dsum = M.d_dsum; a.nshell = M.nshell;
     a.inv = 1.0 / M.real_map; a.real = M.real_map;
     a.nf = M.nf; a.cv0 = M.cv0; a.cv1 = M.cv1;
     a.wshell = M.d_wshell; a.wf = M.wf; a.wc = M.wc;
     a.fom = d_fom; a.cv = d_cv; a.sec = sec;
-    const size_t words = (NDIV + 1) * MAXW + FOM_WARPS * M.nshell * (1 + MAXORG);
-    if (fp64 && sizeof(double) * words > 220 * 1024) return cudaErrorInvalidValue;
-    if (ng > 0) {
-        if (fp64) fom_kernel<double><<<(unsigned)ng, FOM_WARPS * 32, sizeof(double) * words, s>>>(a);
-        else fom_kernel<float><<<(unsigned)ng, FOM_WARPS * 32, sizeof(float) * words, s>>>(a);
+    return a;
+}
+
+constexpr size_t FOM_SMEM = 220 * 1024;
+
+cudaError_t launch_fom_trials(const Match& M, const MHypG* d_groups, long ng, int max_trials, double* d_fom, double* d_cv,
+                              cudaStream_t s, const float* ctf_table, const double2* sec, bool dpr) {
+    if (ng <= 0 || max_trials <= 0) return cudaSuccess;
+    FomArgs a = fom_args(M, d_groups, d_fom, d_cv, ctf_table, sec);
+    const int hmax = M.D / 2;
+    const size_t sums = sizeof(double) * FOM_WARPS * M.nshell * 2 * TRIALS, tables = sizeof(double2) * 2 * (2 * hmax + 1);
+    if (sums > FOM_SMEM) return cudaErrorInvalidValue;
+    a.hmax = sums + tables <= FOM_SMEM ? hmax : -1;
+    const dim3 grid((unsigned)ng, (unsigned)((max_trials + TRIALS - 1) / TRIALS));
+    const size_t smem = sums + (a.hmax >= 0 ? tables : 0);
+    if (dpr) fom_trials_kernel<true><<<grid, FOM_WARPS * 32, smem, s>>>(a, max_trials);
+    else fom_trials_kernel<false><<<grid, FOM_WARPS * 32, smem, s>>>(a, max_trials);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fom(const Match& M, const MHypG* d_groups, long ng, double* d_fom, double* d_cv, cudaStream_t s,
+                       bool fp64, const float* ctf_table, const double2* sec, bool dpr, const float2* psec) {
+    FomArgs a = fom_args(M, d_groups, d_fom, d_cv, ctf_table, sec);
+    a.dpr = dpr ? 1 : 0;
+    a.psec = fp64 ? nullptr : psec;
+    // FP64 sections come gathered (launch_secgather)
+    if (fp64 && !sec) return cudaErrorInvalidValue;
+    const size_t sums = (size_t)FOM_WARPS * M.nshell * (1 + MAXORG);
+    if (ng <= 0) return cudaSuccess;
+    if (fp64) {
+        const int hmax = M.D / 2;
+        const size_t tables = sizeof(double2) * 2 * PHASE_TABLES * (2 * hmax + 1), most = FOM_SMEM;
+        if (sizeof(double) * sums > most) return cudaErrorInvalidValue;
+        a.hmax = sizeof(double) * sums + tables <= most ? hmax : -1;
+        fom_kernel<double><<<(unsigned)ng, FOM_WARPS * 32, sizeof(double) * sums + (a.hmax >= 0 ? tables : 0), s>>>(a);
+    } else {
+        const size_t lut = a.psec ? 0 : (NDIV + 1) * MAXW;
+        fom_kernel<float><<<(unsigned)ng, FOM_WARPS * 32, sizeof(float) * (sums + lut), s>>>(a);
     }
     return cudaGetLastError();
 }
@@ -1074,16 +1420,21 @@ static int ensure_hyps(Match& M, long nh) {
 }
 
 namespace bsg {
-int ensure_groups(Match& M, long ng) {
-    if (ng <= M.grp_cap) return BSG_OK;
-    cudaFree(M.d_grp);
-    cudaFree(M.d_gout);
-    M.d_grp = nullptr;
-    M.d_gout = nullptr;
-    M.grp_cap = 0;
-    MCK(cudaMalloc(&M.d_grp, sizeof(MHypG) * ng));
-    MCK(cudaMalloc(&M.d_gout, sizeof(double) * 2 * MAXORG * ng));
-    M.grp_cap = ng;
+int ensure_groups(Match& M, long ng, int outs) {
+    if (ng > M.grp_cap) {
+        cudaFree(M.d_grp);
+        M.d_grp = nullptr;
+        M.grp_cap = 0;
+        MCK(cudaMalloc(&M.d_grp, sizeof(MHypG) * ng));
+        M.grp_cap = ng;
+    }
+    if (2 * ng * outs > M.gout_cap) {
+        cudaFree(M.d_gout);
+        M.d_gout = nullptr;
+        M.gout_cap = 0;
+        MCK(cudaMalloc(&M.d_gout, sizeof(double) * 2 * ng * outs));
+        M.gout_cap = 2 * ng * outs;
+    }
     return BSG_OK;
 }
 }  // namespace bsg
@@ -1250,8 +1601,36 @@ extern "C" int bsg_match_score(bsg_match* h, const double* hyps, long nhyp, doub
     if (rc2) return rc2;
     cudaStream_t s = M->stream;
     MCK(cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s));
-    MCK(launch_fom(*M, M->d_grp, ng, M->d_gout, M->d_gout + ng * MAXORG, s, (flags & BSG_MATCH_SCORE_FP64) != 0,
-                   nullptr, nullptr, (flags & BSG_MATCH_SCORE_DPR) != 0));
+    const bool dpr = (flags & BSG_MATCH_SCORE_DPR) != 0;
+    if (flags & BSG_MATCH_SCORE_FP64) {
+        // the groups' FP64 sections, at most ~1 GB at a time
+        const long npix = (long)M->h_pix.size();
+        const long chunk = std::max(1L, std::min(ng, (1L << 30) / ((long)sizeof(double2) * std::max(npix, 1L))));
+        std::vector<double> mats(9 * ng);
+        for (long g = 0; g < ng; ++g) {
+            memcpy(&mats[9 * g], groups[g].m, sizeof(groups[g].m));
+            groups[g].sec = (int)(g % chunk);
+        }
+        MCK(cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s));
+        double* d_mats = nullptr;
+        double2* d_sec = nullptr;
+        cudaError_t e = cudaMalloc(&d_mats, sizeof(double) * 9 * ng);
+        if (e == cudaSuccess) e = cudaMalloc(&d_sec, sizeof(double2) * npix * chunk);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d_mats, mats.data(), sizeof(double) * 9 * ng, cudaMemcpyHostToDevice, s);
+        for (long g0 = 0; e == cudaSuccess && g0 < ng; g0 += chunk) {
+            const long cnt = std::min(chunk, ng - g0);
+            e = launch_secgather(*M, d_mats + 9 * g0, cnt, d_sec, s);
+            if (e == cudaSuccess)
+                e = launch_fom(*M, M->d_grp + g0, cnt, M->d_gout + g0 * MAXORG, M->d_gout + (ng + g0) * MAXORG, s, true,
+                               nullptr, d_sec, dpr);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        cudaFree(d_mats);
+        cudaFree(d_sec);
+        MCK(e);
+    } else {
+        MCK(launch_fom(*M, M->d_grp, ng, M->d_gout, M->d_gout + ng * MAXORG, s, false, nullptr, nullptr, dpr));
+    }
     std::vector<double> go(2 * ng * MAXORG);
     MCK(cudaMemcpyAsync(go.data(), M->d_gout, sizeof(double) * go.size(), cudaMemcpyDeviceToHost, s));
     MCK(cudaStreamSynchronize(s));

@@ -15,6 +15,7 @@ namespace bsg {
 constexpr int NDIV = 512;     // FSI_Kernel divisions (FSI_Kernel.h:42)
 constexpr int MAXW = 8;       // widest kernel the warp gather supports
 constexpr int FOM_WARPS = 8;
+constexpr int HALO = 8;       // wrapped planes around the padded reference transform (match.cu)
 
 struct MPix {
     short h, k;     // signed frequency indices
@@ -43,6 +44,8 @@ struct MHypG {
     int norg;
     int ctf;        // row of the CTF table the launch scores with (the image's own: img)
     int sec;        // gathered section of the launch's section buffer (when it has one)
+    int ntr;        // CTF rows tried from row `ctf` on (launch_fom_trials)
+    int pad;
 };
 
 
@@ -210,6 +213,8 @@ struct Match {
     double2* d_tw_map = nullptr;
     double2* d_tw_img = nullptr;
     float2* d_ref = nullptr;           // diam^3
+    float2* d_refpad = nullptr;        // two padded copies of it (the FP64 gather's source)
+    bool refpad_valid = false;
     float2* d_full = nullptr;          // uncut N^3 transform for the projector
     cudaArray_t ref_array = nullptr;   // the same values behind a 3-D texture
     cudaTextureObject_t ref_tex = 0;
@@ -232,8 +237,15 @@ struct Match {
     long hyp_cap = 0;
     double* d_out = nullptr;           // 2 x hyp_cap
     MHypG* d_grp = nullptr;            // hypothesis groups for the exact score
-    double* d_gout = nullptr;          // 2 x MAXORG x grp_cap
-    long grp_cap = 0;
+    double* d_gout = nullptr;          // their figures of merit and cross-validation figures
+    long grp_cap = 0, gout_cap = 0;
+    // refinement's buffers, kept between calls (grow-only; the sections at
+    // most ~1 GB, a chunk's): views, gathered sections, CTF trial rows
+    double* d_rmats = nullptr;
+    double2* d_rsec = nullptr;
+    float* d_rctf = nullptr;
+    ImgCtf* d_rrec = nullptr;
+    long rview_cap = 0, rrow_cap = 0;
     float* h_pin = nullptr;            // pinned staging
     size_t pin_bytes = 0;
     // exhaustive search (search.cu)
@@ -281,17 +293,22 @@ struct Match {
 cudaError_t launch_fom(const Match& M, const MHypG* d_groups, long ng, double* d_fom, double* d_cv, cudaStream_t s,
                        bool fp64 = false, const float* ctf_table = nullptr, const double2* sec = nullptr,
                        bool dpr = false, const float2* psec = nullptr);
+// FP64 scores of ng groups (one origin each) under their H.ntr CTF rows, at
+// most max_trials: d_fom / d_cv get max_trials slots per group
+cudaError_t launch_fom_trials(const Match& M, const MHypG* d_groups, long ng, int max_trials, double* d_fom, double* d_cv,
+                              cudaStream_t s, const float* ctf_table, const double2* sec, bool dpr);
 // FP32 sections of nsec panel views at the figure-of-merit pixels, gathered
 // as fom_kernel<float> gathers them: nsec x npix float2 (0 where a pixel is
 // outside the section)
 cudaError_t launch_panel_exact(const Match& M, const MHyp* d_secs, long nsec, float2* d_out, cudaStream_t s);
 // FP64 section values of nv views (9 doubles each, MHyp's scaled rows) at
 // the figure-of-merit pixels: nv x npix double2
-cudaError_t launch_secgather(const Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s);
+cudaError_t launch_secgather(Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s);
 // CTF table rows (npix floats each) for nrec records on the device
 cudaError_t launch_ctf_rows(const Match& M, const ImgCtf* d_rec, long nrec, float* d_out, cudaStream_t s);
 void group_hypotheses(const std::vector<MHyp>& hyps, std::vector<MHypG>& groups, std::vector<long>& slot);
-int ensure_groups(Match& M, long ng);
+// room for ng groups and `outs` figures of merit each
+int ensure_groups(Match& M, long ng, int outs = MAXORG);
 // view matrix rows 0, 1 scaled by the sampling ratio (img_fit_in_recip_space_grid)
 void match_view_rows(const Match& M, const double* mat, double* m);
 int match_fail(int code, const char* fmt, ...);

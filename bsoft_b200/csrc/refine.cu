@@ -394,36 +394,42 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
     std::vector<MHypG> groups;
     std::vector<long> owner, gfirst;
     std::vector<double> go;
-    float* d_rctf = nullptr;
-    ImgCtf* d_rrec = nullptr;
-    double* d_rmats = nullptr;          // chunk x 27 views, 9 doubles each
-    double2* d_sec = nullptr;           // chunk x 27 gathered sections
     std::vector<double> mats;
     int rc = BSG_OK;
     {
+        // chunk x 27 views (9 doubles each) and their gathered sections
         const long nvmax = std::min(nstart, chunk) * NVIEW;
-        ce = cudaMalloc(&d_rmats, sizeof(double) * 9 * nvmax);
-        if (ce == cudaSuccess) ce = cudaMalloc(&d_sec, sizeof(double2) * (size_t)npix * nvmax);
+        if (nvmax > M->rview_cap) {
+            cudaFree(M->d_rmats);
+            cudaFree(M->d_rsec);
+            M->d_rmats = nullptr;
+            M->d_rsec = nullptr;
+            M->rview_cap = 0;
+            ce = cudaMalloc(&M->d_rmats, sizeof(double) * 9 * nvmax);
+            if (ce == cudaSuccess) ce = cudaMalloc(&M->d_rsec, sizeof(double2) * (size_t)npix * nvmax);
+            if (ce == cudaSuccess) M->rview_cap = nvmax;
+        }
         if (ce != cudaSuccess) {
-            cudaFree(d_rmats);
-            cudaFree(d_sec);
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
             return match_fail(BSG_ERR_NOMEM, "bsg_match_refine: %s", cudaGetErrorString(ce));
         }
     }
+    double* const d_rmats = M->d_rmats;
+    double2* const d_sec = M->d_rsec;
 
-    // score `groups` (FP64) with the given CTF table and gathered sections;
-    // results in go
-    auto score_with = [&](const float* table, const double2* sec) -> int {
-        const long ng = (long)groups.size();
-        int r = ensure_groups(*M, ng);
+    // score `groups` (FP64) with the given CTF table and gathered sections,
+    // at their origins or (trials > 0) under their CTF rows; results in go
+    auto score_with = [&](const float* table, const double2* sec, int trials) -> int {
+        const long ng = (long)groups.size(), outs = trials > 0 ? trials : MAXORG;
+        int r = ensure_groups(*M, ng, (int)outs);
         if (r != BSG_OK) return r;
-        go.resize(2 * ng * MAXORG);
+        go.resize(2 * ng * outs);
         cudaError_t e = cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = cudaEventRecord(e0, s);
         if (e == cudaSuccess)
-            e = launch_fom(*M, M->d_grp, ng, M->d_gout, M->d_gout + ng * MAXORG, s, true, table, sec, dpr);
+            e = trials > 0 ? launch_fom_trials(*M, M->d_grp, ng, trials, M->d_gout, M->d_gout + ng * outs, s, table, sec, dpr)
+                           : launch_fom(*M, M->d_grp, ng, M->d_gout, M->d_gout + ng * outs, s, true, table, sec, dpr);
         if (e == cudaSuccess) e = cudaEventRecord(e1, s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(go.data(), M->d_gout, sizeof(double) * go.size(), cudaMemcpyDeviceToHost, s);
@@ -435,7 +441,7 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
         ++launches;
         return BSG_OK;
     };
-    auto score = [&](const float* table) -> int { return score_with(table, d_sec); };
+    auto score = [&](const float* table, int trials) -> int { return score_with(table, d_sec, trials); };
     // group of the t-th active particle's view v (its gathered section t * 27 + v)
     auto view_group = [&](const Particle& P, long t, int v) {
         MHypG g;
@@ -592,7 +598,7 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
                         }
                     }
                 }
-                r = score_with(table, d_msec);
+                r = score_with(table, d_msec, 0);
                 if (r != BSG_OK) break;
                 for (long t = 0; t < np_; ++t) {
                     Particle& P = parts[p0 + t];
@@ -627,7 +633,7 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
                         groups.push_back(g);
                     }
                 }
-            r = score_with(table, d_msec);
+            r = score_with(table, d_msec, 0);
             if (r != BSG_OK) break;
             const long ng = (long)groups.size();
             const double* gfom = go.data();
@@ -707,15 +713,20 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
                     recs.push_back(C);
                 }
             }
-            cudaFree(d_rctf);
-            cudaFree(d_rrec);
-            d_rctf = nullptr;
-            d_rrec = nullptr;
-            ce = cudaMalloc(&d_rctf, sizeof(float) * npix * recs.size());
-            if (ce == cudaSuccess) ce = cudaMalloc(&d_rrec, sizeof(ImgCtf) * recs.size());
+            ce = cudaSuccess;
+            if ((long)recs.size() > M->rrow_cap) {
+                cudaFree(M->d_rctf);
+                cudaFree(M->d_rrec);
+                M->d_rctf = nullptr;
+                M->d_rrec = nullptr;
+                M->rrow_cap = 0;
+                ce = cudaMalloc(&M->d_rctf, sizeof(float) * npix * recs.size());
+                if (ce == cudaSuccess) ce = cudaMalloc(&M->d_rrec, sizeof(ImgCtf) * recs.size());
+                if (ce == cudaSuccess) M->rrow_cap = (long)recs.size();
+            }
             if (ce == cudaSuccess)
-                ce = cudaMemcpyAsync(d_rrec, recs.data(), sizeof(ImgCtf) * recs.size(), cudaMemcpyHostToDevice, s);
-            if (ce == cudaSuccess) ce = launch_ctf_rows(*M, d_rrec, (long)recs.size(), d_rctf, s);
+                ce = cudaMemcpyAsync(M->d_rrec, recs.data(), sizeof(ImgCtf) * recs.size(), cudaMemcpyHostToDevice, s);
+            if (ce == cudaSuccess) ce = launch_ctf_rows(*M, M->d_rrec, (long)recs.size(), M->d_rctf, s);
             if (ce != cudaSuccess) {
                 rc = match_fail(BSG_ERR_CUDA, "bsg_match_refine: %s", cudaGetErrorString(ce));
                 break;
@@ -770,35 +781,35 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
                 }
             if (dsearch) {
                 groups.clear();
-                gfirst.clear();
+                long most = 0;
                 for (size_t t = 0; t < owner.size(); ++t) {
                     Particle& P = parts[owner[t]];
-                    gfirst.push_back((long)groups.size());
+                    const long nd = (long)P.dvals.size() - 1;
+                    most = std::max(most, nd);
                     for (int v = 0; v < NVIEW; ++v) {
                         MHypG g = view_group(P, (long)t, v);
                         g.norg = 1;
                         g.sx[0] = slope(P.ox);
                         g.sy[0] = slope(P.oy);
-                        for (size_t k = 0; k + 1 < P.dvals.size(); ++k) {
-                            g.ctf = (int)(P.row0 + (long)k);
-                            groups.push_back(g);
-                        }
+                        g.ctf = (int)P.row0;
+                        g.ntr = (int)nd;
+                        groups.push_back(g);
                     }
                 }
-                rc = score(d_rctf);
+                if (most > 0) rc = score(M->d_rctf, (int)most);
                 if (rc != BSG_OK) break;
                 for (size_t t = 0; t < owner.size(); ++t) {
                     Particle& P = parts[owner[t]];
                     const long nd = (long)P.dvals.size() - 1;
                     for (int v = 0; v < NVIEW; ++v)
                         for (long k = 0; k < nd; ++k) {
-                            const long g = gfirst[t] + (long)v * nd + k;
-                            const double f = go[g * MAXORG];
+                            const long g = ((long)t * NVIEW + v) * most + k;
+                            const double f = go[g];
                             P.number++;
                             if (P.vfom[v] < f) {
                                 P.vfom[v] = f;
                                 P.vk[v] = (int)k;
-                                P.vcv[v] = go[(long)groups.size() * MAXORG + g * MAXORG];
+                                P.vcv[v] = go[(long)groups.size() * most + g];
                             }
                         }
                 }
@@ -823,7 +834,7 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
                 }
             }
             if (!groups.empty()) {
-                rc = score(dsearch ? d_rctf : nullptr);
+                rc = score(dsearch ? M->d_rctf : nullptr, 0);
                 if (rc != BSG_OK) break;
             }
             const long ng = (long)groups.size();
@@ -878,10 +889,6 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
         }
         if (rc == BSG_OK && !mags.empty()) rc = mag_stage(c0, c1);
     }
-    cudaFree(d_rctf);
-    cudaFree(d_rrec);
-    cudaFree(d_rmats);
-    cudaFree(d_sec);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (rc != BSG_OK) return rc;
