@@ -22,11 +22,18 @@
 // 64 staged by TMA (128-byte swizzle) through a 4-deep shared-memory ring;
 // one elected thread issues tcgen05.mma (M=128, N=256, K=16) into one of two
 // 256-column TMEM accumulators while four epilogue warps read the other with
-// tcgen05.ld and keep each row's 8 best columns in registers.  Work items
-// are (M tile, range of N tiles) so a CTA carries its rows' top-8 across the
-// whole range; items are ordered so that the ~148 concurrent CTAs cover 10 M
-// tiles x 15 N ranges and share their A and B tiles through L2.  Every wait
-// is bounded (2 s) and reports through a status word.
+// tcgen05.ld and keep each row's 8 best columns in registers.  The M tiles
+// are taken in groups; the CTAs of a group are a grid of its M tiles by
+// stretches of N, so that those of one stretch read the same B tiles at the
+// same time and all share the group's A tiles through L2.  Groups of seven and
+// four M tiles (21 and 37 stretches) keep 147 and 148 of the 148 SMs at work,
+// and the stretches' lengths, which differ by one tile, alternate from group
+// to group (ten M tiles x 15 stretches as 150 work items a group left the
+// last of six rounds nearly empty: 256 images x 25 origins against 68,520
+// sections 6.31 -> 5.48 ms at full clock, 6.09 -> 6.03 under the power cap; one
+// run of tiles per CTA regardless of the stretches, evener still, 7.70: B is
+// then read by one CTA at a time).  A CTA carries its rows' top-8 along its
+// stretch.  Every wait is bounded (2 s) and reports through a status word.
 #include "match.cuh"
 
 #include <cuda.h>
@@ -139,28 +146,60 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// The work of each CTA: in group g (M tiles first(g) .. first(g + 1) - 1) CTA c
+// takes M tile c % size of it and the N tiles of stretch c / size.
+struct Runs {
+    int mtiles, ntiles, ctas;
+    int groups, sevens;               // sevens < 0: groups of nearly equal sizes
+
+    __host__ __device__ static Runs plan(int mtiles, int ntiles) {
+        Runs r{mtiles, ntiles, 148, 0, -1};
+        for (int four = 0; four < 7 && r.sevens < 0; ++four)
+            if (mtiles >= 4 * four && (mtiles - 4 * four) % 7 == 0) {
+                r.sevens = (mtiles - 4 * four) / 7;
+                r.groups = r.sevens + four;
+            }
+        if (r.sevens < 0) r.groups = (mtiles + 6) / 7;     // below 18, where sevens and fours do not add up
+        return r;
+    }
+    __host__ __device__ int first(int g) const {
+        if (sevens < 0) return (int)((long)g * mtiles / groups);
+        return g <= sevens ? 7 * g : 7 * sevens + 4 * (g - sevens);
+    }
+    __host__ __device__ int size(int g) const { return first(g + 1) - first(g); }
+    __host__ __device__ int stretches(int g) const { return ctas / size(g); }
+    // first N tile of stretch r
+    __host__ __device__ int bound(int g, int r) const {
+        const int n = stretches(g);
+        return (int)(((long)r * ntiles + (long)g * n / groups) / n);
+    }
+    __host__ __device__ int group_of(int mtile) const {
+        if (sevens >= 0) return mtile < 7 * sevens ? mtile / 7 : sevens + (mtile - 7 * sevens) / 4;
+        int g = (int)((long)mtile * groups / mtiles);
+        while (first(g) > mtile) --g;
+        while (first(g + 1) <= mtile) ++g;
+        return g;
+    }
+    // CTA c's M tile and N tiles in group g; false: none
+    __host__ __device__ bool work(int g, int c, int& m, int& n0, int& n1) const {
+        const int sz = size(g), r = c / sz;
+        if (r >= stretches(g)) return false;
+        m = first(g) + c % sz;
+        n0 = bound(g, r);
+        n1 = bound(g, r + 1);
+        return n0 < n1;
+    }
+};
+
 struct GemmArgs {
     int kblocks;          // K / 64
     int ncols;            // valid columns (sections)
-    int ntiles_n;         // ceil(ncols / 256)
-    int mtiles;           // M tiles holding rows of this batch
+    Runs runs;            // the batch's M tiles by ceil(ncols / 256) N tiles
     long prow;            // row stride of the partial buffers (batch height)
-    int ranges;           // N ranges
-    int tiles_per_range;
-    int mgroup;           // M tiles per group
-    int items;            // groups * ranges * mgroup
-    float* part_score;    // [ranges][prow][TOPK]
+    float* part_score;    // [stretch][prow][TOPK]
     int* part_idx;
     int* status;
 };
-
-__device__ __forceinline__ bool item_coords(const GemmArgs& a, int item, int& mtile, int& r) {
-    const int per_group = a.ranges * a.mgroup;
-    const int g = item / per_group, rem = item - g * per_group;
-    r = rem / a.mgroup;
-    mtile = g * a.mgroup + (rem - r * a.mgroup);
-    return mtile < a.mtiles;
-}
 
 // keep the 8 largest (value, column) of a row, sorted descending
 struct Top8 {
@@ -192,6 +231,7 @@ search_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(gsm_raw) + 1023u) & ~1023u;   // 1024-aligned stage ring
+    const Runs runs = a.runs;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
@@ -221,11 +261,10 @@ search_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             uint32_t stage = 0, phase = 0;
             uint32_t issued_mask = 0, last_parity = 0;   // per stage: ever issued, parity of its last load
             bool ok = true;
-            for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
-                int mtile, r;
-                if (!item_coords(a, item, mtile, r)) continue;
-                const int t0 = r * a.tiles_per_range, t1 = min(a.ntiles_n, t0 + a.tiles_per_range);
-                for (int nt = t0; ok && nt < t1; ++nt) {
+            for (int g = 0; ok && g < runs.groups; ++g) {
+                int mtile, n0, n1;
+                if (!runs.work(g, blockIdx.x, mtile, n0, n1)) continue;
+                for (int nt = n0; ok && nt < n1; ++nt) {
                     for (int kb = 0; kb < a.kblocks; ++kb) {
                         if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1, abort_v)) { ok = false; break; }
                         const uint32_t fb = smem_u32(&full_bar[stage]);
@@ -257,11 +296,10 @@ search_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (lane == 0) {
             uint32_t stage = 0, phase = 0, acc = 0, aphase = 0;
             bool ok = true;
-            for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
-                int mtile, r;
-                if (!item_coords(a, item, mtile, r)) continue;
-                const int t0 = r * a.tiles_per_range, t1 = min(a.ntiles_n, t0 + a.tiles_per_range);
-                for (int nt = t0; ok && nt < t1; ++nt) {
+            for (int g = 0; ok && g < runs.groups; ++g) {
+                int mtile, n0, n1;
+                if (!runs.work(g, blockIdx.x, mtile, n0, n1)) continue;
+                for (int nt = n0; ok && nt < n1; ++nt) {
                     if (!mbar_wait(smem_u32(&tempty_bar[acc]), aphase ^ 1, abort_v)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t d = tmem + acc * BN;
@@ -296,12 +334,11 @@ search_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         uint32_t acc = 0, aphase = 0;
         Top8 top;
         bool ok = true;
-        for (int item = blockIdx.x; ok && item < a.items; item += gridDim.x) {
-            int mtile, r;
-            if (!item_coords(a, item, mtile, r)) continue;
+        for (int g = 0; ok && g < runs.groups; ++g) {
+            int mtile, n0, n1;
+            if (!runs.work(g, blockIdx.x, mtile, n0, n1)) continue;
             top.reset();
-            const int t0 = r * a.tiles_per_range, t1 = min(a.ntiles_n, t0 + a.tiles_per_range);
-            for (int nt = t0; nt < t1; ++nt) {
+            for (int nt = n0; nt < n1; ++nt) {
                 // one lane waits, the warp follows it (tcgen05.ld is warp-collective)
                 int w = 1;
                 if (lane == 0) w = mbar_wait(smem_u32(&tfull_bar[acc]), aphase, abort_v) ? 1 : 0;
@@ -324,7 +361,7 @@ search_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             }
             if (!ok) break;
             const long row = (long)mtile * BM + quarter * 32 + lane;
-            const long o = ((long)r * a.prow + row) * TOPK;
+            const long o = ((long)(blockIdx.x / runs.size(g)) * a.prow + row) * TOPK;
 #pragma unroll
             for (int t = 0; t < TOPK; ++t) { a.part_score[o + t] = top.s[t]; a.part_idx[o + t] = top.i[t]; }
         }
@@ -436,45 +473,96 @@ __global__ void __launch_bounds__(256) rows_kernel(const float2* __restrict__ sp
     }
 }
 
-// one warp per image: the topk best of its nshift rows x ranges x 8
-// partial candidates (ties: lower section, then lower origin index)
-__global__ void merge_kernel(const float* __restrict__ ps, const int* __restrict__ pi, int ranges, long mrows,
-                             int nshift, int nimg_batch, int topk, long img0, int* __restrict__ cand_sec,
-                             int* __restrict__ cand_org, float* __restrict__ cand_score) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= nimg_batch) return;
-    const int n = nshift * ranges * TOPK;
-    float prev_s = 3.0e38f;
-    long prev_key = -1;
+// One CTA per image: the topk best of the partial candidates of its nshift rows
+// in (score descending, section, origin) order.  A candidate is one number
+// that sorts that way (64 bits; 128 when sections x origins exceed 32),
+// gathered once into shared memory (when they fit:
+// cached = 1), and each pick is the largest below the last (reading the
+// partial buffers again for every pick, one warp per image, took 0.42 ms for
+// 256 images: now 0.07).
+constexpr int MERGE_THREADS = 256;
+constexpr int MERGE_CACHE = 12288;         // candidates that shared memory holds (96 KB)
+
+typedef unsigned __int128 wide_t;
+
+__device__ __forceinline__ unsigned long long shfl_xor_key(unsigned long long v, int o) {
+    return __shfl_xor_sync(0xffffffffu, v, o);
+}
+__device__ __forceinline__ wide_t shfl_xor_key(wide_t v, int o) {
+    return (wide_t)__shfl_xor_sync(0xffffffffu, (unsigned long long)(v >> 64), o) << 64 |
+           __shfl_xor_sync(0xffffffffu, (unsigned long long)v, o);
+}
+
+// K: score in the upper half, the inverted section x origin number in the lower
+template <class K>
+__global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(const float* __restrict__ ps, const int* __restrict__ pi,
+                                                              Runs runs, long mrows, int nshift, int topk, long img0,
+                                                              int cached, int* __restrict__ cand_sec,
+                                                              int* __restrict__ cand_org, float* __restrict__ cand_score) {
+    constexpr int HALF = 4 * sizeof(K);
+    constexpr K LOW = ((K)1 << HALF) - 1;
+    extern __shared__ __align__(16) unsigned char msm[];
+    K* const cache = reinterpret_cast<K*>(msm);
+    __shared__ K best[MERGE_THREADS / 32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // f(candidate) for every candidate: a warp takes a row, its lanes the
+    // row's stretches and places
+    auto each = [&](auto&& f) {
+        int at = 0;
+        for (int s = 0; s < nshift; ++s) {
+            const long row = (long)blockIdx.x * nshift + s;
+            const int g = runs.group_of((int)(row / BM)), n = runs.stretches(g) * TOPK;
+            for (int e = threadIdx.x; e < n; e += MERGE_THREADS) {
+                const int r = e / TOPK;
+                K v = 0;
+                if (runs.bound(g, r) < runs.bound(g, r + 1)) {
+                    const long o = ((long)r * mrows + row) * TOPK + e % TOPK;
+                    const int sec = pi[o];
+                    if (sec >= 0) {
+                        unsigned u = __float_as_uint(ps[o]);
+                        u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;         // sorts as the float does
+                        v = (K)u << HALF | (LOW - ((K)sec * nshift + s));
+                    }
+                }
+                f(at + e, v);
+            }
+            at += n;
+        }
+        return at;
+    };
+    int count = 0;
+    if (cached) count = each([&](int i, K v) { cache[i] = v; });
+    __syncthreads();
+    K prev = ~(K)0;
     for (int t = 0; t < topk; ++t) {
-        float bs = -3.0e38f;
-        long bk = -1;
-        for (int e = lane; e < n; e += 32) {
-            const int s = e / (ranges * TOPK), rem = e - s * ranges * TOPK, r = rem / TOPK, k = rem - r * TOPK;
-            const long o = ((long)r * mrows + (long)warp * nshift + s) * TOPK + k;
-            const int sec = pi[o];
-            if (sec < 0) continue;
-            const float v = ps[o];
-            const long key = (long)sec * nshift + s;
-            // strictly after the previous pick in (score desc, key asc) order
-            const bool after = v < prev_s || (v == prev_s && key > prev_key);
-            if (!after) continue;
-            if (v > bs || (v == bs && (bk < 0 || key < bk))) { bs = v; bk = key; }
+        K b = 0;
+        if (cached) {
+            for (int i = threadIdx.x; i < count; i += MERGE_THREADS) {
+                const K v = cache[i];
+                if (v < prev && v > b) b = v;
+            }
+        } else {
+            each([&](int, K v) { if (v < prev && v > b) b = v; });
         }
         for (int o = 16; o; o >>= 1) {
-            const float os = __shfl_xor_sync(0xffffffffu, bs, o);
-            const long ok = __shfl_xor_sync(0xffffffffu, bk, o);
-            if (ok >= 0 && (os > bs || (os == bs && (bk < 0 || ok < bk)))) { bs = os; bk = ok; }
+            const K v = shfl_xor_key(b, o);
+            if (v > b) b = v;
         }
-        if (lane == 0) {
-            const long c = (img0 + warp) * topk + t;
-            cand_sec[c] = bk >= 0 ? (int)(bk / nshift) : -1;
-            cand_org[c] = bk >= 0 ? (int)(bk % nshift) : -1;
-            cand_score[c] = bs;
+        __syncthreads();                         // the last pick has been read
+        if (lane == 0) best[warp] = b;
+        __syncthreads();
+        for (int w = 0; w < MERGE_THREADS / 32; ++w) if (best[w] > b) b = best[w];
+        if (threadIdx.x == 0) {
+            const long c = (img0 + blockIdx.x) * topk + t;
+            const long key = (long)(LOW - (b & LOW));
+            unsigned u = (unsigned)(b >> HALF);
+            u ^= (u >> 31) ? 0x80000000u : 0xffffffffu;
+            cand_sec[c] = b ? (int)(key / nshift) : -1;
+            cand_org[c] = b ? (int)(key % nshift) : -1;
+            cand_score[c] = b ? __uint_as_float(u) : -3.0e38f;
         }
-        prev_s = bs;
-        prev_key = bk;
-        if (bk < 0) prev_s = -3.0e38f;
+        if (b) prev = b;
+        else prev = 0;                           // nothing is left
     }
 }
 
@@ -795,6 +883,9 @@ extern "C" int bsg_match_set_panel(bsg_match* h, const double* mats, long nsec, 
     std::call_once(g_search_attr, [] {
         g_search_attr_err = cudaFuncSetAttribute(search_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
         if (g_search_attr_err == cudaSuccess)
+            g_search_attr_err = cudaFuncSetAttribute(merge_kernel<unsigned long long>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)sizeof(long long) * MERGE_CACHE);
+        if (g_search_attr_err == cudaSuccess)
             g_search_attr_err = cudaFuncSetAttribute(panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     });
     if (g_search_attr_err != cudaSuccess)
@@ -905,15 +996,16 @@ extern "C" int bsg_match_search(bsg_match* h, const double* origins, int norigin
     const long mrows = ((rows_max + BM - 1) / BM) * BM;
     const int mtiles_max = (int)(mrows / BM);
     const int ntiles = (int)((M->nsec + BN - 1) / BN);
-    // work-item grid: mgroup M tiles x ranges so that ~148 CTAs share tiles
-    int mgroup = std::min(mtiles_max, 10);
-    int ranges = std::max(1, std::min(ntiles, (148 + mgroup - 1) / mgroup));
-    const int tpr = (ntiles + ranges - 1) / ranges;
-    ranges = (ntiles + tpr - 1) / tpr;
+    const Runs full = Runs::plan(mtiles_max, ntiles);
+    const long tail_rows = ((M->nimg - 1) % nb + 1) * norigin;             // the last batch
+    const Runs tail = Runs::plan((int)((tail_rows + BM - 1) / BM), ntiles);
+    long stretches = 1;
+    for (const Runs* r : {&full, &tail})
+        for (int g = 0; g < r->groups; ++g) stretches = std::max(stretches, (long)r->stretches(g));
 
     // scratch (kept between calls)
     const size_t need_A = (size_t)mrows * kpad;
-    const size_t need_part = (size_t)ranges * mrows * TOPK;
+    const size_t need_part = (size_t)stretches * mrows * TOPK;
     const size_t need_cand = (size_t)M->nimg * topk;
     if (need_A > M->a_elems) {
         cudaFree(M->d_A); M->d_A = nullptr; M->a_elems = 0;
@@ -986,23 +1078,20 @@ extern "C" int bsg_match_search(bsg_match* h, const double* origins, int norigin
         GemmArgs ga{};
         ga.kblocks = kpad / BK;
         ga.ncols = (int)M->nsec;
-        ga.ntiles_n = ntiles;
-        ga.mtiles = (int)((rows + BM - 1) / BM);
+        ga.runs = Runs::plan((int)((rows + BM - 1) / BM), ntiles);
         ga.prow = mrows;
-        ga.mgroup = std::min(ga.mtiles, mgroup);
-        ga.ranges = ranges;
-        ga.tiles_per_range = tpr;
-        const int groups = (ga.mtiles + ga.mgroup - 1) / ga.mgroup;
-        ga.items = groups * ranges * ga.mgroup;
         ga.part_score = M->d_pscore;
         ga.part_idx = M->d_pidx;
         ga.status = M->d_status;
-        const int grid = std::min(ga.items, 148);
-        search_gemm_kernel<<<grid, GEMM_THREADS, GEMM_SMEM, s>>>(tmA, tmB, ga);
+        search_gemm_kernel<<<ga.runs.ctas, GEMM_THREADS, GEMM_SMEM, s>>>(tmA, tmB, ga);
         cudaEventRecord(ev[2], s);
-        merge_kernel<<<(unsigned)((cnt * 32 + 255) / 256), 256, 0, s>>>(M->d_pscore, M->d_pidx, ranges, mrows, norigin,
-                                                                         (int)cnt, topk, i0, M->d_csec, M->d_corg,
-                                                                         M->d_cscore);
+        const bool cached = stretches * TOPK * norigin <= MERGE_CACHE;
+        if (M->nsec * (long)norigin < 0xffffffffL)
+            merge_kernel<unsigned long long><<<(unsigned)cnt, MERGE_THREADS, cached ? sizeof(long long) * MERGE_CACHE : 0, s>>>(
+                M->d_pscore, M->d_pidx, ga.runs, mrows, norigin, topk, i0, cached ? 1 : 0, M->d_csec, M->d_corg, M->d_cscore);
+        else
+            merge_kernel<wide_t><<<(unsigned)cnt, MERGE_THREADS, 0, s>>>(
+                M->d_pscore, M->d_pidx, ga.runs, mrows, norigin, topk, i0, 0, M->d_csec, M->d_corg, M->d_cscore);
         cudaEventRecord(ev[3], s);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaEventSynchronize(ev[3]);
