@@ -53,6 +53,8 @@ struct Recon : Context {
     DevParticle* d_partbuf[2] = {nullptr, nullptr};
     DevParticle* d_psymbuf[2] = {nullptr, nullptr};
     size_t psymbuf_cap[2] = {0, 0};
+    TileTest* d_testbuf[2] = {nullptr, nullptr};        // tile tests of the records that are gridded
+    size_t testbuf_cap[2] = {0, 0};
     float2* d_specbuf[2] = {nullptr, nullptr};
     cudaEvent_t copy_done[2] = {nullptr, nullptr};
     cudaEvent_t fft_done[2] = {nullptr, nullptr};       // batch's spectra written
@@ -123,7 +125,6 @@ static void make_dev_particle(const Recon& r, const double* q, DevParticle& d, d
     d.inv2 = inv * inv;
     d.inv_st2 = 1.0 / ((double)d.step * (double)d.step);
     d.inv_step = 1.0f / d.step;
-    for (int i = 0; i < 3; ++i) d.ib[i] = fabsf(d.bf[i]) > 1e-6f ? 1.0f / d.bf[i] : 0.0f;
     double pw = q[15];
     double pad_ratio = (double)g.ft / (double)g.n;     // mg_reconstruct.cpp:192-199
     if (pad_ratio > 1) { pad_ratio *= pad_ratio * 0.6; pw /= pad_ratio; }
@@ -278,7 +279,7 @@ static void free_all(Recon* r) {
     for (int i = 0; i < 2; ++i) {
         F(r->d_imgbuf[i]); F(r->d_vol[i]); F(r->d_w[i]); F(r->d_pow[i]); F(r->d_w2[i]);
         F(r->d_evol[i]); F(r->d_ew[i]);
-        F(r->d_partbuf[i]); F(r->d_psymbuf[i]); F(r->d_specbuf[i]);
+        F(r->d_partbuf[i]); F(r->d_psymbuf[i]); F(r->d_testbuf[i]); F(r->d_specbuf[i]);
         if (r->h_partbuf[i]) cudaFreeHost(r->h_partbuf[i]);
         if (r->copy_done[i]) cudaEventDestroy(r->copy_done[i]);
         if (r->fft_done[i]) cudaEventDestroy(r->fft_done[i]);
@@ -313,8 +314,8 @@ static int run_batch_kernels(Recon* r, int buf, const float* d_img, long np, boo
     if (!insert) return BSG_OK;
     for (int h = 0; h < r->nhalves; ++h) {
         if (r->timing) { cudaEventCreate(&a); cudaEventCreate(&b); cudaEventRecord(a, s); }
-        if (r->nexp > 0) CK(launch_insert(*r, spec_out, r->d_psym, (int)r->nexp, r->nhalves == 2 ? h : -1, s));
-        else CK(launch_insert(*r, spec_out, r->d_part, (int)np, r->nhalves == 2 ? h : -1, s));
+        CK(launch_insert(*r, spec_out, r->nexp > 0 ? r->d_psym : r->d_part, r->d_testbuf[buf],
+                         (int)(r->nexp > 0 ? r->nexp : np), r->nhalves == 2 ? h : -1, s));
         if (r->timing) { cudaEventRecord(b, s); r->timed.push_back({a, b, 0}); }
         r->stats.launches += r->g.fom && r->replicas > 1 ? 2 : 1;     // gridding (+ the FOM path's replica combine)
         r->stats.insert_launches += 1;
@@ -397,8 +398,17 @@ static int upload_params(Recon* r, int buf, const double* params, long np) {
         CK(cudaMemcpyAsync(r->d_psym, r->h_psym.data(), sizeof(DevParticle) * k, cudaMemcpyHostToDevice,
                            r->fft_stream));
     }
-    // the records that are gridded get their phase lattices on the device
-    CK(launch_lattices(*r, r->nexp > 0 ? r->d_psym : r->d_part, r->nexp > 0 ? r->nexp : np, r->fft_stream));
+    // the records that are gridded get their phase lattices and tile tests on
+    // the device
+    const long nrec = r->nexp > 0 ? r->nexp : np;
+    if ((size_t)nrec > r->testbuf_cap[buf]) {
+        if (r->d_testbuf[buf]) cudaFree(r->d_testbuf[buf]);
+        r->d_testbuf[buf] = nullptr;
+        r->testbuf_cap[buf] = 0;
+        CK(cudaMalloc((void**)&r->d_testbuf[buf], sizeof(TileTest) * nrec));
+        r->testbuf_cap[buf] = (size_t)nrec;
+    }
+    CK(launch_lattices(*r, r->nexp > 0 ? r->d_psym : r->d_part, r->d_testbuf[buf], nrec, r->fft_stream));
     r->stats.launches += 1;
     return BSG_OK;
 }
@@ -535,6 +545,8 @@ int bsg_recon_create(const bsg_recon_config* cfg, bsg_recon** out) {
         if (!rc && cudaMallocHost((void**)&r->h_partbuf[i], sizeof(DevParticle) * batch) != cudaSuccess)
             rc = fail(BSG_ERR_NOMEM, "bsg_recon_create: pinned host allocation");
         A((void**)&r->d_partbuf[i], sizeof(DevParticle) * batch);
+        A((void**)&r->d_testbuf[i], sizeof(TileTest) * batch);
+        r->testbuf_cap[i] = (size_t)batch;
         A((void**)&r->d_specbuf[i], sizeof(float2) * (size_t)(ft + 1) * (ft + 2) * batch);
         if (!rc && cudaMemset(r->d_specbuf[i], 0, sizeof(float2) * (size_t)(ft + 1) * (ft + 2) * batch) != cudaSuccess)
             rc = fail(BSG_ERR_CUDA, "bsg_recon_create: clearing the spectra buffer");

@@ -28,29 +28,39 @@ struct alignas(16) DevParticle {
     double bx, by;          // background circle centre (pixels)
     double fs;              // CTF frequency step 1/(ft*pixel)   (mg_ctf.cpp:84-85)
     double c00, c20, c22, c2m2, c40, c11, c1m1;   // aberration weights (ctf.h:321-348)
-    // insertion (fspace_pack_2D, Bimage_reconstruct.cpp:131-160)
+    // insertion (fspace_pack_2D, Bimage_reconstruct.cpp:131-160); the fields a
+    // gridding pair's set-up reads are together, in 16-byte pieces
     double ad[3], bd[3];    // map frequency per unit pixel step: R[:,0]*inv*mscale, R[:,1]*inv*mscale
-    double iad[3], ibd[3];  // 1 / ad, 1 / bd (0 where |.| <= 1e-12): the gridding walks' row and line bounds
+    double iad[3];          // 1 / ad (0 where |.| <= 1e-12): the gridding walks' row bounds
+    double inv_st2;         // 1 / step^2: pixel coordinate per unit of ad.c
+    float  af[3], bf[3];    // float copies of ad / bd
+    float  pw;              // particle weight / (pad_ratio^2 * 0.6)
+    float  inv_step;        // 1 / step
+    int    spec;            // index of this record's spectrum in the batch (symmetry copies share it)
+    int    lat;             // gridding phase lattice lh | lk << 12 | sh << 24 (lattice.h); 0: the
+                            // orientation-independent one
+    float  ezmax;           // max |ewh s2| mscale over the pixels (voxels)
+    float  step;            // |ad| = voxels per pixel step
+    double ibd[3];          // 1 / bd, as iad: the unpaired pixels' lines
     double nrm[3];          // unit plane normal R[:,2]
     double inv2;            // (scale/(ft*pixel))^2: s2 per unit pixel^2
-    double inv_st2;         // 1 / step^2: pixel coordinate per unit of ad.c
     double na, nb;          // image normalisation v * na + nb (breconstruct -rescale; 1, 0 otherwise)
     // Ewald-sphere surface (breconstruct -ewald; Bimage_reconstruct.cpp:157-168):
     // m += ewh s2 cd with s2 = (h^2 + k^2) inv2, one record per surface
     double ewh;             // +-lambda/2 (0: the plane)
     double inv;             // sqrt(inv2): s per unit pixel
     double cd[3];           // R[:,2] * mscale
-    float  ezmax;           // max |ewh s2| mscale over the pixels (voxels)
-    float  ib[3];           // 1 / bf[i] (0 when |bf[i]| <= 1e-6)
-    float  inv_step;        // 1 / step
-    float  af[3], bf[3];    // float copies of ad / bd
-    float  pw;              // particle weight / (pad_ratio^2 * 0.6)
     float  slab;            // sum |nrm_i|: plane reaches a voxel cube iff |n.c| < slab
-    float  step;            // |ad| = voxels per pixel step
     int    half;            // half-map index
-    int    spec;            // index of this record's spectrum in the batch (symmetry copies share it)
-    int    lat;             // gridding phase lattice lh | lk << 12 | sh << 24 (lattice.h); 0: the
-                            // orientation-independent one
+};
+
+// What a tile's test of a gridding record reads (tile_mask), 32 bytes instead
+// of fields spread over the record: the plane's normal, its slab's half width
+// without the tile's, the farthest pixel along each axis, the half map.
+struct alignas(16) TileTest {
+    float n[3], slab;
+    float reach[3];
+    int half;
 };
 
 // Run geometry shared by all kernels of one context.
@@ -79,9 +89,9 @@ struct Context;
 cudaError_t launch_background(const Context& c, const float* img, int nimg, cudaStream_t s);
 cudaError_t launch_rows(const Context& c, const float* img, int nimg, cudaStream_t s);
 cudaError_t launch_cols(const Context& c, int nimg, float2* spectra, cudaStream_t s);
-cudaError_t launch_lattices(const Context& c, DevParticle* parts, long n, cudaStream_t s);
-cudaError_t launch_insert(const Context& c, const float2* spectra, const DevParticle* parts, int np, int half,
-                          cudaStream_t s);
+cudaError_t launch_lattices(const Context& c, DevParticle* parts, TileTest* tests, long n, cudaStream_t s);
+cudaError_t launch_insert(const Context& c, const float2* spectra, const DevParticle* parts, const TileTest* tests,
+                          int np, int half, cudaStream_t s);
 cudaError_t launch_finish(const Context& c, int imap, float* map_out, bool sinc, int* launches, cudaStream_t s);
 cudaError_t launch_sinc_table(double* t, int N, cudaStream_t s);
 size_t fsc_part_elems(const Context& c, int nshell);

@@ -48,6 +48,7 @@ constexpr int WARPS = 4;                  // warps (tiles) per block
 struct InsertArgs {
     const float2* spec;        // batch x (ft+1) x (ft+2), centred
     const DevParticle* part;   // particles of this launch
+    const TileTest* test;      // their tile tests
     int np;
     int half;                  // only particles of this half map (-1: all)
     int N, ft, pitch;
@@ -70,26 +71,20 @@ struct InsertArgs {
     double* w2;
 };
 
-// Does particle P's plane come within reach of the tile for alias
+// Does the record's plane come within reach of the tile for alias
 // combination a (bit i set: axis i shifted by -N)?  Bitmask over the 8.
 template <int TX, int TY, int TZ>
-__device__ __forceinline__ unsigned tile_mask(const DevParticle& P, int x0, int y0, int z0, int N, int ft) {
+__device__ __forceinline__ unsigned tile_mask(const TileTest& t, int x0, int y0, int z0, int N) {
     unsigned mask = 0;
     const float ex = 0.5f * (TX - 1), ey = 0.5f * (TY - 1), ez = 0.5f * (TZ - 1);
-    const float hf = 0.5f * ft;
-    // (an Ewald surface deviates from the plane by up to P.ezmax voxels)
-    const float rx = hf * (fabsf(P.af[0]) + fabsf(P.bf[0])) + 1.0f + P.ezmax;
-    const float ry = hf * (fabsf(P.af[1]) + fabsf(P.bf[1])) + 1.0f + P.ezmax;
-    const float rz = hf * (fabsf(P.af[2]) + fabsf(P.bf[2])) + 1.0f + P.ezmax;
-    const float n0 = (float)P.nrm[0], n1 = (float)P.nrm[1], n2 = (float)P.nrm[2];
-    const float slack = P.slab + fabsf(n0) * ex + fabsf(n1) * ey + fabsf(n2) * ez + 1e-3f + P.ezmax;
+    const float slack = t.slab + fabsf(t.n[0]) * ex + fabsf(t.n[1]) * ey + fabsf(t.n[2]) * ez;
 #pragma unroll
     for (int a = 0; a < 8; ++a) {
         const float cx = x0 - ((a & 1) ? N : 0) + ex;
         const float cy = y0 - ((a & 2) ? N : 0) + ey;
         const float cz = z0 - ((a & 4) ? N : 0) + ez;
-        if (fabsf(cx) - ex > rx || fabsf(cy) - ey > ry || fabsf(cz) - ez > rz) continue;
-        if (fabsf(n0 * cx + n1 * cy + n2 * cz) > slack) continue;
+        if (fabsf(cx) - ex > t.reach[0] || fabsf(cy) - ey > t.reach[1] || fabsf(cz) - ez > t.reach[2]) continue;
+        if (fabsf(t.n[0] * cx + t.n[1] * cy + t.n[2] * cz) > slack) continue;
         mask |= 1u << a;
     }
     return mask;
@@ -658,8 +653,8 @@ __global__ void __launch_bounds__(WARPS * 32) insert_kernel(InsertArgs a) {
         const int p = base + lane;
         unsigned mask = 0;
         if (p < p_hi) {
-            const DevParticle& P = a.part[p];
-            if (P.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(P, x0, y0, z0, N, a.ft);
+            const TileTest t = a.test[p];
+            if (t.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(t, x0, y0, z0, N);
         }
         unsigned todo = __ballot_sync(0xffffffffu, mask != 0);
         while (todo) {
@@ -700,35 +695,66 @@ __global__ void __launch_bounds__(WARPS * 32) insert_kernel(InsertArgs a) {
 // lands on the other side of a cell boundary because of it moves a
 // contribution by that much, and the phase lattices keep a margin above it
 // (lattice.h).
-// One cell's read-modify-write; SLOTS: cells of the tile (the weights follow
-// them).  A corner outside the tile (on = false) loads the tile's first cell
-// and stores nothing: a select and a predicate instead of a branch per corner
-// (as float4 cells, 6.53 -> 5.47 ms per 953 particles at 256^3).
-template <int SLOTS>
-__device__ __forceinline__ void cell_add(unsigned cell0, int index, float2 f, float w, bool on) {
-    const unsigned i = on ? index : 0, at = cell0 + 8u * i, wt = cell0 + 8u * SLOTS + 4u * i;
+// A corner's read-modify-write: the cell at byte address `at` + 8 OFF and its
+// weight at `wt` + 4 OFF.  A corner outside the tile (on = false) is loaded all
+// the same - its address lies within the guards around the arrays (GridSmem) -
+// and not stored, so the eight corners are constant offsets from two registers
+// (953 particles at 256^3: a branch per corner 6.53, a select of its address
+// 5.47 ms with float4 cells; with split cells 256 particles took 1.63 with the
+// select and take 1.56 ms so, with the tile tests read from 32-byte entries).
+template <int OFF>
+__device__ __forceinline__ void cell_add(unsigned at, unsigned wt, float2 f, float w, bool on) {
     float x, y, z;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(at) : "memory");
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(z) : "r"(wt) : "memory");
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2+%3];" : "=f"(x), "=f"(y) : "r"(at), "n"(8 * OFF) : "memory");
+    asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(z) : "r"(wt), "n"(4 * OFF) : "memory");
     x = fmaf(f.x, w, x);
     y = fmaf(f.y, w, y);
     z += w;
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t"
-        "@p st.shared.v2.f32 [%0], {%1, %2};\n\t@p st.shared.f32 [%3], %4;\n\t}" ::"r"(at),
-        "f"(x), "f"(y), "r"(wt), "f"(z), "r"((int)on)
+        "@p st.shared.v2.f32 [%0+%6], {%1, %2};\n\t@p st.shared.f32 [%3+%7], %4;\n\t}" ::"r"(at),
+        "f"(x), "f"(y), "r"(wt), "f"(z), "r"((int)on), "n"(8 * OFF), "n"(4 * OFF)
         : "memory");
 }
 
+// Shared memory of a gridding warp: the queue of pairs, the cells, their
+// weights and what the loads of corners outside the tile can reach.  The first
+// corner of a pixel with a corner in the tile is cell FIRST .. LAST (coordinates
+// -1 .. T - 1), and pixel4 limits it to that, so loads reach from cell FIRST to
+// the eighth corner of cell LAST.
+template <int TX, int TY, int TZ, int PX, int PP>
+struct GridSmem {
+    static constexpr int SLOTS = PP * TZ, CORNER = 1 + PX + PP;
+    static constexpr int FIRST = -CORNER, LAST = (TX - 1) + PX * (TY - 1) + PP * (TZ - 1);
+    static constexpr int PAST = LAST + CORNER + 1 > SLOTS ? LAST + CORNER + 1 - SLOTS : 0;
+    static constexpr int round16(int n) { return (n + 15) & ~15; }
+    static constexpr int larger(int m, int n) { return m > n ? m : n; }
+    static constexpr int QUEUE = 32 * (int)sizeof(int4) + QN * (int)(sizeof(Pair) + sizeof(RowBounds) + sizeof(int));
+    static constexpr int CELLS = round16(larger(QUEUE, 8 * CORNER));       // byte offset of the cells
+    static constexpr int WEIGHTS = CELLS + round16(8 * SLOTS);             // byte offset of the weights
+    static constexpr int BYTES = larger(WEIGHTS + 4 * (SLOTS + PAST), CELLS + 8 * (SLOTS + PAST));
+    static_assert(WEIGHTS - 4 * CORNER >= 0, "loads before the first weight");
+    static_assert(sizeof(Pair) % 16 == 0 && sizeof(RowBounds) % 8 == 0, "alignment in the queue");
+};
+
+// the corners (0, y, z) and (1, y, z) at cell offset OFF
+template <int OFF, int PX, int PP>
+__device__ __forceinline__ void corner_row(unsigned at, unsigned wt, float2 f, float rx, float wyz, const bool* vx, bool on) {
+    cell_add<OFF>(at, wt, f, (1.f - rx) * wyz, vx[0] && on);
+    __syncwarp();
+    cell_add<OFF + 1>(at, wt, f, rx * wyz, vx[1] && on);
+    __syncwarp();
+}
+
 template <bool GATE, bool EW, int TX, int TY, int TZ, int PX, int PP>
-__device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P, const Pair& Q, unsigned cell0,
-                                       float2 f, int h, int k, bool act) {
-    float wt = Q.pw;
+__device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P, const Pair& Q, unsigned cells,
+                                       unsigned weights, float2 f, int h, int k, bool act) {
+    float wt_ = Q.pw;
     if (GATE && act) {
         bool keep;
         const float tw = pixel_weight_gate(a, P, h, k, keep);
         if (!keep) act = false;
-        wt *= tw;
+        wt_ *= tw;
     }
     const float dh = (float)(h - Q.hc), dk = (float)(k - Q.kc);
     float mx = fmaf(dh, Q.ax, fmaf(dk, Q.cx, Q.bx));
@@ -746,13 +772,14 @@ __device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P
     if (a.interp != 2) {
         const float fx = floorf(mx + 0.5f), fy = floorf(my + 0.5f), fz = floorf(mz + 0.5f);
         const int ix = (int)fx, iy = (int)fy, iz = (int)fz;
-        float w = wt;
+        float w = wt_;
         if (a.interp == 1) {
             const float dx = mx - fx, dy = my - fy, dz = mz - fz;
-            w = wt * (1.0f - sqrtf(dx * dx + dy * dy + dz * dz));
+            w = wt_ * (1.0f - sqrtf(dx * dx + dy * dy + dz * dz));
         }
         const bool on = act && (unsigned)ix < TX && (unsigned)iy < TY && (unsigned)iz < TZ && w > 0.f;
-        cell_add<PP * TZ>(cell0, ix + PX * iy + PP * iz, f, w, on);
+        const int i = on ? ix + PX * iy + PP * iz : 0;
+        cell_add<0>(cells + 8 * i, weights + 4 * i, f, w, on);
         __syncwarp();
         return;
     }
@@ -762,22 +789,14 @@ __device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P
     const bool vx[2] = {act && (unsigned)ix < TX, act && (unsigned)(ix + 1) < TX};
     const bool vy[2] = {(unsigned)iy < TY, (unsigned)(iy + 1) < TY};
     const bool vz[2] = {(unsigned)iz < TZ, (unsigned)(iz + 1) < TZ};
-    const int cell = ix + PX * iy + PP * iz;
-#pragma unroll
-    for (int dz = 0; dz < 2; ++dz) {
-        const float wz = (dz ? rz : 1.f - rz) * wt;
-#pragma unroll
-        for (int dy = 0; dy < 2; ++dy) {
-            const float wyz = (dy ? ry : 1.f - ry) * wz;
-            const bool vyz = vy[dy] && vz[dz];
-#pragma unroll
-            for (int dx = 0; dx < 2; ++dx) {
-                cell_add<PP * TZ>(cell0, cell + dx + PX * dy + PP * dz, f, (dx ? rx : 1.f - rx) * wyz,
-                         vx[dx] && vyz);
-                __syncwarp();
-            }
-        }
-    }
+    typedef GridSmem<TX, TY, TZ, PX, PP> Smem;
+    const int cell = act ? min(max(ix + PX * iy + PP * iz, Smem::FIRST), Smem::LAST) : 0;
+    const unsigned at = cells + 8 * cell, wt = weights + 4 * cell;
+    const float z0 = (1.f - rz) * wt_, z1 = rz * wt_;
+    corner_row<0, PX, PP>(at, wt, f, rx, (1.f - ry) * z0, vx, vy[0] && vz[0]);
+    corner_row<PX, PX, PP>(at, wt, f, rx, ry * z0, vx, vy[1] && vz[0]);
+    corner_row<PP, PX, PP>(at, wt, f, rx, (1.f - ry) * z1, vx, vy[0] && vz[1]);
+    corner_row<PP + PX, PX, PP>(at, wt, f, rx, ry * z1, vx, vy[1] && vz[1]);
 }
 
 // The pair's set-up by one lane: the pixels whose tents can reach the tile at
@@ -855,12 +874,14 @@ template <bool GATE, bool EW, int TX, int TY, int TZ, int PX, int PP>
 __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
     constexpr int SLOTS = PP * TZ;
     constexpr int TV = TX * TY * TZ;
-    extern __shared__ float2 s_sum[];                   // SLOTS cells, then their weights
-    float* const s_wt = reinterpret_cast<float*>(s_sum + SLOTS);
-    __shared__ int4 s_rows[32];
-    __shared__ Pair s_pairs[QN];
-    __shared__ RowBounds s_bounds[QN];
-    __shared__ int s_ids[QN];
+    typedef GridSmem<TX, TY, TZ, PX, PP> Smem;
+    extern __shared__ __align__(16) unsigned char s_grid[];
+    int4* const s_rows = reinterpret_cast<int4*>(s_grid);
+    Pair* const s_pairs = reinterpret_cast<Pair*>(s_rows + 32);
+    RowBounds* const s_bounds = reinterpret_cast<RowBounds*>(s_pairs + QN);
+    int* const s_ids = reinterpret_cast<int*>(s_bounds + QN);
+    float2* const s_sum = reinterpret_cast<float2*>(s_grid + Smem::CELLS);
+    float* const s_wt = reinterpret_cast<float*>(s_grid + Smem::WEIGHTS);
     const int lane = threadIdx.x;
     const bool hs = a.zsplit > 0;
     const int items = a.R + (hs ? 1 : 0);               // per tile
@@ -870,7 +891,7 @@ __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
     const int N = a.N;
     const int hf = a.ft / 2;
     const size_t spec_stride = (size_t)(2 * hf + 1) * a.pitch;
-    const unsigned cell0 = (unsigned)__cvta_generic_to_shared(s_sum);
+    const unsigned cells = (unsigned)__cvta_generic_to_shared(s_sum), weights = (unsigned)__cvta_generic_to_shared(s_wt);
     // half-space gridding (walk_edges): tiles at or above zsplit grid only
     // the unpaired pixels; those below it grid the others, and the extra item
     // the unpaired ones into evol / ew
@@ -914,9 +935,9 @@ __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
             if (base < p_hi) {
                 const int p = base + lane;
                 if (p < p_hi) {
-                    const DevParticle& P = a.part[p];
-                    if (P.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(P, x0, y0, z0, N, a.ft);
-                    if (edge_walk && mask) mask = edge_mask<TX, TY, TZ>(P, mask, x0, y0, z0, N, a.ft);
+                    const TileTest t = a.test[p];
+                    if (t.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(t, x0, y0, z0, N);
+                    if (edge_walk && mask) mask = edge_mask<TX, TY, TZ>(a.part[p], mask, x0, y0, z0, N, a.ft);
                 }
                 continue;
             }
@@ -945,7 +966,7 @@ __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
                 return act ? __ldg(S + (long)k * a.pitch + h) : make_float2(0.f, 0.f);
             };
             auto pix = [&](float2 f, int h, int k, bool act) {
-                pixel4<GATE, EW, TX, TY, TZ, PX, PP>(a, P, Q, cell0, f, h, k, act);
+                pixel4<GATE, EW, TX, TY, TZ, PX, PP>(a, P, Q, cells, weights, f, h, k, act);
             };
             if (edge_walk) walk_edges(Q, hf, lane, fetch, pix);
             else walk_groups<TX, TY, TZ>(P, Q, s_bounds[at], EW ? (double)P.ezmax : 0.0,
@@ -1061,11 +1082,9 @@ static cudaError_t set_smem_shape() {
     return cudaFuncSetAttribute(insert_kernel<false, TX, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
-static constexpr int cell_bytes(int slots) { return slots * (int)(sizeof(float2) + sizeof(float)); }
-
 template <int TX, int TY, int TZ, int PX, int PP>
 static cudaError_t set_smem_shape4() {
-    const int smem = cell_bytes(PP * TZ);
+    const int smem = GridSmem<TX, TY, TZ, PX, PP>::BYTES;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(grid4_kernel<true, false, TX, TY, TZ, PX, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(grid4_kernel<false, false, TX, TY, TZ, PX, PP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
@@ -1111,7 +1130,7 @@ static cudaError_t launch_shape4(const InsertArgs& a0, const Context& c, cudaStr
     a.ntz = (N + TZ - 1) / TZ;
     const int ntiles = a.ntx * a.nty * a.ntz;
     const long items = (long)ntiles * (a.R + (a.zsplit > 0 ? 1 : 0));
-    const size_t smem = cell_bytes(PP * TZ);
+    const size_t smem = GridSmem<TX, TY, TZ, PX, PP>::BYTES;
     if (c.g.ewald) {
         if (c.g.gate) grid4_kernel<true, true, TX, TY, TZ, PX, PP><<<(unsigned)items, 32, smem, s>>>(a);
         else grid4_kernel<false, true, TX, TY, TZ, PX, PP><<<(unsigned)items, 32, smem, s>>>(a);
@@ -1122,11 +1141,12 @@ static cudaError_t launch_shape4(const InsertArgs& a0, const Context& c, cudaStr
     return cudaGetLastError();
 }
 
-cudaError_t launch_insert(const Context& c, const float2* spectra, const DevParticle* parts, int np, int half,
-                          cudaStream_t s) {
+cudaError_t launch_insert(const Context& c, const float2* spectra, const DevParticle* parts, const TileTest* tests,
+                          int np, int half, cudaStream_t s) {
     InsertArgs a;
     a.spec = spectra;
     a.part = parts;
+    a.test = tests;
     a.np = np;
     a.half = half;
     a.N = c.g.map;

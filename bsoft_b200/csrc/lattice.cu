@@ -1,5 +1,5 @@
-// lattice.cu - the phase lattices of a batch's gridding records (lattice.h),
-// one warp per record: the lanes test 32 candidates at a time, in
+// lattice.cu - the phase lattices of a batch's gridding records (lattice.h) and
+// their tile-test entries, one warp per record: the lanes test 32 candidates at a time, in
 // choose_lattice's order, and the first safe one is the record's.  On the host
 // the search took 0.5 to 0.7 us a record before the batch's first kernel could
 // start (1.1 of 2.7 ms for 2,000 particles of 64^2); here 12 us for all.
@@ -23,7 +23,8 @@ __device__ __forceinline__ PhaseLattice candidate(int c) {
     return {0, 0, 0};
 }
 
-__global__ void __launch_bounds__(128) lattice_kernel(DevParticle* part, long n, double mscale, int ft) {
+__global__ void __launch_bounds__(128) lattice_kernel(DevParticle* part, TileTest* tests, long n,
+                                                       double mscale, int ft) {
     const long r = blockIdx.x * 4L + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (r >= n) return;
@@ -46,11 +47,23 @@ __global__ void __launch_bounds__(128) lattice_kernel(DevParticle* part, long n,
                     __shfl_sync(0xffffffffu, l.sh, src)};
             break;
         }
-    if (lane == 0) P.lat = pack_lattice(best);
+    if (lane == 0) {
+        P.lat = pack_lattice(best);
+        // (an Ewald surface deviates from the plane by up to P.ezmax voxels)
+        TileTest t;
+        const float hf = 0.5f * ft;
+        for (int i = 0; i < 3; ++i) {
+            t.n[i] = (float)P.nrm[i];
+            t.reach[i] = hf * (fabsf(P.af[i]) + fabsf(P.bf[i])) + 1.0f + P.ezmax;
+        }
+        t.slab = P.slab + 1e-3f + P.ezmax;
+        t.half = P.half;
+        tests[r] = t;
+    }
 }
 
-cudaError_t launch_lattices(const Context& c, DevParticle* parts, long n, cudaStream_t s) {
-    lattice_kernel<<<(unsigned)((n + 3) / 4), 128, 0, s>>>(parts, n, c.g.mscale, c.g.ft);
+cudaError_t launch_lattices(const Context& c, DevParticle* parts, TileTest* tests, long n, cudaStream_t s) {
+    lattice_kernel<<<(unsigned)((n + 3) / 4), 128, 0, s>>>(parts, tests, n, c.g.mscale, c.g.ft);
     return cudaGetLastError();
 }
 
