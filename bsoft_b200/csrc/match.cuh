@@ -257,7 +257,7 @@ struct Match {
     long nsec = 0;
     MHyp* d_secs = nullptr;            // panel views (rows 0, 1 scaled)
     std::vector<MHyp> h_secs;          // host copy
-    float* d_rots = nullptr;           // panel rotations (unscaled, float) for local selection
+    float* d_rots = nullptr;           // panel rotations (unscaled, float, 9 x nsec) for local selection
     __nv_bfloat16* d_panel = nullptr;  // nsec x kpad
     float2* d_pexact = nullptr;        // nsec x npix: the panel's FP32 sections at the figure-of-merit
                                        // pixels, as fom_kernel<float> gathers them (rescoring reads them)

@@ -422,25 +422,61 @@ __global__ void __launch_bounds__(256) panel_kernel(cudaTextureObject_t tex, int
     }
 }
 
-// per image of the batch: 1 / (n_f sqrt(D_j C_j)) per coarse shell
-__global__ void coarse_norm_kernel(const float2* __restrict__ spec, int D, const float* __restrict__ ctf, int npix,
-                                   const MPix* __restrict__ cpix, const int* __restrict__ cstart, int nf, long img0,
-                                   float* __restrict__ gA) {
+// per image of the batch: 1 / (n_f sqrt(D_j C_j)) per coarse shell.  All threads
+// fetch the pixels' terms, NORM_PIX at a time, and a thread per shell adds them
+// in pixel order (a thread per shell that fetched them itself waited for each
+// pixel in turn: 512 images of 128^2 32 us, now 20).
+constexpr int NORM_PIX = 1024;
+constexpr int NORM_SHELLS = 2;             // shells per thread and pass (up to box 512 there are fewer than 512)
+
+__global__ void __launch_bounds__(256) coarse_norm_kernel(const float2* __restrict__ spec, int D,
+                                                          const float* __restrict__ ctf, int npix,
+                                                          const MPix* __restrict__ cpix, const int* __restrict__ cstart,
+                                                          int nf, long img0, float* __restrict__ gA) {
+    __shared__ double2 term[NORM_PIX];
     const long img = img0 + blockIdx.x;
     const float2* X = spec + img * (long)D * D;
     const float* C = ctf + img * (long)npix;
-    for (int j = threadIdx.x; j < nf; j += blockDim.x) {
-        double d = 0, c2 = 0;
-        const int n = cstart[j + 1] - cstart[j];
-        for (int p = cstart[j]; p < cstart[j + 1]; ++p) {
-            const MPix q = cpix[p];
-            const float2 x = X[q.idx];
-            const double c = C[q.pad];
-            d += (double)x.x * x.x + (double)x.y * x.y;
-            c2 += c * c;
+    const int total = cstart[nf];
+    for (int j0 = 0; j0 < nf; j0 += 256 * NORM_SHELLS) {
+        int lo[NORM_SHELLS], hi[NORM_SHELLS];
+        double d[NORM_SHELLS], c2[NORM_SHELLS];
+#pragma unroll
+        for (int i = 0; i < NORM_SHELLS; ++i) {
+            const int j = j0 + threadIdx.x + 256 * i;
+            lo[i] = j < nf ? cstart[j] : 0;
+            hi[i] = j < nf ? cstart[j + 1] : 0;
+            d[i] = c2[i] = 0;
         }
-        const double den = n > 0 ? d * (c2 / n) : 0.0;
-        gA[(long)blockIdx.x * nf + j] = den > 0 ? (float)(1.0 / (nf * sqrt(den))) : 0.f;
+        for (int b = 0; b < total; b += NORM_PIX) {
+            const int m = min(NORM_PIX, total - b);
+#pragma unroll 4
+            for (int p = threadIdx.x; p < m; p += 256) {
+                const MPix q = cpix[b + p];
+                const float2 x = X[q.idx];
+                const double c = C[q.pad];
+                term[p] = make_double2((double)x.x * x.x + (double)x.y * x.y, c * c);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < NORM_SHELLS; ++i) {
+                const int p1 = min(hi[i] - b, m);
+#pragma unroll 8
+                for (int p = max(lo[i] - b, 0); p < p1; ++p) {
+                    const double2 t = term[p];
+                    d[i] += t.x;
+                    c2[i] += t.y;
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int i = 0; i < NORM_SHELLS; ++i) {
+            const int j = j0 + threadIdx.x + 256 * i, n = hi[i] - lo[i];
+            if (j >= nf) continue;
+            const double den = n > 0 ? d[i] * (c2[i] / n) : 0.0;
+            gA[(long)blockIdx.x * nf + j] = den > 0 ? (float)(1.0 / (nf * sqrt(den))) : 0.f;
+        }
     }
 }
 
@@ -475,13 +511,15 @@ __global__ void __launch_bounds__(256) rows_kernel(const float2* __restrict__ sp
 
 // One CTA per image: the topk best of the partial candidates of its nshift rows
 // in (score descending, section, origin) order.  A candidate is one number
-// that sorts that way (64 bits; 128 when sections x origins exceed 32),
-// gathered once into shared memory (when they fit:
-// cached = 1), and each pick is the largest below the last (reading the
-// partial buffers again for every pick, one warp per image, took 0.42 ms for
-// 256 images: now 0.07).
-constexpr int MERGE_THREADS = 256;
-constexpr int MERGE_CACHE = 12288;         // candidates that shared memory holds (96 KB)
+// that sorts that way (64 bits; 128 when sections x origins exceed 32).  Each
+// thread reads its share once and keeps the TOPK best of it in registers, in
+// order; a pick is the largest of the threads' first ones.  Bound by the reads'
+// latency, hence 1,024 threads for a few images.  (256 images of 25 origins:
+// read again for every pick by one warp per image 0.42 ms, by 256 threads from
+// shared memory 0.07, now 0.04; 5 images against 8,580 sections, 29,600
+// candidates an image, 0.84 by the warp and 1.27 when they exceeded shared
+// memory, now 0.08.)
+constexpr int MERGE_MOST = 1024;
 
 typedef unsigned __int128 wide_t;
 
@@ -495,63 +533,66 @@ __device__ __forceinline__ wide_t shfl_xor_key(wide_t v, int o) {
 
 // K: score in the upper half, the inverted section x origin number in the lower
 template <class K>
-__global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(const float* __restrict__ ps, const int* __restrict__ pi,
-                                                              Runs runs, long mrows, int nshift, int topk, long img0,
-                                                              int cached, int* __restrict__ cand_sec,
-                                                              int* __restrict__ cand_org, float* __restrict__ cand_score) {
+__global__ void __launch_bounds__(sizeof(K) == 8 ? MERGE_MOST : MERGE_MOST / 2)
+    merge_kernel(const float* __restrict__ ps, const int* __restrict__ pi, Runs runs, long mrows, int nshift, int topk,
+                 long img0, int* __restrict__ cand_sec, int* __restrict__ cand_org, float* __restrict__ cand_score) {
     constexpr int HALF = 4 * sizeof(K);
     constexpr K LOW = ((K)1 << HALF) - 1;
-    extern __shared__ __align__(16) unsigned char msm[];
-    K* const cache = reinterpret_cast<K*>(msm);
-    __shared__ K best[MERGE_THREADS / 32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // f(candidate) for every candidate: a warp takes a row, its lanes the
-    // row's stretches and places
-    auto each = [&](auto&& f) {
-        int at = 0;
-        for (int s = 0; s < nshift; ++s) {
-            const long row = (long)blockIdx.x * nshift + s;
-            const int g = runs.group_of((int)(row / BM)), n = runs.stretches(g) * TOPK;
-            for (int e = threadIdx.x; e < n; e += MERGE_THREADS) {
-                const int r = e / TOPK;
-                K v = 0;
-                if (runs.bound(g, r) < runs.bound(g, r + 1)) {
-                    const long o = ((long)r * mrows + row) * TOPK + e % TOPK;
-                    const int sec = pi[o];
-                    if (sec >= 0) {
-                        unsigned u = __float_as_uint(ps[o]);
-                        u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;         // sorts as the float does
-                        v = (K)u << HALF | (LOW - ((K)sec * nshift + s));
-                    }
-                }
-                f(at + e, v);
+    __shared__ K best[2][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    K top[TOPK];                                 // this thread's best, largest first
+#pragma unroll
+    for (int i = 0; i < TOPK; ++i) top[i] = 0;
+    // a row's stretches and places, a row after the other: thread t takes every
+    // blockDim.x-th of the image's candidates
+    int e = threadIdx.x, s = 0;
+    long row = (long)blockIdx.x * nshift;
+    int g = runs.group_of((int)(row / BM)), n = runs.stretches(g) * TOPK;
+    while (s < nshift) {
+        if (e >= n) {
+            e -= n;
+            if (++s == nshift) break;
+            ++row;
+            if (row % BM == 0) {
+                g = runs.group_of((int)(row / BM));
+                n = runs.stretches(g) * TOPK;
             }
-            at += n;
+            continue;
         }
-        return at;
-    };
-    int count = 0;
-    if (cached) count = each([&](int i, K v) { cache[i] = v; });
-    __syncthreads();
-    K prev = ~(K)0;
+        const int r = e / TOPK;
+        const long o = ((long)r * mrows + row) * TOPK + e % TOPK;
+        const int sec = __ldg(pi + o);
+        const float score = __ldg(ps + o);
+        if (sec >= 0 && runs.bound(g, r) < runs.bound(g, r + 1)) {
+            unsigned u = __float_as_uint(score);
+            u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;         // sorts as the float does
+            K v = (K)u << HALF | (LOW - ((K)sec * nshift + s));
+            if (v > top[TOPK - 1]) {
+#pragma unroll
+                for (int i = 0; i < TOPK; ++i)
+                    if (v > top[i]) { const K w = top[i]; top[i] = v; v = w; }
+            }
+        }
+        e += blockDim.x;
+    }
     for (int t = 0; t < topk; ++t) {
-        K b = 0;
-        if (cached) {
-            for (int i = threadIdx.x; i < count; i += MERGE_THREADS) {
-                const K v = cache[i];
-                if (v < prev && v > b) b = v;
-            }
-        } else {
-            each([&](int, K v) { if (v < prev && v > b) b = v; });
-        }
+        K b = top[0];
         for (int o = 16; o; o >>= 1) {
             const K v = shfl_xor_key(b, o);
             if (v > b) b = v;
         }
-        __syncthreads();                         // the last pick has been read
-        if (lane == 0) best[warp] = b;
+        if (lane == 0) best[t & 1][warp] = b;
         __syncthreads();
-        for (int w = 0; w < MERGE_THREADS / 32; ++w) if (best[w] > b) b = best[w];
+        b = lane < nwarps ? best[t & 1][lane] : (K)0;
+        for (int o = 16; o; o >>= 1) {
+            const K v = shfl_xor_key(b, o);
+            if (v > b) b = v;
+        }
+        if (b && top[0] == b) {
+#pragma unroll
+            for (int i = 0; i + 1 < TOPK; ++i) top[i] = top[i + 1];
+            top[TOPK - 1] = 0;
+        }
         if (threadIdx.x == 0) {
             const long c = (img0 + blockIdx.x) * topk + t;
             const long key = (long)(LOW - (b & LOW));
@@ -561,8 +602,6 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(const float* __res
             cand_org[c] = b ? (int)(key % nshift) : -1;
             cand_score[c] = b ? __uint_as_float(u) : -3.0e38f;
         }
-        if (b) prev = b;
-        else prev = 0;                           // nothing is left
     }
 }
 
@@ -572,41 +611,86 @@ __global__ void __launch_bounds__(MERGE_THREADS) merge_kernel(const float* __res
 constexpr int LOCAL_MAXC = 1024;    // candidate sections per image
 constexpr int LOCAL_MAXO = 9;       // trial origins per image
 
-// per image: the panel sections whose rotation lies within the angle whose
-// cosine bound is `tr_min` of trace(R_p^T R_s) - in panel order (ordered
-// compaction over 256-section chunks)
-__global__ void __launch_bounds__(256) local_select_kernel(const float* __restrict__ prop, const float* __restrict__ rots,
-                                                           long nsec, float tr_min, long img0,
-                                                           int* __restrict__ cand, int* __restrict__ count) {
-    __shared__ int wsum[8];
-    __shared__ float Rp[9];
+// IMG images per CTA: the panel sections whose rotation lies within the angle
+// whose cosine bound is `tr_min` of trace(R_p^T R_s), in panel order.  rots: nine
+// rows of nsec elements.  The warps take 32 sections each in turn and leave a
+// bit per section and image; then WPI warps per image count their words and
+// write the sections out, a segment of SEL_WORDS words at a time.  Bound by the
+// loads of the rotations: as 36-byte records, one image per CTA and a barrier
+// per 256 sections, 512 images against 68,520 sections took 0.21 ms (now
+// 0.06).
+constexpr int SEL_THREADS = 1024;
+constexpr int SEL_WORDS = 4096;
+
+template <int IMG>
+__global__ void __launch_bounds__(SEL_THREADS) local_select_kernel(const float* __restrict__ prop,
+                                                                   const float* __restrict__ rots, long nsec,
+                                                                   float tr_min, long img0, int nimg, int words,
+                                                                   int* __restrict__ cand, int* __restrict__ count) {
+    constexpr int WARPS = SEL_THREADS / 32, WPI = WARPS / IMG;
+    extern __shared__ unsigned s_bits[];               // IMG x words
+    __shared__ int s_sum[WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long img = img0 + blockIdx.x;
-    if (threadIdx.x < 9) Rp[threadIdx.x] = prop[img * 11 + threadIdx.x];
-    __syncthreads();
-    int base_out = 0;
-    int* my = cand + (long)blockIdx.x * LOCAL_MAXC;
-    for (long c0 = 0; c0 < nsec; c0 += 256) {
-        const long j = c0 + threadIdx.x;
-        bool in = false;
-        if (j < nsec) {
-            const float* r = rots + j * 9;
-            float t = 0.f;
+    const int first = blockIdx.x * IMG;
+    float R[IMG][9];
 #pragma unroll
-            for (int k = 0; k < 9; ++k) t = fmaf(Rp[k], r[k], t);
-            in = t >= tr_min;
+    for (int i = 0; i < IMG; ++i)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) R[i][k] = prop[(img0 + min(first + i, nimg - 1)) * 11 + k];
+    const int mine = warp / WPI, part = warp - mine * WPI;
+    int* out = cand + (long)(first + mine) * LOCAL_MAXC;
+    int base = 0;                                      // sections of earlier segments
+    for (long seg = 0; seg < nsec; seg += 32L * words) {
+        const int here = (int)min((long)words, (nsec - seg + 31) / 32);
+#pragma unroll 2
+        for (int w = warp; w < here; w += WARPS) {
+            const long j = seg + 32L * w + lane;
+            const bool live = j < nsec;
+            float r[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) r[k] = live ? __ldg(rots + k * nsec + j) : 0.f;
+#pragma unroll
+            for (int i = 0; i < IMG; ++i) {
+                float t = 0.f;
+#pragma unroll
+                for (int k = 0; k < 9; ++k) t = fmaf(R[i][k], r[k], t);
+                const unsigned b = __ballot_sync(0xffffffffu, live && t >= tr_min);
+                if (lane == 0) s_bits[i * words + w] = b;
+            }
         }
-        const unsigned b = __ballot_sync(0xffffffffu, in);
-        if (lane == 0) wsum[warp] = __popc(b);
         __syncthreads();
-        int before = 0, total = 0;
-        for (int w = 0; w < 8; ++w) { if (w < warp) before += wsum[w]; total += wsum[w]; }
-        const int pos = base_out + before + __popc(b & ((1u << lane) - 1u));
-        if (in && pos < LOCAL_MAXC) my[pos] = (int)j;
-        base_out += total;
+        const unsigned* bits = s_bits + mine * words;
+        const int per = (here + WPI - 1) / WPI, w0 = min(here, part * per), w1 = min(here, w0 + per);
+        int n = 0;
+        for (int w = w0 + lane; w < w1; w += 32) n += __popc(bits[w]);
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) s_sum[warp] = n;
         __syncthreads();
+        int at = base;
+        for (int q = 0; q < WPI; ++q) {
+            const int v = s_sum[mine * WPI + q];
+            if (q < part) at += v;
+            base += v;
+        }
+        if (n > 0 && first + mine < nimg)
+            for (int wb = w0; wb < w1; wb += 32) {
+                unsigned word = wb + lane < w1 ? bits[wb + lane] : 0u;
+                const int c = __popc(word);
+                int incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                for (int pos = at + incl - c; word && pos < LOCAL_MAXC; ++pos) {
+                    out[pos] = (int)(seg + 32L * (wb + lane) + __ffs(word) - 1);
+                    word &= word - 1;
+                }
+                at += __shfl_sync(0xffffffffu, incl, 31);
+            }
+        __syncthreads();                               // before the next segment's bits
     }
-    if (threadIdx.x == 0) count[blockIdx.x] = base_out;
+    if (part == 0 && lane == 0 && first + mine < nimg) count[first + mine] = base;
 }
 
 __device__ __forceinline__ float2 bf2f(uint32_t u) {
@@ -614,107 +698,149 @@ __device__ __forceinline__ float2 bf2f(uint32_t u) {
 }
 
 // per image: its A rows at its local origins in shared memory (BF16, as
-// rows_kernel writes them), then every candidate section's panel row dotted
-// with each of them by one warp; the topk (section, origin) pairs by score
-// go to the candidate arrays in (score desc, section, origin) order
-__global__ void __launch_bounds__(256) local_score_kernel(
+// rows_kernel writes them), then the candidate sections' panel rows dotted with
+// them, a warp taking two sections and LOCAL_O origins at a time; the topk
+// (section, origin) pairs by score go to the candidate arrays in (score desc,
+// section, origin) order.  A lane's products of one pair are added in the order
+// of the row, whatever the split.  The A rows fill an SM's shared memory for
+// large boxes (115 KB at 128^2 and half the Nyquist frequency), so one CTA has
+// to bring enough warps: 256 threads, one section at a time with all nine
+// origins and a single warp's search for the best pairs took 0.77 ms for 512
+// images of 128^2 (now 0.18).
+constexpr int LOCAL_O = 3;
+constexpr int LOCAL_THREADS = 1024;
+constexpr int LOCAL_SMEM = 227 * 1024 - 512;       // dynamic, beside the picks' 512 bytes (rows of 10,816 values at most)
+
+__global__ void __launch_bounds__(LOCAL_THREADS, 1) local_score_kernel(
     const float2* __restrict__ spec, int D, const float* __restrict__ ctf, int npix, const MPix* __restrict__ cpix,
     int ncpix, int nf, const float* __restrict__ gA, const double2* __restrict__ slopes,
     const int* __restrict__ lorg, const int* __restrict__ nlorg, const int* __restrict__ cand,
     const int* __restrict__ count, const __nv_bfloat16* __restrict__ panel, int kpad, int topk, long img0,
     int* __restrict__ out_sec, int* __restrict__ out_org, float* __restrict__ out_score) {
     extern __shared__ uint4 lsm[];
+    __shared__ unsigned long long best[64];
     const int b = blockIdx.x;
     const long img = img0 + b;
     const int no = nlorg[b];
     const int nc = min(count[b], LOCAL_MAXC);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     __nv_bfloat162* A = reinterpret_cast<__nv_bfloat162*>(lsm);           // no x kpad/2
     float* sc = reinterpret_cast<float*>(A + (size_t)LOCAL_MAXO * (kpad / 2));   // LOCAL_MAXC x LOCAL_MAXO
+    double2* s_slope = reinterpret_cast<double2*>(sc);                    // before the scores
+    if (threadIdx.x < no) s_slope[threadIdx.x] = slopes[lorg[b * LOCAL_MAXO + threadIdx.x]];
+    __syncthreads();
     const float2* X = spec + img * (long)D * D;
     const float* C = ctf + img * (long)npix;
     const float* g = gA + (long)b * nf;
-    for (int o = 0; o < no; ++o) {
-        const double2 sl = slopes[lorg[b * LOCAL_MAXO + o]];
-        for (int p = threadIdx.x; p < kpad / 2; p += blockDim.x) {
+    for (int p = threadIdx.x; p < kpad / 2; p += blockDim.x) {
+        MPix q = {};
+        float2 x = make_float2(0.f, 0.f);
+        float f = 0.f;
+        const bool live = p < ncpix;
+        if (live) {
+            q = cpix[p];
+            x = X[q.idx];
+            f = C[q.pad] * g[q.shell];
+        }
+        for (int o = 0; o < no; ++o) {
             float2 v = make_float2(0.f, 0.f);
-            if (p < ncpix) {
-                const MPix q = cpix[p];
-                const float2 x = X[q.idx];
+            if (live) {
+                const double2 sl = s_slope[o];
                 double phi = q.h * sl.x + q.k * sl.y;
                 phi -= 6.283185307179586 * rint(phi * 0.15915494309189535);
                 float sn, cs;
                 sincosf((float)phi, &sn, &cs);
-                const float f = C[q.pad] * g[q.shell];
                 v = make_float2((x.x * cs - x.y * sn) * f, (x.x * sn + x.y * cs) * f);
             }
             A[(size_t)o * (kpad / 2) + p] = __floats2bfloat162_rn(v.x, v.y);
         }
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = nc * LOCAL_MAXO;
+    for (int e = threadIdx.x; e < n; e += blockDim.x) sc[e] = __int_as_float(0x7fffffff);    // no such origin
+    __syncthreads();
     const uint4* As = reinterpret_cast<const uint4*>(A);
     const int k8 = kpad / 8;                 // 16-byte chunks per row
-    for (int ci = warp; ci < nc; ci += 8) {
-        const int sec = cand[(long)b * LOCAL_MAXC + ci];
-        const uint4* row = reinterpret_cast<const uint4*>(panel + (size_t)sec * kpad);
-        float acc[LOCAL_MAXO];
+    const int og = (no + LOCAL_O - 1) / LOCAL_O, items = (nc + 1) / 2 * og;
+    for (int it = warp; it < items; it += nwarps) {
+        const int pair = it / og, o0 = (it - pair * og) * LOCAL_O;
+        const int c0 = 2 * pair, c1 = min(c0 + 1, nc - 1);
+        const uint4* r0 = reinterpret_cast<const uint4*>(panel + (size_t)cand[(long)b * LOCAL_MAXC + c0] * kpad);
+        const uint4* r1 = reinterpret_cast<const uint4*>(panel + (size_t)cand[(long)b * LOCAL_MAXC + c1] * kpad);
+        float acc[2][LOCAL_O];
 #pragma unroll
-        for (int o = 0; o < LOCAL_MAXO; ++o) acc[o] = 0.f;
+        for (int o = 0; o < LOCAL_O; ++o) acc[0][o] = acc[1][o] = 0.f;
+#pragma unroll 2
         for (int p = lane; p < k8; p += 32) {
-            const uint4 pb = __ldg(row + p);
-            const float2 b0 = bf2f(pb.x), b1 = bf2f(pb.y), b2 = bf2f(pb.z), b3 = bf2f(pb.w);
+            const uint4 p0 = __ldg(r0 + p), p1 = __ldg(r1 + p);
+            const float2 b0[4] = {bf2f(p0.x), bf2f(p0.y), bf2f(p0.z), bf2f(p0.w)};
+            const float2 b1[4] = {bf2f(p1.x), bf2f(p1.y), bf2f(p1.z), bf2f(p1.w)};
 #pragma unroll
-            for (int o = 0; o < LOCAL_MAXO; ++o) {
-                if (o < no) {
-                    const uint4 ab = As[(size_t)o * k8 + p];
-                    const float2 a0 = bf2f(ab.x), a1 = bf2f(ab.y), a2 = bf2f(ab.z), a3 = bf2f(ab.w);
-                    float t = acc[o];
-                    t = fmaf(a0.x, b0.x, t); t = fmaf(a0.y, b0.y, t);
-                    t = fmaf(a1.x, b1.x, t); t = fmaf(a1.y, b1.y, t);
-                    t = fmaf(a2.x, b2.x, t); t = fmaf(a2.y, b2.y, t);
-                    t = fmaf(a3.x, b3.x, t); t = fmaf(a3.y, b3.y, t);
-                    acc[o] = t;
+            for (int o = 0; o < LOCAL_O; ++o) {
+                const uint4 ab = As[(size_t)min(o0 + o, no - 1) * k8 + p];
+                const float2 a[4] = {bf2f(ab.x), bf2f(ab.y), bf2f(ab.z), bf2f(ab.w)};
+                float t = acc[0][o], u = acc[1][o];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    t = fmaf(a[k].x, b0[k].x, t); t = fmaf(a[k].y, b0[k].y, t);
+                    u = fmaf(a[k].x, b1[k].x, u); u = fmaf(a[k].y, b1[k].y, u);
                 }
+                acc[0][o] = t;
+                acc[1][o] = u;
             }
         }
 #pragma unroll
-        for (int o = 0; o < LOCAL_MAXO; ++o) {
-            float t = acc[o];
+        for (int o = 0; o < LOCAL_O; ++o) {
+            float t = acc[0][o], u = acc[1][o];
 #pragma unroll
-            for (int k = 16; k; k >>= 1) t += __shfl_xor_sync(0xffffffffu, t, k);
-            if (lane == 0 && o < no) sc[ci * LOCAL_MAXO + o] = t;
+            for (int k = 16; k; k >>= 1) {
+                t += __shfl_xor_sync(0xffffffffu, t, k);
+                u += __shfl_xor_sync(0xffffffffu, u, k);
+            }
+            if (lane == 0 && o0 + o < no) {
+                sc[c0 * LOCAL_MAXO + o0 + o] = t;
+                if (c1 > c0) sc[c1 * LOCAL_MAXO + o0 + o] = u;
+            }
         }
     }
     __syncthreads();
-    if (warp == 0) {
-        const int n = nc * no;
-        float prev_s = 3.0e38f;
-        long prev_k = -1;
-        for (int t = 0; t < topk; ++t) {
-            float bs = -3.0e38f;
-            long bk = -1;
-            for (int e = lane; e < n; e += 32) {
-                const int ci = e / no, o = e - ci * no;
-                const float v = sc[ci * LOCAL_MAXO + o];
-                const long key = (long)cand[(long)b * LOCAL_MAXC + ci] * LOCAL_MAXO + o;
-                const bool after = v < prev_s || (v == prev_s && key > prev_k);
-                if (!after) continue;
-                if (v > bs || (v == bs && (bk < 0 || key < bk))) { bs = v; bk = key; }
-            }
-            for (int k = 16; k; k >>= 1) {
-                const float os = __shfl_xor_sync(0xffffffffu, bs, k);
-                const long ok = __shfl_xor_sync(0xffffffffu, bk, k);
-                if (ok >= 0 && (os > bs || (os == bs && (bk < 0 || ok < bk)))) { bs = os; bk = ok; }
-            }
-            if (lane == 0) {
-                const long c = img * topk + t;
-                out_sec[c] = bk >= 0 ? (int)(bk / LOCAL_MAXO) : -1;
-                out_org[c] = bk >= 0 ? lorg[b * LOCAL_MAXO + (int)(bk % LOCAL_MAXO)] : -1;
-                out_score[c] = bs;
-            }
-            prev_s = bk >= 0 ? bs : -3.0e38f;
-            prev_k = bk;
+    // A pair as one number that sorts in the order of the picks (the candidates
+    // are in section order), 0 for none; each pick is the largest below the last.
+    auto key = [&](int e) -> unsigned long long {
+        const float v = sc[e];
+        if (!(v >= -3.0e38f && v <= 3.0e38f)) return 0ull;
+        unsigned u = __float_as_uint(v + 0.f);
+        u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;
+        return (unsigned long long)u << 32 | (0xffffffffu - (unsigned)e);
+    };
+    unsigned long long prev = ~0ull;
+    for (int t = 0; t < topk; ++t) {
+        unsigned long long top = 0;
+        for (int e = threadIdx.x; e < n; e += blockDim.x) {
+            const unsigned long long v = key(e);
+            if (v < prev && v > top) top = v;
         }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, top, o);
+            if (v > top) top = v;
+        }
+        if (lane == 0) best[(t & 1) * 32 + warp] = top;
+        __syncthreads();
+        top = lane < nwarps ? best[(t & 1) * 32 + lane] : 0ull;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, top, o);
+            if (v > top) top = v;
+        }
+        if (threadIdx.x == 0) {
+            const long c = img * topk + t;
+            const int e = (int)(0xffffffffu - (unsigned)top);
+            out_sec[c] = top ? cand[(long)b * LOCAL_MAXC + e / LOCAL_MAXO] : -1;
+            out_org[c] = top ? lorg[b * LOCAL_MAXO + e % LOCAL_MAXO] : -1;
+            out_score[c] = top ? sc[e] : -3.0e38f;
+        }
+        prev = top;                                    // (0: nothing is left)
     }
 }
 
@@ -849,14 +975,18 @@ static cudaError_t rescore_candidates(Match& Mr, int topk, const std::vector<dou
         }
     }
     for (long i = 0; i < M->nimg; ++i) {
-        std::vector<int> ord(topk);
-        for (int t = 0; t < topk; ++t) ord[t] = t;
+        int ord[TOPK];
         const long b = i * topk;
-        std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) {
+        auto before = [&](int x, int y) {
             const bool vx = csec[b + x] >= 0, vy = csec[b + y] >= 0;
             if (vx != vy) return vx;
             return cf[b + x] > cf[b + y];
-        });
+        };
+        for (int t = 0; t < topk; ++t) {
+            int j = t;
+            for (; j > 0 && before(t, ord[j - 1]); --j) ord[j] = ord[j - 1];
+            ord[j] = t;
+        }
         for (int t = 0; t < topk; ++t) {
             const long c = b + ord[t];
             double* o = out + (b + t) * BSG_MATCH_RESULT_DOUBLES;
@@ -882,9 +1012,6 @@ extern "C" int bsg_match_set_panel(bsg_match* h, const double* mats, long nsec, 
     if (e != cudaSuccess) return match_fail(BSG_ERR_CUDA, "bsg_match_set_panel: %s", cudaGetErrorString(e));
     std::call_once(g_search_attr, [] {
         g_search_attr_err = cudaFuncSetAttribute(search_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-        if (g_search_attr_err == cudaSuccess)
-            g_search_attr_err = cudaFuncSetAttribute(merge_kernel<unsigned long long>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)sizeof(long long) * MERGE_CACHE);
         if (g_search_attr_err == cudaSuccess)
             g_search_attr_err = cudaFuncSetAttribute(panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     });
@@ -918,7 +1045,8 @@ extern "C" int bsg_match_set_panel(bsg_match* h, const double* mats, long nsec, 
     if (e == cudaSuccess) e = cudaMemcpyAsync(M->d_cstart, M->h_cstart.data(), sizeof(int) * (M->nf + 1), cudaMemcpyHostToDevice, s);
     {
         std::vector<float> rf((size_t)9 * nsec);
-        for (long i = 0; i < 9 * nsec; ++i) rf[i] = (float)mats[i];
+        for (long i = 0; i < nsec; ++i)
+            for (int k = 0; k < 9; ++k) rf[k * nsec + i] = (float)mats[9 * i + k];
         if (e == cudaSuccess) e = cudaMemcpyAsync(M->d_rots, rf.data(), sizeof(float) * rf.size(), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
@@ -1068,7 +1196,7 @@ extern "C" int bsg_match_search(bsg_match* h, const double* origins, int norigin
         const long cnt = std::min(nb, M->nimg - i0);
         const long rows = cnt * norigin;
         cudaEventRecord(ev[0], s);
-        coarse_norm_kernel<<<(unsigned)cnt, 64, 0, s>>>(M->d_spec, M->D, M->d_ctf, (int)M->h_pix.size(), M->d_cpix,
+        coarse_norm_kernel<<<(unsigned)cnt, 256, 0, s>>>(M->d_spec, M->D, M->d_ctf, (int)M->h_pix.size(), M->d_cpix,
                                                          M->d_cstart, nf, i0, M->d_gA);
         rows_kernel<<<(unsigned)rows, 256, 0, s>>>(M->d_spec, M->D, M->d_ctf, (int)M->h_pix.size(), M->d_cpix, M->ncpix,
                                                     nf, M->d_gA, M->d_slopes, norigin, i0, kpad, M->d_A);
@@ -1085,13 +1213,14 @@ extern "C" int bsg_match_search(bsg_match* h, const double* origins, int norigin
         ga.status = M->d_status;
         search_gemm_kernel<<<ga.runs.ctas, GEMM_THREADS, GEMM_SMEM, s>>>(tmA, tmB, ga);
         cudaEventRecord(ev[2], s);
-        const bool cached = stretches * TOPK * norigin <= MERGE_CACHE;
+        // two CTAs of half the threads share an SM (256 images 38 against 45 us, 16 images 29 against 26)
+        const int half = MERGE_MOST / 2, threads = cnt > 148 ? half : MERGE_MOST;
         if (M->nsec * (long)norigin < 0xffffffffL)
-            merge_kernel<unsigned long long><<<(unsigned)cnt, MERGE_THREADS, cached ? sizeof(long long) * MERGE_CACHE : 0, s>>>(
-                M->d_pscore, M->d_pidx, ga.runs, mrows, norigin, topk, i0, cached ? 1 : 0, M->d_csec, M->d_corg, M->d_cscore);
+            merge_kernel<unsigned long long><<<(unsigned)cnt, threads, 0, s>>>(
+                M->d_pscore, M->d_pidx, ga.runs, mrows, norigin, topk, i0, M->d_csec, M->d_corg, M->d_cscore);
         else
-            merge_kernel<wide_t><<<(unsigned)cnt, MERGE_THREADS, 0, s>>>(
-                M->d_pscore, M->d_pidx, ga.runs, mrows, norigin, topk, i0, 0, M->d_csec, M->d_corg, M->d_cscore);
+            merge_kernel<wide_t><<<(unsigned)cnt, half, 0, s>>>(
+                M->d_pscore, M->d_pidx, ga.runs, mrows, norigin, topk, i0, M->d_csec, M->d_corg, M->d_cscore);
         cudaEventRecord(ev[3], s);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaEventSynchronize(ev[3]);
@@ -1163,37 +1292,23 @@ extern "C" int bsg_match_search_local(bsg_match* h, const float* proposals, doub
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(local_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        attr = cudaFuncSetAttribute(local_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LOCAL_SMEM);
+        if (attr == cudaSuccess)
+            attr = cudaFuncSetAttribute(local_select_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(unsigned) * 4 * SEL_WORDS);
     });
     const size_t lsmem = sizeof(__nv_bfloat16) * (size_t)LOCAL_MAXO * M->kpad + sizeof(float) * LOCAL_MAXC * LOCAL_MAXO;
-    if (attr != cudaSuccess || lsmem > 227 * 1024)
+    if (attr != cudaSuccess || lsmem > LOCAL_SMEM)
         return match_fail(BSG_ERR_ARG, "bsg_match_search_local: %d coarse values per row exceed the kernel's shared memory",
                           M->kpad);
     cudaStream_t s = M->stream;
     const long nimg = M->nimg;
     const int nf = M->nf;
-    // local trial origins of each image: those within origin_radius of the
-    // proposed origin (box centre + proposed shift), nearest first, at most 9
+    // (the proposals are on the host too, for the choice of the trial origins)
     std::vector<float> prop((size_t)nimg * 11);
     e = cudaMemcpy(prop.data(), proposals, sizeof(float) * prop.size(),
                    (flags & BSG_DEVICE_PTR) ? cudaMemcpyDeviceToHost : cudaMemcpyHostToHost);
     if (e != cudaSuccess) return match_fail(BSG_ERR_CUDA, "bsg_match_search_local: %s", cudaGetErrorString(e));
-    std::vector<int> lorg((size_t)nimg * LOCAL_MAXO, 0), nlorg(nimg, 0);
-    for (long i = 0; i < nimg; ++i) {
-        const double px = M->n / 2 + prop[i * 11 + 9], py = M->n / 2 + prop[i * 11 + 10];
-        std::vector<std::pair<double, int>> d;
-        for (int o = 0; o < norigin; ++o) {
-            const double dx = origins[2 * o] - px, dy = origins[2 * o + 1] - py;
-            d.push_back({dx * dx + dy * dy, o});
-        }
-        std::stable_sort(d.begin(), d.end());
-        int k = 0;
-        for (auto& t : d) {
-            if (k >= LOCAL_MAXO || (t.first > origin_radius * origin_radius && k > 0)) break;
-            lorg[i * LOCAL_MAXO + k++] = t.second;
-        }
-        nlorg[i] = k;
-    }
     std::vector<double2> sl(norigin);
     for (int i = 0; i < norigin; ++i)
         sl[i] = make_double2(M->cut_scale * origins[2 * i] / M->D * 2 * M_PI, M->cut_scale * origins[2 * i + 1] / M->D * 2 * M_PI);
@@ -1245,22 +1360,60 @@ extern "C" int bsg_match_search_local(bsg_match* h, const float* proposals, doub
     float* d_prop = M->d_lprop;
     int *d_lorg = M->d_lorg, *d_nlorg = M->d_nlorg, *d_cand = M->d_lcand, *d_count = M->d_lcount;
     e = cudaMemcpyAsync(d_prop, prop.data(), sizeof(float) * prop.size(), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_lorg, lorg.data(), sizeof(int) * lorg.size(), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_nlorg, nlorg.data(), sizeof(int) * nimg, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(M->d_slopes, sl.data(), sizeof(double2) * norigin, cudaMemcpyHostToDevice, s);
     const float tr_min = (float)(1.0 + 2.0 * cos(radius));
     cudaEvent_t ev[2];
     cudaEventCreate(&ev[0]);
     cudaEventCreate(&ev[1]);
     cudaEventRecord(ev[0], s);
+    // Four images per CTA once that fills the SMs: the rotations are read once
+    // for them (512 images against 68,520 sections 176 us with one, 61
+    // with four; 64 images 34 and 54).
+    const int words = (int)std::min<long>(SEL_WORDS, (M->nsec + 31) / 32);
+    auto select = [&](long i0, long cnt) {
+        if (cnt > 148)
+            local_select_kernel<4><<<(unsigned)((cnt + 3) / 4), SEL_THREADS, sizeof(unsigned) * 4 * words, s>>>(
+                d_prop, M->d_rots, M->nsec, tr_min, i0, (int)cnt, words, d_cand, d_count);
+        else
+            local_select_kernel<1><<<(unsigned)cnt, SEL_THREADS, sizeof(unsigned) * words, s>>>(
+                d_prop, M->d_rots, M->nsec, tr_min, i0, (int)cnt, words, d_cand, d_count);
+        coarse_norm_kernel<<<(unsigned)cnt, 256, 0, s>>>(M->d_spec, M->D, M->d_ctf, (int)M->h_pix.size(), M->d_cpix,
+                                                         M->d_cstart, nf, i0, M->d_gA);
+        return cudaGetLastError();
+    };
+    if (e == cudaSuccess) e = select(0, std::min(nb, nimg));
+    // meanwhile, the local trial origins of each image: those within
+    // origin_radius of the proposed origin (box centre + proposed shift), nearest
+    // first, at most LOCAL_MAXO
+    std::vector<int> lorg((size_t)nimg * LOCAL_MAXO, 0), nlorg(nimg, 0);
+    for (long i = 0; i < nimg; ++i) {
+        const double px = M->n / 2 + prop[i * 11 + 9], py = M->n / 2 + prop[i * 11 + 10];
+        double d[LOCAL_MAXO];
+        int* at = &lorg[i * LOCAL_MAXO];
+        int k = 0;
+        for (int o = 0; o < norigin; ++o) {
+            const double dx = origins[2 * o] - px, dy = origins[2 * o + 1] - py, v = dx * dx + dy * dy;
+            if (k == LOCAL_MAXO && !(v < d[k - 1])) continue;
+            int j = k < LOCAL_MAXO ? k++ : k - 1;
+            for (; j > 0 && v < d[j - 1]; --j) { d[j] = d[j - 1]; at[j] = at[j - 1]; }
+            d[j] = v;
+            at[j] = o;
+        }
+        int within = 1;
+        while (within < k && !(d[within] > origin_radius * origin_radius)) ++within;
+        for (int j = within; j < k; ++j) at[j] = 0;
+        nlorg[i] = within;
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_lorg, lorg.data(), sizeof(int) * lorg.size(), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_nlorg, nlorg.data(), sizeof(int) * nimg, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(M->d_slopes, sl.data(), sizeof(double2) * norigin, cudaMemcpyHostToDevice, s);
     long launches = 0, considered = 0;
     std::vector<int> cnt_h(nb);
+    // (as many threads as an SM's registers hold beside what its shared memory does)
+    const int threads = lsmem > 75 * 1024 ? LOCAL_THREADS : LOCAL_THREADS / 2;
     for (long i0 = 0; e == cudaSuccess && i0 < nimg; i0 += nb) {
         const long cnt = std::min(nb, nimg - i0);
-        local_select_kernel<<<(unsigned)cnt, 256, 0, s>>>(d_prop, M->d_rots, M->nsec, tr_min, i0, d_cand, d_count);
-        coarse_norm_kernel<<<(unsigned)cnt, 64, 0, s>>>(M->d_spec, M->D, M->d_ctf, (int)M->h_pix.size(), M->d_cpix,
-                                                         M->d_cstart, nf, i0, M->d_gA);
-        local_score_kernel<<<(unsigned)cnt, 256, lsmem, s>>>(
+        if (i0 > 0 && (e = select(i0, cnt)) != cudaSuccess) break;
+        local_score_kernel<<<(unsigned)cnt, threads, lsmem, s>>>(
             M->d_spec, M->D, M->d_ctf, (int)M->h_pix.size(), M->d_cpix, M->ncpix, nf, M->d_gA, M->d_slopes,
             d_lorg + i0 * LOCAL_MAXO, d_nlorg + i0, d_cand, d_count, M->d_panel, M->kpad, topk, i0, M->d_csec,
             M->d_corg, M->d_cscore);

@@ -1,6 +1,6 @@
 """The search's division of row tiles and panel tiles over the SMs: batches of
 one to twenty row tiles (even groups, sevens and fours, a ragged last batch),
-panels of one to several tiles, merges in and beyond shared memory.  How the
+panels of one to several tiles, merges of few and many candidates.  How the
 work is cut changes no bit, so every division gives the one-image batches'
 result, and the best candidate's correlation is the FP64 one's to BF16 rounding
 (tested elsewhere)."""
@@ -15,7 +15,9 @@ pytestmark = pytest.mark.gpu
     (7, 25, 700),      # two row tiles, three panel tiles
     (96, 25, 700),     # 19 row tiles
     (104, 25, 1100),   # 21: three sevens
-    (12, 49, 3000),    # more candidates an image than shared memory holds
+    (12, 49, 3000),    # many candidates an image
+    (5, 25, 38000),    # one row tile over every SM, more panel tiles than stretches
+    (150, 9, 300),     # merges of two CTAs per SM
 ])
 def test_divisions_agree(nimg, norigin, nsec):
     from bsoft_b200.match import Matcher, ctf_record
