@@ -121,16 +121,133 @@ __global__ void __launch_bounds__(SWL * 32) strided64_kernel(double2* data, int 
     }
 }
 
-// real values -> complex (float)(v * scale[b] + shift[b]) (the rescaled
-// image is stored as float, Bimage_rescale.cpp:41-44); scale/shift per image
-// b of `per` values (NULL: 1 and 0)
-__global__ void to_complex_kernel(const float* __restrict__ in, double2* __restrict__ out, long count, long per,
-                                  const double* __restrict__ scale, const double* __restrict__ shift) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count; i += (long)gridDim.x * blockDim.x) {
-        double v = in[i];
-        if (scale) { const long b = i / per; v = v * scale[b] + shift[b]; }
-        out[i] = make_double2((double)(float)v, 0.0);
+__global__ void to_complex_kernel(const float* __restrict__ in, double2* __restrict__ out, long count) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count; i += (long)gridDim.x * blockDim.x)
+        out[i] = make_double2((double)in[i], 0.0);
+}
+
+__device__ __forceinline__ int crop_src(int xx, int nu, int size) { return xx > (nu - 1) / 2 ? xx + size - nu : xx; }
+// crop_src's inverse: the cut transform's index of index i of the full one, -1 outside the cut
+__device__ __forceinline__ int crop_dst(int i, int nu, int size) {
+    if (i <= (nu - 1) / 2) return i;
+    const int xx = i - size + nu;
+    return xx > (nu - 1) / 2 ? xx : -1;
+}
+
+// The images' transforms, rows then columns, as warp_fft64's stages taken two
+// at a time in registers: the same products and sums, so the same bits.  The
+// first pass reads its four inputs from global memory (bit-reversed order is a
+// permutation of consecutive quarter lines), the last one writes the cut
+// transform only, so the rows leave D of n columns and the columns' CTAs run
+// on those D.  Bound by the FP64 traffic through shared memory and L2: with
+// whole lines in bit-reversed order, a pass per stage, and separate passes for
+// the conversion and the cut, 512 images of 128^2 (cut to 118^2) took 0.41 ms,
+// now 0.12.
+__device__ __forceinline__ void two_stages(double2* v, double2 w1, double2 w2, double2 w3) {
+    const double2 t1 = zmul(v[1], w1), t3 = zmul(v[3], w1);
+    const double2 a = make_double2(v[0].x + t1.x, v[0].y + t1.y), b = make_double2(v[0].x - t1.x, v[0].y - t1.y);
+    const double2 c = make_double2(v[2].x + t3.x, v[2].y + t3.y), d = make_double2(v[2].x - t3.x, v[2].y - t3.y);
+    const double2 tc = zmul(c, w2), td = zmul(d, w3);
+    v[0] = make_double2(a.x + tc.x, a.y + tc.y);
+    v[2] = make_double2(a.x - tc.x, a.y - tc.y);
+    v[1] = make_double2(b.x + td.x, b.y + td.y);
+    v[3] = make_double2(b.x - td.x, b.y - td.y);
+}
+
+// One line's passes by `step` threads (this one the first-th): load(i) gives
+// input i, buf(i) is the line's element i in shared memory, store(i, value)
+// takes output i, sync() separates passes.  L a power of two >= 8.
+template <class Load, class Buf, class Store, class Sync>
+__device__ __forceinline__ void line_passes(int L, int logL, const double2* tw, int first, int step, Load&& load,
+                                            Buf&& buf, Store&& store, Sync&& sync) {
+    const int quarter = L >> 2;
+    for (int q = first; q < quarter; q += step) {
+        const int r = bitrev(q, logL - 2);
+        double2 v[4] = {load(r), load(r + 2 * quarter), load(r + quarter), load(r + 3 * quarter)};
+        two_stages(v, tw[0], tw[0], tw[quarter]);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) buf(4 * q + m) = v[m];
     }
+    sync();
+    int s = 3;
+    for (; s < logL; s += 2) {
+        const int h = 1 << (s - 1);
+        const bool last = s + 1 == logL;
+        for (int q = first; q < quarter; q += step) {
+            const int j = q & (h - 1), i = ((q >> (s - 1)) << (s + 1)) + j;
+            double2 v[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) v[m] = buf(i + m * h);
+            two_stages(v, tw[j * (L >> s)], tw[j * (L >> (s + 1))], tw[(j + h) * (L >> (s + 1))]);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                if (last) store(i + m * h, v[m]);
+                else buf(i + m * h) = v[m];
+            }
+        }
+        if (!last) sync();
+    }
+    if (s == logL)
+        for (int j = first; j < L / 2; j += step) {
+            const double2 u = buf(j), t = zmul(buf(j + L / 2), tw[j]);
+            store(j, make_double2(u.x + t.x, u.y + t.y));
+            store(j + L / 2, make_double2(u.x - t.x, u.y - t.y));
+        }
+}
+
+// rows: (float)(v * scale + shift) per image (the rescaled image is stored as
+// float, Bimage_rescale.cpp:41-44), a warp per row; elements 8 i + 0..7 are
+// padded by one so that the first pass's stores do not collide
+constexpr int IRW = 4;
+__global__ void __launch_bounds__(IRW * 32) img_rows64_kernel(const float* __restrict__ img,
+                                                              const double* __restrict__ scale,
+                                                              const double* __restrict__ shift, long nlines, int n,
+                                                              int logn, int D, const double2* __restrict__ tw,
+                                                              double2* __restrict__ out) {
+    extern __shared__ double2 zsm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double2* stw = zsm;
+    double2* line_buf = zsm + n / 2 + warp * (n + n / 8);
+    for (int i = threadIdx.x; i < n / 2; i += blockDim.x) stw[i] = tw[i];
+    __syncthreads();
+    const long line = (long)blockIdx.x * IRW + warp;
+    if (line >= nlines) return;
+    const float* p = img + line * n;
+    const double sc = scale[line / n], sh = shift[line / n];
+    line_passes(
+        n, logn, stw, lane, 32,
+        [&](int i) { const double v = p[i]; return make_double2((double)(float)(v * sc + sh), 0.0); },
+        [&](int i) -> double2& { return line_buf[i + (i >> 3)]; },
+        [&](int i, double2 v) {
+            const int c = crop_dst(i, D, n);
+            if (c >= 0) out[line * D + c] = v;
+        },
+        [] { __syncwarp(); });
+}
+
+// columns of the cut rows, eight per CTA (consecutive in shared memory and in
+// the rows); rounded to float, the zero-frequency term cleared
+constexpr int ICL = 8;
+__global__ void __launch_bounds__(ICL * 32) img_cols64_kernel(const double2* __restrict__ rows, int n, int logn, int D,
+                                                              const double2* __restrict__ tw,
+                                                              float2* __restrict__ out) {
+    extern __shared__ double2 zsm[];
+    double2* stw = zsm;
+    double2* tile = zsm + n / 2;
+    for (int i = threadIdx.x; i < n / 2; i += blockDim.x) stw[i] = tw[i];
+    const int c = threadIdx.x % ICL, x = blockIdx.x * ICL + c;
+    const double2* src = rows + (long)blockIdx.y * n * D;
+    float2* dst = out + (long)blockIdx.y * D * D;
+    __syncthreads();
+    line_passes(
+        n, logn, stw, threadIdx.x / ICL, 32,
+        [&](int i) { return x < D ? src[(long)i * D + x] : make_double2(0.0, 0.0); },
+        [&](int i) -> double2& { return tile[i * ICL + c]; },
+        [&](int i, double2 v) {
+            const int y = crop_dst(i, D, n);
+            if (x < D && y >= 0) dst[(long)y * D + x] = x == 0 && y == 0 ? make_float2(0.f, 0.f) : make_float2((float)v.x, (float)v.y);
+        },
+        [] { __syncthreads(); });
 }
 
 // per-image population statistics (Bimage::statistics(long)) -> the
@@ -157,8 +274,6 @@ __global__ void __launch_bounds__(256) image_stats_kernel(const float* __restric
         shift[blockIdx.x] = -avg * sc;
     }
 }
-
-__device__ __forceinline__ int crop_src(int xx, int nu, int size) { return xx > (nu - 1) / 2 ? xx + size - nu : xx; }
 
 // full N^3 transform -> cut diam^3, x norm, zero-frequency term cleared,
 // phase shift exp(i (h sx + k sy + l sz)) in FP64 (Bimage_complex.cpp:490-534)
@@ -260,47 +375,79 @@ __global__ void proj_real_kernel(const double2* __restrict__ in, long count, dou
         out[i] = (float)(in[i].x * norm);
 }
 
-// full n^2 transforms -> cut diam^2 with the zero-frequency term cleared
-__global__ void img_cut_kernel(const double2* __restrict__ full, int n, int D, long nimg, float2* __restrict__ out) {
-    const long per = (long)D * D, total = per * nimg;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const long b = i / per;
-        const int x = (int)(i % D), y = (int)((i % per) / D);
-        const double2 f = full[(size_t)b * n * n + (size_t)crop_src(y, D, n) * n + crop_src(x, D, n)];
-        float2 v = make_float2((float)f.x, (float)f.y);
-        if (x == 0 && y == 0) v = make_float2(0.f, 0.f);
-        out[i] = v;
+// sin and cos of twice each pixel's angle, which the CTF's astigmatism needs
+// (they were evaluated per image: two thirds of img_shells_kernel's FP64 work)
+__global__ void pix_angle_kernel(const MPix* __restrict__ pix, int npix, double2* __restrict__ out) {
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
+        const double a = atan2((double)pix[p].k, (double)pix[p].h);
+        out[p] = make_double2(sin(2 * a), cos(2 * a));
     }
 }
 
-
 // per image: CTF at the figure-of-merit pixels (ctf.h:321-365 with
-// s = index / (n * pixel)) and the image power per shell (fixed order)
+// s = index / (n * pixel)) and the image power per shell (fixed order).  The
+// pixels' CTF is split over gridDim.y CTAs; in the first one all threads fetch
+// the powers, SHELL_PIX at a time, and a thread per shell adds them in pixel
+// order (512 images of 128^2 0.12 -> 0.06 ms with pix_angle_kernel's table,
+// 16 images 70 -> 30 us).
+constexpr int SHELL_PIX = 1024;
+constexpr int SHELL_SLOTS = 2;       // shells per thread and pass
+
 __global__ void __launch_bounds__(256) img_shells_kernel(const float2* __restrict__ spec, int D,
-                                                         const MPix* __restrict__ pix, int npix,
+                                                         const MPix* __restrict__ pix,
+                                                         const double2* __restrict__ angle, int npix,
                                                          const int* __restrict__ shell_start, int nshell,
                                                          const ImgCtf* __restrict__ ctf, double fs,
                                                          float* __restrict__ ctf_out, double* __restrict__ dsum) {
+    __shared__ double term[SHELL_PIX];
     const long b = blockIdx.x;
     const float2* X = spec + b * (long)D * D;
-    const ImgCtf C = ctf[b];
-    for (int p = threadIdx.x; p < npix; p += blockDim.x) ctf_out[b * npix + p] = ctf_factor(C, pix[p], fs);
-    for (int j = threadIdx.x; j < nshell; j += blockDim.x) {
-        double d = 0;
-        for (int p = shell_start[j]; p < shell_start[j + 1]; ++p) {
-            const float2 x = X[pix[p].idx];
-            d += (double)x.x * x.x + (double)x.y * x.y;
+    if (blockIdx.y == 0)
+        for (int j0 = 0; j0 < nshell; j0 += 256 * SHELL_SLOTS) {
+            const int total = shell_start[nshell];
+            int lo[SHELL_SLOTS], hi[SHELL_SLOTS];
+            double d[SHELL_SLOTS];
+#pragma unroll
+            for (int i = 0; i < SHELL_SLOTS; ++i) {
+                const int j = j0 + threadIdx.x + 256 * i;
+                lo[i] = j < nshell ? shell_start[j] : 0;
+                hi[i] = j < nshell ? shell_start[j + 1] : 0;
+                d[i] = 0;
+            }
+            for (int p0 = 0; p0 < total; p0 += SHELL_PIX) {
+                const int m = min(SHELL_PIX, total - p0);
+#pragma unroll 4
+                for (int p = threadIdx.x; p < m; p += 256) {
+                    const float2 x = X[pix[p0 + p].idx];
+                    term[p] = (double)x.x * x.x + (double)x.y * x.y;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int i = 0; i < SHELL_SLOTS; ++i) {
+                    const int p1 = min(hi[i] - p0, m);
+#pragma unroll 8
+                    for (int p = max(lo[i] - p0, 0); p < p1; ++p) d[i] += term[p];
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int i = 0; i < SHELL_SLOTS; ++i) {
+                const int j = j0 + threadIdx.x + 256 * i;
+                if (j < nshell) dsum[b * nshell + j] = d[i];
+            }
         }
-        dsum[b * nshell + j] = d;
-    }
+    const ImgCtf C = ctf[b];
+    for (int p = blockIdx.y * 256 + threadIdx.x; p < npix; p += 256 * gridDim.y)
+        ctf_out[b * npix + p] = ctf_factor(C, pix[p], angle[p], fs);
 }
 
 // CTF rows for arbitrary records (the refinement's defocus trials)
 __global__ void __launch_bounds__(256) ctf_rows_kernel(const ImgCtf* __restrict__ rec, const MPix* __restrict__ pix,
-                                                       int npix, double fs, float* __restrict__ out) {
+                                                       const double2* __restrict__ angle, int npix, double fs,
+                                                       float* __restrict__ out) {
     const long b = blockIdx.x;
     const ImgCtf C = rec[b];
-    for (int p = threadIdx.x; p < npix; p += blockDim.x) out[b * npix + p] = ctf_factor(C, pix[p], fs);
+    for (int p = threadIdx.x; p < npix; p += blockDim.x) out[b * npix + p] = ctf_factor(C, pix[p], angle[p], fs);
 }
 
 // central sections for output: one CTA per view over the pixel list of the
@@ -753,6 +900,7 @@ cudaError_t g_attr_err = cudaSuccess;
 void set_attributes() {
     const int big = 100 * 1024;
     cudaError_t e = cudaFuncSetAttribute(strided64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(img_cols64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(fom_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e == cudaSuccess)
@@ -924,6 +1072,7 @@ extern "C" int bsg_match_create(const bsg_match_config* cfg, bsg_match** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&M->stream, cudaStreamNonBlocking);
 #define ALLOC(p, bytes) if (e == cudaSuccess) e = cudaMalloc((void**)&(p), (bytes))
     ALLOC(M->d_pix, sizeof(MPix) * std::max<size_t>(1, M->h_pix.size()));
+    ALLOC(M->d_pixang, sizeof(double2) * std::max<size_t>(1, M->h_pix.size()));
     ALLOC(M->d_shell_start, sizeof(int) * M->h_shell_start.size());
     ALLOC(M->d_secpix, sizeof(MPix) * std::max<size_t>(1, M->h_secpix.size()));
     ALLOC(M->d_lut, sizeof(double) * lut.size());
@@ -935,7 +1084,13 @@ extern "C" int bsg_match_create(const bsg_match_config* cfg, bsg_match** out) {
 #undef ALLOC
     if (e == cudaSuccess)
         e = cudaMemcpy(M->d_wshell, M->h_wshell.data(), sizeof(double) * M->h_wshell.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(M->d_pix, M->h_pix.data(), sizeof(MPix) * M->h_pix.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(M->d_pix, M->h_pix.data(), sizeof(MPix) * M->h_pix.size(), cudaMemcpyHostToDevice, M->stream);
+    if (e == cudaSuccess && !M->h_pix.empty()) {
+        pix_angle_kernel<<<(unsigned)((M->h_pix.size() + 255) / 256), 256, 0, M->stream>>>(M->d_pix, (int)M->h_pix.size(),
+                                                                                           M->d_pixang);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess)
         e = cudaMemcpy(M->d_shell_start, M->h_shell_start.data(), sizeof(int) * M->h_shell_start.size(),
                        cudaMemcpyHostToDevice);
@@ -961,7 +1116,7 @@ extern "C" void bsg_match_destroy(bsg_match* h) {
     if (!M) return;
     cudaSetDevice(M->device);
     if (M->stream) cudaStreamSynchronize(M->stream);
-    void* ptrs[] = {M->d_pix, M->d_shell_start, M->d_secpix, M->d_lut, M->d_lutf, M->d_tw_map, M->d_tw_img, M->d_ref, M->d_refpad,
+    void* ptrs[] = {M->d_pix, M->d_pixang, M->d_shell_start, M->d_secpix, M->d_lut, M->d_lutf, M->d_tw_map, M->d_tw_img, M->d_ref, M->d_refpad,
                     M->d_spec, M->d_ctf, M->d_dsum, M->d_real, M->d_work, M->d_scale, M->d_shift, M->d_ictf,
                     M->d_hyp, M->d_out, M->d_full, M->d_grp, M->d_gout, M->d_rmats, M->d_rsec, M->d_rctf, M->d_rrec, M->d_cpix, M->d_cstart, M->d_secs, M->d_panel, M->d_A, M->d_pscore,
                     M->d_pidx, M->d_csec, M->d_corg, M->d_cscore, M->d_rots, M->d_gA, M->d_slopes,
@@ -1009,7 +1164,7 @@ extern "C" int bsg_match_set_reference(bsg_match* h, const float* map, const dou
         MCK(cudaMemcpyAsync(M->d_real, map, sizeof(float) * n3, cudaMemcpyHostToDevice, s));
         src = M->d_real;
     }
-    to_complex_kernel<<<148 * 8, 256, 0, s>>>(src, M->d_work, (long)n3, (long)n3, nullptr, nullptr);
+    to_complex_kernel<<<148 * 8, 256, 0, s>>>(src, M->d_work, (long)n3);
     MCK(cudaGetLastError());
     // 3-D forward transform: x lines, then y and z as strided lines
     const int logN = ilog2i(N);
@@ -1314,7 +1469,7 @@ cudaError_t launch_panel_exact(const Match& M, const MHyp* d_secs, long nsec, fl
 
 cudaError_t launch_ctf_rows(const Match& M, const ImgCtf* d_rec, long nrec, float* d_out, cudaStream_t s) {
     if (nrec > 0)
-        ctf_rows_kernel<<<(unsigned)nrec, 256, 0, s>>>(d_rec, M.d_pix, (int)M.h_pix.size(), 1.0 / M.real_img, d_out);
+        ctf_rows_kernel<<<(unsigned)nrec, 256, 0, s>>>(d_rec, M.d_pix, M.d_pixang, (int)M.h_pix.size(), 1.0 / M.real_img, d_out);
     return cudaGetLastError();
 }
 
@@ -1543,15 +1698,20 @@ extern "C" int bsg_match_set_images(bsg_match* h, const float* images, long nimg
             image_stats_kernel<<<(unsigned)cnt, 256, 0, s>>>(src, (int)n2, M->d_scale + b0, M->d_shift + b0);
             MCK(cudaGetLastError());
         }
-        to_complex_kernel<<<148 * 8, 256, 0, s>>>(src, M->d_work, n2 * cnt, n2, M->d_scale + b0, M->d_shift + b0);
+        const int logn = ilog2i(n);
+        img_rows64_kernel<<<(unsigned)((n * cnt + IRW - 1) / IRW), IRW * 32,
+                            sizeof(double2) * (n / 2 + IRW * (n + n / 8)), s>>>(
+            src, M->d_scale + b0, M->d_shift + b0, n * cnt, n, logn, D, M->d_tw_img, M->d_work);
         MCK(cudaGetLastError());
-        MCK(fft2_forward(M->d_work, n, cnt, M->d_tw_img, s));
-        img_cut_kernel<<<148 * 8, 256, 0, s>>>(M->d_work, n, D, cnt, M->d_spec + (size_t)b0 * D * D);
+        img_cols64_kernel<<<dim3((unsigned)((D + ICL - 1) / ICL), (unsigned)cnt), ICL * 32,
+                            sizeof(double2) * (n / 2 + ICL * n), s>>>(M->d_work, n, logn, D, M->d_tw_img,
+                                                                      M->d_spec + (size_t)b0 * D * D);
         MCK(cudaGetLastError());
-        img_shells_kernel<<<(unsigned)cnt, 256, 0, s>>>(M->d_spec + (size_t)b0 * D * D, D, M->d_pix, npix,
-                                                         M->d_shell_start, M->nshell, M->d_ictf + b0,
-                                                         1.0 / M->real_img, M->d_ctf + (size_t)b0 * npix,
-                                                         M->d_dsum + (size_t)b0 * M->nshell);
+        // (as many CTAs as the SMs hold for a few images)
+        const unsigned parts = (unsigned)std::max(1L, std::min((npix + 255L) / 256, 592 / cnt));
+        img_shells_kernel<<<dim3((unsigned)cnt, parts), 256, 0, s>>>(
+            M->d_spec + (size_t)b0 * D * D, D, M->d_pix, M->d_pixang, npix, M->d_shell_start, M->nshell, M->d_ictf + b0,
+            1.0 / M->real_img, M->d_ctf + (size_t)b0 * npix, M->d_dsum + (size_t)b0 * M->nshell);
         MCK(cudaGetLastError());
         if (!(flags & BSG_DEVICE_PTR)) MCK(cudaStreamSynchronize(s));   // staging reuse
     }

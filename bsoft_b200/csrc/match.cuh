@@ -168,14 +168,14 @@ struct ImgCtf {
 
 // sin(chi) of one figure-of-merit pixel (img_recip_space_fom's CTF factor,
 // mg_refine.cpp:700-740; chi as CTFparam::calculate_aberration_even,
-// ctf.h:321-334); 1 when the record does not apply
-__device__ __forceinline__ float ctf_factor(const ImgCtf& C, const MPix& q, double fs) {
+// ctf.h:321-334); 1 when the record does not apply.  angle: sin, cos of twice
+// the pixel's angle atan2(k, h)
+__device__ __forceinline__ float ctf_factor(const ImgCtf& C, const MPix& q, double2 angle, double fs) {
     if (!C.apply) return 1.f;
     double sx2 = (C.fsx > 0 ? C.fsx : fs) * q.h; sx2 *= sx2;
     double sy2 = (C.fsy > 0 ? C.fsy : fs) * q.k; sy2 *= sy2;
     const double s2 = sx2 + sy2;
-    const double a = atan2((double)q.k, (double)q.h);
-    const double chi = C.c[0] + s2 * (C.c[3] * sin(2 * a) + C.c[1] + C.c[2] * cos(2 * a)) + s2 * s2 * C.c[4];
+    const double chi = C.c[0] + s2 * (C.c[3] * angle.x + C.c[1] + C.c[2] * angle.y) + s2 * s2 * C.c[4];
     double s = sin(chi);
     if (C.invert) s = -s;
     return (float)s;
@@ -206,6 +206,7 @@ struct Match {
     std::vector<int> h_shell_start;
     std::vector<MPix> h_secpix;        // section pixels
     MPix* d_pix = nullptr;
+    double2* d_pixang = nullptr;       // sin, cos of twice the pixels' angles
     int* d_shell_start = nullptr;
     MPix* d_secpix = nullptr;
     double* d_lut = nullptr;           // FSI table, FP64 (sections output)
