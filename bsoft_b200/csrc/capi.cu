@@ -338,12 +338,21 @@ static int upload_params(Recon* r, int buf, const double* params, long np) {
     // least ft/2 pixel steps from the origin, and no pixel lies beyond the
     // transform's corner, ft/2 sqrt(2) steps
     {
-        double smin = 1e300, smax = 0;
+        const double hf = r->g.ft / 2.0;
+        double smin = 1e300, smax = 0, far = 0;
         for (long i = 0; i < np; ++i) {
             smin = std::min(smin, (double)hp[i].step);
             smax = std::max(smax, (double)hp[i].step);
+            // the farther corner, |ad +- bd| hf (symmetry copies' are the same)
+            double aa = 0, bb = 0, ab = 0;
+            for (int k = 0; k < 3; ++k) {
+                aa += hp[i].ad[k] * hp[i].ad[k];
+                bb += hp[i].bd[k] * hp[i].bd[k];
+                ab += hp[i].ad[k] * hp[i].bd[k];
+            }
+            far = std::max(far, hf * sqrt(aa + bb + 2.0 * fabs(ab)) + hp[i].ezmax);
         }
-        const double hf = r->g.ft / 2.0;
+        r->rmax = (float)(far * (1.0 + 1e-5) + 2.0);     // (a tent's corner lies sqrt(3) away at most)
         r->edge_rmin = np ? hf * smin * (1.0 - 1e-6) - 1e-3 : 0.0;
         r->edge_rmax = hf * smax * 1.4142136 * (1.0 + 1e-6) + 2.0;
     }

@@ -68,6 +68,7 @@ struct Context {
     double2* d_evol[2] = {nullptr, nullptr};   // half-space: unpaired pixels' sums below zsplit (zsplit N^2)
     double* d_ew[2] = {nullptr, nullptr};
     double edge_rmin = 0, edge_rmax = 0;       // current batch: unpaired pixels' least |m|, any pixel's largest
+    float rmax = 0;                            // current batch: no pixel's tent reaches farther from the origin (voxels)
     void* d_part_sums = nullptr;     // replica partial sums (replicas > 1): float per tile, FOM path double per map
     unsigned* d_arrived = nullptr;   // replicas of each tile that are done (grid4_kernel)
     int* d_status = nullptr;         // device view of h_status (mapped)

@@ -55,14 +55,16 @@ struct InsertArgs {
     int ntx, nty, ntz;         // tiles per axis
     const int* order;          // tile visiting order (heaviest first)
     int R;                     // replicas per tile (each takes a slice of the particles)
+    int nlow;                  // tiles below the split (grid4_kernel)
     float* psum;               // R > 1: replica partial sums, tiles x R x 3 x tile voxels
     unsigned* arrived;         // per tile: replicas done (bits 0-7) and which stored sums (8 + rep)
     double* fsum;              // FOM path, R > 1: replica partial sums, R x 5 x N^3
     int zsplit;                // > 0: half-space gridding (walk_edges)
     double2* evol;             // half-space: unpaired pixels' sums below zsplit (zsplit x N^2)
     double* ew;
-    double edge_rmin;          // unpaired pixels lie at least this far from the origin (voxels)
-    double edge_rmax;          // and no pixel farther than this
+    float edge_rmin;           // unpaired pixels lie at least this far from the origin (voxels)
+    float edge_rmax;           // and no pixel farther than this
+    float rmax;                // nor, with its tent and an Ewald surface's curvature, than this
     int interp;
     double maxs2, mins2, mscale;
     double2* vol;
@@ -71,15 +73,32 @@ struct InsertArgs {
     double* w2;
 };
 
-// Does the record's plane come within reach of the tile for alias
-// combination a (bit i set: axis i shifted by -N)?  Bitmask over the 8.
+// The alias combinations (bit i: axis i shifted by -N) under which a pixel at
+// most rmax voxels from the origin can reach the tile: for most tiles one or two
+// of the eight that tile_mask then has to test for every record.
 template <int TX, int TY, int TZ>
-__device__ __forceinline__ unsigned tile_mask(const TileTest& t, int x0, int y0, int z0, int N) {
+__device__ __forceinline__ unsigned tile_aliases(int x0, int y0, int z0, int N, float rmax) {
+    const float ex = 0.5f * (TX - 1), ey = 0.5f * (TY - 1), ez = 0.5f * (TZ - 1);
+    unsigned set = 0;
+    for (int a = 0; a < 8; ++a) {
+        const float dx = fmaxf(0.f, fabsf(x0 - ((a & 1) ? N : 0) + ex) - ex);
+        const float dy = fmaxf(0.f, fabsf(y0 - ((a & 2) ? N : 0) + ey) - ey);
+        const float dz = fmaxf(0.f, fabsf(z0 - ((a & 4) ? N : 0) + ez) - ez);
+        if (dx * dx + dy * dy + dz * dz <= rmax * rmax) set |= 1u << a;
+    }
+    return set;
+}
+
+// Does the record's plane come within reach of the tile for the alias
+// combinations in `aliases`?  Bitmask over the 8.
+template <int TX, int TY, int TZ>
+__device__ __forceinline__ unsigned tile_mask(const TileTest& t, unsigned aliases, int x0, int y0, int z0, int N) {
     unsigned mask = 0;
     const float ex = 0.5f * (TX - 1), ey = 0.5f * (TY - 1), ez = 0.5f * (TZ - 1);
     const float slack = t.slab + fabsf(t.n[0]) * ex + fabsf(t.n[1]) * ey + fabsf(t.n[2]) * ez;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
+#pragma unroll 1
+    for (unsigned left = aliases; left; left &= left - 1) {
+        const int a = __ffs(left) - 1;
         const float cx = x0 - ((a & 1) ? N : 0) + ex;
         const float cy = y0 - ((a & 2) ? N : 0) + ey;
         const float cz = z0 - ((a & 4) ? N : 0) + ez;
@@ -564,20 +583,20 @@ __device__ __forceinline__ unsigned edge_mask(const DevParticle& P, unsigned mas
 }
 
 // Can an unpaired pixel (at least rmin voxels from the origin, and no pixel
-// beyond rmax) reach the tile, under some wrap-around alias?
+// beyond rmax) reach the tile, under some wrap-around alias?  (FP32 with a
+// margin: a superset.)
 template <int TX, int TY, int TZ>
-__device__ __forceinline__ bool tile_reaches_edges(int x0, int y0, int z0, int N, double rmin, double rmax) {
+__device__ __forceinline__ bool tile_reaches_edges(int x0, int y0, int z0, int N, float rmin, float rmax) {
     const int o[3] = {x0, y0, z0}, T[3] = {TX, TY, TZ};
     for (int a = 0; a < 8; ++a) {
-        double nr = 0, fr = 0;
+        float nr = 0, fr = 0;
         for (int i = 0; i < 3; ++i) {
-            const double lo = o[i] - (((a >> i) & 1) ? N : 0) - 1.0, hi = lo + T[i] + 1.0;
-            const double n = (lo <= 0 && hi >= 0) ? 0.0 : fmin(fabs(lo), fabs(hi));
-            const double f = fmax(fabs(lo), fabs(hi));
+            const float lo = o[i] - (((a >> i) & 1) ? N : 0) - 1.0f, hi = lo + T[i] + 1.0f;
+            const float n = fmaxf(0.f, fmaxf(lo, -hi)), f = fmaxf(fabsf(lo), fabsf(hi));
             nr += n * n;
             fr += f * f;
         }
-        if (nr <= rmax * rmax && fr >= rmin * rmin) return true;
+        if (nr <= rmax * rmax * 1.00001f && fr * 1.00001f >= rmin * rmin) return true;
     }
     return false;
 }
@@ -649,12 +668,13 @@ __global__ void __launch_bounds__(WARPS * 32) insert_kernel(InsertArgs a) {
     for (int i = lane; i < NCH * TV; i += 32) my_acc[i] = 0;
     __syncwarp();
 
+    const unsigned aliases = tile_aliases<TX, TY, TZ>(x0, y0, z0, N, a.rmax);
     for (int base = p_lo; base < p_hi; base += 32) {
         const int p = base + lane;
         unsigned mask = 0;
         if (p < p_hi) {
             const TileTest t = a.test[p];
-            if (t.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(t, x0, y0, z0, N);
+            if (t.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(t, aliases, x0, y0, z0, N);
         }
         unsigned todo = __ballot_sync(0xffffffffu, mask != 0);
         while (todo) {
@@ -734,6 +754,7 @@ struct GridSmem {
     static constexpr int WEIGHTS = CELLS + round16(8 * SLOTS);             // byte offset of the weights
     static constexpr int BYTES = larger(WEIGHTS + 4 * (SLOTS + PAST), CELLS + 8 * (SLOTS + PAST));
     static_assert(WEIGHTS - 4 * CORNER >= 0, "loads before the first weight");
+    static_assert(4 * SLOTS % 16 == 0, "cleared in 16-byte pieces");
     static_assert(sizeof(Pair) % 16 == 0 && sizeof(RowBounds) % 8 == 0, "alignment in the queue");
 };
 
@@ -884,8 +905,18 @@ __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
     float* const s_wt = reinterpret_cast<float*>(s_grid + Smem::WEIGHTS);
     const int lane = threadIdx.x;
     const bool hs = a.zsplit > 0;
-    const int items = a.R + (hs ? 1 : 0);               // per tile
-    const int slot = blockIdx.x / items, rep = blockIdx.x - slot * items;
+    // per tile: R items, and one for the unpaired pixels below the split (those
+    // tiles come first)
+    int slot, rep;
+    if (hs && blockIdx.x < (unsigned)a.nlow * (a.R + 1)) {
+        slot = blockIdx.x / (a.R + 1);
+        rep = blockIdx.x - slot * (a.R + 1);
+    } else {
+        const unsigned b = blockIdx.x - (hs ? (unsigned)a.nlow * (a.R + 1) : 0u);
+        slot = b / a.R;
+        rep = b - slot * a.R;
+        if (hs) slot += a.nlow;
+    }
     const int tile = a.order[slot];
     const int x0 = (tile % a.ntx) * TX, y0 = ((tile / a.ntx) % a.nty) * TY, z0 = (tile / (a.ntx * a.nty)) * TZ;
     const int N = a.N;
@@ -897,20 +928,20 @@ __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
     // the unpaired ones into evol / ew
     const bool upper = hs && z0 >= a.zsplit;
     const bool extra = rep == a.R;
-    if (extra && upper) return;
     const bool edge_walk = extra || upper;
     // (a tile that no unpaired pixel reaches skips the edge walks)
     const bool none = edge_walk && !tile_reaches_edges<TX, TY, TZ>(x0, y0, z0, N, a.edge_rmin, a.edge_rmax);
     if (extra && none) return;
     const int p_lo = extra ? 0 : (int)((long)a.np * rep / a.R);
     const int p_hi = none ? p_lo : extra ? a.np : (int)((long)a.np * (rep + 1) / a.R);
-    for (int i = lane; i < SLOTS; i += 32) {
-        s_sum[i] = make_float2(0.f, 0.f);
-        s_wt[i] = 0.f;
-    }
+    for (int i = lane; i < (Smem::WEIGHTS - Smem::CELLS + 4 * SLOTS) / 16; i += 32)
+        reinterpret_cast<float4*>(s_grid + Smem::CELLS)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
 
     bool any = false;                // some pair reached the tile
+    const unsigned aliases = tile_aliases<TX, TY, TZ>(x0, y0, z0, N, a.rmax);
+    TileTest ahead;                  // this lane's next test, on its way
+    if (p_lo + lane < p_hi) ahead = a.test[p_lo + lane];
     int base = p_lo - 32, qn = 0;
     unsigned mask = 0;               // this lane's particle's aliases still to be queued
     for (;;) {
@@ -935,8 +966,9 @@ __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
             if (base < p_hi) {
                 const int p = base + lane;
                 if (p < p_hi) {
-                    const TileTest t = a.test[p];
-                    if (t.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(t, x0, y0, z0, N);
+                    const TileTest t = ahead;
+                    if (p + 32 < p_hi) ahead = a.test[p + 32];
+                    if (t.half == a.half || a.half < 0) mask = tile_mask<TX, TY, TZ>(t, aliases, x0, y0, z0, N);
                     if (edge_walk && mask) mask = edge_mask<TX, TY, TZ>(a.part[p], mask, x0, y0, z0, N, a.ft);
                 }
                 continue;
@@ -977,72 +1009,124 @@ __global__ void __launch_bounds__(32, 20) grid4_kernel(InsertArgs a) {
         __syncwarp();
     }
     // tile sums -> HBM.  One replica (and the unpaired pixels' item) adds to
-    // the map; of several, each stores its FP32 partial sums, and the one that
-    // arrives last adds them in replica order while they are still in L2 (a
-    // separate pass over FP64 partial sums took 0.86 ms of a 256^3 map's
-    // 14.9 ms and 0.93 ms per batch and half map at 384^3).  Replicas that no
-    // pair reached store nothing.
-    const size_t N2 = (size_t)N * N;
-    auto voxel = [&](int i, size_t& idx) {
-        const int x = x0 + i % TX, y = y0 + (i / TX) % TY, z = z0 + i / (TX * TY);
-        idx = (size_t)z * N2 + (size_t)y * N + x;
-        return x < N && y < N && z < N;
-    };
-    if (extra || a.R == 1) {
-        double2* const vol = extra ? a.evol : a.vol;
-        double* const wgt = extra ? a.ew : a.w;
+    // the map; of several, the one that arrives last adds the FP32 partial sums
+    // in replica order: its own from shared memory, the others', which they
+    // stored, while they are still in L2 (a separate pass over FP64 partial sums
+    // took 0.86 ms of a 256^3 map's 14.9 ms and 0.93 ms per batch and half map
+    // at 384^3).  Replicas that no pair reached store nothing.  Four voxels at a
+    // time where the map's rows allow it: a voxel at a time left one warp
+    // waiting for 16 trips to L2 and HBM in turn (0.29 of the 1.56 ms of 256
+    // particles at 256^3; now 0.11 of 1.35).
+    const bool sole = extra || a.R == 1;
+    unsigned have = 0;               // whose partial sums there are
+    float* const mine = a.psum + ((size_t)tile * a.R + rep) * 3 * TV;
+    if (sole) {
         if (!any) return;
+    } else {
+        const unsigned self = any ? 256u << rep : 0u;
+        unsigned old = 0;
+        if (lane == 0) old = *(volatile unsigned*)&a.arrived[tile];
+        old = __shfl_sync(0xffffffffu, old, 0);
+        if ((int)(old & 255u) != a.R - 1) {            // the others are not all done
+            if (any) {
 #pragma unroll 2
-        for (int i = lane; i < TV; i += 32) {
-            const int ci = i % TX + PX * ((i / TX) % TY) + PP * (i / (TX * TY));
-            size_t idx;
-            if (!voxel(i, idx)) continue;
-            double2 o = vol[idx];
-            o.x += s_sum[ci].x;
-            o.y += s_sum[ci].y;
-            vol[idx] = o;
-            wgt[idx] += s_wt[ci];
+                for (int i = 4 * lane; i < TV; i += 128) {
+                    const int ci = i % TX + PX * ((i / TX) % TY) + PP * (i / (TX * TY));
+                    const float2 c0 = s_sum[ci], c1 = s_sum[ci + 1], c2 = s_sum[ci + 2], c3 = s_sum[ci + 3];
+                    *reinterpret_cast<float4*>(mine + i) = make_float4(c0.x, c1.x, c2.x, c3.x);
+                    *reinterpret_cast<float4*>(mine + TV + i) = make_float4(c0.y, c1.y, c2.y, c3.y);
+                    *reinterpret_cast<float4*>(mine + 2 * TV + i) = make_float4(s_wt[ci], s_wt[ci + 1], s_wt[ci + 2], s_wt[ci + 3]);
+                }
+                __threadfence();
+            }
+            __syncwarp();
+            if (lane == 0) old = atomicAdd(&a.arrived[tile], 1u | self);
+            old = __shfl_sync(0xffffffffu, old, 0);
+            if ((int)(old & 255u) != a.R - 1) return;
+        }
+        have = (old | self) >> 8;
+        if (lane == 0) a.arrived[tile] = 0;           // for the next launch
+        if (!have) return;
+        __threadfence();
+    }
+    const size_t N2 = (size_t)N * N;
+    const float* const all = a.psum + (size_t)tile * a.R * 3 * TV;
+    double2* const vol = extra ? a.evol : a.vol;
+    double* const wgt = extra ? a.ew : a.w;
+    if ((N & 3) == 0) {
+#pragma unroll 1
+        for (int i = 4 * lane; i < TV; i += 128) {
+            const int lx = i % TX, ly = (i / TX) % TY, lz = i / (TX * TY);
+            if (x0 + lx >= N || y0 + ly >= N || z0 + lz >= N) continue;
+            const size_t idx = (size_t)(z0 + lz) * N2 + (size_t)(y0 + ly) * N + x0 + lx;
+            const int ci = lx + PX * ly + PP * lz;
+            double2* const wq = reinterpret_cast<double2*>(wgt + idx);
+            double2 o[4] = {vol[idx], vol[idx + 1], vol[idx + 2], vol[idx + 3]}, w0 = wq[0], w1 = wq[1];
+            if (sole) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    o[k].x += s_sum[ci + k].x;
+                    o[k].y += s_sum[ci + k].y;
+                }
+                w0.x += s_wt[ci]; w0.y += s_wt[ci + 1];
+                w1.x += s_wt[ci + 2]; w1.y += s_wt[ci + 3];
+            } else {
+                double re[4] = {}, im[4] = {}, w[4] = {};
+#pragma unroll 2
+                for (int r = 0; r < a.R; ++r) {
+                    if (!((have >> r) & 1u)) continue;
+                    float4 p, q, v;
+                    if (r == rep) {
+                        p = make_float4(s_sum[ci].x, s_sum[ci + 1].x, s_sum[ci + 2].x, s_sum[ci + 3].x);
+                        q = make_float4(s_sum[ci].y, s_sum[ci + 1].y, s_sum[ci + 2].y, s_sum[ci + 3].y);
+                        v = make_float4(s_wt[ci], s_wt[ci + 1], s_wt[ci + 2], s_wt[ci + 3]);
+                    } else {
+                        const float* src = all + (size_t)r * 3 * TV + i;
+                        p = __ldcg(reinterpret_cast<const float4*>(src));
+                        q = __ldcg(reinterpret_cast<const float4*>(src + TV));
+                        v = __ldcg(reinterpret_cast<const float4*>(src + 2 * TV));
+                    }
+                    re[0] += p.x; re[1] += p.y; re[2] += p.z; re[3] += p.w;
+                    im[0] += q.x; im[1] += q.y; im[2] += q.z; im[3] += q.w;
+                    w[0] += v.x; w[1] += v.y; w[2] += v.z; w[3] += v.w;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) { o[k].x += re[k]; o[k].y += im[k]; }
+                w0.x += w[0]; w0.y += w[1];
+                w1.x += w[2]; w1.y += w[3];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) vol[idx + k] = o[k];
+            wq[0] = w0;
+            wq[1] = w1;
         }
         return;
     }
-    float* const mine = a.psum + ((size_t)tile * a.R + rep) * 3 * TV;
-    if (any) {
-#pragma unroll 2
-        for (int i = lane; i < TV; i += 32) {
-            const int ci = i % TX + PX * ((i / TX) % TY) + PP * (i / (TX * TY));
-            mine[i] = s_sum[ci].x;
-            mine[TV + i] = s_sum[ci].y;
-            mine[2 * TV + i] = s_wt[ci];
-        }
-        __threadfence();
-    }
-    __syncwarp();
-    unsigned old = 0;
-    if (lane == 0) old = atomicAdd(&a.arrived[tile], 1u | (any ? 256u << rep : 0u));
-    old = __shfl_sync(0xffffffffu, old, 0);
-    if ((int)(old & 255u) != a.R - 1) return;
-    const unsigned have = (old >> 8) | (any ? 1u << rep : 0u);
-    if (lane == 0) a.arrived[tile] = 0;               // for the next launch
-    if (!have) return;
-    __threadfence();
-    const float* const all = a.psum + (size_t)tile * a.R * 3 * TV;
 #pragma unroll 1
     for (int i = lane; i < TV; i += 32) {
-        size_t idx;
-        if (!voxel(i, idx)) continue;
+        const int lx = i % TX, ly = (i / TX) % TY, lz = i / (TX * TY);
+        if (x0 + lx >= N || y0 + ly >= N || z0 + lz >= N) continue;
+        const size_t idx = (size_t)(z0 + lz) * N2 + (size_t)(y0 + ly) * N + x0 + lx;
+        const int ci = lx + PX * ly + PP * lz;
         double re = 0, im = 0, w = 0;
-        for (int r = 0; r < a.R; ++r) {
-            if (!((have >> r) & 1u)) continue;
-            const float* q = all + (size_t)r * 3 * TV + i;
-            re += __ldcg(q);
-            im += __ldcg(q + TV);
-            w += __ldcg(q + 2 * TV);
+        if (sole) {
+            re = s_sum[ci].x;
+            im = s_sum[ci].y;
+            w = s_wt[ci];
+        } else {
+            for (int r = 0; r < a.R; ++r) {
+                if (!((have >> r) & 1u)) continue;
+                const float* q = all + (size_t)r * 3 * TV + i;
+                re += r == rep ? s_sum[ci].x : __ldcg(q);
+                im += r == rep ? s_sum[ci].y : __ldcg(q + TV);
+                w += r == rep ? s_wt[ci] : __ldcg(q + 2 * TV);
+            }
         }
-        double2 o = a.vol[idx];
+        double2 o = vol[idx];
         o.x += re;
         o.y += im;
-        a.vol[idx] = o;
-        a.w[idx] += w;
+        vol[idx] = o;
+        wgt[idx] += w;
     }
 }
 
@@ -1129,7 +1213,8 @@ static cudaError_t launch_shape4(const InsertArgs& a0, const Context& c, cudaStr
     a.nty = (N + TY - 1) / TY;
     a.ntz = (N + TZ - 1) / TZ;
     const int ntiles = a.ntx * a.nty * a.ntz;
-    const long items = (long)ntiles * (a.R + (a.zsplit > 0 ? 1 : 0));
+    a.nlow = a.zsplit > 0 ? a.ntx * a.nty * ((a.zsplit + TZ - 1) / TZ) : 0;
+    const long items = (long)ntiles * a.R + a.nlow;
     const size_t smem = GridSmem<TX, TY, TZ, PX, PP>::BYTES;
     if (c.g.ewald) {
         if (c.g.gate) grid4_kernel<true, true, TX, TY, TZ, PX, PP><<<(unsigned)items, 32, smem, s>>>(a);
@@ -1169,8 +1254,9 @@ cudaError_t launch_insert(const Context& c, const float2* spectra, const DevPart
     a.zsplit = c.g.fom ? 0 : c.zsplit;
     a.evol = c.d_evol[h];
     a.ew = c.d_ew[h];
-    a.edge_rmin = c.edge_rmin;
-    a.edge_rmax = c.edge_rmax;
+    a.edge_rmin = (float)c.edge_rmin;
+    a.edge_rmax = (float)c.edge_rmax;
+    a.rmax = c.rmax;
     if (!c.g.fom) {
         switch (c.shape) {
             case 0: return launch_shape4<8, 8, 8, 8, 67>(a, c, s);

@@ -64,6 +64,8 @@ def _grid(F, mats, N, ft, scale, weight, halves):
     (64, 64, 24, 1, "C1"),       # whole-voxel steps
     (32, 128, 30, 1, "D2"),      # step 0.25; four records a particle
     (8, 32, 40, 1, "C1"),        # one tile, all aliases
+    (42, 128, 24, 2, "C1"),      # rows that are folded a voxel at a time, half maps
+    (12, 32, 33, 1, "C1"),       # rows folded by fours, the last tile cut after one
 ])
 def test_sums_match_fp64_gridding(N, ft, P, nmaps, sym):
     from bsoft_b200.recon import Reconstructor
