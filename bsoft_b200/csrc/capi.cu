@@ -209,7 +209,7 @@ static int set_shape(Recon* r, int shape) {
 }
 
 // Switch half-space gridding on or off.  Off: the accumulators become the
-// full map's sums (read_sums, in place).  On: only while they are empty (a
+// full map's sums (launch_map_sums, in place).  On: only while they are empty (a
 // full map's sums cannot be split into paired and unpaired parts).
 static int set_half_space(Recon* r, bool on) {
     const int old = r->zsplit;

@@ -1,4 +1,4 @@
-// fft_tile.cuh - transforms of a tile of 16 lines by one CTA, for the 3-D map
+// fft_tile.cuh - transforms of a tile of 16 or 8 lines by one CTA, for the 3-D map
 // transform.
 //
 // The tile sits in shared memory as [element][line], so the 16 lines of an
@@ -179,12 +179,12 @@ __device__ __forceinline__ void dft(float2* v) {
     }
 }
 
-template <int R, bool INV>
+template <int R, bool INV, int LINES>
 __device__ __forceinline__ void tile_stage(const float2* src, float2* dst, int n, int ns, int magic,
                                            const float2* roots, int rstride, int pitch) {
     const int nr = n / R, tstep = n / (ns * R) * rstride;
-    for (int i = threadIdx.x; i < nr * TILE_LINES; i += blockDim.x) {
-        const int c = i & (TILE_LINES - 1), j = i / TILE_LINES;
+    for (int i = threadIdx.x; i < nr * LINES; i += blockDim.x) {
+        const int c = i & (LINES - 1), j = i / LINES;
         const int q = (j * magic) >> 20, k = j - q * ns;
         float2 v[R];
 #pragma unroll
@@ -204,23 +204,23 @@ __device__ __forceinline__ void tile_stage(const float2* src, float2* dst, int n
     }
 }
 
-// Transform the tile in a (p.n x 16, element pitch `pitch`) with b as the
+// Transform the tile in a (p.n x LINES, element pitch `pitch`) with b as the
 // other buffer; all threads of the CTA, which have synchronised after filling
 // a.  roots: exp(-2 pi i t / (p.n rstride)), t < p.n rstride, in shared
 // memory.  Returns the buffer holding the result (synchronised).
-template <bool INV>
+template <bool INV, int LINES = TILE_LINES>
 __device__ __forceinline__ float2* tile_fft(float2* a, float2* b, const TilePlan& p, const float2* roots, int rstride,
                                             int pitch) {
     for (int s = 0; s < p.nstage; ++s) {
         const int ns = p.ns[s], mg = p.magic[s];
         switch (p.radix[s]) {
-            case 2: tile_stage<2, INV>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
-            case 3: tile_stage<3, INV>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
-            case 4: tile_stage<4, INV>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
-            case 5: tile_stage<5, INV>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
-            case 6: tile_stage<6, INV>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
-            case 7: tile_stage<7, INV>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
-            default: tile_stage<8, INV>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
+            case 2: tile_stage<2, INV, LINES>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
+            case 3: tile_stage<3, INV, LINES>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
+            case 4: tile_stage<4, INV, LINES>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
+            case 5: tile_stage<5, INV, LINES>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
+            case 6: tile_stage<6, INV, LINES>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
+            case 7: tile_stage<7, INV, LINES>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
+            default: tile_stage<8, INV, LINES>(a, b, p.n, ns, mg, roots, rstride, pitch); break;
         }
         __syncthreads();
         float2* t = a;

@@ -46,41 +46,60 @@ __device__ __forceinline__ size_t mirror_index(size_t x, size_t y, size_t z, siz
     return ((((N - z) % N) * N + (N - y) % N) * N + (N - x) % N);
 }
 
-// The map's sums at voxel i.  Half-space accumulators (zsplit > 0) hold
-// the paired pixels' sums P below zsplit, with the unpaired pixels' sums U
-// there in (e, ew), and U alone at and above zsplit: the map is P(v) + U(v)
-// below the split and conj(P(-v)) + U(v) above it.
-__device__ __forceinline__ void read_sums(const double2* vol, const double* w, const double2* e, const double* ew,
-                                          size_t i, size_t N, int zsplit, double2& v, double& wt) {
-    v = vol[i];
-    wt = w[i];
-    if (zsplit <= 0) return;
-    const size_t z = i / (N * N);
-    if (z >= (size_t)zsplit) {
-        const size_t m = mirror_index(i % N, (i / N) % N, z, N);
-        const double2 u = vol[m];
-        v.x += u.x;
-        v.y -= u.y;
-        wt += w[m];
+// One half map's sums at voxel v = (x, y, z) and at its mirror -v = (xm, ym, zm).
+// Half-space accumulators (zsplit > 0) hold the paired pixels' sums P below
+// zsplit, with the unpaired pixels' sums U there in (e, ew), and U alone at and
+// above zsplit: the map is P(v) + U(v) below the split and conj(P(-v)) + U(v)
+// above it.  Of v and -v one at least lies below (zsplit > N/2).
+struct VoxelPair {
+    double2 v, vm;
+    double w, wm;
+};
+
+__device__ __forceinline__ VoxelPair half_pair(const HalfSums& h, int x, int y, int z, int xm, int ym, int zm, int N,
+                                               int zsplit) {
+    const size_t i = ((size_t)z * N + y) * N + x, m = ((size_t)zm * N + ym) * N + xm;
+    VoxelPair s{h.vol[i], h.vol[m], h.w[i], h.w[m]};
+    if (zsplit <= 0) return s;
+    const bool low = z < zsplit, lowm = zm < zsplit;
+    const double2 p = s.v, pm = s.vm;
+    const double wp = s.w, wpm = s.wm;
+    if (low) {
+        const double2 u = h.e[i];
+        s.v.x += u.x;
+        s.v.y += u.y;
+        s.w += h.ew[i];
     } else {
-        const double2 u = e[i];
-        v.x += u.x;
-        v.y += u.y;
-        wt += ew[i];
+        s.v.x += pm.x;
+        s.v.y -= pm.y;
+        s.w += wpm;
     }
+    if (lowm) {
+        const double2 u = h.e[m];
+        s.vm.x += u.x;
+        s.vm.y += u.y;
+        s.wm += h.ew[m];
+    } else {
+        s.vm.x += p.x;
+        s.vm.y -= p.y;
+        s.wm += wp;
+    }
+    return s;
 }
 
-// A voxel's sums over the halves that are added.
-__device__ __forceinline__ void voxel_sums(const WeighArgs& a, size_t i, double2& v, double& w) {
-    read_sums(a.h[0].vol, a.h[0].w, a.h[0].e, a.h[0].ew, i, a.N, a.zsplit, v, w);
+// The pair's sums over the halves that are added.
+__device__ __forceinline__ VoxelPair voxel_pair(const WeighArgs& a, int x, int y, int z, int xm, int ym, int zm) {
+    VoxelPair s = half_pair(a.h[0], x, y, z, xm, ym, zm, a.N, a.zsplit);
     if (a.nh > 1) {
-        double2 v1;
-        double w1;
-        read_sums(a.h[1].vol, a.h[1].w, a.h[1].e, a.h[1].ew, i, a.N, a.zsplit, v1, w1);
-        v.x += v1.x;
-        v.y += v1.y;
-        w += w1;
+        const VoxelPair t = half_pair(a.h[1], x, y, z, xm, ym, zm, a.N, a.zsplit);
+        s.v.x += t.v.x;
+        s.v.y += t.v.y;
+        s.w += t.w;
+        s.vm.x += t.vm.x;
+        s.vm.y += t.vm.y;
+        s.wm += t.wm;
     }
+    return s;
 }
 
 // fspace_reconstruction_weigh: the sum over the weight, as float
@@ -94,9 +113,14 @@ __device__ __forceinline__ float2 weighed(double2 v, double w) {
 __global__ void snr_kernel(WeighArgs a) {
     const size_t N = a.N, N3 = N * N * N;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N3; i += (size_t)gridDim.x * blockDim.x) {
-        double2 v;
-        double w;
-        voxel_sums(a, i, v, w);
+        double2 v = a.h[0].vol[i];
+        double w = a.h[0].w[i];
+        if (a.nh > 1) {
+            const double2 u = a.h[1].vol[i];
+            v.x += u.x;
+            v.y += u.y;
+            w += a.h[1].w[i];
+        }
         double p = a.h[0].p[i], q = a.h[0].q[i];
         if (a.nh > 1) { p += a.h[1].p[i]; q += a.h[1].q[i]; }
         const float2 F = weighed(v, w);
@@ -120,7 +144,7 @@ __global__ void snr_kernel(WeighArgs a) {
 
 // ---- 3-D inverse transform ----------------------------------------------------
 //
-// 384^3, both half maps and their FSC: 24.8 -> 5.5 ms; the passes were
+// 384^3, both half maps and their FSC: 24.8 -> 4.3 ms; the passes were
 // full complex volumes through runtime-radix line transforms (an index
 // division per element and local-memory butterflies) at 1.4 TB/s.
 
@@ -129,6 +153,10 @@ constexpr int FIN_THREADS = 256;
 // of a transposed x tile (odd, so that a warp's consecutive elements of one
 // line fall in distinct banks)
 constexpr int YZ_PITCH = TILE_LINES, X_PITCH = TILE_LINES + 1;
+// weigh_y's tiles: 8 lines leave room for twice the CTAs, whose loads of the
+// sums it waits for, and a pitch of 9 spreads the radix-8 stages' stores over
+// the banks (384^3: 16 lines 0.86, 8 lines 0.97, with the pitch 0.65 ms a map)
+constexpr int W_LINES = 8, W_PITCH = 9;
 
 struct IfftArgs {
     float2* g;         // N x N x pitch: the half volume
@@ -140,39 +168,37 @@ struct IfftArgs {
     const double* sinc;   // weight by squared distance from the map centre, or null
 };
 
-// y lines: 16 adjacent x of one z, G formed from the sums on the way in
+// y lines: 8 adjacent x of one z, G formed from the sums on the way in.  Bound
+// by the reads of the sums' two ends: 1.25 -> 0.65 ms a map at 384^3, half of it
+// from the coordinates of -v, which 64-bit divisions of the index gave.
 __global__ void __launch_bounds__(FIN_THREADS) weigh_y_kernel(const __grid_constant__ WeighArgs w,
                                                               const __grid_constant__ IfftArgs a) {
     extern __shared__ float2 sm[];
     const int N = a.N, XH = N / 2 + 1;
     float2* roots = sm;
     float2* t0 = sm + N;
-    float2* t1 = t0 + N * YZ_PITCH;
+    float2* t1 = t0 + N * W_PITCH;
     for (int i = threadIdx.x; i < N; i += FIN_THREADS) roots[i] = a.tw[i];
-    const int x0 = blockIdx.x * TILE_LINES, z = blockIdx.y, zm = z ? N - z : 0;
-    for (int i = threadIdx.x; i < N * TILE_LINES; i += FIN_THREADS) {
-        const int c = i & (TILE_LINES - 1), y = i / TILE_LINES, x = x0 + c;
+    const int x0 = blockIdx.x * W_LINES, z = blockIdx.y, zm = z ? N - z : 0;
+    for (int i = threadIdx.x; i < N * W_LINES; i += FIN_THREADS) {
+        const int c = i & (W_LINES - 1), y = i / W_LINES, x = x0 + c;
         float2 g = make_float2(0.f, 0.f);
         if (x < XH) {
             const int ym = y ? N - y : 0, xm = x ? N - x : 0;
-            double2 v;
-            double wt;
-            voxel_sums(w, ((size_t)z * N + y) * N + x, v, wt);
-            const float2 f = weighed(v, wt);
-            voxel_sums(w, ((size_t)zm * N + ym) * N + xm, v, wt);
-            const float2 m = weighed(v, wt);
+            const VoxelPair q = voxel_pair(w, x, y, z, xm, ym, zm);
+            const float2 f = weighed(q.v, q.w), m = weighed(q.vm, q.wm);
             // half the sum; phase_shift_to_center is (-1)^(h+k+l), the same
             // for both (signed and unsigned indices share parity for even N)
             const float s = ((x + y + z) & 1) ? -0.5f : 0.5f;
             g = make_float2(s * (f.x + m.x), s * (f.y - m.y));
         }
-        t0[y * YZ_PITCH + c] = g;
+        t0[y * W_PITCH + c] = g;
     }
     __syncthreads();
-    const float2* r = tile_fft<true>(t0, t1, a.plan, roots, 1, YZ_PITCH);
-    for (int i = threadIdx.x; i < N * TILE_LINES; i += FIN_THREADS) {
-        const int c = i & (TILE_LINES - 1), y = i / TILE_LINES, x = x0 + c;
-        if (x < XH) a.g[((size_t)z * N + y) * a.pitch + x] = r[y * YZ_PITCH + c];
+    const float2* r = tile_fft<true, W_LINES>(t0, t1, a.plan, roots, 1, W_PITCH);
+    for (int i = threadIdx.x; i < N * W_LINES; i += FIN_THREADS) {
+        const int c = i & (W_LINES - 1), y = i / W_LINES, x = x0 + c;
+        if (x < XH) a.g[((size_t)z * N + y) * a.pitch + x] = r[y * W_PITCH + c];
     }
 }
 
@@ -284,6 +310,7 @@ static WeighArgs weigh_args(const Context& c, int imap) {
 }
 
 static size_t yz_smem(int N) { return sizeof(float2) * ((size_t)N + 2 * (size_t)N * YZ_PITCH); }
+static size_t weigh_smem(int N) { return sizeof(float2) * ((size_t)N + 2 * (size_t)N * W_PITCH); }
 static size_t x_smem(int N) { return sizeof(float2) * ((size_t)N + 2 * (size_t)(N / 2 + 1) * X_PITCH); }
 
 // Map imap (0: the halves added) of the context's sums: weighed, transformed,
@@ -308,7 +335,7 @@ cudaError_t launch_finish(const Context& c, int imap, float* map_out, bool sinc,
     a.pitch = (XH + 3) / 4 * 4;
     if (!tile_plan(N, &a.plan)) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)((XH + TILE_LINES - 1) / TILE_LINES), (unsigned)N);
-    weigh_y_kernel<<<grid, FIN_THREADS, yz_smem(N), s>>>(w, a);
+    weigh_y_kernel<<<dim3((unsigned)((XH + W_LINES - 1) / W_LINES), (unsigned)N), FIN_THREADS, weigh_smem(N), s>>>(w, a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     fft_z_kernel<<<grid, FIN_THREADS, yz_smem(N), s>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -320,7 +347,7 @@ cudaError_t launch_finish(const Context& c, int imap, float* map_out, bool sinc,
     return cudaGetLastError();
 }
 
-// Half-space accumulators -> the map's sums (read_sums), into (dv, dw); in
+// Half-space accumulators -> the map's sums (half_pair), into (dv, dw); in
 // place (dv == vol) too: the voxels at and above zsplit are written first,
 // from the paired sums below it, then (e, ew) is added below it.
 __global__ void map_sums_upper_kernel(double2* dv, double* dw, const double2* vol, const double* w, int N,
@@ -375,7 +402,7 @@ cudaError_t launch_map_sums(double2* dv, double* dw, const double2* vol, const d
 // shared memory.  Rows, warps and CTAs in fixed order: deterministic, FP64
 // throughout.  Bound by the FP64 pipe and the reads of the sums; a thread per
 // shell scanning a whole plane (384 CTAs, every voxel's square root two to
-// four times) took 5.4 ms at 384^3 after 2.0 ms of weighing.
+// four times) took 5.4 ms at 384^3 after 2.0 ms of weighing, now 1.7.
 __device__ __forceinline__ double fsc_radius(int h, int k, int l, double real) {
     const double fs = 1.0 / real;
     double rx = h * fs, ry = k * fs, rz = l * fs;
@@ -410,15 +437,12 @@ __global__ void __launch_bounds__(FSC_WARPS * 32) fsc_rows_kernel(const __grid_c
             if (!__any_sync(0xffffffffu, in)) break;            // the radius only grows
             double num = 0, d1 = 0, d2 = 0;
             if (in) {
+                const int hm = h ? N - h : 0;
+                const VoxelPair q1 = voxel_pair(a.w[0], h, y, z, hm, ym, zm), q2 = voxel_pair(a.w[1], h, y, z, hm, ym, zm);
                 for (int m = 0; m < 2; ++m) {
                     if (m && (h == 0 || h == H)) continue;       // its mate is another row's
-                    const size_t i = m ? ((size_t)zm * N + ym) * N + (N - h) : ((size_t)z * N + y) * N + h;
-                    double2 v;
-                    double w;
-                    voxel_sums(a.w[0], i, v, w);
-                    const float2 f1 = weighed(v, w);
-                    voxel_sums(a.w[1], i, v, w);
-                    const float2 f2 = weighed(v, w);
+                    const float2 f1 = m ? weighed(q1.vm, q1.wm) : weighed(q1.v, q1.w);
+                    const float2 f2 = m ? weighed(q2.vm, q2.wm) : weighed(q2.v, q2.w);
                     num += (double)f1.x * f2.x + (double)f1.y * f2.y;
                     d1 += (double)f1.x * f1.x + (double)f1.y * f1.y;
                     d2 += (double)f2.x * f2.x + (double)f2.y * f2.y;
