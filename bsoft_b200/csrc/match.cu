@@ -1304,8 +1304,10 @@ static cudaError_t ensure_padded(Match& M, cudaStream_t s) {
 // x weights applied to the sums, and eight pixels' lane sums added by one
 // exchange tree.  Loads come from the padded copies: the texture unit delivers
 // four 8-byte texels a clock per SM, which bounded the gather through it
-// (5,184 views of 9,900 pixels 25.7 -> 14.3 ms, now the
-// float-to-double conversions').  gridDim.y CTAs share a
+// (5,184 views of 9,900 pixels 25.7 -> 14.3 ms).  Bound by what the loads write
+// into registers, 4 KB a pixel at 64 bytes a clock per SM: 64 of the 74 clocks a
+// pixel takes (integer instructions for half of the float-to-double conversions,
+// and pixels in compact tiles, which hit L1, changed nothing).  gridDim.y CTAs share a
 // view's pixels, so that a few hundred views fill the SMs evenly.  Positions
 // beyond the padding, and other kernel widths, take the general gather.
 __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureObject_t tex, int D, int wd,
