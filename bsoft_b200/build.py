@@ -30,7 +30,7 @@ def up_to_date() -> bool:
     if not os.path.exists(OUT):
         return False
     t = os.path.getmtime(OUT)
-    deps = sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + [os.path.join(HERE, "..", "include", "bsgpu.h")]
+    deps = sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + [os.path.join(HERE, "..", "include", "bsgpu.h")]
     return all(os.path.getmtime(d) <= t for d in deps if os.path.exists(d))
 
 
