@@ -30,6 +30,11 @@ namespace bsg {
 
 constexpr size_t SCRATCH_BYTES = BSG_NOALLOC_SCRATCH_BYTES;
 
+// what a particle record takes of the area: fixed, so that the number of
+// particles that fit does not follow the record's layout
+constexpr size_t RECORD_BYTES = 368;
+static_assert(sizeof(DevParticle) <= RECORD_BYTES, "record's share of the scratch area");
+
 static __device__ __align__(256) unsigned char g_noalloc_scratch[SCRATCH_BYTES];
 
 cudaError_t launch_background(const Context& c, const float* img, int nimg, cudaStream_t s);
@@ -59,7 +64,7 @@ Layout layout(int n, int ft, long np) {
     Layout L;
     size_t off = 0;
     L.tw = off;    off += align256(sizeof(float2) * (size_t)(ft / 2));
-    L.part = off;  off += align256(sizeof(DevParticle) * (size_t)np);
+    L.part = off;  off += align256(RECORD_BYTES * (size_t)np);
     L.bkg = off;   off += align256(sizeof(double) * (size_t)np);
     L.phase = off; off += align256(sizeof(float2) * 2 * (size_t)ft * np);
     L.rows = off;  off += align256(sizeof(float2) * (size_t)n * (ft / 2 + 1) * np);
