@@ -25,14 +25,16 @@
 // tcgen05.ld and keep each row's 8 best columns in registers.  The M tiles
 // are taken in groups; the CTAs of a group are a grid of its M tiles by
 // stretches of N, so that those of one stretch read the same B tiles at the
-// same time and all share the group's A tiles through L2.  Groups of seven and
-// four M tiles (21 and 37 stretches) keep 147 and 148 of the 148 SMs at work,
-// and the stretches' lengths, which differ by one tile, alternate from group
-// to group (ten M tiles x 15 stretches as 150 work items a group left the
-// last of six rounds nearly empty: 256 images x 25 origins against 68,520
-// sections 6.31 -> 5.48 ms at full clock, 6.09 -> 6.03 under the power cap; one
-// run of tiles per CTA regardless of the stretches, evener still, 7.70: B is
-// then read by one CTA at a time).  A CTA carries its rows' top-8 along its
+// same time and all share the group's A tiles through L2.  Groups of 21, seven
+// and four M tiles (7, 21 and 37 stretches) keep 147 and 148 of the 148 SMs at
+// work, and the stretches' lengths, which differ by one tile, alternate from
+// group to group.  Larger groups read B from HBM fewer times, which the power
+// cap rewards; the A tiles of 21 fit L2 at 128^2.  256 images x 25 origins
+// against 68,520 sections, the whole call: ten M tiles x 15 stretches as 150
+// work items a group (the last of six rounds nearly empty) 7.70, sevens and
+// fours 7.21, with 21s 7.04 ms; 2,048 images against 550,320 sections: 523,
+// 568 and 522 ms of GEMM.  One run of tiles per CTA regardless of the
+// stretches, evener still, 7.70: B is then read by one CTA at a time.  A CTA carries its rows' top-8 along its
 // stretch.  Every wait is bounded (2 s) and reports through a status word.
 #include "match.cuh"
 
@@ -150,21 +152,26 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r) {
 // takes M tile c % size of it and the N tiles of stretch c / size.
 struct Runs {
     int mtiles, ntiles, ctas;
-    int groups, sevens;               // sevens < 0: groups of nearly equal sizes
+    int groups, large, sevens;        // large groups of 21, then sevens, then fours; sevens < 0: groups of
+                                      // nearly equal sizes
 
     __host__ __device__ static Runs plan(int mtiles, int ntiles) {
-        Runs r{mtiles, ntiles, 148, 0, -1};
+        Runs r{mtiles, ntiles, 148, 0, 0, -1};
         for (int four = 0; four < 7 && r.sevens < 0; ++four)
             if (mtiles >= 4 * four && (mtiles - 4 * four) % 7 == 0) {
                 r.sevens = (mtiles - 4 * four) / 7;
-                r.groups = r.sevens + four;
+                r.large = r.sevens / 3;
+                r.sevens -= 3 * r.large;
+                r.groups = r.large + r.sevens + four;
             }
         if (r.sevens < 0) r.groups = (mtiles + 6) / 7;     // below 18, where sevens and fours do not add up
         return r;
     }
     __host__ __device__ int first(int g) const {
         if (sevens < 0) return (int)((long)g * mtiles / groups);
-        return g <= sevens ? 7 * g : 7 * sevens + 4 * (g - sevens);
+        if (g <= large) return 21 * g;
+        g -= large;
+        return 21 * large + (g <= sevens ? 7 * g : 7 * sevens + 4 * (g - sevens));
     }
     __host__ __device__ int size(int g) const { return first(g + 1) - first(g); }
     __host__ __device__ int stretches(int g) const { return ctas / size(g); }
@@ -174,7 +181,11 @@ struct Runs {
         return (int)(((long)r * ntiles + (long)g * n / groups) / n);
     }
     __host__ __device__ int group_of(int mtile) const {
-        if (sevens >= 0) return mtile < 7 * sevens ? mtile / 7 : sevens + (mtile - 7 * sevens) / 4;
+        if (sevens >= 0) {
+            if (mtile < 21 * large) return mtile / 21;
+            const int m = mtile - 21 * large;
+            return large + (m < 7 * sevens ? m / 7 : sevens + (m - 7 * sevens) / 4);
+        }
         int g = (int)((long)mtile * groups / mtiles);
         while (first(g) > mtile) --g;
         while (first(g + 1) <= mtile) ++g;

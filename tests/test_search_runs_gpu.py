@@ -1,5 +1,5 @@
 """The search's division of row tiles and panel tiles over the SMs: batches of
-one to twenty row tiles (even groups, sevens and fours, a ragged last batch),
+one to 53 row tiles (even groups, groups of 21, 7 and 4, a ragged last batch),
 panels of one to several tiles, merges of few and many candidates.  How the
 work is cut changes no bit, so every division gives the one-image batches'
 result, and the best candidate's correlation is the FP64 one's to BF16 rounding
@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
     (1, 1, 5),         # one tile of each
     (7, 25, 700),      # two row tiles, three panel tiles
     (96, 25, 700),     # 19 row tiles
-    (104, 25, 1100),   # 21: three sevens
+    (104, 25, 1100),   # 21: one large group
+    (128, 25, 700),    # 25: a large group and a four
+    (270, 25, 1500),   # 53: two large groups, a seven, a four
     (12, 49, 3000),    # many candidates an image
     (5, 25, 38000),    # one row tile over every SM, more panel tiles than stretches
     (150, 9, 300),     # merges of two CTAs per SM
