@@ -760,11 +760,12 @@ struct GridSmem {
 
 // the corners (0, y, z) and (1, y, z) at cell offset OFF
 template <int OFF, int PX, int PP>
-__device__ __forceinline__ void corner_row(unsigned at, unsigned wt, float2 f, float rx, float wyz, const bool* vx, bool on) {
+__device__ __forceinline__ void corner_row(unsigned at, unsigned wt, float2 f, float rx, float wyz, const bool* vx, bool on,
+                                           unsigned lanes) {
     cell_add<OFF>(at, wt, f, (1.f - rx) * wyz, vx[0] && on);
-    __syncwarp();
+    __syncwarp(lanes);
     cell_add<OFF + 1>(at, wt, f, rx * wyz, vx[1] && on);
-    __syncwarp();
+    __syncwarp(lanes);
 }
 
 template <bool GATE, bool EW, int TX, int TY, int TZ, int PX, int PP>
@@ -804,20 +805,26 @@ __device__ __forceinline__ void pixel4(const InsertArgs& a, const DevParticle& P
         __syncwarp();
         return;
     }
-    const float flx = floorf(mx), fly = floorf(my), flz = floorf(mz);
-    const int ix = (int)flx, iy = (int)fly, iz = (int)flz;
-    const float rx = mx - flx, ry = my - fly, rz = mz - flz;
-    const bool vx[2] = {act && (unsigned)ix < TX, act && (unsigned)(ix + 1) < TX};
-    const bool vy[2] = {(unsigned)iy < TY, (unsigned)(iy + 1) < TY};
-    const bool vz[2] = {(unsigned)iz < TZ, (unsigned)(iz + 1) < TZ};
-    typedef GridSmem<TX, TY, TZ, PX, PP> Smem;
-    const int cell = act ? min(max(ix + PX * iy + PP * iz, Smem::FIRST), Smem::LAST) : 0;
-    const unsigned at = cells + 8 * cell, wt = weights + 4 * cell;
-    const float z0 = (1.f - rz) * wt_, z1 = rz * wt_;
-    corner_row<0, PX, PP>(at, wt, f, rx, (1.f - ry) * z0, vx, vy[0] && vz[0]);
-    corner_row<PX, PX, PP>(at, wt, f, rx, ry * z0, vx, vy[1] && vz[0]);
-    corner_row<PP, PX, PP>(at, wt, f, rx, (1.f - ry) * z1, vx, vy[0] && vz[1]);
-    corner_row<PP + PX, PX, PP>(at, wt, f, rx, ry * z1, vx, vy[1] && vz[1]);
+    // only the lanes with a pixel (4 of 32 on average) go on: the others would
+    // load too, and a load's two half warps cost a wavefront each
+    const unsigned lanes = __ballot_sync(0xffffffffu, act);
+    if (act) {
+        const float flx = floorf(mx), fly = floorf(my), flz = floorf(mz);
+        const int ix = (int)flx, iy = (int)fly, iz = (int)flz;
+        const float rx = mx - flx, ry = my - fly, rz = mz - flz;
+        const bool vx[2] = {(unsigned)ix < TX, (unsigned)(ix + 1) < TX};
+        const bool vy[2] = {(unsigned)iy < TY, (unsigned)(iy + 1) < TY};
+        const bool vz[2] = {(unsigned)iz < TZ, (unsigned)(iz + 1) < TZ};
+        typedef GridSmem<TX, TY, TZ, PX, PP> Smem;
+        const int cell = min(max(ix + PX * iy + PP * iz, Smem::FIRST), Smem::LAST);
+        const unsigned at = cells + 8 * cell, wt = weights + 4 * cell;
+        const float z0 = (1.f - rz) * wt_, z1 = rz * wt_;
+        corner_row<0, PX, PP>(at, wt, f, rx, (1.f - ry) * z0, vx, vy[0] && vz[0], lanes);
+        corner_row<PX, PX, PP>(at, wt, f, rx, ry * z0, vx, vy[1] && vz[0], lanes);
+        corner_row<PP, PX, PP>(at, wt, f, rx, (1.f - ry) * z1, vx, vy[0] && vz[1], lanes);
+        corner_row<PP + PX, PX, PP>(at, wt, f, rx, ry * z1, vx, vy[1] && vz[1], lanes);
+    }
+    __syncwarp();
 }
 
 // The pair's set-up by one lane: the pixels whose tents can reach the tile at
