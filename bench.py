@@ -1012,14 +1012,14 @@ def main():
         per_particle = 22.0 * BOX * BOX
         avg_launch_ms = ins_ms / max(1, ins_launch)
         achieved = per_particle * B / (avg_launch_ms / 1e3) / 1e9
-        # DRAM bytes of one gridding launch, from one ncu capture of this
-        # kernel (8^3 tiles, two replicas, half-space gridding, 256^3 map) on
-        # a 256-particle batch of this workload: reads 574.2 MB (mostly the
-        # spectra, 2.243 MB per particle: the tiles below the split read each
-        # particle's spectrum about once) and writes 922.7 MB (the two
-        # replicas' partial sums and the unpaired pixels' sums, fixed per
-        # launch); scaled to the launch's batch
-        traffic = (2.243e6 * B + 0.923e9) if (int(shape) == 0 and BOX == 256) else None
+        # DRAM bytes of one gridding launch, from ncu captures of this kernel
+        # (two replicas, half-space gridding, 256^3 map) on a 256-particle
+        # batch of this workload: reads 754.8 MB with 8^3 tiles and 870.2 MB
+        # with 16 x 8 x 8 (mostly the spectra, so per particle), writes 447.4
+        # and 713.7 MB (the sums, fixed per launch); scaled to the launch's
+        # batch
+        per = {0: (2.948e6, 0.447e9), 2: (3.399e6, 0.714e9)}.get(int(shape))
+        traffic = per[0] * B + per[1] if per and BOX == 256 else None
         roof = {"kernel": "grid4_kernel", "bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                 "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
                 "traffic_unit": ("bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum of a "
