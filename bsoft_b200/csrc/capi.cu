@@ -91,6 +91,13 @@ static void host_twiddles(int L, std::vector<float2>& out) {
     if (L / 2 == 0) out[0] = make_float2(1.f, 0.f);
 }
 
+// Largest distance (voxels) of an Ewald surface s_z = ewh s^2 from its plane:
+// at the transform's corner, ft/2 steps along both axes.
+static double ewald_reach(const Geometry& g, double ewh, double inv2) {
+    const double hf = g.ft / 2.0;
+    return fabs(ewh) * 2.0 * hf * hf * inv2 * g.mscale * 1.0001;
+}
+
 // 32-double C-ABI record -> device record (see bsgpu.h for the layout)
 // ewh: the Ewald surface's +-lambda/2 for this record (0: the plane)
 static void make_dev_particle(const Recon& r, const double* q, DevParticle& d, double ewh = 0.0) {
@@ -133,8 +140,7 @@ static void make_dev_particle(const Recon& r, const double* q, DevParticle& d, d
     // the Ewald surface's largest offset (its lattice bounds the curvature:
     // ewh inv2 mscale |p + q| <= ewh inv2 mscale ft sqrt(2) per pixel step)
     d.ewh = ewh;
-    const double hf = g.ft / 2.0;
-    d.ezmax = (float)(fabs(d.ewh) * 2.0 * hf * hf * d.inv2 * g.mscale * 1.0001);
+    d.ezmax = (float)ewald_reach(g, d.ewh, d.inv2);
     // particle_reconstruct's rescale_to_avg_std(0, 1) under -rescale
     // (mg_reconstruct.cpp:155): v * scale + shift, scale 0 = none
     d.na = q[24] != 0 ? q[24] : 1.0;
@@ -343,14 +349,17 @@ static int upload_params(Recon* r, int buf, const double* params, long np) {
         for (long i = 0; i < np; ++i) {
             smin = std::min(smin, (double)hp[i].step);
             smax = std::max(smax, (double)hp[i].step);
-            // the farther corner, |ad +- bd| hf (symmetry copies' are the same)
+            // the farther corner, |ad +- bd| hf (symmetry copies' are the
+            // same), and there the Ewald surfaces' distance from the plane
+            // (hp holds the planes' records: the wavelength is in params)
             double aa = 0, bb = 0, ab = 0;
             for (int k = 0; k < 3; ++k) {
                 aa += hp[i].ad[k] * hp[i].ad[k];
                 bb += hp[i].bd[k] * hp[i].bd[k];
                 ab += hp[i].ad[k] * hp[i].bd[k];
             }
-            far = std::max(far, hf * sqrt(aa + bb + 2.0 * fabs(ab)) + hp[i].ezmax);
+            const double ez = ewald_reach(r->g, params[i * BSG_PARTICLE_DOUBLES + 26] / 2, hp[i].inv2);
+            far = std::max(far, hf * sqrt(aa + bb + 2.0 * fabs(ab)) + ez);
         }
         r->rmax = (float)(far * (1.0 + 1e-5) + 2.0);     // (a tent's corner lies sqrt(3) away at most)
         r->edge_rmin = np ? hf * smin * (1.0 - 1e-6) - 1e-3 : 0.0;
