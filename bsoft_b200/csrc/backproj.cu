@@ -294,19 +294,27 @@ constexpr int BP_EDGE = 16;          // edge of a CTA's square of voxels
 constexpr int BP_CHUNK = 64;         // image parameters staged in shared memory at a time
 
 // An image's parameters for one plane z of the map: its coordinates at voxel
-// offset (c0, c1) are (xx c0 + xy c1 + x0, yx c0 + yy c1 + y0).
+// offset (c0, c1) are (xx c0 + xy c1 + x0, yx c0 + yy c1 + y0), x0 = xz + ox.
+// With h the high word of a coordinate, h - low < in: it lies inside the image's
+// last row and column whatever its rounding; neither h - low < out nor |h| < low:
+// outside the image.
 struct PlaneImage {
     double xx, xy, x0, yx, yy, y0, fill;
+    unsigned low, in, out;
     int map;
+    double xz, ox, yz, oy;
 };
 
 // A 16 x 16 square of a plane z per CTA, 8 x 8 per warp and two voxels per
 // thread (an 8 x 4 patch of voxels samples a patch of the image about as wide
 // in every direction; a row of 32 sampled up to 32 image rows), every image of
 // the batch in order; the map(s) read once and written once per batch.  Inside the image the four samples' weights sum to one, so
-// the reference's weighted mean is a bilinear interpolation in FP64; at its
-// last row and column, where samples are left out and the weights flip,
-// interpolate2 follows the reference.  Floor and fraction come from additions
+// the reference's weighted mean is a bilinear interpolation in FP64.  At its
+// border the last bit of a coordinate decides between a sample and the
+// background (and between two weightings in the last column), so there the
+// coordinates are the reference's products and sums one by one, and
+// interpolate2 follows its steps, also in the last row and column, where
+// samples are left out and the weights flip.  Floor and fraction come from additions
 // of 2^52, rounded down, instead of conversions.  Bound by the L1 reads of the
 // samples, then FP64 issue and the six float / double conversions a sample
 // (pixels stored as doubles 1.62 ms, as single floats 1.26).  200 images of
@@ -345,8 +353,18 @@ __global__ void __launch_bounds__(BP_THREADS) backproject_kernel(const float2* _
         for (int t = threadIdx.x; t < cnt; t += BP_THREADS) {
             const BpImage& q = par[k0 + t];
             PlaneImage& s = sp[t];
-            s.xx = q.m[0]; s.xy = q.m[1]; s.x0 = fma(q.m[2], c2, q.ox);
-            s.yx = q.m[3]; s.yy = q.m[4]; s.y0 = fma(q.m[5], c2, q.oy);
+            s.xx = q.m[0]; s.xy = q.m[1]; s.xz = dmul(q.m[2], c2); s.ox = q.ox;
+            s.yx = q.m[3]; s.yy = q.m[4]; s.yz = dmul(q.m[5], c2); s.oy = q.oy;
+            s.x0 = s.xz + q.ox;
+            s.y0 = s.yz + q.oy;
+            // the two forms of a coordinate differ by at most ten roundings
+            // (1.1e-16) of its terms' sum
+            const double e = 2e-15 * ((fabs(s.xx) + fabs(s.xy) + fabs(s.yx) + fabs(s.yy)) * o + fabs(s.xz) +
+                                      fabs(s.yz) + fabs(q.ox) + fabs(q.oy) + n);
+            s.low = __double2hiint(e) + 1;
+            const int last = __double2hiint((n - 1) - e);
+            s.in = last > (int)s.low ? last - s.low : 0u;
+            s.out = __double2hiint(n + e) + 1 - s.low;
             s.fill = q.fill;
             s.map = q.map;
         }
@@ -360,18 +378,19 @@ __global__ void __launch_bounds__(BP_THREADS) backproject_kernel(const float2* _
                 const double X = fma(q.xx, c0[u], fma(q.xy, c1[u], q.x0));
                 const double Y = fma(q.yx, c0[u], fma(q.yy, c1[u], q.y0));
                 double v = q.fill;
-                if (X >= 0 && X < n && Y >= 0 && Y < n) {
+                const unsigned hx = __double2hiint(X), hy = __double2hiint(Y);
+                if (hx - q.low < q.in && hy - q.low < q.in) {
                     const double tx = __dadd_rd(X, big), ty = __dadd_rd(Y, big);
                     const int ix = __double2loint(tx), iy = __double2loint(ty);
-                    if (ix < n - 1 && iy < n - 1) {
-                        const float2 a = __ldg(im + iy * n + ix), b = __ldg(im + (iy + 1) * n + ix);
-                        const double fx = X - (tx - big), fy = Y - (ty - big);
-                        const double top = fma(fx, (double)a.y - (double)a.x, (double)a.x);
-                        const double bot = fma(fx, (double)b.y - (double)b.x, (double)b.x);
-                        v = fma(fy, bot - top, top);
-                    } else {
-                        v = interpolate2(im, n, X, Y, q.fill);
-                    }
+                    const float2 a = __ldg(im + iy * n + ix), b = __ldg(im + (iy + 1) * n + ix);
+                    const double fx = X - (tx - big), fy = Y - (ty - big);
+                    const double top = fma(fx, (double)a.y - (double)a.x, (double)a.x);
+                    const double bot = fma(fx, (double)b.y - (double)b.x, (double)b.x);
+                    v = fma(fy, bot - top, top);
+                } else if ((hx - q.low < q.out || 2 * hx < 2 * q.low) && (hy - q.low < q.out || 2 * hy < 2 * q.low)) {
+                    const PlaneImage& p = sp[t];
+                    v = interpolate2(im, n, dadd(dadd(dadd(dmul(p.xx, c0[u]), dmul(p.xy, c1[u])), p.xz), p.ox),
+                                     dadd(dadd(dadd(dmul(p.yx, c0[u]), dmul(p.yy, c1[u])), p.yz), p.oy), p.fill);
                 }
                 if (q.map) acc1[u] = (float)((double)acc1[u] + v);
                 else acc0[u] = (float)((double)acc0[u] + v);
