@@ -6,6 +6,7 @@
 
 #include <math.h>
 #include <stdarg.h>
+#include <stdint.h>
 #include <stdio.h>
 #include <string.h>
 
@@ -690,7 +691,10 @@ int bsg_recon_finish(bsg_recon* h, int imap, float* map_out, float* fom_out, int
     if (rc) return rc;
     const bool sinc = (flags & BSG_SINC) != 0;
     const bool dev = (flags & BSG_DEVICE_PTR) != 0;
-    float* dst = dev ? map_out : r->d_map;
+    // (the last pass stores pairs of voxels: a destination on an odd float gets
+    // its map by a copy)
+    const bool direct = dev && (reinterpret_cast<uintptr_t>(map_out) & 7) == 0;
+    float* dst = direct ? map_out : r->d_map;
     const bool symz = !r->symz_orders.empty(), resc = r->rescale_std > 0;
     // with symmetrization after reconstruction (mode 1) and rescaling, the
     // sinc weight follows them, as breconstruct applies filter_sinc to the
@@ -720,7 +724,8 @@ int bsg_recon_finish(bsg_recon* h, int imap, float* map_out, float* fom_out, int
         r->stats.launches += 2;
     }
     const size_t N3 = r->vol_elems();
-    if (!dev) CK(cudaMemcpyAsync(map_out, r->d_map, sizeof(float) * N3, cudaMemcpyDeviceToHost, r->stream));
+    if (!direct) CK(cudaMemcpyAsync(map_out, r->d_map, sizeof(float) * N3,
+                                    dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, r->stream));
     if (fom_out) CK(cudaMemcpyAsync(fom_out, r->d_fom, sizeof(float) * N3,
                                     dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, r->stream));
     CK(cudaStreamSynchronize(r->stream));
