@@ -589,8 +589,12 @@ int bsg_recon_create(const bsg_recon_config* cfg, bsg_recon** out) {
     if (!rc && cudaHostGetDevicePointer((void**)&r->d_status, r->h_status, 0) != cudaSuccess)
         rc = fail(BSG_ERR_CUDA, "bsg_recon_create: status word mapping");
     if (!rc) *r->h_status = 0;
-    // (the shapes' tiles are at least 8 x 8 x 8 or 16 x 16 x 4 voxels)
-    const size_t most_tiles = (size_t)((N + 7) / 8) * ((N + 7) / 8) * ((N + 7) / 8);
+    size_t most_tiles = 0;                     // of any shape (8^3 voxels are two tiles of 16 x 16 x 4)
+    for (int i = 0; i < insert_num_shapes(); ++i) {
+        int tx, ty, tz;
+        insert_shape(i, &tx, &ty, &tz);
+        most_tiles = std::max(most_tiles, (size_t)((N + tx - 1) / tx) * ((N + ty - 1) / ty) * ((N + tz - 1) / tz));
+    }
     if (!rc) rc = alloc((void**)&r->d_tile_order, sizeof(int) * most_tiles);
     if (!rc) rc = alloc((void**)&r->d_arrived, sizeof(unsigned) * most_tiles);
     if (rc) { free_all(r); delete r; return rc; }
