@@ -38,6 +38,7 @@
 // box (once for all phases that walk that row), a warp scan turns the row
 // counts into offsets, and lanes take points in order.
 #include "context.cuh"
+#include "row_range.h"
 
 #include <math.h>
 
@@ -419,10 +420,10 @@ __device__ __forceinline__ void walk_groups(const DevParticle& P, const Pair& Q,
                     ha = fminf(ha, q + B.hi_a[i]);
                     hb = fminf(hb, q + B.hi_b[i]);
                 }
-                hmin = max(h_lo, Q.hc + __float2int_ru(la));
-                hmax = min(h_hi, Q.hc + __float2int_rd(hb));
-                sure = hmin > hmax || (hmin == max(h_lo, Q.hc + __float2int_ru(lb)) &&
-                                       hmax == min(h_hi, Q.hc + __float2int_rd(ha)));
+                const RowRange r = row_range(Q.hc, h_lo, h_hi, la, lb, ha, hb);
+                hmin = r.lo;
+                hmax = r.hi;
+                sure = r.sure;
             }
             if (__any_sync(0xffffffffu, !sure) && row) {
                 const int2 r = row_bounds<TX, TY, TZ>(P, k, h_lo, h_hi, ox, oy, oz, e);
