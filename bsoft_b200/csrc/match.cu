@@ -1286,7 +1286,11 @@ static cudaError_t ensure_padded(Match& M, cudaStream_t s) {
     if (M.refpad_valid) return cudaSuccess;
     if (!M.d_refpad) {
         const cudaError_t e = cudaMalloc(&M.d_refpad, sizeof(float2) * 2 * pad_elems(M.D));
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            cudaGetLastError();              // (the next launch's check would find it)
+            M.d_refpad = nullptr;
+            return e;
+        }
     }
     pad_reference_kernel<<<148 * 8, 256, 0, s>>>(M.d_ref, M.D, M.d_refpad);
     const cudaError_t e = cudaGetLastError();
@@ -1309,7 +1313,8 @@ static cudaError_t ensure_padded(Match& M, cudaStream_t s) {
 // pixel takes (integer instructions for half of the float-to-double conversions,
 // and pixels in compact tiles, which hit L1, changed nothing).  gridDim.y CTAs share a
 // view's pixels, so that a few hundred views fill the SMs evenly.  Positions
-// beyond the padding, and other kernel widths, take the general gather.
+// beyond the padding, other kernel widths, and all pixels when there are no
+// copies (pad null), take the general gather.
 __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureObject_t tex, int D, int wd,
                                                                    const float2* __restrict__ pad,
                                                                    const double* __restrict__ lut_g,
@@ -1342,7 +1347,7 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureOb
                 const int bx = (int)fx - 3 + lim, by = (int)fy - 3 + lim, bz = (int)fz - 3 + lim;
                 kxy = (int)((mx - fx) * NDIV + 0.5) | ((int)((my - fy) * NDIV + 0.5) << 16);
                 kz = (int)((mz - fz) * NDIV + 0.5);
-                general = wd != 8 || min(bx, min(by, bz)) < 0 || max(bx, max(by, bz)) > P - 8;
+                general = wd != 8 || !pad || min(bx, min(by, bz)) < 0 || max(bx, max(by, bz)) > P - 8;
                 at = general ? 0 : (bz * P + by) * P + bx;
             }
         }
@@ -1407,15 +1412,18 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureOb
 
 cudaError_t launch_secgather(Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s) {
     if (nv <= 0) return cudaSuccess;
+    // without memory for the copies (2.4 GB for a cut edge of 512) every pixel
+    // takes the general gather
     const cudaError_t e = ensure_padded(M, s);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return e;
+    const float2* const pad = M.refpad_valid ? M.d_refpad : nullptr;
     // CTAs per view: about eight waves of three CTAs per SM, each with at
     // least two blocks of 32 pixels per warp
     const int npix = (int)M.h_pix.size();
     const long most = std::max(1L, (long)npix / (64 * FOM_WARPS));
     const unsigned split = (unsigned)std::max(1L, std::min(most, 148L * 3 * 8 / nv));
     secgather_kernel<<<dim3((unsigned)nv, split), FOM_WARPS * 32, 0, s>>>(
-        M.ref_tex, M.D, M.wd, M.d_refpad, M.d_lut, M.d_pix, npix, d_mats, 1.0 / M.real_map, M.real_map, d_out);
+        M.ref_tex, M.D, M.wd, pad, M.d_lut, M.d_pix, npix, d_mats, 1.0 / M.real_map, M.real_map, d_out);
     return cudaGetLastError();
 }
 

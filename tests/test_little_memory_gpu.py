@@ -47,6 +47,18 @@ def _hypotheses(n):
     return [hypothesis(i % 2, r * np.linalg.det(r), (64.3, 63.6)) for i, r in enumerate(q)]
 
 
+def test_fp64_score_without_the_padded_copies():
+    """The FP64 gather's padded copies (40 MB here) do not fit: the gather
+    through the texture takes over (FP64 sums of 512 taps in another order:
+    1e-12 of the figure)."""
+    hyps = _hypotheses(27)
+    with _matcher() as m:
+        ref = m.score(hyps, fp64=True)                     # (loads the kernels, too)
+    with _matcher() as m, _leave(24 * MB):
+        got = m.score(hyps, fp64=True)
+    assert np.abs(got[0] - ref[0]).max() < 1e-11 and np.abs(got[1] - ref[1]).max() < 1e-11
+
+
 def test_repeated_fp64_scores_allocate_nothing():
     hyps = _hypotheses(60)
     with _matcher() as m:
