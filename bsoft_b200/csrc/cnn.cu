@@ -1428,18 +1428,24 @@ extern "C" int bsg_cnn_predict(bsg_cnn* h, const float* images, long n, float* o
     // blocks for 148 SMs.
     int B = std::max(1, std::min<int>(c->cfg.batch > 0 ? c->cfg.batch : 256, (int)std::min<long>(n, 1 << 20)));
     const long wide = std::min<long>(std::min<long>(n, 16384), (long)(1500000000 / image_bytes(*c)));
-    int rc = BSG_OK;
-    if (wide > B && ensure_batch(*c, (int)wide) == BSG_OK) {
+    const size_t npix = (size_t)c->cfg.box * c->cfg.box;
+    const bool dev = (flags & BSG_DEVICE_PTR) != 0;
+    // the activations of b images, and host images' copy
+    auto room = [&](int b) {
+        const int rc = ensure_batch(*c, b);
+        return rc || dev ? rc : ensure_src(*c, npix * b);
+    };
+    if (wide > B && room((int)wide) == BSG_OK) {
         B = (int)wide;
     } else {
-        cudaGetLastError();                      // the wide buffers did not fit
-        rc = ensure_batch(*c, B);
+        if (wide > B) {                          // they did not fit together
+            cudaGetLastError();
+            free_forward(*c);
+        }
+        const int rc = room(B);
         if (rc) return rc;
     }
-    const int npix = c->cfg.box * c->cfg.box;
     cudaStream_t s = c->stream;
-    const bool dev = (flags & BSG_DEVICE_PTR) != 0;
-    if (!dev && (rc = ensure_src(*c, (size_t)npix * B))) return rc;
     cudaError_t e = cudaSuccess;
     for (long b0 = 0; e == cudaSuccess && b0 < n; b0 += B) {
         const int cnt = (int)std::min<long>(B, n - b0);

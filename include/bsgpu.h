@@ -507,7 +507,7 @@ typedef struct {
     int    box;            /* image edge: power of two, 64..512             */
     int    channels[6];    /* output channels of the 6 convolutions         */
     int    hidden;         /* width of the dense layer                      */
-    int    batch;          /* mini-batch (training) / chunk (inference)     */
+    int    batch;          /* mini-batch (training); inference: see predict */
     float  shift_weight;   /* lambda of the shift term of the loss          */
     int    device;
     unsigned long long seed;   /* initialisation and batch sampling         */
@@ -520,7 +520,10 @@ void bsg_cnn_destroy(bsg_cnn* c);
 long bsg_cnn_num_params(const bsg_cnn* c);
 int  bsg_cnn_get_params(bsg_cnn* c, float* out);
 int  bsg_cnn_set_params(bsg_cnn* c, const float* in);      /* resets the optimiser */
-/* n images (box^2 float32 each) -> n x BSG_CNN_RESULT_FLOATS */
+/* n images (box^2 float32 each) -> n x BSG_CNN_RESULT_FLOATS.  They are taken
+ * cfg.batch at a time, or more where up to 1.5 GB of activations hold more and
+ * there is memory for that; the buffers stay with the context.  An image's
+ * result does not depend on the pass it is in. */
 int  bsg_cnn_predict(bsg_cnn* c, const float* images, long n, float* out, int flags);
 /* mean loss and its gradient (all parameters) for n host images with host
  * targets (n x BSG_CNN_RESULT_FLOATS: true rotation and shift) */

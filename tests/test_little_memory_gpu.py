@@ -68,3 +68,18 @@ def test_repeated_fp64_scores_allocate_nothing():
             few = m.score(hyps[:3], fp64=True)
     assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
     assert np.array_equal(few[0], ref[0][:3])
+
+
+def test_proposer_goes_back_to_its_batch():
+    """The wide pass's activations fit, the copy of the host images beside
+    them does not: passes of the context's batch give the same poses."""
+    from bsoft_b200.cnn import Proposer
+    images = np.random.default_rng(6).normal(size=(1024, 128, 128)).astype(np.float32)
+    with Proposer(box=128, batch=8, seed=3) as p:
+        free, _ = torch.cuda.mem_get_info()
+        ref = p.predict(images)
+        used = free - torch.cuda.mem_get_info()[0]
+    assert used > 64 * MB                                  # (the images' copy alone)
+    with Proposer(box=128, batch=8, seed=3) as p, _leave(used - 32 * MB):
+        got = p.predict(images)
+    assert np.array_equal(got, ref)
