@@ -18,7 +18,11 @@ namespace bsg {
 
 static thread_local char g_err[1024] = "";
 
+// The message of a failed call.  A failed allocation or launch stays the
+// runtime's last error until it is read, and the next call's first launch check
+// would find it: it is read here.
 void set_error(const char* fmt, ...) {
+    cudaGetLastError();
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(g_err, sizeof(g_err), fmt, ap);
@@ -69,6 +73,7 @@ struct Recon : Context {
 static bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
 static int fail(int code, const char* fmt, ...) {
+    cudaGetLastError();                      // (set_error)
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(g_err, sizeof(g_err), fmt, ap);
@@ -208,6 +213,7 @@ static int set_shape(Recon* r, int shape) {
     if (r->d_part_sums) { cudaFree(r->d_part_sums); r->d_part_sums = nullptr; }
     if (cudaMalloc((void**)&r->d_part_sums, need) != cudaSuccess) {
         // not enough memory for replicas: run each tile in one warp
+        cudaGetLastError();
         r->d_part_sums = nullptr;
         R = 1;
     }

@@ -83,3 +83,46 @@ def test_proposer_goes_back_to_its_batch():
     with Proposer(box=128, batch=8, seed=3) as p, _leave(used - 32 * MB):
         got = p.predict(images)
     assert np.array_equal(got, ref)
+
+
+def test_failed_allocations_do_not_fail_the_next_call():
+    """A call that ran out of memory leaves nothing behind for the next ones."""
+    from bsoft_b200._lib import BsgError
+    hyps = _hypotheses(3)
+    with _matcher() as m:
+        ref = m.score(hyps, fp64=True)
+        with _leave(64 * MB), pytest.raises(BsgError):
+            m.set_panel(np.tile(np.eye(3), (100000, 1, 1)))
+        with _matcher() as other:
+            got = other.score(hyps, fp64=True)
+        again = m.score(hyps, fp64=True)
+    assert np.array_equal(got[0], ref[0]) and np.array_equal(again[0], ref[0])
+
+
+def test_gridding_without_replicas():
+    """Without memory for the replicas' partial sums one warp grids a tile: the
+    same contributions in one FP32 sum instead of several (1e-6 of the norm)."""
+    from bsoft_b200.recon import Reconstructor
+    from bsoft_b200.plan import P_CTF, P_MAT, P_ORIGIN, P_PIXEL, P_SCALE, P_WEIGHT, ReconPlan
+    rng = np.random.default_rng(8)
+    q, _ = np.linalg.qr(rng.normal(size=(60, 3, 3)))
+    rec = np.zeros((60, 32))
+    rec[:, P_MAT:P_MAT + 9] = (q * np.linalg.det(q)[:, None, None]).reshape(60, 9)
+    rec[:, P_ORIGIN:P_ORIGIN + 2] = 64
+    rec[:, P_PIXEL] = 1.5
+    rec[:, P_SCALE] = rec[:, P_WEIGHT] = 1
+    rec[:, P_CTF + 1] = -500.0
+    plan = ReconPlan(n=128, ft=256, map=128, map_sampling=1.5, hi_res=1.0, interp=2, ctf_action=0, wiener=0.0, params=rec,
+                     nmaps=1)
+    images = rng.normal(size=(60, 128, 128)).astype(np.float32)
+    free, _ = torch.cuda.mem_get_info()
+    with Reconstructor(plan, batch=64) as r:
+        used = free - torch.cuda.mem_get_info()[0]
+        r.insert(images, rec)
+        v, w = r.accumulators(0)
+    assert used > 400 * MB                                 # 16 replicas of 25 MB among it
+    with _leave(used - 200 * MB), Reconstructor(plan, batch=64) as r:
+        r.insert(images, rec)
+        v1, w1 = r.accumulators(0)
+    assert np.linalg.norm(w1 - w) < 1e-6 * np.linalg.norm(w)
+    assert np.linalg.norm((v1 - v).ravel()) < 1e-6 * np.linalg.norm(v.ravel())
