@@ -8,21 +8,6 @@
 
 namespace bsg {
 
-constexpr int MAX_PHASES = 16;
-constexpr int CANDIDATES = 220;          // lattices (lh, lk, sh) with lh lk <= 16
-
-// candidate number c: by phases lh lk, then rows lk, then shift
-__device__ __forceinline__ PhaseLattice candidate(int c) {
-    for (int d = 1; d <= MAX_PHASES; ++d)
-        for (int lk = 1; lk <= d; ++lk) {
-            if (d % lk) continue;
-            const int lh = d / lk;
-            if (c < lh) return {lh, lk, c};
-            c -= lh;
-        }
-    return {0, 0, 0};
-}
-
 __global__ void __launch_bounds__(128) lattice_kernel(DevParticle* part, TileTest* tests, long n,
                                                        double mscale, int ft) {
     const long r = blockIdx.x * 4L + (threadIdx.x >> 5);
@@ -37,8 +22,8 @@ __global__ void __launch_bounds__(128) lattice_kernel(DevParticle* part, TileTes
     const double reach = lattice_reach(ad, bd, curve);
     PhaseLattice best = square_lattice(reach);
     if (reach < 64.0)
-        for (int c0 = 0; c0 < CANDIDATES; c0 += 32) {
-            const PhaseLattice l = candidate(c0 + lane);
+        for (int c0 = 0; c0 < LATTICE_CANDIDATES; c0 += 32) {
+            const PhaseLattice l = lattice_candidate(c0 + lane);
             const bool ok = l.lh > 0 && lattice_ok(ad, bd, l.lh, l.lk, l.sh, reach, curve);
             const unsigned some = __ballot_sync(0xffffffffu, ok);
             if (!some) continue;

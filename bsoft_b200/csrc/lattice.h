@@ -1,5 +1,5 @@
-// lattice.h - the phase lattice of the gridding scatter, chosen per particle
-// (plain C++ on the host; lattice.cu runs the same arithmetic on the device).
+// lattice.h - the phase lattice of the gridding scatter, chosen per particle on
+// the device (lattice.cu); plain C++ on the host for the tests.
 //
 // The gridding kernel walks a particle's pixels phase by phase: the pixels
 // (h0 + lh i + sh j, k0 + lk j) of one phase are gridded by the 32 lanes of
@@ -101,19 +101,38 @@ BSG_LATTICE_FN bool lattice_ok(const double ad[3], const double bd[3], int lh, i
     return true;
 }
 
-// The safe lattice with the fewest phases lh * lk (up to max_phases; fewest
-// rows lk first, then the smallest shift), else the square lattice of side
-// ceil(reach), which no vector shorter than `reach` belongs to; {0, 0, 0}
-// when that side would not fit the 12-bit fields of pack_lattice.
-// curve: bound on the extra displacement (voxels per pixel step of the
-// lattice vector) of a curved insertion surface; 0 for the plane.
+// The square lattice of side ceil(reach), which no vector shorter than `reach`
+// belongs to; {0, 0, 0} when that side would not fit the 12-bit fields of
+// pack_lattice.
 BSG_LATTICE_FN PhaseLattice square_lattice(double reach) {
     if (!(reach < 4095.0)) return {0, 0, 0};
     const int L = (int)ceil(reach);
     return {L > 1 ? L : 1, L > 1 ? L : 1, 0};
 }
 
-inline PhaseLattice choose_lattice(const double ad[3], const double bd[3], int max_phases = 16, double curve = 0.0) {
+constexpr int LATTICE_PHASES = 16;           // most phases lh * lk tried
+constexpr int LATTICE_CANDIDATES = 220;      // lattices (lh, lk, sh) with lh lk <= 16
+
+// Lattice number c in the order of preference: fewest phases lh lk, then
+// fewest rows lk, then the smallest shift ({0, 0, 0} past the last).
+BSG_LATTICE_FN PhaseLattice lattice_candidate(int c) {
+    for (int d = 1; d <= LATTICE_PHASES; ++d)
+        for (int lk = 1; lk <= d; ++lk) {
+            if (d % lk) continue;
+            const int lh = d / lk;
+            if (c < lh) return {lh, lk, c};
+            c -= lh;
+        }
+    return {0, 0, 0};
+}
+
+// The safe lattice with the fewest phases (up to max_phases; lattice_candidate's
+// order), else the square one.  lattice.cu makes this choice on the device, 32
+// candidates at a time; this form is what the tests hold it to.
+// curve: bound on the extra displacement (voxels per pixel step of the
+// lattice vector) of a curved insertion surface; 0 for the plane.
+inline PhaseLattice choose_lattice(const double ad[3], const double bd[3], int max_phases = LATTICE_PHASES,
+                                   double curve = 0.0) {
     const double reach = lattice_reach(ad, bd, curve);
     if (reach < 64.0) {
         for (int d = 1; d <= max_phases; ++d)
