@@ -23,7 +23,7 @@
 // one elected thread issues tcgen05.mma (M=128, N=256, K=16) into one of two
 // 256-column TMEM accumulators while four epilogue warps read the other with
 // tcgen05.ld and keep each row's 8 best columns in registers.  The M tiles
-// are taken in groups; the CTAs of a group are a grid of its M tiles by
+// are taken in groups (search_runs.h; short panels are cut into runs instead); the CTAs of a group are a grid of its M tiles by
 // stretches of N, so that those of one stretch read the same B tiles at the
 // same time and all share the group's A tiles through L2.  Groups of 21, seven
 // and four M tiles (7, 21 and 37 stretches) keep 147 and 148 of the 148 SMs at
@@ -34,9 +34,10 @@
 // work items a group (the last of six rounds nearly empty) 7.70, sevens and
 // fours 7.21, with 21s 7.04 ms; 2,048 images against 550,320 sections: 523,
 // 568 and 522 ms of GEMM.  One run of tiles per CTA regardless of the
-// stretches, evener still, 7.70: B is then read by one CTA at a time.  A CTA carries its rows' top-8 along its
-// stretch.  Every wait is bounded (2 s) and reports through a status word.
+// stretches, evener still, 7.70: B is then read by one CTA at a time.  A CTA
+// carries its rows' top-8 along its stretch.  Every wait is bounded (2 s) and reports through a status word.
 #include "match.cuh"
+#include "search_runs.h"
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -148,66 +149,12 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// The work of each CTA: in group g (M tiles first(g) .. first(g + 1) - 1) CTA c
-// takes M tile c % size of it and the N tiles of stretch c / size.
-struct Runs {
-    int mtiles, ntiles, ctas;
-    int groups, large, sevens;        // large groups of 21, then sevens, then fours; sevens < 0: groups of
-                                      // nearly equal sizes
-
-    __host__ __device__ static Runs plan(int mtiles, int ntiles) {
-        Runs r{mtiles, ntiles, 148, 0, 0, -1};
-        for (int four = 0; four < 7 && r.sevens < 0; ++four)
-            if (mtiles >= 4 * four && (mtiles - 4 * four) % 7 == 0) {
-                r.sevens = (mtiles - 4 * four) / 7;
-                r.large = r.sevens / 3;
-                r.sevens -= 3 * r.large;
-                r.groups = r.large + r.sevens + four;
-            }
-        if (r.sevens < 0) r.groups = (mtiles + 6) / 7;     // below 18, where sevens and fours do not add up
-        return r;
-    }
-    __host__ __device__ int first(int g) const {
-        if (sevens < 0) return (int)((long)g * mtiles / groups);
-        if (g <= large) return 21 * g;
-        g -= large;
-        return 21 * large + (g <= sevens ? 7 * g : 7 * sevens + 4 * (g - sevens));
-    }
-    __host__ __device__ int size(int g) const { return first(g + 1) - first(g); }
-    __host__ __device__ int stretches(int g) const { return ctas / size(g); }
-    // first N tile of stretch r
-    __host__ __device__ int bound(int g, int r) const {
-        const int n = stretches(g);
-        return (int)(((long)r * ntiles + (long)g * n / groups) / n);
-    }
-    __host__ __device__ int group_of(int mtile) const {
-        if (sevens >= 0) {
-            if (mtile < 21 * large) return mtile / 21;
-            const int m = mtile - 21 * large;
-            return large + (m < 7 * sevens ? m / 7 : sevens + (m - 7 * sevens) / 4);
-        }
-        int g = (int)((long)mtile * groups / mtiles);
-        while (first(g) > mtile) --g;
-        while (first(g + 1) <= mtile) ++g;
-        return g;
-    }
-    // CTA c's M tile and N tiles in group g; false: none
-    __host__ __device__ bool work(int g, int c, int& m, int& n0, int& n1) const {
-        const int sz = size(g), r = c / sz;
-        if (r >= stretches(g)) return false;
-        m = first(g) + c % sz;
-        n0 = bound(g, r);
-        n1 = bound(g, r + 1);
-        return n0 < n1;
-    }
-};
-
 struct GemmArgs {
     int kblocks;          // K / 64
     int ncols;            // valid columns (sections)
     Runs runs;            // the batch's M tiles by ceil(ncols / 256) N tiles
     long prow;            // row stride of the partial buffers (batch height)
-    float* part_score;    // [stretch][prow][TOPK]
+    float* part_score;    // [slot][prow][TOPK]
     int* part_idx;
     int* status;
 };
@@ -372,7 +319,7 @@ search_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             }
             if (!ok) break;
             const long row = (long)mtile * BM + quarter * 32 + lane;
-            const long o = ((long)(blockIdx.x / runs.size(g)) * a.prow + row) * TOPK;
+            const long o = ((long)runs.slot(g, blockIdx.x) * a.prow + row) * TOPK;
 #pragma unroll
             for (int t = 0; t < TOPK; ++t) { a.part_score[o + t] = top.s[t]; a.part_idx[o + t] = top.i[t]; }
         }
@@ -527,9 +474,8 @@ __global__ void __launch_bounds__(256) rows_kernel(const float2* __restrict__ sp
 // order; a pick is the largest of the threads' first ones.  Bound by the reads'
 // latency, hence 1,024 threads for a few images.  (256 images of 25 origins:
 // read again for every pick by one warp per image 0.42 ms, by 256 threads from
-// shared memory 0.07, now 0.04; 5 images against 8,580 sections, 29,600
-// candidates an image, 0.84 by the warp and 1.27 when they exceeded shared
-// memory, now 0.08.)
+// shared memory 0.07, now 0.04; 5 images against 8,580 sections, 0.84 by the
+// warp, 0.08 with 148 places a row, most of them empty, now 34 and 0.02.)
 constexpr int MERGE_MOST = 1024;
 
 typedef unsigned __int128 wide_t;
@@ -554,27 +500,24 @@ __global__ void __launch_bounds__(sizeof(K) == 8 ? MERGE_MOST : MERGE_MOST / 2)
     K top[TOPK];                                 // this thread's best, largest first
 #pragma unroll
     for (int i = 0; i < TOPK; ++i) top[i] = 0;
-    // a row's stretches and places, a row after the other: thread t takes every
+    // a row's slots and places, a row after the other: thread t takes every
     // blockDim.x-th of the image's candidates
     int e = threadIdx.x, s = 0;
     long row = (long)blockIdx.x * nshift;
-    int g = runs.group_of((int)(row / BM)), n = runs.stretches(g) * TOPK;
+    int n = runs.slots((int)(row / BM)) * TOPK;
     while (s < nshift) {
         if (e >= n) {
             e -= n;
             if (++s == nshift) break;
             ++row;
-            if (row % BM == 0) {
-                g = runs.group_of((int)(row / BM));
-                n = runs.stretches(g) * TOPK;
-            }
+            if (row % BM == 0) n = runs.slots((int)(row / BM)) * TOPK;
             continue;
         }
         const int r = e / TOPK;
         const long o = ((long)r * mrows + row) * TOPK + e % TOPK;
         const int sec = __ldg(pi + o);
         const float score = __ldg(ps + o);
-        if (sec >= 0 && runs.bound(g, r) < runs.bound(g, r + 1)) {
+        if (sec >= 0) {
             unsigned u = __float_as_uint(score);
             u ^= (u >> 31) ? 0xffffffffu : 0x80000000u;         // sorts as the float does
             K v = (K)u << HALF | (LOW - ((K)sec * nshift + s));
@@ -1138,13 +1081,13 @@ extern "C" int bsg_match_search(bsg_match* h, const double* origins, int norigin
     const Runs full = Runs::plan(mtiles_max, ntiles);
     const long tail_rows = ((M->nimg - 1) % nb + 1) * norigin;             // the last batch
     const Runs tail = Runs::plan((int)((tail_rows + BM - 1) / BM), ntiles);
-    long stretches = 1;
+    long slots = 1;
     for (const Runs* r : {&full, &tail})
-        for (int g = 0; g < r->groups; ++g) stretches = std::max(stretches, (long)r->stretches(g));
+        for (int m = 0; m < r->mtiles; ++m) slots = std::max(slots, (long)r->slots(m));
 
     // scratch (kept between calls)
     const size_t need_A = (size_t)mrows * kpad;
-    const size_t need_part = (size_t)stretches * mrows * TOPK;
+    const size_t need_part = (size_t)slots * mrows * TOPK;
     const size_t need_cand = (size_t)M->nimg * topk;
     if (need_A > M->a_elems) {
         cudaFree(M->d_A); M->d_A = nullptr; M->a_elems = 0;
