@@ -1313,18 +1313,21 @@ static cudaError_t ensure_padded(Match& M, cudaStream_t s) {
 // pixel takes (integer instructions for half of the float-to-double conversions,
 // and pixels in compact tiles, which hit L1, changed nothing).  gridDim.y CTAs share a
 // view's pixels, so that a few hundred views fill the SMs evenly.  Positions
-// beyond the padding, other kernel widths, and all pixels when there are no
-// copies (pad null), take the general gather.
-__global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureObject_t tex, int D, int wd,
+// beyond the padding take the general gather; so do all with other kernel widths
+// and without the copies, in a kernel of its own (PADDED false), whose registers
+// let more warps wait for the texture unit.
+template <bool PADDED>
+__global__ void __launch_bounds__(FOM_WARPS * 32, PADDED ? 2 : 3) secgather_kernel(cudaTextureObject_t tex, int D, int wd,
                                                                    const float2* __restrict__ pad,
                                                                    const double* __restrict__ lut_g,
                                                                    const MPix* __restrict__ pix, int npix,
-                                                                   const double* __restrict__ mats, double inv,
-                                                                   double real, double2* __restrict__ out) {
+                                                                   const double* __restrict__ mats, int stride,
+                                                                   double inv, double real,
+                                                                   double2* __restrict__ out) {
     __shared__ __align__(16) double lut[(NDIV + 1) * MAXW];
     for (int i = threadIdx.x; i < (NDIV + 1) * wd; i += blockDim.x) lut[i] = lut_g[i];
     __syncthreads();
-    const double* m = mats + 9 * (long)blockIdx.x;
+    const double* m = mats + stride * (long)blockIdx.x;
     const int warp = blockIdx.y * FOM_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int P = pad_edge(D), lim = D / 2 + HALO;
     const int xp = lane & 3, yl = lane >> 2;
@@ -1338,7 +1341,9 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureOb
         bool general = false;
         if (lane < cnt) {
             const MPix pq = pix[base + lane];
-            if (pq.insec) {
+            if constexpr (!PADDED) {
+                general = pq.insec;
+            } else if (pq.insec) {
                 const double ix = pq.h * inv, iy = pq.k * inv;
                 const double mx = (m[0] * ix + m[1] * iy) * real;
                 const double my = (m[3] * ix + m[4] * iy) * real;
@@ -1347,13 +1352,13 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureOb
                 const int bx = (int)fx - 3 + lim, by = (int)fy - 3 + lim, bz = (int)fz - 3 + lim;
                 kxy = (int)((mx - fx) * NDIV + 0.5) | ((int)((my - fy) * NDIV + 0.5) << 16);
                 kz = (int)((mz - fz) * NDIV + 0.5);
-                general = wd != 8 || !pad || min(bx, min(by, bz)) < 0 || max(bx, max(by, bz)) > P - 8;
+                general = min(bx, min(by, bz)) < 0 || max(bx, max(by, bz)) > P - 8;
                 at = general ? 0 : (bz * P + by) * P + bx;
             }
         }
         const unsigned far = __ballot_sync(0xffffffffu, general);
-        const unsigned live = __ballot_sync(0xffffffffu, at >= 0) & ~far;
-        for (int q0 = 0; q0 < cnt; q0 += 8) {
+        const unsigned live = PADDED ? __ballot_sync(0xffffffffu, at >= 0) & ~far : 0u;
+        for (int q0 = 0; PADDED && q0 < cnt; q0 += 8) {
             if (!((live >> q0) & 255u)) continue;
             double t[16];
 #pragma unroll
@@ -1410,20 +1415,23 @@ __global__ void __launch_bounds__(FOM_WARPS * 32) secgather_kernel(cudaTextureOb
     }
 }
 
-cudaError_t launch_secgather(Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s) {
+cudaError_t launch_secgather(Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s, int stride) {
     if (nv <= 0) return cudaSuccess;
     // without memory for the copies (2.4 GB for a cut edge of 512) every pixel
     // takes the general gather
-    const cudaError_t e = ensure_padded(M, s);
+    const cudaError_t e = M.wd == 8 ? ensure_padded(M, s) : cudaErrorMemoryAllocation;
     if (e != cudaSuccess && e != cudaErrorMemoryAllocation) return e;
-    const float2* const pad = M.refpad_valid ? M.d_refpad : nullptr;
     // CTAs per view: about eight waves of three CTAs per SM, each with at
     // least two blocks of 32 pixels per warp
     const int npix = (int)M.h_pix.size();
     const long most = std::max(1L, (long)npix / (64 * FOM_WARPS));
     const unsigned split = (unsigned)std::max(1L, std::min(most, 148L * 3 * 8 / nv));
-    secgather_kernel<<<dim3((unsigned)nv, split), FOM_WARPS * 32, 0, s>>>(
-        M.ref_tex, M.D, M.wd, pad, M.d_lut, M.d_pix, npix, d_mats, 1.0 / M.real_map, M.real_map, d_out);
+    auto launch = [&](auto kernel) {
+        kernel<<<dim3((unsigned)nv, split), FOM_WARPS * 32, 0, s>>>(M.ref_tex, M.D, M.wd, M.d_refpad, M.d_lut, M.d_pix, npix,
+                                                                   d_mats, stride, 1.0 / M.real_map, M.real_map, d_out);
+    };
+    if (e == cudaSuccess) launch(secgather_kernel<true>);
+    else launch(secgather_kernel<false>);
     return cudaGetLastError();
 }
 
@@ -1602,6 +1610,20 @@ int ensure_groups(Match& M, long ng, int outs) {
     }
     return BSG_OK;
 }
+
+cudaError_t ensure_views(Match& M, long nv) {
+    if (nv <= M.rview_cap) return cudaSuccess;
+    cudaFree(M.d_rmats);
+    cudaFree(M.d_rsec);
+    M.d_rmats = nullptr;
+    M.d_rsec = nullptr;
+    M.rview_cap = 0;
+    cudaError_t e = cudaMalloc(&M.d_rmats, sizeof(double) * 9 * nv);
+    if (e == cudaSuccess) e = cudaMalloc(&M.d_rsec, sizeof(double2) * std::max<size_t>(1, M.h_pix.size()) * nv);
+    if (e == cudaSuccess) M.rview_cap = nv;
+    else cudaGetLastError();                 // (the next launch's check would find it)
+    return e;
+}
 }  // namespace bsg
 
 extern "C" int bsg_match_sections(bsg_match* h, const double* mats, long nviews, float* out, int flags) {
@@ -1772,27 +1794,32 @@ extern "C" int bsg_match_score(bsg_match* h, const double* hyps, long nhyp, doub
     cudaStream_t s = M->stream;
     const bool dpr = (flags & BSG_MATCH_SCORE_DPR) != 0;
     if (flags & BSG_MATCH_SCORE_FP64) {
-        // as many groups' FP64 sections at a time as the work buffer holds (the
-        // reference's transform went through it: map edge^3 elements at least);
-        // their views take the place of the hypotheses.  With buffers of its
-        // own, allocated and freed in every call, 27 hypotheses of 64^2 took
-        // 0.78 ms, now 0.13.
-        const long npix = (long)M->h_pix.size();
-        const long chunk = std::max(1L, std::min(ng, (long)M->work_elems / std::max(npix, 1L)));
-        std::vector<double> mats(9 * ng);
-        for (long g = 0; g < ng; ++g) {
-            memcpy(&mats[9 * g], groups[g].m, sizeof(groups[g].m));
-            groups[g].sec = (int)(g % chunk);
+        // the groups' FP64 sections: in the work buffer when it holds them all
+        // (the reference's transform went through it: map edge^3 elements at
+        // least), else in refinement's kept buffer, up to ~1 GB at a time, or,
+        // without memory for that, as many as the work buffer holds.  (In a
+        // buffer allocated and freed in every call 27 hypotheses of 64^2 took
+        // 0.78 ms, now 0.13; 2,000 of 32^2 took 0.43 in pieces of 68 through the
+        // work buffer.)
+        const long npix = std::max(1L, (long)M->h_pix.size());
+        long chunk = std::max(1L, std::min(ng, (long)M->work_elems / npix));
+        double2* d_sec = M->d_work;
+        if (chunk < ng) {
+            const long wide = std::min(ng, (1L << 30) / ((long)sizeof(double2) * npix));
+            if (wide > chunk && ensure_views(*M, wide) == cudaSuccess) {
+                chunk = wide;
+                d_sec = M->d_rsec;
+            }
         }
-        static_assert(sizeof(MHyp) >= 9 * sizeof(double), "views in the hypotheses' buffer");
-        double* const d_mats = reinterpret_cast<double*>(M->d_hyp);
+        for (long g = 0; g < ng; ++g) groups[g].sec = (int)(g % chunk);
         MCK(cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s));
-        MCK(cudaMemcpyAsync(d_mats, mats.data(), sizeof(double) * 9 * ng, cudaMemcpyHostToDevice, s));
+        static_assert(offsetof(MHypG, m) == 0 && sizeof(MHypG) % sizeof(double) == 0, "a group starts with its view");
         for (long g0 = 0; g0 < ng; g0 += chunk) {
             const long cnt = std::min(chunk, ng - g0);
-            MCK(launch_secgather(*M, d_mats + 9 * g0, cnt, M->d_work, s));
+            MCK(launch_secgather(*M, reinterpret_cast<const double*>(M->d_grp + g0), cnt, d_sec, s,
+                                 (int)(sizeof(MHypG) / sizeof(double))));
             MCK(launch_fom(*M, M->d_grp + g0, cnt, M->d_gout + g0 * MAXORG, M->d_gout + (ng + g0) * MAXORG, s, true,
-                           nullptr, M->d_work, dpr));
+                           nullptr, d_sec, dpr));
         }
     } else {
         MCK(cudaMemcpyAsync(M->d_grp, groups.data(), sizeof(MHypG) * ng, cudaMemcpyHostToDevice, s));

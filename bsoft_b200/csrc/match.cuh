@@ -241,7 +241,8 @@ struct Match {
     double* d_gout = nullptr;          // their figures of merit and cross-validation figures
     long grp_cap = 0, gout_cap = 0;
     // refinement's buffers, kept between calls (grow-only; the sections at
-    // most ~1 GB, a chunk's): views, gathered sections, CTF trial rows
+    // most ~1 GB, a chunk's; FP64 scores of many hypotheses use them too):
+    // views, gathered sections, CTF trial rows
     double* d_rmats = nullptr;
     double2* d_rsec = nullptr;
     float* d_rctf = nullptr;
@@ -302,14 +303,16 @@ cudaError_t launch_fom_trials(const Match& M, const MHypG* d_groups, long ng, in
 // as fom_kernel<float> gathers them: nsec x npix float2 (0 where a pixel is
 // outside the section)
 cudaError_t launch_panel_exact(const Match& M, const MHyp* d_secs, long nsec, float2* d_out, cudaStream_t s);
-// FP64 section values of nv views (9 doubles each, MHyp's scaled rows) at
-// the figure-of-merit pixels: nv x npix double2
-cudaError_t launch_secgather(Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s);
+// FP64 section values of nv views (9 doubles each, MHyp's scaled rows, `stride`
+// doubles apart) at the figure-of-merit pixels: nv x npix double2
+cudaError_t launch_secgather(Match& M, const double* d_mats, long nv, double2* d_out, cudaStream_t s, int stride = 9);
 // CTF table rows (npix floats each) for nrec records on the device
 cudaError_t launch_ctf_rows(const Match& M, const ImgCtf* d_rec, long nrec, float* d_out, cudaStream_t s);
 void group_hypotheses(const std::vector<MHyp>& hyps, std::vector<MHypG>& groups, std::vector<long>& slot);
 // room for ng groups and `outs` figures of merit each
 int ensure_groups(Match& M, long ng, int outs = MAXORG);
+// room for nv views (d_rmats) and their gathered sections (d_rsec)
+cudaError_t ensure_views(Match& M, long nv);
 // view matrix rows 0, 1 scaled by the sampling ratio (img_fit_in_recip_space_grid)
 void match_view_rows(const Match& M, const double* mat, double* m);
 int match_fail(int code, const char* fmt, ...);

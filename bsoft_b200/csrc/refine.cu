@@ -398,17 +398,7 @@ extern "C" int bsg_match_refine(bsg_match* h, const double* start, long nstart, 
     int rc = BSG_OK;
     {
         // chunk x 27 views (9 doubles each) and their gathered sections
-        const long nvmax = std::min(nstart, chunk) * NVIEW;
-        if (nvmax > M->rview_cap) {
-            cudaFree(M->d_rmats);
-            cudaFree(M->d_rsec);
-            M->d_rmats = nullptr;
-            M->d_rsec = nullptr;
-            M->rview_cap = 0;
-            ce = cudaMalloc(&M->d_rmats, sizeof(double) * 9 * nvmax);
-            if (ce == cudaSuccess) ce = cudaMalloc(&M->d_rsec, sizeof(double2) * (size_t)npix * nvmax);
-            if (ce == cudaSuccess) M->rview_cap = nvmax;
-        }
+        ce = ensure_views(*M, std::min(nstart, chunk) * NVIEW);
         if (ce != cudaSuccess) {
             cudaEventDestroy(e0);
             cudaEventDestroy(e1);
