@@ -3,6 +3,7 @@
 // pipeline (image upload, 2-D stage, gridding) and map finishing.
 #include "context.cuh"
 #include "fft_dev.cuh"
+#include "lattice.h"
 
 #include <math.h>
 #include <stdarg.h>
@@ -59,6 +60,7 @@ struct Recon : Context {
     DevParticle* d_psymbuf[2] = {nullptr, nullptr};
     size_t psymbuf_cap[2] = {0, 0};
     TileTest* d_testbuf[2] = {nullptr, nullptr};        // tile tests of the records that are gridded
+    const TileTest* d_test = nullptr;                   // the current batch's: there, or behind its records
     size_t testbuf_cap[2] = {0, 0};
     float2* d_specbuf[2] = {nullptr, nullptr};
     cudaEvent_t copy_done[2] = {nullptr, nullptr};
@@ -327,7 +329,7 @@ static int run_batch_kernels(Recon* r, int buf, const float* d_img, long np, boo
     if (!insert) return BSG_OK;
     for (int h = 0; h < r->nhalves; ++h) {
         if (r->timing) { cudaEventCreate(&a); cudaEventCreate(&b); cudaEventRecord(a, s); }
-        CK(launch_insert(*r, spec_out, r->nexp > 0 ? r->d_psym : r->d_part, r->d_testbuf[buf],
+        CK(launch_insert(*r, spec_out, r->nexp > 0 ? r->d_psym : r->d_part, r->d_test,
                          (int)(r->nexp > 0 ? r->nexp : np), r->nhalves == 2 ? h : -1, s));
         if (r->timing) { cudaEventRecord(b, s); r->timed.push_back({a, b, 0}); }
         r->stats.launches += r->g.fom && r->replicas > 1 ? 2 : 1;     // gridding (+ the FOM path's replica combine)
@@ -337,8 +339,15 @@ static int run_batch_kernels(Recon* r, int buf, const float* d_img, long np, boo
     return BSG_OK;
 }
 
-// Upload one batch's particle records through a pinned staging buffer.
-static int upload_params(Recon* r, int buf, const double* params, long np) {
+// Batches of up to this many particles get their phase lattices and tile tests on
+// the host, in the records' copy: 0.6 us a particle, where a kernel for them lies
+// 8 us before the batch's first (one particle of 32^2 69 us a call, 77 with the
+// kernel).
+constexpr int FEW = 8;
+
+// Upload one batch's particle records through a pinned staging buffer; `grid`:
+// they will be gridded.
+static int upload_params(Recon* r, int buf, const double* params, long np, bool grid) {
     // the staging buffer may still feed an in-flight copy from two batches ago
     CK(cudaEventSynchronize(r->compute_done[buf]));
     DevParticle* hp = r->h_partbuf[buf];
@@ -373,10 +382,20 @@ static int upload_params(Recon* r, int buf, const double* params, long np) {
         r->edge_rmax = hf * smax * 1.4142136 * (1.0 + 1e-6) + 2.0;
     }
     r->d_part = r->d_partbuf[buf];
-    CK(cudaMemcpyAsync(r->d_part, hp, sizeof(DevParticle) * np, cudaMemcpyHostToDevice, r->fft_stream));
     const long nsym = std::max(1L, (long)r->sym.size() / 9);
     bool ewald = false;
     for (long i = 0; i < np && !ewald; ++i) ewald = params[i * BSG_PARTICLE_DOUBLES + 26] != 0;
+    const bool few = grid && np <= FEW && nsym == 1 && !ewald;
+    size_t bytes = sizeof(DevParticle) * np;
+    if (few) {
+        TileTest* tests = reinterpret_cast<TileTest*>(hp + np);
+        for (long i = 0; i < np; ++i) {
+            hp[i].lat = pack_lattice(choose_lattice(hp[i].ad, hp[i].bd));
+            tests[i] = tile_test(hp[i], r->g.ft);
+        }
+        bytes += sizeof(TileTest) * np;
+    }
+    CK(cudaMemcpyAsync(r->d_part, hp, bytes, cudaMemcpyHostToDevice, r->fft_stream));
     r->nexp = 0;
     r->g.ewald = ewald ? 1 : 0;
     if (nsym > 1 || ewald) {
@@ -423,6 +442,8 @@ static int upload_params(Recon* r, int buf, const double* params, long np) {
         CK(cudaMemcpyAsync(r->d_psym, r->h_psym.data(), sizeof(DevParticle) * k, cudaMemcpyHostToDevice,
                            r->fft_stream));
     }
+    if (few) r->d_test = reinterpret_cast<const TileTest*>(r->d_part + np);
+    if (few || !grid) return BSG_OK;
     // the records that are gridded get their phase lattices and tile tests on
     // the device
     const long nrec = r->nexp > 0 ? r->nexp : np;
@@ -433,6 +454,7 @@ static int upload_params(Recon* r, int buf, const double* params, long np) {
         CK(cudaMalloc((void**)&r->d_testbuf[buf], sizeof(TileTest) * nrec));
         r->testbuf_cap[buf] = (size_t)nrec;
     }
+    r->d_test = r->d_testbuf[buf];
     CK(launch_lattices(*r, r->nexp > 0 ? r->d_psym : r->d_part, r->d_testbuf[buf], nrec, r->fft_stream));
     r->stats.launches += 1;
     return BSG_OK;
@@ -447,7 +469,7 @@ static int process(Recon* r, const float* images, const double* params, long npa
         // alternate the staging buffers across calls too, so that one call's
         // upload overlaps the previous call's kernels
         const int buf = (int)(r->seq++ & 1);
-        int rc = upload_params(r, buf, params + off * BSG_PARTICLE_DOUBLES, np);
+        int rc = upload_params(r, buf, params + off * BSG_PARTICLE_DOUBLES, np, !spectra_out);
         if (rc) return rc;
         if (!spectra_out && r->g.ewald && !r->ewald_seen) {
             // an Ewald surface is not Hermitian: the full map from here on
@@ -564,12 +586,12 @@ int bsg_recon_create(const bsg_recon_config* cfg, bsg_recon** out) {
         free_all(r); delete r;
         return fail(BSG_ERR_CUDA, "bsg_recon_create: stream creation failed");
     }
-    const size_t N3 = (size_t)N * N * N;
+    const size_t N3 = (size_t)N * N * N, part_bytes = sizeof(DevParticle) * batch + sizeof(TileTest) * FEW;
     for (int i = 0; i < 2; ++i) {
         A((void**)&r->d_imgbuf[i], sizeof(float) * (size_t)n * n * batch);
-        if (!rc && cudaMallocHost((void**)&r->h_partbuf[i], sizeof(DevParticle) * batch) != cudaSuccess)
+        if (!rc && cudaMallocHost((void**)&r->h_partbuf[i], part_bytes) != cudaSuccess)
             rc = fail(BSG_ERR_NOMEM, "bsg_recon_create: pinned host allocation");
-        A((void**)&r->d_partbuf[i], sizeof(DevParticle) * batch);
+        A((void**)&r->d_partbuf[i], part_bytes);
         A((void**)&r->d_testbuf[i], sizeof(TileTest) * batch);
         r->testbuf_cap[i] = (size_t)batch;
         A((void**)&r->d_specbuf[i], sizeof(float2) * (size_t)(ft + 1) * (ft + 2) * batch);

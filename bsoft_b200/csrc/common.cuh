@@ -63,6 +63,18 @@ struct alignas(16) TileTest {
     int half;
 };
 
+// (an Ewald surface deviates from the plane by up to P.ezmax voxels)
+__host__ __device__ inline TileTest tile_test(const DevParticle& P, int ft) {
+    TileTest t;
+    for (int i = 0; i < 3; ++i) {
+        t.n[i] = (float)P.nrm[i];
+        t.reach[i] = fmaf(0.5f * ft, fabsf(P.af[i]) + fabsf(P.bf[i]), 1.0f) + P.ezmax;
+    }
+    t.slab = P.slab + 1e-3f + P.ezmax;
+    t.half = P.half;
+    return t;
+}
+
 // Run geometry shared by all kernels of one context.
 struct Geometry {
     int n, ft, map, logft;

@@ -2,7 +2,8 @@
 // their tile-test entries, one warp per record: the lanes test 32 candidates at a time, in
 // choose_lattice's order, and the first safe one is the record's.  On the host
 // the search took 0.5 to 0.7 us a record before the batch's first kernel could
-// start (1.1 of 2.7 ms for 2,000 particles of 64^2); here 12 us for all.
+// start (1.1 of 2.7 ms for 2,000 particles of 64^2); here 12 us for all.  (A batch
+// of a few particles stays on the host: capi.cu, upload_params.)
 #include "context.cuh"
 #include "lattice.h"
 
@@ -34,16 +35,7 @@ __global__ void __launch_bounds__(128) lattice_kernel(DevParticle* part, TileTes
         }
     if (lane == 0) {
         P.lat = pack_lattice(best);
-        // (an Ewald surface deviates from the plane by up to P.ezmax voxels)
-        TileTest t;
-        const float hf = 0.5f * ft;
-        for (int i = 0; i < 3; ++i) {
-            t.n[i] = (float)P.nrm[i];
-            t.reach[i] = hf * (fabsf(P.af[i]) + fabsf(P.bf[i])) + 1.0f + P.ezmax;
-        }
-        t.slab = P.slab + 1e-3f + P.ezmax;
-        t.half = P.half;
-        tests[r] = t;
+        tests[r] = tile_test(P, ft);
     }
 }
 

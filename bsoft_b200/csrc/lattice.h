@@ -1,5 +1,5 @@
-// lattice.h - the phase lattice of the gridding scatter, chosen per particle on
-// the device (lattice.cu); plain C++ on the host for the tests.
+// lattice.h - the phase lattice of the gridding scatter, chosen per particle, on
+// the device (lattice.cu) or, for a few, on the host; plain C++ there.
 //
 // The gridding kernel walks a particle's pixels phase by phase: the pixels
 // (h0 + lh i + sh j, k0 + lk j) of one phase are gridded by the 32 lanes of
@@ -128,7 +128,7 @@ BSG_LATTICE_FN PhaseLattice lattice_candidate(int c) {
 
 // The safe lattice with the fewest phases (up to max_phases; lattice_candidate's
 // order), else the square one.  lattice.cu makes this choice on the device, 32
-// candidates at a time; this form is what the tests hold it to.
+// candidates at a time; this is the host's form, and what the tests hold that to.
 // curve: bound on the extra displacement (voxels per pixel step of the
 // lattice vector) of a curved insertion surface; 0 for the plane.
 inline PhaseLattice choose_lattice(const double ad[3], const double bd[3], int max_phases = LATTICE_PHASES,
