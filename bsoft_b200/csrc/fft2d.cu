@@ -31,7 +31,7 @@
 // bit for bit); the line changes hands through shared memory once (up to 256
 // elements) or twice.  Lines in shared memory with a round trip per two stages
 // took 3.59 (columns) and 0.99 ms (rows) per 2,000 particles of 256^2 at ft
-// 512, bound by those trips; now 1.90 and 0.67.
+// 512, bound by those trips; now 1.81 and 0.65.
 #include "context.cuh"
 #include "fft_dev.cuh"
 
@@ -214,17 +214,20 @@ __device__ __forceinline__ void line_fft(float2* v, int t, const float2* tw, Put
 }
 
 // ------------------------------------------------------------------ rows
-constexpr int ROW_THREADS = 256;
-
-// 256 / T row pairs per CTA, T = ft / 16 threads each; 32 KB of lines.
+// (a box of 32 has 16 pairs: 64 threads at ft 64, where 256 left three quarters
+// idle; 500 particles 13.2 -> 7.3 us)
 template <int LOG>
-__global__ void __launch_bounds__(ROW_THREADS)
+constexpr int ROW_THREADS = LOG <= 6 ? 64 : 256;
+
+// ROW_THREADS / T row pairs per CTA, T = ft / 16 threads each; at most 32 KB of lines.
+template <int LOG>
+__global__ void __launch_bounds__(ROW_THREADS<LOG>)
 rows_kernel(const float* __restrict__ img, const double* __restrict__ bkg, const float2* __restrict__ tw,
             const DevParticle* __restrict__ part, int n, float2* __restrict__ rows) {
-    constexpr int ft = 1 << LOG, T = ft / E, LINES = ROW_THREADS / T;
+    constexpr int ft = 1 << LOG, T = ft / E, THREADS = ROW_THREADS<LOG>, LINES = THREADS / T;
     __shared__ float2 stw[ft / 2];
     __shared__ float2 lines[LINES * ft];
-    for (int i = threadIdx.x; i < ft / 2; i += ROW_THREADS) stw[swz(i)] = tw[i];
+    for (int i = threadIdx.x; i < ft / 2; i += THREADS) stw[swz(i)] = tw[i];
     __syncthreads();
     const int b = blockIdx.y, t = threadIdx.x % T;
     const int pair = blockIdx.x * LINES + threadIdx.x / T;
@@ -348,7 +351,10 @@ __device__ __forceinline__ float2 pixel_factor(const ColArgs& a, const CtfTerms&
 // apart in shared memory so that the columns of one element are adjacent.
 // A thread's outputs are 16 pixels (h, k) of one column: it writes each and
 // its mate (-h, -k) = conj, whose even CTF factor is the same, so the FP64
-// aberration is evaluated once for the two.
+// aberration is evaluated once for the two.  Four pixels of the epilogue at a
+// time: with all 16 unrolled a launch waited for the instructions to arrive, 21 us
+// for the smallest, now 10 (500 particles of ft 512 480 -> 452 us, of ft 64 23 ->
+// 14; two at a time 458 and 15, one 474 and 15).
 template <int LOG>
 __global__ void __launch_bounds__(COL_W * (1 << (LOG - 4)), LOG <= 9 ? 1024 / (COL_W * (1 << (LOG - 4))) : 1)
 cols_kernel(ColArgs a) {
@@ -387,19 +393,24 @@ cols_kernel(ColArgs a) {
     const bool mate = hidx >= 1 && hidx < hf;
     const float2 exh = ex[hidx];
     const double sx = (double)h * P.fs;
+    // (back to the places in shared memory that this thread read last, so that
+    // the loop below need not be unrolled)
 #pragma unroll
+    for (int q = 0; q < E; ++q) buf[line_output<LOG>(t, q) * COL_W + c] = v[q];
+#pragma unroll 4
     for (int q = 0; q < E; ++q) {
         const int kk = line_output<LOG>(t, q), k = sfreq(kk, ft);
+        const float2 g = buf[kk * COL_W + c];
         const double sy = (double)k * P.fs;
         const float w = a.ctf_action ? even_ctf(a, P, sx, sy) : 0.f;
-        out[(long)k * pitch + h] = value_times(v[q], pixel_factor(a, P, sc, phase_of(exh, sey[kk]), w, sx, sy));
+        out[(long)k * pitch + h] = value_times(g, pixel_factor(a, P, sc, phase_of(exh, sey[kk]), w, sx, sy));
         if (mate) {
             // F(-h, -k) = conj(G(h, k)) * factor(-h, -k); -(-ft/2) is -ft/2
             const int km = (ft - kk) & (ft - 1), k2 = sfreq(km, ft);
             const double sy2 = (double)k2 * P.fs;
             const float w2 = k2 == -k || !a.ctf_action ? w : even_ctf(a, P, -sx, sy2);
             out[(long)k2 * pitch - h] = value_times(
-                make_float2(v[q].x, -v[q].y), pixel_factor(a, P, sc, mate_phase_of(exh, sey[km]), w2, -sx, sy2));
+                make_float2(g.x, -g.y), pixel_factor(a, P, sc, mate_phase_of(exh, sey[km]), w2, -sx, sy2));
         }
     }
 }
@@ -430,10 +441,10 @@ struct RowsLaunch {
     cudaStream_t s;
     template <int LOG>
     cudaError_t operator()() const {
-        constexpr int LINES = ROW_THREADS / ((1 << LOG) / E);
+        constexpr int LINES = ROW_THREADS<LOG> / ((1 << LOG) / E);
         const int npairs = (c.g.n + 1) / 2;
         const dim3 grid((npairs + LINES - 1) / LINES, nimg);
-        rows_kernel<LOG><<<grid, ROW_THREADS, 0, s>>>(img, c.d_bkg, c.d_tw, c.d_part, c.g.n, c.d_rows);
+        rows_kernel<LOG><<<grid, ROW_THREADS<LOG>, 0, s>>>(img, c.d_bkg, c.d_tw, c.d_part, c.g.n, c.d_rows);
         return cudaGetLastError();
     }
 };
