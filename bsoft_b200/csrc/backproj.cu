@@ -320,8 +320,9 @@ struct PlaneImage {
 // (pixels stored as doubles 1.62 ms, as single floats 1.26).  200 images of
 // 128^2 into 128^3: the reference's operations one by one (12 products and
 // sums for the coordinates, 18 for weights and sums, a division) 2.31 ms,
-// now 1.23.
-__global__ void __launch_bounds__(BP_THREADS) backproject_kernel(const float2* __restrict__ img,
+// now 1.20 (with eight CTAs per SM; the border's coordinates take 72 registers
+// when they are let, seven CTAs and 1.29).
+__global__ void __launch_bounds__(BP_THREADS, 8) backproject_kernel(const float2* __restrict__ img,
                                                                  const BpImage* __restrict__ par, int nimg, int n,
                                                                  int N, float* map0, float* map1) {
     __shared__ PlaneImage sp[BP_CHUNK];
