@@ -31,12 +31,16 @@
 // heaviest first (nearest to the Fourier origin, where every particle's
 // plane passes) so the long ones do not trail the launch, and each tile has
 // R replica warps that take consecutive slices of the particle list into
-// private partial sums; a combine pass adds the replicas in order.
+// private partial sums, added in replica order by the last of them to arrive
+// (grid4_kernel) or, with the FOM channels, by a combine pass.
 //
-// Each phase's lattice points are enumerated exactly: lane j computes the
-// h-interval of lattice row j from the three slab constraints of the tile
-// box (once for all phases that walk that row), a warp scan turns the row
-// counts into offsets, and lanes take points in order.
+// A row's pixels are found exactly from the three slab constraints of the tile
+// box.  grid4_kernel bounds them in FP32 where that settles the integers, gives
+// each lane a group of a row's pixels, one of each column phase, and steps
+// through the phases together (walk_groups).  The FOM path enumerates phase by
+// phase: lane j computes the h-interval of lattice row j (once for all phases
+// that walk it), a warp scan turns the row counts into offsets, and lanes take
+// points in order (walk_pair).
 #include "context.cuh"
 #include "row_range.h"
 

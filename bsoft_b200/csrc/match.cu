@@ -1308,7 +1308,7 @@ static cudaError_t ensure_padded(Match& M, cudaStream_t s) {
 // x weights applied to the sums, and eight pixels' lane sums added by one
 // exchange tree.  Loads come from the padded copies: the texture unit delivers
 // four 8-byte texels a clock per SM, which bounded the gather through it
-// (5,184 views of 9,900 pixels 25.7 -> 14.3 ms).  Bound by what the loads write
+// (5,184 views of 9,900 pixels 25.7 -> 13.2 ms).  Bound by what the loads write
 // into registers, 4 KB a pixel at 64 bytes a clock per SM: 64 of the 74 clocks a
 // pixel takes (integer instructions for half of the float-to-double conversions,
 // and pixels in compact tiles, which hit L1, changed nothing).  gridDim.y CTAs share a
